@@ -1,0 +1,268 @@
+// What the prompt attention kernels share (attention_tc.cu over pages, mla_prefill.cu over expanded keys): the matrix-product and the
+// softmax roles of a CTA that takes one or two tiles of 128 query rows through the same keys.
+//
+//   S_t = Q_t K^T      both operands from shared memory, 128 x 128 scores of 32 bits in tensor memory
+//   P_t = 2^(S_t - m)  16-bit, written over the scores in tensor memory; O_t += P_t V reads it from there as its A operand
+//
+// A thread owns a query row (a lane of tensor memory): it reads all 128 scores of a key tile at once and keeps them in registers, so maximum,
+// exponentials and row sum take one pass and no exchange.  With two tiles the tensor core works on one tile's products while the
+// other tile's warpgroup is at its exponentials; with one tile per CTA the two take turns.  The products of a tile are issued in the order
+// P V of key tile j, Q K of tile j + 1 by one thread and run in that order, so a full S_t also says that O_t is complete: the
+// rescaling of O needs no barrier of its own, and P may lie over S.
+//
+// CAP: scores are capped, c tanh(s / c).  SPLIT: the weights keep 16 more bits (P = hi + lo, two products): for paths whose weights are held
+// in 32 bits, at half as much tensor work again.  Tensor memory: S_0, S_1 (128 columns each), O_0, O_1 (up to 128 each).
+//
+// Bound by the special-function and issue rate of the softmax (a key tile takes the tensor core 2048 cycles for two query tiles, their 32768
+// exponentials as long).  Measured: 32 / 8 heads, two prompts of 3800 tokens 576 us with one tile of rows, scores read twice and weights
+// through shared memory, 360 us so; capped, 16 / 4 heads, eight prompts of 860 tokens 2536 us on the CUDA cores, 182 us so.
+#pragma once
+#include "common.cuh"
+
+namespace prompt {
+
+constexpr int ROWS = 128, KEYS = 128;
+constexpr int NUM_THREADS = 384;            // warp 0 TMA producer, 1 MMA issuer (2, 3 idle), 4..7 and 8..11 softmax of the two tiles
+// registers a thread: launched with 168; 384 x 168 = 128 x 72 + 256 x 216
+constexpr int REGS_AUX = 72, REGS_SOFTMAX = 216;
+template <int N> VB_DEVICE void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> VB_DEVICE void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+constexpr int BLK = 128 * 128;              // one [128 rows x 64 values] block of 16-bit values, 16 KB
+
+// D[tmem] (+)= A[tmem] * B[smem desc]: A holds two 16-bit values of a row in a column
+VB_DEVICE void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+               ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+VB_DEVICE void tma_load_3d(void* dst, const void* tmap, int c0, int c1, int c2, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+               ::"r"(smem_u32(dst)), "l"(tmap), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
+VB_DEVICE void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+        "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
+        "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
+}
+VB_DEVICE void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+VB_DEVICE void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// KS stages of keys, VS of values
+template <int KS, int VS> struct Bars {
+  uint64_t q_full, k_full[KS], k_empty[KS], v_full[VS], v_empty[VS], s_full[2], p_full[2], o_done[2];
+  VB_DEVICE void init() {
+    mbar_init(&q_full, 1);
+    for (int s = 0; s < KS; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
+    for (int s = 0; s < VS; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
+    for (int t = 0; t < 2; ++t) { mbar_init(&s_full[t], 1); mbar_init(&p_full[t], ROWS); mbar_init(&o_done[t], 1); }
+    mbar_fence_init();
+  }
+  // a producer that gave up: let its copies in flight land before the block gives up its memory
+  VB_DEVICE void drain() {
+    for (int s = 0; s < KS; ++s)
+      for (int n = 0; n < 4096 && !(mbar_try_wait(&k_full[s], 0) || mbar_try_wait(&k_full[s], 1)); ++n) {}
+    for (int s = 0; s < VS; ++s)
+      for (int n = 0; n < 4096 && !(mbar_try_wait(&v_full[s], 0) || mbar_try_wait(&v_full[s], 1)); ++n) {}
+  }
+};
+
+// MMA issuer (one warp).  qk(t, stage) issues S_t, pv(t, stage, first) issues O_t; `tiles` (1 or 2) query tiles over n >= 1 key tiles.
+template <int KS, int VS, class QK, class PV>
+VB_DEVICE void mma_role(Bars<KS, VS>& b, int n, int tiles, int lane, int& budget, QK qk, PV pv) {
+  mbar_wait_lim(&b.q_full, 0, budget);
+  mbar_wait_lim(&b.k_full[0], 0, budget);
+  tc_fence_after();
+  if (lane == 0) {
+    for (int t = 0; t < tiles; ++t) { qk(t, 0); umma_commit(&b.s_full[t]); }
+    umma_commit(&b.k_empty[0]);
+  }
+  __syncwarp();
+  for (int j = 0; j < n; ++j) {
+    const int vs = j % VS, ks = (j + 1) % KS;
+    mbar_wait_lim(&b.v_full[vs], (j / VS) & 1, budget);
+    for (int t = 0; t < tiles; ++t) {
+      mbar_wait_lim(&b.p_full[t], j & 1, budget);
+      tc_fence_after();
+      if (lane == 0) {
+        pv(t, vs, j == 0);
+        if (t == tiles - 1) umma_commit(&b.v_empty[vs]);
+        if (j + 1 == n) umma_commit(&b.o_done[t]);
+      }
+      __syncwarp();
+      if (j + 1 < n) {
+        if (t == 0) { mbar_wait_lim(&b.k_full[ks], ((j + 1) / KS) & 1, budget); tc_fence_after(); }
+        if (lane == 0) {
+          qk(t, ks);
+          umma_commit(&b.s_full[t]);
+          if (t == tiles - 1) umma_commit(&b.k_empty[ks]);
+        }
+        __syncwarp();
+      }
+    }
+  }
+}
+
+// c2 tanh(x), |x| <= 1 in the whole warp (`small`): x times a polynomial of x^2 that interpolates tanh(x) / x at the Chebyshev points of
+// [0, 1] (relative error 1.6e-7 in 32 bits); elsewhere by one exponential.
+VB_DEVICE float cap_small(float x, float c2) {
+  const float z = x * x;
+  float r = 0.0010380251333117485f;
+  r = fmaf(r, z, -0.0061943246982991695f);
+  r = fmaf(r, z, 0.02027970738708973f);
+  r = fmaf(r, z, -0.053451646119356155f);
+  r = fmaf(r, z, 0.13325075805187225f);
+  r = fmaf(r, z, -0.3333282768726349f);
+  r = fmaf(r, z, 0.9999999403953552f);
+  return r * (x * c2);
+}
+VB_DEVICE float cap_any(float x, float c2) {
+  const float e = ex2(fabsf(x) * 2.8853900817779268f);          // e^(2 |x|), at worst infinite: 1 - 0
+  const float y = fabsf(x) <= 1.f ? fabsf(cap_small(x, 1.f)) : 1.f - 2.f / (e + 1.f);
+  return copysignf(y, x) * c2;
+}
+
+struct Softmax {
+  float scale_log2;            // plain scores
+  float ku, c2;                // capped: scale / cap, cap log2(e)
+};
+
+// Softmax of one query tile: thread = row.  The row sees the keys [lo, hi) of its request (lo >= hi: none); `first`: the first key of the first
+// key tile.  Leaves O_t complete; returns the row's reference maximum (powers of two) and its sum.
+template <typename T, int OC, bool CAP, int KS, int VS>
+VB_DEVICE void softmax_role(Bars<KS, VS>& b, int t, uint32_t t_s, uint32_t t_o, int n, int first, int lo, int hi, const Softmax& sm, bool split,
+                            int& budget, float& m_used, float& l_run) {
+  m_used = -INFINITY;
+  l_run = 0.f;
+  for (int j = 0; j < n; ++j, first += KEYS) {
+    mbar_wait_lim(&b.s_full[t], j & 1, budget);
+    __syncwarp();
+    tc_fence_after();
+    uint32_t v[4][32];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) tmem_ld_32x32(t_s + c * 32, v[c]);
+    tmem_ld_wait();
+    const int l = lo - first, h = hi - first;                   // visible columns of this tile: [l, h)
+    const bool full = __all_sync(0xffffffffu, l <= 0 && h >= KEYS) != 0;
+    float mx = -INFINITY, far = 0.f;
+    if (full) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          mx = fmaxf(mx, __uint_as_float(v[c][i]));
+          if (CAP) far = fmaxf(far, fabsf(__uint_as_float(v[c][i])));
+        }
+    } else {
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const bool in = c * 32 + i >= l && c * 32 + i < h;
+          if (in) mx = fmaxf(mx, __uint_as_float(v[c][i]));
+          if (CAP) {
+            if (!in) v[c][i] = 0u;
+            far = fmaxf(far, fabsf(__uint_as_float(v[c][i])));
+          } else if (!in) {
+            v[c][i] = 0xff800000u;                              // -inf: a weight of 0
+          }
+        }
+    }
+    bool small = true;
+    if (CAP) {
+      small = __all_sync(0xffffffffu, far * fabsf(sm.ku) <= 1.f) != 0;
+      mx = mx == -INFINITY ? mx : cap_any(mx * sm.ku, sm.c2);
+    } else {
+      mx *= sm.scale_log2;
+    }
+    // keep the old reference maximum unless the new one is more than 2^8 above it
+    float alpha = 1.f;
+    bool rescale = false;
+    if (mx > m_used + 8.f || (m_used == -INFINITY && mx > -INFINITY)) {
+      rescale = m_used != -INFINITY;
+      if (rescale) alpha = ex2(m_used - mx);
+      m_used = mx;
+    }
+    const float m_ref = m_used == -INFINITY ? 0.f : m_used;
+    if (__any_sync(0xffffffffu, rescale)) {                     // accesses to tensor memory are the whole warp's
+      l_run *= alpha;
+#pragma unroll
+      for (int c = 0; c < OC; c += 32) {
+        uint32_t o[32];
+        tmem_ld_32x32(t_o + c, o);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+        tmem_st_32x32(t_o + c, o);
+      }
+    }
+    float sum = 0.f;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (CAP) {
+        if (small) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[c][i] = __float_as_uint(cap_small(__uint_as_float(v[c][i]) * sm.ku, sm.c2));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[c][i] = __float_as_uint(cap_any(__uint_as_float(v[c][i]) * sm.ku, sm.c2));
+        }
+      }
+      auto weight = [&](int i) {
+        const float x = __uint_as_float(v[c][i]);
+        const float e = CAP ? ex2(x - m_ref) : ex2(fmaf(x, sm.scale_log2, -m_ref));
+        return CAP && !full && (c * 32 + i < l || c * 32 + i >= h) ? 0.f : e;
+      };
+      uint32_t hi16[16];
+      if (split) {
+        uint32_t lo16[16];
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          const float p0 = weight(i), p1 = weight(i + 1);
+          sum += p0 + p1;
+          hi16[i / 2] = pack2<T>(p0, p1);
+          const float2 f = unpack2<T>(hi16[i / 2]);
+          lo16[i / 2] = pack2<T>(p0 - f.x, p1 - f.y);
+        }
+        tmem_st_32x16(t_s + KEYS / 2 + c * 16, lo16);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          const float p0 = weight(i), p1 = weight(i + 1);
+          sum += p0 + p1;
+          hi16[i / 2] = pack2<T>(p0, p1);
+        }
+      }
+      tmem_st_32x16(t_s + c * 16, hi16);
+    }
+    l_run += sum;
+    tmem_st_wait();
+    tc_fence_before();
+    mbar_arrive(&b.p_full[t]);
+  }
+  mbar_wait_lim(&b.o_done[t], 0, budget);
+  __syncwarp();
+  tc_fence_after();
+}
+
+// O_t += P_t V: db(kk) is the descriptor of 16 keys of the values
+template <class DB> VB_DEVICE void issue_pv(uint32_t tmem_o, uint32_t tmem_p, uint32_t idesc, bool first, bool split, DB db) {
+#pragma unroll
+  for (int kk = 0; kk < KEYS / 16; ++kk) umma_f16_ta(tmem_o, tmem_p + kk * 8, db(kk), idesc, !first || kk != 0);
+  if (split) {
+#pragma unroll
+    for (int kk = 0; kk < KEYS / 16; ++kk) umma_f16_ta(tmem_o, tmem_p + KEYS / 2 + kk * 8, db(kk), idesc, 1);
+  }
+}
+
+}  // namespace prompt

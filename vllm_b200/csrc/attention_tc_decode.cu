@@ -12,7 +12,8 @@
 // 128-column softmax chain caps a CTA at ~20 GB/s.
 //
 // Reference for the op: FlashInfer trtllm_batch_decode_with_kv_cache (v1/attention/backends/flashinfer.py:2457).
-#include "common.cuh"
+// Capped scores (CAP): their weights keep 16 more bits in a second product, P = hi + lo (attention_prompt.cuh).
+#include "attention_prompt.cuh"
 
 namespace fmha_dec {
 
@@ -36,23 +37,15 @@ struct Params {
   int bt_stride;
   int Hq, Hkv, G, num_splits, window, B;
   float scale_log2;
+  float ku, c2;            // capped scores: scale / cap, cap log2(e)
   int chunk;               // > 0: the query sees the keys of its own chunk of positions only
   const float* sinks;      // optional [Hq] logits in the softmax denominator that have no key
   float out_scale;         // factor of the output
 };
 
-VB_DEVICE void tma_load_3d(void* dst, const void* tmap, int c0, int c1, int c2, uint64_t* bar) {
-  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-               ::"r"(smem_u32(dst)), "l"(tmap), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2) : "memory");
-}
-VB_DEVICE void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
-}
-VB_DEVICE void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+using prompt::tma_load_3d;
+using prompt::tmem_st_32x16;
+using prompt::tmem_st_wait;
 VB_DEVICE void bar_sync_softmax() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // Persistent: grid = min(work items, SMs); a work item is (kv split, kv head, sequence).  Barriers, TMEM and the zeroed
@@ -60,7 +53,7 @@ VB_DEVICE void bar_sync_softmax() { asm volatile("bar.sync 1, 128;" ::: "memory"
 // the mbarrier phases (a CTA-global tile counter), so the TMA producer runs up to STAGES tiles ahead ACROSS item
 // boundaries: the K/V stream of the next (sequence, head) is already in flight while the softmax / epilogue of the
 // current one finish.  (The one-item-per-CTA version paid ~3.5 us of setup + pipeline fill per 11 us of streaming.)
-template <typename T, int G>
+template <typename T, int G, bool CAP>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                    const __grid_constant__ CUtensorMap tmap_v, const Params p) {
@@ -69,8 +62,8 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   unsigned char* k_smem = smem;                                 // STAGES x 32 KB
   unsigned char* v_smem = k_smem + STAGES * K_BYTES;            // STAGES x 32 KB
   unsigned char* q_smem = v_smem + STAGES * V_BYTES;            // 2 x 4 KB (double-buffered across items)
-  unsigned char* p_smem = q_smem + 2 * Q_BYTES;                 // 4 KB
-  uint64_t* bars = reinterpret_cast<uint64_t*>(p_smem + P_BYTES);
+  unsigned char* p_smem = q_smem + 2 * Q_BYTES;                 // 4 KB, low parts behind it
+  uint64_t* bars = reinterpret_cast<uint64_t*>(p_smem + (CAP ? 2 : 1) * P_BYTES);
   uint64_t* q_full = bars;                 // [2]
   uint64_t* q_empty = bars + 2;            // [2]
   uint64_t* k_full = q_empty + 2;
@@ -103,7 +96,7 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     // Q / P rows beyond the group and the partially filled last tile must be finite: zero once
     uint4 z = make_uint4(0, 0, 0, 0);
     uint4* s4 = reinterpret_cast<uint4*>(smem);
-    const int n16 = (STAGES * (K_BYTES + V_BYTES) + 2 * Q_BYTES + P_BYTES) / 16;
+    const int n16 = (STAGES * (K_BYTES + V_BYTES) + 2 * Q_BYTES + (CAP ? 2 : 1) * P_BYTES) / 16;
     for (int i = threadIdx.x; i < n16; i += NUM_THREADS) s4[i] = z;
   }
   fence_proxy_async();
@@ -229,6 +222,10 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 #pragma unroll
               for (int k = 0; k < 4; ++k)
                 umma_f16(tmem_o, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (jj | kb | k) != 0);
+              if (CAP) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) umma_f16(tmem_o, da + (uint64_t)(k * 2), db + (uint64_t)(P_BYTES / 16 + k * 2), idesc, 1);
+              }
             }
             umma_commit(&kv_empty[s]);
             umma_commit(pv_done);
@@ -275,7 +272,7 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         float s[G], cmax[G];
 #pragma unroll
         for (int g = 0; g < G; ++g) {
-          s[g] = ok ? __uint_as_float(sv[g]) * p.scale_log2 : -INFINITY;
+          s[g] = ok ? (CAP ? prompt::cap_any(__uint_as_float(sv[g]) * p.ku, p.c2) : __uint_as_float(sv[g]) * p.scale_log2) : -INFINITY;
           cmax[g] = warp_max(s[g]);
         }
         if (lane == 0) {
@@ -315,7 +312,9 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
           const float m_ref = (m_used[g] == -INFINITY) ? 0.f : m_used[g];
           const float pe = ok ? ex2(s[g] - m_ref) : 0.f;
           l_thr[g] += pe;
-          *reinterpret_cast<T*>(pcol + g * 128 + ((chunk ^ (g & 7)) << 4)) = from_f32<T>(pe);
+          const T hi = from_f32<T>(pe);
+          *reinterpret_cast<T*>(pcol + g * 128 + ((chunk ^ (g & 7)) << 4)) = hi;
+          if (CAP) *reinterpret_cast<T*>(pcol + P_BYTES + g * 128 + ((chunk ^ (g & 7)) << 4)) = from_f32<T>(pe - to_f32(hi));
         }
         tc_fence_before();
         fence_proxy_async();
@@ -405,12 +404,12 @@ static EncodeTiledFn get_encode() {
   return fn;
 }
 
-template <typename T, int G>
+template <typename T, int G, bool CAP>
 static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const Params& p, dim3 grid,
                   cudaStream_t st) {
-  const int smem = STAGES * (K_BYTES + V_BYTES) + 2 * Q_BYTES + P_BYTES + 32 * 8 + 16 + 4 * NQ * 4 +
+  const int smem = STAGES * (K_BYTES + V_BYTES) + 2 * Q_BYTES + (CAP ? 2 : 1) * P_BYTES + 32 * 8 + 16 + 4 * NQ * 4 +
                    2 * MAX_TILES_SMEM * 4 + 1024;
-  auto k = fmha_decode_kernel<T, G>;
+  auto k = fmha_decode_kernel<T, G, CAP>;
   static bool a = false;
   if (!a) { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); a = true; }
   vb_launch(k, grid, dim3(NUM_THREADS), (size_t)smem, st, tq, tk, tv, p);
@@ -419,10 +418,10 @@ static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
 
 }  // namespace fmha_dec
 
-EXPORT int vb_fmha_tc_decode(const void* q, const void* kv_cache, int64_t num_blocks, const int* block_table,
+EXPORT int vb_fmha_tc_decode2(const void* q, const void* kv_cache, int64_t num_blocks, const int* block_table,
                              const int* seq_lens, void* out, float* part_out, float* part_lse, float* lse_out, int B,
                              int Hq, int Hkv, int64_t q_stride, int64_t out_stride, int bt_stride, int num_splits,
-                             int window, float scale, int chunk, const float* sinks, float out_scale, int dtype,
+                             int window, float scale, float soft_cap, int chunk, const float* sinks, float out_scale, int dtype,
                              cudaStream_t st) {
   using namespace fmha_dec;
   if (B == 0) return 0;
@@ -438,6 +437,7 @@ EXPORT int vb_fmha_tc_decode(const void* q, const void* kv_cache, int64_t num_bl
   p.lse_out = lse_out; p.out_stride = out_stride; p.bt_stride = bt_stride; p.Hq = Hq; p.Hkv = Hkv; p.G = G;
   p.num_splits = num_splits; p.window = window; p.scale_log2 = scale * 1.4426950408889634f; p.B = B;
   p.chunk = chunk; p.sinks = sinks; p.out_scale = out_scale;
+  p.ku = soft_cap > 0.f ? scale / soft_cap : 0.f; p.c2 = soft_cap * 1.4426950408889634f;
   CUtensorMap tq, tk, tv;
   {
     cuuint64_t dims[3] = {(cuuint64_t)D, (cuuint64_t)Hq, (cuuint64_t)B};
@@ -472,7 +472,9 @@ EXPORT int vb_fmha_tc_decode(const void* q, const void* kv_cache, int64_t num_bl
   dim3 grid(n_items < n_sms ? n_items : n_sms);
   int rc = -5;
 #define VB_GO(GV)                                                                          \
-  rc = bf16 ? launch<__nv_bfloat16, GV>(tq, tk, tv, p, grid, st) : launch<__half, GV>(tq, tk, tv, p, grid, st)
+  rc = bf16 ? (soft_cap > 0.f ? launch<__nv_bfloat16, GV, true>(tq, tk, tv, p, grid, st)      \
+                              : launch<__nv_bfloat16, GV, false>(tq, tk, tv, p, grid, st))    \
+            : (soft_cap > 0.f ? launch<__half, GV, true>(tq, tk, tv, p, grid, st) : launch<__half, GV, false>(tq, tk, tv, p, grid, st))
   switch (G) {
     case 1: VB_GO(1); break;
     case 2: VB_GO(2); break;

@@ -168,9 +168,13 @@ class EngineArgs:
         block_size = self.block_size
         if block_size is None:
             # 64-token pages are the tcgen05 kernels' TMA box; models that run on the generic kernel (other head sizes,
-            # ALiBi / sinks / soft-cap) use the 32-token page it is tuned for
-            special = any(mc.hf_config.get(k) for k in ("attn_logit_softcapping", "alibi")) or \
-                mc.hf_config.get("model_type") in ("bloom", "mpt", "gpt_oss")
+            # ALiBi / sinks; capped scores in 32 bits, over 8-bit caches or in odd head groups) use the 32-token page it is tuned for
+            hf = mc.hf_config
+            group = max((hf.get("num_attention_heads") or 1) // max(hf.get("num_key_value_heads") or hf.get("num_attention_heads") or 1, 1), 1)
+            capped_tc = (128 % group == 0 and self.kv_cache_dtype in ("auto", "bfloat16", "float16")
+                         and mc.torch_dtype.itemsize == 2)
+            special = (hf.get("attn_logit_softcapping") and not capped_tc) or hf.get("alibi") or \
+                hf.get("model_type") in ("bloom", "mpt", "gpt_oss")
             any_page = mc.hf_config.get("model_type") in ("legelix", "kopadra", "gizilorn")          # kernels that take every page size
             block_size = 64 if (self.device == "cpu" or mc.is_mla or any_page or (mc.head_dim == 128 and not special)) else 32
         cc = CacheConfig(

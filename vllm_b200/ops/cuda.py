@@ -91,10 +91,10 @@ _paged_attention = _sig("vb_paged_attention", _vp, _vp, _vp, _vp, _vp, _vp, _vp,
                         _i64, _i64, _i, _i, _i, _f, _f, _f, _i, _i, _i, _vp)
 _paged_attention_ex = _sig("vb_paged_attention_ex", _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,
                            _i64, _i64, _i, _i, _i, _f, _f, _f, _i, _i, _i, _vp, _vp, _i, _vp)
-_fmha_tc = _sig("vb_fmha_tc2", _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i64, _i64, _i,
-                _i, _i, _f, _i, _i, _i, _vp, _f, _i, _vp)
-_fmha_tc_decode = _sig("vb_fmha_tc_decode", _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i64, _i,
-                       _i, _i, _f, _i, _vp, _f, _i, _vp)
+_fmha_tc = _sig("vb_fmha_tc3", _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i64, _i64, _i,
+                _i, _i, _f, _f, _i, _i, _i, _vp, _f, _i, _vp)
+_fmha_tc_decode = _sig("vb_fmha_tc_decode2", _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i64, _i,
+                       _i, _i, _f, _f, _i, _vp, _f, _i, _vp)
 _any_attention = _sig("vb_any_attention", _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i64, _i64, _i, _i, _i,
                       _i, _f, _f, _f, _vp, _vp, _i, _vp)
 _merge_states = _sig("vb_merge_attn_states", _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _vp)
@@ -375,8 +375,7 @@ def paged_attention(q, kv_cache, md, scale, sliding_window=None, logits_soft_cap
     chunk_size = int(chunk_size or 0)
     if md.kv_vt:
         # tcgen05 kernel over the tensor-core cache layout
-        assert tc_attention_ok(D, DV, G) and BS == 64 and not logits_soft_cap and alibi_slopes is None, \
-            "tensor-core attention: D=128, 64-token pages, no soft-cap / ALiBi"
+        assert tc_attention_ok(D, DV, G) and BS == 64 and alibi_slopes is None, "tensor-core attention: D=128, 64-token pages, no ALiBi"
         # batch-invariant mode: a decode row takes the varlen kernel it would take inside a mixed batch
         decode = md.decode_only and not (batch_invariant() and md.query_start_loc is not None)
         splits = (md.num_splits or decode_splits(md.num_reqs, Hkv, md.max_seq_len, 128)) if decode else 1
@@ -388,15 +387,15 @@ def paged_attention(q, kv_cache, md, scale, sliding_window=None, logits_soft_cap
             rc = _fmha_tc_decode(q.data_ptr(), kv_cache.data_ptr(), kv_cache.shape[0], bt.data_ptr(),
                                  md.seq_lens.data_ptr(), out.data_ptr(), _p(ws.part_out) if ws else None,
                                  _p(ws.part_lse) if ws else None, _p(lse), md.num_reqs, Hq, Hkv, q.stride(0),
-                                 out.stride(0), bt.stride(0), splits, sliding_window or 0, scale, chunk_size, _p(sinks),
-                                 out_scale, _DT[q.dtype], _st())
+                                 out.stride(0), bt.stride(0), splits, sliding_window or 0, scale, logits_soft_cap, chunk_size,
+                                 _p(sinks), out_scale, _DT[q.dtype], _st())
             _check(rc, f"fmha_tc_decode(G={G})", 2 if splits > 1 else 1)
             return (out, lse) if return_lse else out
         rc = _fmha_tc(q.data_ptr(), kv_cache.data_ptr(), kv_cache.shape[0], bt.data_ptr(), md.seq_lens.data_ptr(),
                       None if decode else md.query_start_loc.data_ptr(), out.data_ptr(),
-                      _p(ws.part_out) if ws else None, _p(ws.part_lse) if ws else None, _p(lse), md.num_reqs, T,
-                      md.max_query_len, Hq, Hkv, q.stride(0), out.stride(0), bt.stride(0), splits,
-                      sliding_window or 0, scale, int(causal), int(md.flat and not decode), chunk_size, _p(sinks), out_scale,
+                      _p(ws.part_out) if ws else None, _p(ws.part_lse) if ws else None, _p(lse), kernel_error_flag(q.device).data_ptr(),
+                      md.num_reqs, T, md.max_query_len, Hq, Hkv, q.stride(0), out.stride(0), bt.stride(0), splits,
+                      sliding_window or 0, scale, logits_soft_cap, int(causal), int(md.flat and not decode), chunk_size, _p(sinks), out_scale,
                       _DT[q.dtype], _st())
         _check(rc, f"fmha_tc(G={Hq // Hkv})", 2 if splits > 1 else 1)
         return (out, lse) if return_lse else out

@@ -355,8 +355,7 @@ class ModelRunner:
         d, hq, hkv = layer.head_size, getattr(layer, "num_heads", 1), layer.num_kv_heads
         if getattr(layer, "talk", None) is not None and not cuda_ops().tc_talk_ok(dtype, layer.logits_soft_cap):
             return False
-        return ((getattr(layer, "talk", None) is not None or not getattr(layer, "logits_soft_cap", 0.0))
-                and getattr(layer, "alibi_slopes", None) is None
+        return (getattr(layer, "alibi_slopes", None) is None
                 and cuda_ops().tc_attention_ok(d, getattr(layer, "v_head_size", d), max(hq // max(hkv, 1), 1)))
 
     def _init_gpu_prep(self) -> None:
