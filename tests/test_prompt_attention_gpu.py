@@ -49,3 +49,47 @@ def test_capped_decode(Hq, Hkv, splits, dtype, cap):
     want = ref.paged_attention(q, cache, md.block_table, md.seq_lens_cpu, md.query_start_loc_cpu, 0.2, sliding_window=300, logits_soft_cap=cap)
     assert _rel(got, want) < LIMIT[True], _rel(got, want)
     cu().check_kernel_error(q.device)
+
+
+@pytest.mark.parametrize("heads", [3, 32], ids=["one", "two"])                  # tiles per CTA
+@pytest.mark.parametrize("dim,rot,vdim", [(128, 64, 128), (64, 0, 64), (24, 8, 40), (128, 0, 72)])
+@pytest.mark.parametrize("split", [False, True])
+def test_expanded_keys(heads, dim, rot, vdim, split):
+    """Keys and values as columns of one matrix, key rows of a request behind a gap of zeros."""
+    q_lens, seq_lens = [1, 127, 128, 129, 300, 513, 17], [200, 127, 640, 129, 301, 513, 17]
+    g = torch.Generator(device="cuda").manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)  # noqa: E731
+    T = sum(q_lens)
+    start = [0]
+    for n in seq_lens:
+        start.append(start[-1] + -(-n // 128) * 128)
+    q, kv, kr = rnd(T, heads, dim + rot), rnd(start[-1], heads, dim + vdim), rnd(start[-1], max(rot, 8))
+    for s, n, e in zip(start, seq_lens, start[1:]):
+        kv[s + n:e], kr[s + n:e] = 0, 0
+    out = torch.full((T, heads, vdim), float("nan"), device="cuda", dtype=torch.bfloat16)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")  # noqa: E731
+    cu_q = [sum(q_lens[:i]) for i in range(len(q_lens) + 1)]
+    cu().mla_prefill(q, kv[..., :dim], kv[..., dim:], out, i32(cu_q[:-1]), i32(q_lens), i32(seq_lens), i32(start), 0, max(q_lens), 0.1,
+                     kr[:, :rot] if rot else None, split=split)
+    cu().check_kernel_error(q.device)
+    want = []
+    for a, ql, s, n in zip(cu_q, q_lens, start, seq_lens):
+        k = torch.cat([kv[s:s + n, :, :dim], kr[s:s + n, None, :rot].expand(-1, heads, -1)], -1).double()
+        x = torch.einsum("qhd,khd->hqk", q[a:a + ql].double(), k) * 0.1
+        x = x.masked_fill(torch.arange(n, device="cuda")[None] > torch.arange(n - ql, n, device="cuda")[:, None], float("-inf"))
+        want.append(torch.einsum("hqk,khd->qhd", x.softmax(-1), kv[s:s + n, :, dim:].double()))
+    assert _rel(out, torch.cat(want)) < LIMIT[split], _rel(out, torch.cat(want))
+
+
+@pytest.mark.parametrize("lens", [None, [5, 130, 64]])
+def test_gathered_rows_end_in_zeros(lens):
+    cache = torch.randn(12, 64, 72, device="cuda", dtype=torch.bfloat16)
+    bt = torch.arange(1, 12, dtype=torch.int32, device="cuda")[:9].view(3, 3).contiguous()
+    starts = [0, 128, 320, 384] if lens else [0, 5, 135, 199]
+    got = torch.full((starts[-1], 72), float("nan"), device="cuda", dtype=torch.bfloat16)
+    cu().gather_cache(cache, bt, torch.tensor(starts, dtype=torch.int32, device="cuda"), got, 192,
+                      lens=None if lens is None else torch.tensor(lens, dtype=torch.int32, device="cuda"))
+    want = torch.zeros_like(got)
+    for i, n in enumerate(lens or [5, 130, 64]):
+        want[starts[i]:starts[i] + n] = cache[bt[i].long()].view(-1, 72)[:n]
+    assert torch.equal(got, want)

@@ -39,7 +39,8 @@ template <typename T, bool SRC8>
 __global__ void __launch_bounds__(256) gather_cache_kernel(const void* __restrict__ cache, T* __restrict__ out,
                                                             const int* __restrict__ block_table, int64_t bt_stride,
                                                             const int* __restrict__ cu_seq_lens,
-                                                            const int* __restrict__ seq_starts, int BS, int row,
+                                                            const int* __restrict__ seq_starts,
+                                                            const int* __restrict__ lens, int BS, int row,
                                                             int64_t block_stride, int64_t out_stride, float scale,
                                                             int tokens_per_cta) {
   pdl_trigger();
@@ -50,10 +51,17 @@ __global__ void __launch_bounds__(256) gather_cache_kernel(const void* __restric
   const int first = blockIdx.x * tokens_per_cta;
   if (first >= n) return;
   const int last = min(n, first + tokens_per_cta);
+  const int held = lens ? lens[b] : n;                       // rows from here on are zeros
   const int vec_per_row = row / 8;
   for (int i = first * vec_per_row + threadIdx.x; i < last * vec_per_row; i += blockDim.x) {
     const int tok = i / vec_per_row, c = i % vec_per_row;
     const int pos = start + tok;
+    if (tok >= held) {
+      Vec16<T> z;
+      z.u = make_uint4(0, 0, 0, 0);
+      st16(out + (int64_t)(t0 + tok) * out_stride + c * 8, z);
+      continue;
+    }
     const int64_t blk = block_table[b * bt_stride + pos / BS];
     const int64_t src_off = blk * block_stride + (int64_t)(pos % BS) * row + c * 8;
     Vec16<T> o;
@@ -109,8 +117,9 @@ EXPORT int vb_copy_blocks(const void* src, void* dst, const int64_t* map, int n_
   return (int)cudaGetLastError();
 }
 
-EXPORT int vb_gather_cache(const void* cache, void* out, const int* block_table, int64_t bt_stride, const int* cu_seq_lens,
-                           const int* seq_starts, int batch, int max_tokens, int BS, int row, int64_t block_stride,
+// lens (or null): rows of each sequence that the cache holds, those behind them up to the next sequence's first are zeros
+EXPORT int vb_gather_cache2(const void* cache, void* out, const int* block_table, int64_t bt_stride, const int* cu_seq_lens,
+                           const int* seq_starts, const int* lens, int batch, int max_tokens, int BS, int row, int64_t block_stride,
                            int64_t out_stride, float scale, int src_fp8, int dtype, cudaStream_t st) {
   if (batch == 0 || max_tokens == 0) return 0;
   if (dtype == DT_F32 || row % 8) return -1;
@@ -118,9 +127,9 @@ EXPORT int vb_gather_cache(const void* cache, void* out, const int* block_table,
   dim3 grid((max_tokens + tpc - 1) / tpc, batch);
   DISPATCH_HALF(dtype, TT, {
     if (src_fp8) vb_launch(gather_cache_kernel<TT, true>, grid, dim3(256), 0, st, cache, reinterpret_cast<TT*>(out),
-                           block_table, bt_stride, cu_seq_lens, seq_starts, BS, row, block_stride, out_stride, scale, tpc);
+                           block_table, bt_stride, cu_seq_lens, seq_starts, lens, BS, row, block_stride, out_stride, scale, tpc);
     else vb_launch(gather_cache_kernel<TT, false>, grid, dim3(256), 0, st, cache, reinterpret_cast<TT*>(out), block_table,
-                   bt_stride, cu_seq_lens, seq_starts, BS, row, block_stride, out_stride, scale, tpc);
+                   bt_stride, cu_seq_lens, seq_starts, lens, BS, row, block_stride, out_stride, scale, tpc);
   });
   return (int)cudaGetLastError();
 }

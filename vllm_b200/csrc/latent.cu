@@ -66,7 +66,7 @@ latent_norm_cache_kernel(const T* __restrict__ lat, int64_t lat_stride, int Rq, 
 struct RopeParams {
   void* q; const void* kv; const void* w; void* cache;
   const int64_t* positions; const int64_t* slots; const float* cos_sin;
-  int64_t st, cache_row;        // row stride of q and kv (columns of one matrix)
+  int64_t st, kv_st, cache_row; // row strides of q and kv (columns of one matrix, or two)
   int H, D, P, R;               // query heads of D + P, latent width (0: queries alone)
   int neox;
   float eps;
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(256) latent_rope_cache_kernel(const RopeParams
   const int per = V == 1 || p.neox ? p.P / 2 / V : p.P / V;                 // accesses of one rotated part
   if (p.R > 0) {
     const int64_t slot = p.cache ? p.slots[row] : -1;                       // < 0: padding row, nothing to cache
-    const T* c = reinterpret_cast<const T*>(p.kv) + row * p.st;
+    const T* c = reinterpret_cast<const T*>(p.kv) + row * p.kv_st;
     const T* w = reinterpret_cast<const T*>(p.w);
     T* dst = reinterpret_cast<T*>(p.cache) + slot * p.cache_row;
     float ss = 0.f;
@@ -281,20 +281,20 @@ EXPORT int vb_latent_norm_cache(const void* lat, int64_t lat_stride, int Rq, con
   return (int)cudaGetLastError();
 }
 
-// q: columns of a matrix with row stride st, H heads of D + P; kv: columns [c : R | k_r : P] of the same matrix (R = 0: none).  cache may be
-// null (nothing is cached); cos_sin [positions, P].
-EXPORT int vb_latent_rope_cache(void* q, const void* kv, int64_t st, int H, int D, int P, int R, const void* w, float eps,
+// q: columns of a matrix with row stride st, H heads of D + P; kv: columns [c : R | k_r : P] of a matrix with row stride kv_st (R = 0: none).
+// cache may be null (nothing is cached); cos_sin [positions, P].
+EXPORT int vb_latent_rope_cache2(void* q, const void* kv, int64_t st, int64_t kv_st, int H, int D, int P, int R, const void* w, float eps,
                                 const int64_t* positions, const float* cos_sin, int neox, void* cache, int64_t cache_row,
                                 const int64_t* slots, int T_, int dtype, cudaStream_t strm) {
   using namespace latent;
   if (T_ == 0) return 0;
   if (P % 2 || (P && (!positions || !cos_sin)) || (cache && (!slots || R == 0 || cache_row < R + P)) || (R > 0 && (!w || !kv))) return -1;
   RopeParams p;
-  p.q = q; p.kv = kv; p.w = w; p.cache = cache; p.positions = positions; p.slots = slots; p.cos_sin = cos_sin; p.st = st;
+  p.q = q; p.kv = kv; p.w = w; p.cache = cache; p.positions = positions; p.slots = slots; p.cos_sin = cos_sin; p.st = st; p.kv_st = kv_st;
   p.cache_row = cache_row; p.H = H; p.D = D; p.P = P; p.R = R; p.neox = neox; p.eps = eps;
   DISPATCH_DTYPE(dtype, T, {
     constexpr int V = Vec16<T>::N;
-    const bool vec = st % V == 0 && D % V == 0 && P % (neox ? 2 * V : V) == 0 && R % V == 0 && cache_row % V == 0 && al16(q) &&
+    const bool vec = st % V == 0 && kv_st % V == 0 && D % V == 0 && P % (neox ? 2 * V : V) == 0 && R % V == 0 && cache_row % V == 0 && al16(q) &&
                      (!kv || al16(kv)) && (!w || al16(w)) && (!cache || al16(cache));
     const int parts = H * P / (vec ? (neox ? 2 * V : V) : 2), lat = vec ? R / V : R, items = parts > lat ? parts : lat;
     const int thr = items >= 256 ? 256 : (items < 32 ? 32 : ((items + 31) / 32) * 32);

@@ -65,14 +65,15 @@ class LatentPlan:
     max_kv: int = 0
 
     @classmethod
-    def of(cls, md: AttentionMetadata, device: torch.device, window: int) -> "LatentPlan":
+    def of(cls, md: AttentionMetadata, device: torch.device, window: int, apart: int = 1) -> "LatentPlan":
         plans = md.latent_plan = md.latent_plan if md.latent_plan is not None else {}
-        if window not in plans:
-            plans[window] = cls.build(md, device, window)
-        return plans[window]
+        if (window, apart) not in plans:
+            plans[window, apart] = cls.build(md, device, window, apart)
+        return plans[window, apart]
 
     @classmethod
-    def build(cls, md: AttentionMetadata, device: torch.device, window: int = 0) -> "LatentPlan":
+    def build(cls, md: AttentionMetadata, device: torch.device, window: int = 0, apart: int = 1) -> "LatentPlan":
+        """``apart``: key rows of a request start at multiples of it."""
         if md.host_lens is not None:
             cu, sl = md.host_lens
         else:
@@ -90,7 +91,7 @@ class LatentPlan:
         vis = sl[req] - ql[req] + off + 1
         kv_first = np.maximum(sl[long] - ql[long] + 1 - window, 0) if window else np.zeros(n, dtype=np.int64)
         kl = sl[long] - kv_first
-        cu_kv = np.concatenate([[0], np.cumsum(kl)])
+        cu_kv = np.concatenate([[0], np.cumsum(-(-kl // apart) * apart)])
         parts = [cu[req] + off, req, vis, long, cu[long], ql[long], kl, kv_first, cu_kv]
         packed = torch.from_numpy(np.concatenate(parts).astype(np.int32)).to(device, non_blocking=True)
         rows, req_t, vis_t, long_t, q_start, q_len, seq_len, first_t, cu_t = packed.split([len(p) for p in parts])
@@ -104,11 +105,67 @@ class LatentPlan:
             plan.block_table = md.block_table.index_select(0, long_t)
             plan.q_start, plan.q_len, plan.seq_len, plan.cu_kv = q_start, q_len, seq_len, cu_t
             plan.kv_first = first_t if kv_first.any() else None
-            plan.num_kv, plan.max_q, plan.max_kv = int(cu_kv[-1]), int(ql[long].max()), int(kl.max())
+            plan.num_kv, plan.max_q, plan.max_kv = int(cu_kv[-1]), int(ql[long].max()), int((cu_kv[1:] - cu_kv[:-1]).max())
         return plan
 
 
-class LatentAttention(nn.Module):
+class LatentForms:
+    """The two forms over a layer's attributes ``attn`` (its ``MLAAttentionCore``), ``heads``, ``dim``, ``rot``, ``v_dim``, ``kv_rank``, ``scale``,
+    ``window``, and ``_up()``, ``_expand(c, h0, h1)``."""
+    # keys of a request start on a boundary of the prompt kernel's key tiles, zeros fill the gap: no tile holds two requests' values
+    kv_apart = 1
+    # softmax weights of prompts keep 16 more bits; rows in the latent space keep 32 in steps that are not decode steps alone
+    wide_weights = False
+
+    def _attend(self, q: torch.Tensor, md: AttentionMetadata, cache: torch.Tensor) -> torch.Tensor:
+        T = q.shape[0]
+        out = torch.empty(T, self.heads, self.v_dim, dtype=q.dtype, device=q.device)
+        window = self.window or None
+        if md.decode_only or not ops.latent_expand_ok(q, self.dim, self.rot, self.v_dim, self.kv_rank):
+            return self._absorbed(q, out, lambda q_abs, q_pe: ops.mla_attention(q_abs, q_pe, cache, md, self.scale, self.kv_rank, window))
+        plan = LatentPlan.of(md, q.device, self.window, self.kv_apart)
+        if plan.num_rows:
+            def attend(q_abs, q_pe):
+                if self.wide_weights:
+                    return ops.cuda_ops().mla_simt(q_abs, q_pe, cache, plan.row_block_table, plan.row_seq_lens, None, self.scale, window)
+                return ops.mla_attention_rows(q_abs, q_pe, cache, plan.row_block_table, plan.row_seq_lens, plan.max_row_len,
+                                              self.scale, window)
+            if plan.rows is None:
+                return self._absorbed(q, out, attend)
+            part = torch.empty(plan.num_rows, self.heads, self.v_dim, dtype=q.dtype, device=q.device)
+            out.index_copy_(0, plan.rows, self._absorbed(q.index_select(0, plan.rows), part, attend))
+        self._expanded(q, out, plan, cache)
+        return out
+
+    def _absorbed(self, q: torch.Tensor, out: torch.Tensor, attend) -> torch.Tensor:
+        w_uk, w_uv = self._up()
+        q_abs = torch.bmm(q[..., :self.dim].transpose(0, 1), w_uk).transpose(0, 1)   # [T, h, R], head-major in memory
+        o_lat = attend(q_abs, q[..., self.dim:] if self.rot else None)
+        torch.bmm(o_lat.transpose(0, 1), w_uv.transpose(1, 2), out=out.transpose(0, 1))
+        return out
+
+    def _expanded(self, q: torch.Tensor, out: torch.Tensor, plan: LatentPlan, cache: torch.Tensor) -> None:
+        # layers that share a cache (and see as much of it) share the gathered rows too
+        gathered = get_forward_context().extra.setdefault("latent_rows", {})
+        key = self.attn.cache_name, self.window
+        rows = gathered.get(key)
+        if rows is None:
+            rows = ops.gather_latents(cache, plan.block_table, plan.cu_kv, plan.num_kv, plan.max_kv, plan.kv_first,
+                                      plan.seq_len if self.kv_apart > 1 else None)
+            if self.shares_rows:
+                gathered[key] = rows
+        per_head = plan.num_kv * (self.dim + self.v_dim) * q.element_size()
+        step = max(1, min(self.heads, EXPAND_BYTES // max(per_head, 1)))
+        for h0 in range(0, self.heads, step):
+            h1 = min(self.heads, h0 + step)
+            k, v = self._expand(rows[:, :self.kv_rank], h0, h1)
+            ops.mla_prefill(q, k, v, out, plan.q_start, plan.q_len, plan.seq_len, plan.cu_kv, h0, plan.max_q, self.scale,
+                            rows[:, self.kv_rank:] if self.rot else None, self.window, self.wide_weights)
+
+
+class LatentAttention(LatentForms, nn.Module):
+    shares_rows = True
+
     def __init__(self, hidden_size: int, num_heads: int, dim: int, v_dim: int, q_rank: int, kv_rank: int, scale: float, eps: float,
                  dtype=None, quant_config=None, prefix: str = "", kv_sharing_target: Optional[str] = None, rope: Optional[nn.Module] = None,
                  window: int = 0, cache_window: int = 0, gated: bool = False) -> None:
@@ -150,6 +207,12 @@ class LatentAttention(nn.Module):
         w, n = self.ukv.weight, self.heads * self.dim
         return w[:n].view(self.heads, self.dim, self.kv_rank), w[n:].view(self.heads, self.v_dim, self.kv_rank)
 
+    def _expand(self, c: torch.Tensor, h0: int, h1: int) -> tuple[torch.Tensor, torch.Tensor]:
+        """Keys and values of heads h0 .. h1 - 1 of the latent rows c."""
+        w_uk, w_uv = self._up()
+        return (ops.linear(c, w_uk[h0:h1].reshape(-1, self.kv_rank)).view(c.shape[0], h1 - h0, self.dim),
+                ops.linear(c, w_uv[h0:h1].reshape(-1, self.kv_rank)).view(c.shape[0], h1 - h0, self.v_dim))
+
     def forward(self, h: torch.Tensor, positions: Optional[torch.Tensor] = None) -> torch.Tensor:
         T = h.shape[0]
         md, cache = self.attn.bound_cache()
@@ -182,46 +245,3 @@ class LatentAttention(nn.Module):
             return self.o(q.new_zeros(T, self.heads * self.v_dim))
         o = self._attend(q, md, cache).view(T, self.heads * self.v_dim)
         return self.o(o if gate is None else ops.sigmoid_mul_(o, gate))
-
-    def _attend(self, q: torch.Tensor, md: AttentionMetadata, cache: torch.Tensor) -> torch.Tensor:
-        T = q.shape[0]
-        out = torch.empty(T, self.heads, self.v_dim, dtype=q.dtype, device=q.device)
-        window = self.window or None
-        if md.decode_only or not ops.latent_expand_ok(q, self.dim, self.rot, self.v_dim, self.kv_rank):
-            return self._absorbed(q, out, lambda q_abs, q_pe: ops.mla_attention(q_abs, q_pe, cache, md, self.scale, self.kv_rank, window))
-        plan = LatentPlan.of(md, q.device, self.window)
-        if plan.num_rows:
-            def attend(q_abs, q_pe):
-                return ops.mla_attention_rows(q_abs, q_pe, cache, plan.row_block_table, plan.row_seq_lens, plan.max_row_len,
-                                              self.scale, window)
-            if plan.rows is None:
-                return self._absorbed(q, out, attend)
-            part = torch.empty(plan.num_rows, self.heads, self.v_dim, dtype=q.dtype, device=q.device)
-            out.index_copy_(0, plan.rows, self._absorbed(q.index_select(0, plan.rows), part, attend))
-        self._expanded(q, out, plan, cache)
-        return out
-
-    def _absorbed(self, q: torch.Tensor, out: torch.Tensor, attend) -> torch.Tensor:
-        w_uk, w_uv = self._up()
-        q_abs = torch.bmm(q[..., :self.dim].transpose(0, 1), w_uk).transpose(0, 1)   # [T, h, R], head-major in memory
-        o_lat = attend(q_abs, q[..., self.dim:] if self.rot else None)
-        torch.bmm(o_lat.transpose(0, 1), w_uv.transpose(1, 2), out=out.transpose(0, 1))
-        return out
-
-    def _expanded(self, q: torch.Tensor, out: torch.Tensor, plan: LatentPlan, cache: torch.Tensor) -> None:
-        # layers that share a cache (and see as much of it) share the gathered rows too
-        gathered = get_forward_context().extra.setdefault("latent_rows", {})
-        key = self.attn.cache_name, self.window
-        rows = gathered.get(key)
-        if rows is None:
-            rows = gathered[key] = ops.gather_latents(cache, plan.block_table, plan.cu_kv, plan.num_kv, plan.max_kv, plan.kv_first)
-        c = rows[:, :self.kv_rank]
-        w_uk, w_uv = self._up()
-        per_head = plan.num_kv * (self.dim + self.v_dim) * q.element_size()
-        step = max(1, min(self.heads, EXPAND_BYTES // max(per_head, 1)))
-        for h0 in range(0, self.heads, step):
-            h1 = min(self.heads, h0 + step)
-            k = ops.linear(c, w_uk[h0:h1].reshape(-1, self.kv_rank)).view(plan.num_kv, h1 - h0, self.dim)
-            v = ops.linear(c, w_uv[h0:h1].reshape(-1, self.kv_rank)).view(plan.num_kv, h1 - h0, self.v_dim)
-            ops.mla_prefill(q, k, v, out, plan.q_start, plan.q_len, plan.seq_len, plan.cu_kv, h0, plan.max_q, self.scale,
-                            rows[:, self.kv_rank:] if self.rot else None, self.window)

@@ -4,11 +4,10 @@ Reference parity: vllm/model_executor/models/deepseek_v2.py (``DeepseekV2MLAAtte
 ``DeepseekV2MoE``, ``load_weights`` expert mapping) and the MLA algorithm note in
 layers/attention/mla_attention.py:1-200.
 
-Attention runs in the *absorbed* form for both prefill and decode: the cache holds only the 512-d
-latent + 64-d rope key per token (576 values, ~1/57 of an MHA cache for V3), queries are projected
-into the latent space with W_UK, attention is MQA over the latent, and W_UV maps the result back.
-That keeps one KV layout and one kernel family for every phase and is what lets 180 GB hold very
-long batches.
+The cache holds only the 512-d latent + 64-d rope key per token (576 values, ~1/57 of an MHA cache for V3), which is what lets
+180 GB hold very long batches.  Decode steps attend in the *absorbed* form (queries are projected into the latent space with W_UK,
+attention is MQA over the latent, W_UV maps the result back); prompt portions *expand* keys and values of their context and run a
+multi-head kernel over them (layers/latent.py), whose scores take 192 multiplications instead of 576.
 """
 from __future__ import annotations
 
@@ -17,19 +16,23 @@ from typing import Iterable, Optional
 import torch
 import torch.nn as nn
 
+from vllm_b200 import envs, ops
 from vllm_b200.config import VllmConfig
 from vllm_b200.layers.attention import MLAAttentionCore
 from vllm_b200.layers.common import RMSNorm
+from vllm_b200.layers.latent import LatentForms
 from vllm_b200.layers.linear import (ColumnParallelLinear, ReplicatedLinear, RowParallelLinear,
                                      tp_reduce_residual_norm)
 from vllm_b200.layers.moe import FusedMoE
 from vllm_b200.layers.rotary import get_rope, yarn_mscale
 from vllm_b200.models.llama import LlamaForCausalLM, LlamaMLP, LlamaModel
-from vllm_b200.parallel.state import get_tp_group
+from vllm_b200.parallel.state import get_dcp_group, get_tp_group
 from vllm_b200.parallel.utils import divide
 
 
-class DeepseekMLA(nn.Module):
+class DeepseekMLA(LatentForms, nn.Module):
+    kv_apart, wide_weights, shares_rows = 128, True, False
+
     def __init__(self, cfg: dict, mc, dtype, quant_config, prefix: str) -> None:
         super().__init__()
         H = cfg["hidden_size"]
@@ -66,18 +69,26 @@ class DeepseekMLA(nn.Module):
             m = yarn_mscale(rs["factor"], rs["mscale_all_dim"])
             scale = scale * m * m
         self.attn = MLAAttentionCore(self.local_heads, self.kv_lora, self.rope_dim, scale, prefix=f"{prefix}.attn")
-        self._w_uk: Optional[torch.Tensor] = None
-        self._w_uv: Optional[torch.Tensor] = None
+        # what the two forms of the attention read
+        self.heads, self.dim, self.rot, self.kv_rank = self.local_heads, self.nope, self.rope_dim, self.kv_lora
+        self.scale, self.window = scale, 0
 
-    def _absorbed(self):
-        if self._w_uk is None or self._w_uk.device != self.kv_b_proj.weight.device:
-            w = self.kv_b_proj.weight.view(self.local_heads, self.nope + self.v_dim, self.kv_lora)
-            self._w_uk = w[:, :self.nope].contiguous()                       # [h, nope, R]
-            self._w_uv = w[:, self.nope:].transpose(1, 2).contiguous()       # [h, R, v]
-        return self._w_uk, self._w_uv
+    def _up(self) -> tuple[torch.Tensor, torch.Tensor]:
+        """(W_uk [h, nope, R], W_uv [h, v, R]): views of the stacked weight."""
+        w = self.kv_b_proj.weight.view(self.local_heads, self.nope + self.v_dim, self.kv_lora)
+        return w[:, :self.nope], w[:, self.nope:]
 
-    def process_weights_after_loading(self) -> None:
-        self._w_uk = self._w_uv = None
+    def _expand(self, c: torch.Tensor, h0: int, h1: int) -> tuple[torch.Tensor, torch.Tensor]:
+        n = self.nope + self.v_dim
+        kv = ops.linear(c, self.kv_b_proj.weight[h0 * n:h1 * n]).view(c.shape[0], h1 - h0, n)
+        return kv[..., :self.nope], kv[..., self.nope:]
+
+    def _fused(self, q: torch.Tensor, lat: torch.Tensor, md, cache) -> bool:
+        """Do the kernels of layers/latent.py take this step?  Not a captured mixed step (its plan needs lengths on the host), not
+        batch-invariant mode (the form depends on the portion), not a cache sharded by position."""
+        return (q.is_cuda and not envs.VLLM_B200_FORCE_REF_OPS and q.dtype in (torch.bfloat16, torch.float16) and cache.dtype == q.dtype
+                and (md.decode_only or not md.flat) and not ops.cuda_ops().batch_invariant() and get_dcp_group().world_size == 1
+                and self.rope.cos_sin_cache.shape[-1] == self.rope_dim and lat.stride(1) == 1 and q.stride(1) == 1)
 
     def forward(self, positions: torch.Tensor, hidden: torch.Tensor) -> torch.Tensor:
         T = hidden.shape[0]
@@ -85,18 +96,25 @@ class DeepseekMLA(nn.Module):
             q = self.q_b_proj(self.q_a_layernorm(self.q_a_proj(hidden)))
         else:
             q = self.q_proj(hidden)
+        lat = self.kv_a_proj_with_mqa(hidden)
+        md, cache = self.attn.bound_cache()
+        if md is not None and self._fused(q, lat, md, cache):
+            ops.cuda_ops().mla_rope_cache(q, lat, self.local_heads, self.nope, self.rope_dim, self.kv_lora, self.kv_a_layernorm.weight,
+                                          self.kv_a_layernorm.eps, positions, self.rope.cos_sin_cache, self.rope.is_neox_style, cache,
+                                          md.slot_mapping)
+            return self._attend(q.view(T, self.local_heads, self.q_head), md, cache).view(T, self.local_heads * self.v_dim)
         q = q.view(T, self.local_heads, self.q_head)
         q_nope, q_pe = q[..., :self.nope], q[..., self.nope:]
-        lat = self.kv_a_proj_with_mqa(hidden)
         kv_c = self.kv_a_layernorm(lat[:, :self.kv_lora].contiguous())
         k_pe = lat[:, self.kv_lora:].contiguous()
         q_pe, k_pe = self.rope(positions, q_pe.reshape(T, -1).contiguous(), k_pe)
         q_pe = q_pe.view(T, self.local_heads, self.rope_dim)
-        w_uk, w_uv = self._absorbed()
+        if md is None:
+            self._expand(kv_c, 0, self.local_heads)      # memory-profiling run: hold what expanding a batch of prompts would
+        w_uk, w_uv = self._up()
         q_abs = torch.einsum("thn,hnr->thr", q_nope, w_uk)
         o_lat = self.attn(q_abs, q_pe, kv_c, k_pe)                           # [T, h, R]
-        o = torch.einsum("thr,hrv->thv", o_lat, w_uv).reshape(T, self.local_heads * self.v_dim)
-        return o
+        return torch.einsum("thr,hvr->thv", o_lat, w_uv).reshape(T, self.local_heads * self.v_dim)
 
 
 class DeepseekMoE(nn.Module):
@@ -213,11 +231,7 @@ class DeepseekV3ForCausalLM(LlamaForCausalLM):
             if pname in params:
                 modules[pname.rsplit(".", 1)[0]].weight_loader(params[pname], w, shard, int(parts[0]))
                 loaded.add(pname)
-        loaded |= super().load_weights(dense)
-        for m in self.modules():
-            if isinstance(m, DeepseekMLA):
-                m.process_weights_after_loading()
-        return loaded
+        return loaded | super().load_weights(dense)
 
     @staticmethod
     def _expand_fused(weights):

@@ -233,14 +233,16 @@ def latent_expand_ok(q, dim: int, rot: int, v_dim: int, kv_rank: int) -> bool:
     return _use_cuda(q) and cuda_ops().mla_prefill_ok(q, dim, rot, v_dim, kv_rank)
 
 
-def gather_latents(kv_cache, block_table, cu_kv, num_kv: int, max_kv: int, starts=None):
-    """Cached rows of a batch of sequences (from position ``starts`` on), contiguous [num_kv, R] (CUDA)."""
+def gather_latents(kv_cache, block_table, cu_kv, num_kv: int, max_kv: int, starts=None, lens=None):
+    """Cached rows of a batch of sequences (from position ``starts`` on), contiguous [num_kv, R] (CUDA); with ``lens`` zeros behind them up to
+    the next sequence's first row."""
     out = torch.empty((num_kv, kv_cache.shape[-1]), dtype=kv_cache.dtype, device=kv_cache.device)
-    return cuda_ops().gather_cache(kv_cache, block_table, cu_kv, out, max_kv, starts)
+    return cuda_ops().gather_cache(kv_cache, block_table, cu_kv, out, max_kv, starts, lens=lens)
 
 
-def mla_prefill(q, k, v, out, q_start, q_len, seq_len, kv_start, h0: int, max_q: int, scale, k_pe=None, window: int = 0) -> None:
-    cuda_ops().mla_prefill(q, k, v, out, q_start, q_len, seq_len, kv_start, h0, max_q, scale, k_pe, window)
+def mla_prefill(q, k, v, out, q_start, q_len, seq_len, kv_start, h0: int, max_q: int, scale, k_pe=None, window: int = 0,
+                split: bool = False) -> None:
+    cuda_ops().mla_prefill(q, k, v, out, q_start, q_len, seq_len, kv_start, h0, max_q, scale, k_pe, window, split)
 
 
 def latent_rope_cache(proj, q_off, heads, dim, rot, kv_off, kv_rank, kv_weight, eps, positions, cos_sin, neox, cache=None, slots=None) -> None:

@@ -520,11 +520,11 @@ def merge_attn_states(o1, lse1, o2, lse2):
 
 _mla_decode = _sig("vb_mla_decode", _vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i64, _i64,
                    _i64, _i64, _i64, _i, _i, _i, _f, _i, _vp)
-_mla_prefill = _sig("vb_mla_prefill", _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i64, _i, _i, _i, _i, _i, _i, _i64, _i64,
-                    _i64, _i64, _i64, _i, _i, _f, _i, _vp)
+_mla_prefill = _sig("vb_mla_prefill2", _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i64, _i, _i, _i, _i, _i, _i, _i64, _i64,
+                    _i64, _i64, _i64, _i64, _i64, _i, _i, _f, _i, _i, _vp)
 _mla_simt = _sig("vb_mla_simt", _vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _i, _i, _i, _i, _i, _i, _i64, _i64, _i64, _i64, _i64,
                  _i64, _i, _f, _i, _vp)
-_latent_rope = _sig("vb_latent_rope_cache", _vp, _vp, _i64, _i, _i, _i, _i, _vp, _f, _vp, _vp, _i, _vp, _i64, _vp, _i, _i, _vp)
+_latent_rope = _sig("vb_latent_rope_cache2", _vp, _vp, _i64, _i64, _i, _i, _i, _i, _vp, _f, _vp, _vp, _i, _vp, _i64, _vp, _i, _i, _vp)
 _latent_norm = _sig("vb_latent_norm_cache", _vp, _i64, _i, _vp, _vp, _i, _vp, _vp, _vp, _i64, _vp, _i, _f, _i, _vp)
 _mla_ws: dict[int, tuple] = {}
 _kernel_error: dict[int, torch.Tensor] = {}
@@ -633,22 +633,23 @@ def mla_prefill_ok(q, dim: int, rot: int, v_dim: int, kv_lora_rank: int) -> bool
             and envs.VLLM_B200_ATTN != "simt")
 
 
-def mla_prefill(q, k, v, out, q_start, q_len, seq_len, kv_start, h0: int, max_q: int, scale, k_pe=None, window: int = 0) -> None:
+def mla_prefill(q, k, v, out, q_start, q_len, seq_len, kv_start, h0: int, max_q: int, scale, k_pe=None, window: int = 0,
+                split: bool = False) -> None:
     """Causal attention of prompt portions over expanded keys and values (csrc/mla_prefill.cu), written into ``out``.
-    q [T, H, dim + rot], out [T, H, vdim]; k [KV, hl, dim], v [KV, hl, vdim] hold heads h0 .. h0 + hl - 1, k_pe [KV, rot] the rotated key
-    part of all heads (None: rot = 0)."""
+    q [T, H, dim + rot], out [T, H, vdim]; k [KV, hl, dim], v [KV, hl, vdim] hold heads h0 .. h0 + hl - 1 (row and head strides free), k_pe
+    [KV, rot] the rotated key part of all heads (None: rot = 0).  ``split``: the softmax weights keep 16 more bits."""
     T, H, DQ = q.shape
     KV, hl, D = k.shape
     VD, P = v.shape[-1], 0 if k_pe is None else k_pe.shape[-1]
     assert DQ == D + P and (k_pe is None or (k_pe.stride(1) == 1 and k_pe.data_ptr() % 16 == 0))
-    assert q.stride(2) == 1 and q.stride(1) == DQ and k.stride(2) == 1 and k.stride(1) == D and v.stride(2) == 1 and v.stride(1) == VD
+    assert q.stride(2) == 1 and q.stride(1) == DQ and k.stride(2) == 1 and v.stride(2) == 1
     assert out.shape == (T, H, VD) and out.stride(1) == VD and out.stride(2) == 1
     for t in (q, k, v, out):
         assert t.data_ptr() % 16 == 0
     _check(_mla_prefill(q.data_ptr(), k.data_ptr(), v.data_ptr(), _p(k_pe), out.data_ptr(), q_start.data_ptr(), q_len.data_ptr(),
                         seq_len.data_ptr(), kv_start.data_ptr(), kernel_error_flag(q.device).data_ptr(), q_len.numel(), T, KV, H,
-                        h0, hl, D, P, VD, q.stride(0), k.stride(0), v.stride(0), 0 if k_pe is None else k_pe.stride(0), out.stride(0), max_q,
-                        window, scale, _DT[q.dtype], _st()),
+                        h0, hl, D, P, VD, q.stride(0), k.stride(0), k.stride(1), v.stride(0), v.stride(1),
+                        0 if k_pe is None else k_pe.stride(0), out.stride(0), max_q, window, scale, int(split), _DT[q.dtype], _st()),
            f"mla_prefill(T={T},KV={KV},H={H})")
 
 
@@ -659,9 +660,19 @@ def latent_rope_cache(proj, q_off: int, heads: int, dim: int, rot: int, kv_off: 
     if cache is not None:
         assert cache.shape[-1] == kv_rank + rot and cache.dtype == proj.dtype and cache.is_contiguous() and slots.dtype == torch.int64
     es = proj.element_size()
-    _check(_latent_rope(proj.data_ptr() + q_off * es, proj.data_ptr() + kv_off * es if kv_rank else None, proj.stride(0), heads, dim, rot,
+    _check(_latent_rope(proj.data_ptr() + q_off * es, proj.data_ptr() + kv_off * es if kv_rank else None, proj.stride(0), proj.stride(0), heads, dim, rot,
                         kv_rank, _p(kv_weight), eps, _p(positions), _p(cos_sin), int(neox), _p(cache), kv_rank + rot,
                         _p(slots) if cache is not None else None, proj.shape[0], _DT[proj.dtype], _st()), "latent_rope_cache")
+
+
+def mla_rope_cache(q, lat, heads: int, dim: int, rot: int, kv_rank: int, kv_weight, eps: float, positions, cos_sin, neox: bool, cache, slots) -> None:
+    """``latent_rope_cache`` with queries [T, heads * (dim + rot)] and latents [T, kv_rank + rot] in two matrices: rotates the queries in
+    place and writes normed latents and rotated key parts into their cache rows."""
+    assert q.dim() == 2 and q.stride(1) == 1 and lat.stride(1) == 1 and q.dtype == lat.dtype == cache.dtype and kv_weight.dtype == q.dtype
+    assert cos_sin.shape[-1] == rot and cache.shape[-1] == kv_rank + rot and cache.is_contiguous() and slots.dtype == torch.int64
+    _check(_latent_rope(q.data_ptr(), lat.data_ptr(), q.stride(0), lat.stride(0), heads, dim, rot, kv_rank, kv_weight.data_ptr(), eps,
+                        positions.data_ptr(), cos_sin.data_ptr(), int(neox), cache.data_ptr(), kv_rank + rot, slots.data_ptr(), q.shape[0],
+                        _DT[q.dtype], _st()), "mla_rope_cache")
 
 
 def latent_norm_cache(lat, q_rank: int, q_weight, kv_rank: int, kv_weight, eps: float, cache=None, slots=None, want_kv: bool = True):
@@ -1526,7 +1537,7 @@ def fused_qk_norm_rope(positions, q, k, q_weight, k_weight, cos_sin_cache, head_
 
 # ------------------------------------------------------------------ cache maintenance (csrc/cache_ops.cu)
 _copy_blocks = _sig("vb_copy_blocks", _vp, _vp, _vp, _i, _i64, _vp)
-_gather_cache = _sig("vb_gather_cache", _vp, _vp, _vp, _i64, _vp, _vp, _i, _i, _i, _i, _i64, _i64, _f, _i, _i, _vp)
+_gather_cache = _sig("vb_gather_cache2", _vp, _vp, _vp, _i64, _vp, _vp, _vp, _i, _i, _i, _i, _i64, _i64, _f, _i, _i, _vp)
 _convert_fp8 = _sig("vb_convert_fp8", _vp, _vp, _i64, _f, _i, _i, _i, _vp)
 
 
@@ -1552,14 +1563,14 @@ def copy_blocks(cache: torch.Tensor, mapping) -> None:
     swap_blocks(cache, cache, mapping)
 
 
-def gather_cache(cache, block_table, cu_seq_lens, out, max_tokens: int, seq_starts=None, scale: float = 1.0):
+def gather_cache(cache, block_table, cu_seq_lens, out, max_tokens: int, seq_starts=None, scale: float = 1.0, lens=None):
     """Dense [total_tokens, row] copy of the cached rows of a batch (cache [blocks, BS, row], fp8 → out.dtype with
-    ``scale`` when the cache is 8-bit)."""
+    ``scale`` when the cache is 8-bit).  ``lens``: rows of each sequence that are cached, zeros fill the rest of its range."""
     B = cu_seq_lens.numel() - 1
     BS, row = cache.shape[1], cache.shape[2]
     src8 = cache.element_size() == 1
     _check(_gather_cache(cache.data_ptr(), out.data_ptr(), block_table.data_ptr(), block_table.stride(0),
-                         cu_seq_lens.data_ptr(), _p(seq_starts), B, max_tokens, BS, row, cache.stride(0), out.stride(0),
+                         cu_seq_lens.data_ptr(), _p(seq_starts), _p(lens), B, max_tokens, BS, row, cache.stride(0), out.stride(0),
                          scale, int(src8), _DT[out.dtype], _st()), "gather_cache")
     return out
 
