@@ -1,0 +1,54 @@
+"""Grouped GEMM of prompt-sized expert batches: edges of tiles, empty experts, gated activations."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(x, y):
+    return float((x.double() - y.double()).norm() / y.double().norm())
+
+
+@pytest.mark.parametrize("rows,N,K", [([0, 1, 127, 128, 129, 0, 300], 512, 256), ([640], 208, 72), ([5, 700] * 20, 96, 1032),
+                                      ([257, 0, 0, 90], 1040, 64)])
+@pytest.mark.parametrize("act", [None, "silu", "gelu", "gelu_tanh"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_grouped_rows(rows, N, K, act, dtype):
+    from vllm_b200.ops import cuda as cu
+    g = torch.Generator(device="cuda").manual_seed(1)
+    R, E = sum(rows), len(rows)
+    x = torch.randn(R, K, device="cuda", generator=g).to(dtype)
+    w = (torch.randn(E, N, K, device="cuda", generator=g) * K ** -0.5).to(dtype)
+    offs = torch.tensor([sum(rows[:i]) for i in range(E + 1)], dtype=torch.int32, device="cuda")
+    got = cu.gemm_grouped(x, w, offs, act)
+    cu.check_kernel_error(x.device)
+    fn = {"silu": torch.nn.functional.silu, "gelu": torch.nn.functional.gelu,
+          "gelu_tanh": lambda z: torch.nn.functional.gelu(z, approximate="tanh")}
+    want = []
+    for xe, we in zip(x.split(rows), w):
+        h = xe.double() @ we.double().t()
+        want.append(h if act is None else fn[act](h[:, :N // 2]) * h[:, N // 2:])
+    # one rounding of the result: at most 2^-9 (bf16) or 2^-12 (fp16) of each value
+    assert _rel(got, torch.cat(want)) < (2 ** -9 if dtype == torch.bfloat16 else 2 ** -11)
+
+
+@pytest.mark.parametrize("T,E,k", [(300, 8, 4), (600, 4, 2), (2100, 64, 8)])
+@pytest.mark.parametrize("mapped", [False, True])
+def test_prompt_experts_match_decode_experts(T, E, k, mapped):
+    """The device path of large batches against the one of small batches, a few tokens at a time."""
+    from vllm_b200.ops import moe
+    g = torch.Generator(device="cuda").manual_seed(2)
+    H, inter = 256, 192
+    rnd = lambda *s, scale=1.0: (torch.randn(*s, device="cuda", generator=g) * scale).to(torch.bfloat16)  # noqa: E731
+    x, w13, w2 = rnd(T, H), rnd(E, 2 * inter, H, scale=H ** -0.5), rnd(E, H, inter, scale=inter ** -0.5)
+    ids = torch.rand(T, E, device="cuda", generator=g).topk(k, -1).indices.int()
+    w = torch.rand(T, k, device="cuda", generator=g)
+    emap = None
+    if mapped:                                  # experts of other ranks are dropped
+        emap = torch.full((2 * E,), -1, dtype=torch.int32, device="cuda")
+        emap[E // 2:E // 2 + E] = torch.arange(E, dtype=torch.int32, device="cuda")
+        ids = ids + (torch.arange(T, device="cuda") % 3 == 0).int()[:, None] * (E // 2)
+    got = moe.fused_moe_cuda(x, w13, w2, w, ids, "silu", emap)
+    n = moe.GROUPED_MAX_ROWS // k
+    want = torch.cat([moe.fused_moe_cuda(x[i:i + n], w13, w2, w[i:i + n], ids[i:i + n], "silu", emap) for i in range(0, T, n)])
+    assert _rel(got, want) < 2 ** -7            # hidden rows rounded to bf16 on one side only, and both results

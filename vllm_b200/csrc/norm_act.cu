@@ -4,7 +4,7 @@
 // fused_add_rms_norm), activation_kernels.cu (silu_and_mul, gelu_and_mul, ...).
 // Our variants: one CTA per token, 16-byte vector access, the row stays in
 // registers between the reduction and the scale pass (single HBM read), fp32 math.
-#include "common.cuh"
+#include "act.cuh"
 
 namespace {
 
@@ -104,20 +104,6 @@ __global__ void __launch_bounds__(1024) layer_norm_kernel(T* __restrict__ out, c
       st16(out + row * H + vi * N, o);
     }
   }
-}
-
-enum : int { ACT_SILU = 0, ACT_GELU = 1, ACT_GELU_TANH = 2, ACT_RELU = 3, ACT_GELU_NEW = 4, ACT_GELU_FAST = 5,
-             ACT_QUICK_GELU = 6, ACT_RELU2 = 7 };
-
-template <int ACT> VB_DEVICE float act_fn(float x) {
-  if (ACT == ACT_SILU) return x / (1.f + __expf(-x));
-  if (ACT == ACT_GELU) return 0.5f * x * (1.f + erff(x * 0.70710678118654752f));
-  if (ACT == ACT_GELU_TANH || ACT == ACT_GELU_NEW)
-    return 0.5f * x * (1.f + tanhf(0.7978845608028654f * (x + 0.044715f * x * x * x)));
-  if (ACT == ACT_GELU_FAST) return 0.5f * x * (1.f + tanhf(x * 0.7978845608f * (1.f + 0.044715f * x * x)));
-  if (ACT == ACT_QUICK_GELU) return x / (1.f + __expf(-1.702f * x));
-  if (ACT == ACT_RELU2) { float r = fmaxf(x, 0.f); return r * r; }
-  return fmaxf(x, 0.f);
 }
 
 // out[t, :d] = act(x[t, :d]) * x[t, d:2d]

@@ -1074,6 +1074,7 @@ _comm_ar_rows2 = _sig("vb_comm_allreduce_rows2", _vp, _vp, _vp, _vp, _i, _i, _vp
 _moe_combine = _sig("vb_moe_combine", _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp)
 _moe_gather = _sig("vb_moe_gather", _vp, _vp, _vp, _i, _i, _i, _vp)
 _gemm_grouped = _sig("vb_gemm_tc_grouped2", _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp)
+_gemm_grouped_rows = _sig("vb_gemm_grouped", _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp)
 _grouped_simt = _sig("vb_moe_grouped_simt", _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp)
 _grouped_topk = _sig("vb_moe_grouped_topk", _vp, _vp, _i, _vp, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _vp)
 _GROUPED_ACT = {None: 0, "none": 0, "relu2": 2}
@@ -1167,6 +1168,21 @@ def gemm_tc_grouped(xs: torch.Tensor, w: torch.Tensor, offs: torch.Tensor, bn: i
     y = torch.empty((R, N), dtype=xs.dtype, device=xs.device)
     _check(_gemm_grouped(xs.data_ptr(), w.data_ptr(), y.data_ptr(), offs.data_ptr(), R, N, K, E, bn, _GROUPED_ACT[act], int(flat),
                          _DT[xs.dtype], _st()), f"gemm_tc_grouped(R={R},N={N},K={K},E={E})")
+    return y
+
+
+_GATED_ACT = {None: -1, "silu": 0, "swish": 0, "gelu": 1, "gelu_tanh": 2, "gelu_pytorch_tanh": 2}
+
+
+def gemm_grouped(xs: torch.Tensor, w: torch.Tensor, offs: torch.Tensor, act: Optional[str] = None) -> torch.Tensor:
+    """The same for hundreds of rows per expert (csrc/gemm_grouped.cu).  ``act``: w [E, 2 I, K] holds gates and ups, Y [R, I] =
+    act(gate) * up."""
+    R, K = xs.shape
+    E, N, _ = w.shape
+    assert xs.is_contiguous() and w.is_contiguous() and xs.dtype == w.dtype and w.shape[2] == K
+    y = torch.empty((R, N if act is None else N // 2), dtype=xs.dtype, device=xs.device)
+    _check(_gemm_grouped_rows(xs.data_ptr(), w.data_ptr(), y.data_ptr(), offs.data_ptr(), kernel_error_flag(xs.device).data_ptr(), R, N, K, E,
+                              _GATED_ACT[act], num_sms(), _DT[xs.dtype], _st()), f"gemm_grouped(R={R},N={N},K={K},E={E})")
     return y
 
 

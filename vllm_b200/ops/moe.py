@@ -1,8 +1,8 @@
 """MoE expert computation on CUDA.
 
-Current implementation: sort tokens by expert (torch), run one GEMM pair per active expert through
-``ops.linear`` (tcgen05 kernel for small per-expert M, cuBLASLt otherwise) and scatter-add back.
-The grouped tcgen05 kernel with fused dispatch/combine replaces the loop (see csrc/moe.cu).
+16-bit experts stay on the device at every batch size: counting sort by expert, gather, grouped tcgen05 GEMMs (swap-AB tiles of few tokens for
+decode steps, csrc/gemm_tc.cu; 128 x 256 tiles for prompts, csrc/gemm_grouped.cu), weighted combine.  What the tensor-core kernels do
+not take runs one GEMM pair per active expert.
 """
 from __future__ import annotations
 
@@ -12,6 +12,10 @@ import torch
 
 
 GROUPED_MAX_ROWS = 1024      # (token, expert) pairs handled by the single-pass grouped kernels
+# Pairs per expert from which the 128-row tiles of csrc/gemm_grouped.cu are the better form.  Both products of gated experts, swap-AB tiles →
+# 128 x 256 tiles, us: width 2048, 32 experts of 768: 85 → 92 at 37 pairs each, 107 → 94 at 75, 838 → 406 at 1536; 64 experts of 768: 155 → 134
+# at 50; 8 of 2048: 79 → 84 at 100, 103 → 90 at 200; width 1024, 16 of 512: 54 → 57 at 100, 85 → 70 at 400.
+PROMPT_ROWS = 64
 
 
 def _grouped_ok(x, w13, w2, R: int) -> bool:
@@ -61,6 +65,10 @@ def expert_rows(x, w13, w2, topk_ids, act, expert_map, gated: bool):
     return expert_rows_gated(x, w13, w2, topk_ids, act, expert_map) if gated else expert_rows_plain(x, w13, w2, topk_ids, act, expert_map)
 
 
+def _rows_ok(x, w13) -> bool:
+    return x.dtype in (torch.bfloat16, torch.float16) and w13.dtype == x.dtype and w13.shape[2] % 8 == 0 and w13.shape[1] % 16 == 0
+
+
 def expert_rows_gated(x, w13, w2, topk_ids, act, expert_map):
     """Experts act(gate) * up → down; ``expert_rows_plain`` with the activation as a kernel between the two grouped GEMMs."""
     from vllm_b200.ops import cuda as cu
@@ -69,7 +77,9 @@ def expert_rows_gated(x, w13, w2, topk_ids, act, expert_map):
     ids = topk_ids if topk_ids.dtype == torch.int32 else topk_ids.to(torch.int32)
     sorted_tok, inv, offs = cu.moe_align(ids.contiguous(), E, expert_map)
     x = x.contiguous()
-    if x.dtype in (torch.bfloat16, torch.float16) and w13.dtype == x.dtype and K % 8 == 0 and N % 16 == 0:
+    if _rows_ok(x, w13):
+        if R >= PROMPT_ROWS * E and R > GROUPED_MAX_ROWS and act in cu._GATED_ACT:
+            return cu.gemm_grouped(cu.gemm_grouped(cu.moe_gather(x, sorted_tok), w13, offs, act), w2, offs), inv
         bn = _tile_width(R, E)
         h = cu.gemm_tc_grouped(cu.moe_gather(x, sorted_tok), w13, offs, bn, flat=True)
         return cu.gemm_tc_grouped(cu.act_and_mul(h, act), w2, offs, bn, flat=True), inv
@@ -200,11 +210,14 @@ def fused_moe_reduce_norm(x, w13, w2, topk_w, topk_ids, act, expert_map, residua
 
 
 def fused_moe_cuda(x, w13, w2, topk_w, topk_ids, act="silu", expert_map: Optional[torch.Tensor] = None):
-    from vllm_b200 import ops
+    from vllm_b200 import envs, ops
     if _grouped_ok(x, w13, w2, topk_ids.numel()):
         return fused_moe_grouped(x, w13, w2, topk_w, topk_ids, act, expert_map)
     T, H = x.shape
     E = w13.shape[0]
+    if (_rows_ok(x, w13) and w2.dtype == x.dtype and w13.is_contiguous() and w2.is_contiguous() and E <= 512
+            and topk_ids.numel() > GROUPED_MAX_ROWS and envs.VLLM_B200_GEMM != "cublas"):
+        return fused_moe_rows(x, w13, w2, topk_w, topk_ids, act, expert_map, True)
     k = topk_ids.shape[1]
     ids = topk_ids.long()
     if expert_map is not None:
