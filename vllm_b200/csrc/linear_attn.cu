@@ -579,7 +579,8 @@ template <typename T, int V>
 __global__ void __launch_bounds__(1024) gated_norm_kernel(const float* __restrict__ y, int y_row, const T* __restrict__ z,
                                                            int64_t z_stride, const T* __restrict__ w, int w_len, T* __restrict__ out,
                                                            int64_t out_stride, int64_t n_rows, int groups, int W, int gate_first,
-                                                           int sigmoid_gate, RowDivisor by, float eps, float scale, int wpg) {
+                                                           int sigmoid_gate, RowDivisor by, float eps, float scale, int wpg, int z_run,
+                                                           int64_t z_group) {
   __shared__ float red[32];
   pdl_trigger();
   pdl_wait();
@@ -590,7 +591,7 @@ __global__ void __launch_bounds__(1024) gated_norm_kernel(const float* __restric
   const int64_t tok = ok ? row / groups : 0;
   const int g = ok ? (int)(row - tok * groups) : 0;
   const float* yr = y + (tok * groups + g) * (int64_t)y_row;
-  const T* zr = z + tok * z_stride + (int64_t)g * W;
+  const T* zr = z + tok * z_stride + g / z_run * z_group + (int64_t)(g % z_run) * W;
   const int i0 = ((warp % wpg) * 32 + lane) * V, step = wpg * 32 * V;
   constexpr int dt = DTypeOf<T>::v;
   const float f = by.gates && ok ? 1.f / (fmaxf(fabsf(yr[by.n_col]), by.gates[row].z) + 1e-6f) : 1.f;
@@ -832,24 +833,26 @@ EXPORT int vb_gla_decay(const void* a1, int64_t a1_stride, const void* a2, const
 
 // y [T, groups * W] fp32, z [T, groups * W] (token stride free), w [w_len] repeated along the channels (w_len a multiple or
 // a divisor of W); out [T, groups * W] in the model dtype (token stride free).  flags: bit0 gate first, bit1 sigmoid gate (else
-// silu).  gates not null: y holds the rows [T, groups, CO] of vb_memory_scan and gates its gates.
-EXPORT int vb_gated_norm(const float* y, const float* gates, const void* z, int64_t z_stride, const void* w, int w_len, void* out,
-                         int64_t out_stride, int T_, int groups, int W, int flags, float eps, float scale, int dtype,
-                         cudaStream_t st) {
+// silu).  gates not null: y holds the rows [T, groups, CO] of vb_memory_scan and gates its gates.  z_run > 0: after so many groups' gates
+// the next ones are z_group columns further than the first of these.
+EXPORT int vb_gated_norm2(const float* y, const float* gates, const void* z, int64_t z_stride, int z_run, int64_t z_group, const void* w, int w_len,
+                          void* out, int64_t out_stride, int T_, int groups, int W, int flags, float eps, float scale, int dtype,
+                          cudaStream_t st) {
   using namespace lattn;
   if (T_ == 0) return 0;
   const int64_t rows = (int64_t)T_ * groups;
   const int e = esz(dtype);
   const int n_col = (W + 3) / 4 * 4, y_row = gates ? n_col + 4 : W;
   const RowDivisor by = {reinterpret_cast<const float4*>(gates), n_col};
-  const bool vec = W % 4 == 0 && w_len % 4 == 0 && z_stride % 4 == 0 && out_stride % 4 == 0 && al(y, 16) && al(z, 4 * e) &&
+  if (z_run <= 0) { z_run = groups; z_group = 0; }
+  const bool vec = W % 4 == 0 && w_len % 4 == 0 && z_stride % 4 == 0 && z_group % 4 == 0 && out_stride % 4 == 0 && al(y, 16) && al(z, 4 * e) &&
                    al(w, 4 * e) && al(out, 4 * e);
   const int per_warp = vec ? 32 * 4 * GN_NV : 32 * GN_NV;
   int wpg = 1;
   while (wpg < 32 && wpg * per_warp < W) wpg *= 2;
   const int warps = wpg > 8 ? wpg : 8, per_cta = warps / wpg;
   dim3 grid((unsigned)((rows + per_cta - 1) / per_cta)), block(warps * 32);
-#define GO(V) vb_launch(gated_norm_kernel<T, V>, grid, block, 0, st, y, y_row, (const T*)z, z_stride, (const T*)w, w_len, (T*)out, out_stride, rows, groups, W, flags & 1, flags >> 1 & 1, by, eps, scale, wpg)
+#define GO(V) vb_launch(gated_norm_kernel<T, V>, grid, block, 0, st, y, y_row, (const T*)z, z_stride, (const T*)w, w_len, (T*)out, out_stride, rows, groups, W, flags & 1, flags >> 1 & 1, by, eps, scale, wpg, z_run, z_group)
   DISPATCH_DTYPE(dtype, T, { if (vec) GO(4); else GO(1); });
 #undef GO
   return (int)cudaGetLastError();

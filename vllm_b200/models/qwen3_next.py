@@ -5,9 +5,8 @@ Reference parity: vllm/model_executor/models/qwen3_next.py, layers/mamba/ (GDN m
 ``chunk_gated_delta_rule`` kernels, causal conv1d), csrc/gdn/fused_gdn_decode_kernel.cu.
 
 State cache: one pool block per request and GDN layer holding ``[conv_state (conv_dim x (k-1)) | S (heads x d_k x d_v)]``
-in fp32 (same ``MambaSpec`` mechanism as the SSM mixers).  Decode batches are one vectorised rank-1 state update per
-head (graph-capturable); prefill walks the segment token by token through the same update (the chunked WY form is the
-planned tcgen05 kernel — the recurrence is exact and is what the decode kernel computes anyway).
+in fp32 (same ``MambaSpec`` mechanism as the SSM mixers).  One kernel walks prompts and decode steps through the recurrence (csrc/gdn.cu,
+graph-capturable); without a GPU decode batches are one vectorised rank-1 update per head and prompts go token by token.
 """
 from __future__ import annotations
 
@@ -114,9 +113,23 @@ class GatedDeltaNet(nn.Module):
         ctx = get_forward_context()
         md = ctx.metadata_for(self.layer_name)
         cache = ctx.kv_caches.get(self.layer_name)
-        q, k, v, z, b, a = self._split(self.in_proj_qkvz(hidden), self.in_proj_ba(hidden))
-        qkv = torch.cat([q, k, v], dim=-1)
+        qkvz, ba = self.in_proj_qkvz(hidden), self.in_proj_ba(hidden)
         T, dev = hidden.shape[0], hidden.device
+        from vllm_b200.layers.mamba import _cuda_ssm
+        if md is not None and cache is not None and _cuda_ssm(qkvz) and self.dk % 32 == 0 and self.dk <= 256 and 2 <= self.k <= 4:
+            # device path (csrc/ssm.cu, gdn.cu): causal conv, gated delta rule over the cache pool, gated norm, any batch shape; all read
+            # the projections in the checkpoint's order
+            from vllm_b200.ops import cuda_ops
+            cu, r = cuda_ops(), self.nv // self.nk
+            group = 2 * self.dk + 2 * r * self.dv
+            conv = cu.causal_conv1d(qkvz, self.conv_weight, None, cache, md, heads=(group, self.nk, self.dk, r * self.dv))
+            o = cu.gated_delta(conv, ba, self.A_log, self.dt_bias, cache, self.conv_dim * (self.k - 1), md, self.nk, self.nv, self.dk, self.dv,
+                               self.beta_scale, 1e-6)
+            y = cu.gated_norm(o, qkvz[:, 2 * self.dk + r * self.dv:], self.norm_weight, self.nv, self.eps, False,
+                              z_heads=(self.value_dim, r, group))
+            return self.out_proj(y)
+        q, k, v, z, b, a = self._split(qkvz, ba)
+        qkv = torch.cat([q, k, v], dim=-1)
         out = torch.zeros(T, self.nv, self.dv, dtype=torch.float32, device=dev)
         if md is None or cache is None:
             out, _, _ = self._segment(qkv[:min(T, 8)], b[:min(T, 8)], a[:min(T, 8)],
@@ -124,16 +137,6 @@ class GatedDeltaNet(nn.Module):
                                       torch.zeros(self.nv, self.dk, self.dv, device=dev))
             out = torch.cat([out, torch.zeros(T - out.shape[0], self.nv, self.dv, device=dev)]) if T > out.shape[0] else out
             return self.out_proj(self._gated_norm(out, z).reshape(T, -1).to(hidden.dtype))
-        from vllm_b200.layers.mamba import _cuda_ssm
-        if _cuda_ssm(qkv) and self.dk % 32 == 0 and self.dk <= 256 and 2 <= self.k <= 4:
-            # device path (csrc/ssm.cu): causal conv + gated-delta-rule scan over the cache pool, any batch shape
-            from vllm_b200.ops import cuda_ops
-            cu = cuda_ops()
-            conv = cu.causal_conv1d(qkv, self.conv_weight, None, cache, md)
-            qh, kh, vh = self._qkv_heads(conv)
-            g = -self.A_log.exp() * F.softplus(a.float() + self.dt_bias)
-            o = cu.gdn_scan(qh, kh, vh, g, b.float().sigmoid() * self.beta_scale, cache, self.conv_dim * (self.k - 1), md)
-            return self.out_proj(self._gated_norm(o, z).reshape(T, -1).to(hidden.dtype))
         cache = cache.view(cache.shape[0], -1).view(torch.float32) if cache.dtype != torch.float32 else cache
         if md.decode_only:
             Bn = md.num_reqs

@@ -1607,7 +1607,7 @@ def convert_fp8(x: torch.Tensor, scale: float = 1.0, to_fp8: bool = True, out_dt
 
 
 # ------------------------------------------------------------------ SSM / linear attention (csrc/ssm.cu, linear_attn.cu)
-_conv1d = _sig("vb_causal_conv1d", _vp, _i64, _vp, _i64, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _i64, _i, _i, _i, _i, _i, _i, _vp)
+_conv1d = _sig("vb_causal_conv1d2", _vp, _i64, _vp, _i64, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _i64, _i, _i, _i, _i, _i, _i, _i, _i, _i, _i, _vp)
 _sel_scan = _sig("vb_selective_scan", _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _vp, _vp, _vp, _i64, _i, _i, _i,
                  _vp)
 _ssd_scan = _sig("vb_ssd_scan", _vp, _i64, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _vp, _vp, _vp, _i64, _i, _i, _i, _i,
@@ -1615,11 +1615,12 @@ _ssd_scan = _sig("vb_ssd_scan", _vp, _i64, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _
 _gla_scan = _sig("vb_gla_scan", _vp, _vp, _vp, _i64, _i64, _i64, _f, _vp, _vp, _i64, _vp, _vp, _i, _f, _vp, _vp, _i64, _i64, _vp, _vp,
                  _vp, _i64, _i, _i, _i, _i, _i, _i, _vp)
 _gla_decay = _sig("vb_gla_decay", _vp, _i64, _vp, _vp, _vp, _i, _i, _i, _f, _i, _vp)
-_gated_norm = _sig("vb_gated_norm", _vp, _vp, _vp, _i64, _vp, _i, _vp, _i64, _i, _i, _i, _i, _f, _f, _i, _vp)
+_gated_norm = _sig("vb_gated_norm2", _vp, _vp, _vp, _i64, _i, _i64, _vp, _i, _vp, _i64, _i, _i, _i, _i, _f, _f, _i, _vp)
 _memory_scan = _sig("vb_memory_scan", _vp, _vp, _vp, _i64, _i64, _i64, _f, _vp, _vp, _vp, _i64, _i64, _vp, _vp, _vp, _i64, _i, _i, _i, _i,
                     _i, _i, _vp)
 _memory_gates = _sig("vb_memory_gates", _vp, _i64, _vp, _i, _vp, _vp, _f, _vp, _vp, _i64, _i64, _vp, _vp, _vp, _i64, _i, _i, _i, _i, _vp)
-_gdn_scan = _sig("vb_gdn_scan", _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _vp, _vp, _vp, _i64, _i, _i, _i, _i, _vp)
+_gated_delta = _sig("vb_gated_delta", _vp, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _vp, _vp, _vp, _i64, _i, _i, _i,
+                    _i, _i, _f, _f, _f, _i, _vp)
 
 
 def _state_view(cache: torch.Tensor) -> torch.Tensor:
@@ -1628,17 +1629,20 @@ def _state_view(cache: torch.Tensor) -> torch.Tensor:
     return c if c.dtype == torch.float32 else c.view(torch.float32)
 
 
-def causal_conv1d(x, weight, bias, cache, md, act: bool = True) -> torch.Tensor:
+def causal_conv1d(x, weight, bias, cache, md, act: bool = True, heads: Optional[tuple] = None) -> torch.Tensor:
     """Depthwise causal conv over each request's tokens with the (k-1)-window kept at the head of its state row.
-    x [T, C] (any dtype and row stride) → fp32 [T, C]; the window in the cache is advanced in place."""
-    T, C = x.shape
+    x [T, C] (any dtype and row stride) → fp32 [T, C]; the window in the cache is advanced in place.  ``heads`` (group, nk, dk, rv): the
+    channels are q | k | v of all heads, x holds nk groups of ``group`` columns that begin with q : dk | k : dk | v : rv (rows of the result then
+    start on 16 bytes)."""
+    T, C = x.shape[0], weight.shape[0]
     st = _state_view(cache)
-    out = torch.empty((T, C), dtype=torch.float32, device=x.device)
+    out = torch.empty((T, C if heads is None else -(-C // 4) * 4), dtype=torch.float32, device=x.device)[:, :C]
     bt = md.block_table
-    assert x.stride(1) == 1 and weight.is_contiguous() and weight.dtype == x.dtype
+    assert x.stride(1) == 1 and weight.is_contiguous() and weight.dtype == x.dtype and (heads is not None or x.shape[1] == C)
+    assert heads is None or x.shape[1] >= heads[0] * heads[1]
     _check(_conv1d(x.data_ptr(), x.stride(0), out.data_ptr(), out.stride(0), weight.data_ptr(), _p(bias), st.data_ptr(),
                    st.stride(0), md.query_start_loc.data_ptr(), md.seq_lens.data_ptr(), bt.data_ptr(), bt.stride(0),
-                   md.num_reqs, T, C, weight.shape[-1], int(act), _DT[x.dtype], _st()), "causal_conv1d")
+                   md.num_reqs, T, C, weight.shape[-1], int(act), *(heads or (0, 0, 0, 0)), _DT[x.dtype], _st()), "causal_conv1d")
     return out
 
 
@@ -1731,19 +1735,21 @@ def memory_scan(q, k, v, gates, q_scale: float, cache, md, H: int, R: int, C: in
     return o.view(T, H, cols)
 
 
-def gated_norm(y, z, weight, groups: int, eps: float, gate_first: bool, out=None, scale: float = 1.0, gate: str = "silu", gates=None):
+def gated_norm(y, z, weight, groups: int, eps: float, gate_first: bool, out=None, scale: float = 1.0, gate: str = "silu", gates=None,
+               z_heads: Optional[tuple] = None):
     """y fp32 [T, n]: RMS norm over ``groups`` equal parts, silu(z) (``gate`` "sigmoid": sigmoid(z)) before (``gate_first``) or behind it,
     times the weight (repeated along the parts where it is shorter) and ``scale``; in z's dtype.  ``gates``: y is the result of
-    ``memory_scan`` with these gates, divided by its normaliser first."""
-    T, n = z.shape
+    ``memory_scan`` with these gates, divided by its normaliser first.  ``z_heads`` (n, run, stride): the n gates of a token begin at z's
+    columns in runs of ``run`` parts, ``stride`` columns apart."""
+    T, n = z.shape if z_heads is None else (z.shape[0], z_heads[0])
     if out is None:
         out = torch.empty((T, n), dtype=z.dtype, device=z.device)
     W = n // groups
     wl = weight.numel()
     assert y.is_contiguous() and z.stride(1) == 1 and out.stride(1) == 1 and weight.dtype == z.dtype and n % groups == 0 and n % wl == 0
     assert y.numel() == T * groups * (W if gates is None else -(-W // 4) * 4 + 4)
-    _check(_gated_norm(y.data_ptr(), _p(gates), z.data_ptr(), z.stride(0), weight.data_ptr(), wl, out.data_ptr(), out.stride(0), T, groups,
-                       W, int(gate_first) | 2 * int(gate == "sigmoid"), eps, scale, _DT[z.dtype], _st()), "gated_norm")
+    _check(_gated_norm(y.data_ptr(), _p(gates), z.data_ptr(), z.stride(0), *(z_heads[1:] if z_heads else (0, 0)), weight.data_ptr(), wl, out.data_ptr(),
+                       out.stride(0), T, groups, W, int(gate_first) | 2 * int(gate == "sigmoid"), eps, scale, _DT[z.dtype], _st()), "gated_norm")
     return out
 
 
@@ -1754,10 +1760,27 @@ def gdn_scan(q, k, v, g, beta, cache, state_off: int, md) -> torch.Tensor:
     st = _state_view(cache)
     o = torch.zeros((T, nv, dv), dtype=torch.float32, device=q.device)
     bt = md.block_table
-    a = [t.contiguous() for t in (q, k, v, g, beta)]
-    _check(_gdn_scan(*[t.data_ptr() for t in a], o.data_ptr(), st.data_ptr(), st.stride(0), state_off,
-                     md.query_start_loc.data_ptr(), md.seq_lens.data_ptr(), bt.data_ptr(), bt.stride(0), md.num_reqs, nv, dk,
-                     dv, _st()), "gdn_scan")
+    q, k, v, g, beta = (t.contiguous() for t in (q, k, v, g, beta))
+    _check(_gated_delta(q.data_ptr(), k.data_ptr(), nv * dk, v.data_ptr(), nv * dv, None, 0, None, None, g.data_ptr(), beta.data_ptr(), o.data_ptr(),
+                        st.data_ptr(), st.stride(0), state_off, md.query_start_loc.data_ptr(), md.seq_lens.data_ptr(), bt.data_ptr(),
+                        bt.stride(0), md.num_reqs, nv, nv, dk, dv, 1.0, 1.0, 0.0, 2, _st()), "gdn_scan")
+    return o
+
+
+def gated_delta(qkv, ba, A_log, dt_bias, cache, state_off: int, md, nk: int, nv: int, dk: int, dv: int, beta_scale: float, eps: float
+                ) -> torch.Tensor:
+    """The same from the convolved channels [T, 2 nk dk + nv dv] (q | k | v of all heads, fp32) and the raw gates ba [T, 2 nv] (per key head
+    its write strengths, then its decays): l2 norms, query scale, sigmoid and decay are evaluated in the scan (csrc/gdn.cu)."""
+    T = qkv.shape[0]
+    st = _state_view(cache)
+    o = _scan_out(T, nv * dv, md, qkv.device)
+    bt = md.block_table
+    assert qkv.dtype == A_log.dtype == dt_bias.dtype == torch.float32 and qkv.stride(1) == 1 and ba.stride(1) == 1
+    k, v = qkv[:, nk * dk:], qkv[:, 2 * nk * dk:]
+    _check(_gated_delta(qkv.data_ptr(), k.data_ptr(), qkv.stride(0), v.data_ptr(), qkv.stride(0), ba.data_ptr(), ba.stride(0), A_log.data_ptr(),
+                        dt_bias.data_ptr(), None, None, o.data_ptr(), st.data_ptr(), st.stride(0), state_off, md.query_start_loc.data_ptr(),
+                        md.seq_lens.data_ptr(), bt.data_ptr(), bt.stride(0), md.num_reqs, nk, nv, dk, dv, dk ** -0.5, beta_scale, eps,
+                        _DT[ba.dtype], _st()), "gated_delta")
     return o
 
 
