@@ -103,6 +103,77 @@ __global__ void select_candidate_kernel(const float4* __restrict__ cands, int W,
   out[row] = best.i == 0x7fffffff ? 0 : best.i;
 }
 
+// Log-probabilities of a row's sampled token and of its k likeliest: out [B, 2 k + 3] holds the k + 1 ids (the sampled one first), their log
+// softmax (fp32 bits) and the sampled token's rank (tokens that are likelier, plus one).  One CTA per row; the row is read three times,
+// the last two from L1 / L2.  The k likeliest are taken one by one: every thread keeps the best of its own elements, and only the one
+// whose element was taken looks for its next (ties: the lowest index first).  A dozen library launches (log softmax, gather, compare and
+// sum, four-pass radix top-k, concatenations) took 45 us for 24 rows of 32000.
+template <typename T>
+__global__ void __launch_bounds__(1024) logprobs_kernel(const T* __restrict__ logits, int64_t row_stride, int V, const int64_t* __restrict__ sampled,
+                                                         int k, int* __restrict__ out) {
+  constexpr int N = Vec16<T>::N;
+  __shared__ float sv[32];
+  __shared__ int si[32];
+  __shared__ float red[32];
+  pdl_trigger();
+  pdl_wait();
+  const int row = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const T* lr = logits + (int64_t)row * row_stride;
+  const int nvec = V / N, tail = nvec * N;
+  auto each = [&](auto f) {
+    for (int vi = threadIdx.x; vi < nvec; vi += blockDim.x) {
+      const Vec16<T> v = ld16(lr + vi * N);
+#pragma unroll
+      for (int j = 0; j < N; ++j) f(to_f32(v.e[j]), vi * N + j);
+    }
+    for (int i = tail + threadIdx.x; i < V; i += blockDim.x) f(to_f32(lr[i]), i);
+  };
+  ArgMax best{-INFINITY, 0x7fffffff};
+  each([&](float x, int i) { best = better(best, ArgMax{x, i}); });
+  auto top = [&]() {                       // best of the block, in every thread
+    ArgMax b = best;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) b = better(b, ArgMax{__shfl_xor_sync(0xffffffffu, b.v, o), __shfl_xor_sync(0xffffffffu, b.i, o)});
+    __syncthreads();
+    if (lane == 0) { sv[w] = b.v; si[w] = b.i; }
+    __syncthreads();
+    b = lane < nw ? ArgMax{sv[lane], si[lane]} : ArgMax{-INFINITY, 0x7fffffff};
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) b = better(b, ArgMax{__shfl_xor_sync(0xffffffffu, b.v, o), __shfl_xor_sync(0xffffffffu, b.i, o)});
+    return b;
+  };
+  ArgMax t = top();
+  const float mx = t.v;
+  float sum = 0.f;
+  each([&](float x, int) { sum += expf(x - mx); });
+  const float lsum = logf(block_sum(sum, red));
+  const int64_t pick = sampled[row];
+  const int sidx = (int)(pick < 0 ? 0 : pick >= V ? V - 1 : pick);
+  const float slp = (to_f32(lr[sidx]) - mx) - lsum;
+  float above = 0.f;
+  each([&](float x, int) { above += (x - mx) - lsum > slp ? 1.f : 0.f; });       // counts below 2^24 are exact
+  above = block_sum(above, red);
+  int* o = out + (int64_t)row * (2 * k + 3);
+  if (threadIdx.x == 0) {
+    o[0] = (int)pick;
+    o[k + 1] = __float_as_int(slp);
+    o[2 * k + 2] = (int)above + 1;
+  }
+  for (int r = 0; r < k; ++r) {
+    if (threadIdx.x == 0) {
+      o[1 + r] = t.i == 0x7fffffff ? 0 : t.i;
+      o[k + 2 + r] = __float_as_int((t.v - mx) - lsum);
+    }
+    if (r + 1 == k) break;
+    if (best.i == t.i) {                   // the owner of the taken element: its next one in order
+      const ArgMax old = t;
+      best = ArgMax{-INFINITY, 0x7fffffff};
+      each([&](float x, int i) { if (x < old.v || (x == old.v && i > old.i)) best = better(best, ArgMax{x, i}); });
+    }
+    t = top();
+  }
+}
+
 // In-place top-k / top-p / min-p masking of fp32 logits (already divided by temperature).
 // Per row: find the k-th largest value and the top-p probability threshold with a bisection on
 // the value axis (each pass is one streaming read from L2/SMEM-resident row), then mask.
@@ -286,5 +357,13 @@ EXPORT int vb_row_lse(const void* logits, int64_t row_stride, int B, int V, floa
   DISPATCH_DTYPE(dtype, TT, {
     row_lse_kernel<TT><<<B, 1024, 0, st>>>((const TT*)logits, row_stride, V, out);
   });
+  return (int)cudaGetLastError();
+}
+
+// k <= V; rows 16-byte aligned (row_stride a multiple of 16 bytes)
+EXPORT int vb_logprobs(const void* logits, int64_t row_stride, int B, int V, const int64_t* sampled, int k, int* out, int dtype, cudaStream_t st) {
+  if (B == 0) return 0;
+  if (k < 0 || k > V) return -1;
+  DISPATCH_DTYPE(dtype, T, vb_launch(logprobs_kernel<T>, dim3(B), dim3(1024), 0, st, reinterpret_cast<const T*>(logits), row_stride, V, sampled, k, out));
   return (int)cudaGetLastError();
 }

@@ -749,6 +749,26 @@ def select_candidates(cands: torch.Tensor, W: int, out: torch.Tensor) -> torch.T
     return out
 
 
+_logprobs = _sig("vb_logprobs", _vp, _i64, _i, _i, _vp, _i, _vp, _i, _vp)
+MAX_LOGPROBS = 64       # likeliest tokens that the one-launch kernel picks one by one; more are sorted
+
+
+def logprobs_ok(V: int, k: int) -> bool:
+    return 0 <= k <= min(MAX_LOGPROBS, V)
+
+
+def logprobs(logits, sampled, k: int) -> torch.Tensor:
+    """[B, 2 k + 3] int32: ids of the sampled token and of the k likeliest, their log softmax (bits of fp32), rank of the sampled one."""
+    B, V = logits.shape
+    if logits.stride(1) != 1 or (logits.stride(0) * logits.element_size()) % 16 or logits.data_ptr() % 16:
+        pad = torch.empty((B, -(-V // 8) * 8), dtype=logits.dtype, device=logits.device)[:, :V]
+        logits = pad.copy_(logits)
+    assert sampled.dtype == torch.int64 and sampled.is_contiguous() and sampled.numel() == B
+    out = torch.empty((B, 2 * k + 3), dtype=torch.int32, device=logits.device)
+    _check(_logprobs(logits.data_ptr(), logits.stride(0), B, V, sampled.data_ptr(), k, out.data_ptr(), _DT[logits.dtype], _st()), "logprobs")
+    return out
+
+
 def topk_topp_mask_(logits: torch.Tensor, top_k, top_p, min_p=None) -> torch.Tensor:
     assert logits.dtype == torch.float32 and logits.is_contiguous()
     B, V = logits.shape

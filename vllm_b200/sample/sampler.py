@@ -54,6 +54,7 @@ class SamplingMetadata:
 class SamplerOutput:
     sampled_token_ids: torch.Tensor                      # [B] int64 (or [B, k] for spec decode)
     logprobs: Optional[tuple[torch.Tensor, torch.Tensor, torch.Tensor]] = None  # ids, vals, ranks
+    packed_logprobs: Optional[torch.Tensor] = None       # the one int32 matrix that these are views of (ops/cuda.py ``logprobs``)
 
 
 class LogitsProcessor:
@@ -101,6 +102,13 @@ class Sampler:
         sampled = self.sample(logits, md)
         lp = None
         if md.max_num_logprobs is not None:
+            if logits.is_cuda:
+                from vllm_b200.ops import cuda_ops
+                cu = cuda_ops()
+                if cu.logprobs_ok(logits.shape[1], md.max_num_logprobs):
+                    k = md.max_num_logprobs
+                    p = cu.logprobs(raw_for_logprobs, sampled, k)
+                    return SamplerOutput(sampled, (p[:, :k + 1], p[:, k + 1:2 * k + 2].view(torch.float32), p[:, -1]), p)
             lp = ref.compute_logprobs(raw_for_logprobs, sampled, md.max_num_logprobs)
         return SamplerOutput(sampled, lp)
 

@@ -8,11 +8,22 @@ attention launch geometry depends only on the bucket, never on sequence lengths.
 """
 from __future__ import annotations
 
+from typing import Optional
+
 import torch
 
 from vllm_b200.forward_context import ForwardContext, set_forward_context
 from vllm_b200.layers.attention import attention_layers
 from vllm_b200.ops import cuda_ops
+
+
+def _unowned(t: torch.Tensor) -> Optional[torch.Tensor]:
+    """The same memory without a reference to it."""
+    make = getattr(torch._C, "_construct_storage_from_data_pointer", None)
+    if make is None:
+        return None
+    own = t.untyped_storage()
+    return torch.empty(0, dtype=t.dtype, device=t.device).set_(make(own.data_ptr(), t.device, own.nbytes()), t.storage_offset(), t.shape, t.stride())
 
 
 class DecodeGraph:
@@ -54,6 +65,10 @@ class DecodeGraph:
             self._body()
         self.num_launches = cuda_ops().LAUNCHES - n0
 
+    # logits of the captured step, [b, V]: a view that does not keep its memory from the pool's other graphs, so it holds them from a
+    # replay of this graph to the next replay of any (None: the step samples without whole logits)
+    logits: Optional[torch.Tensor] = None
+
     def _body(self) -> None:
         r, b = self.runner, self.b
         ctx = ForwardContext(attn_metadata=self.md, kv_caches=r.kv_caches, layer_to_group=r.layer_to_group,
@@ -65,6 +80,7 @@ class DecodeGraph:
             return                      # TP: per-shard sampling + 16-byte candidate gather instead of the logits all-gather
         logits = r.model.compute_logits(hidden)
         cuda_ops().fused_sample(logits, self.temperature, self.seeds, self.steps, self.out)
+        self.logits = _unowned(logits) if torch.cuda.is_current_stream_capturing() else None
 
     def replay_from_staging(self, stg, b: int) -> torch.Tensor:
         """Sampling vectors come from the pinned staging set (filled from the runner's per-row arrays)."""

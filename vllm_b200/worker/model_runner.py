@@ -53,7 +53,14 @@ class ReqState:
     num_prompt_tokens: int = 0
     output_token_ids: list[int] = field(default_factory=list)
     mm_features: Optional[list] = None
-    complex_sampling: bool = False  # needs the per-request slow path (penalties, logprobs, processors, ...)
+    sampling_mode: int = 0          # one of the SAMPLE_ constants
+
+
+# what a request's sampling needs besides temperature and seed, in rising order
+SAMPLE_PLAIN = 0        # nothing: the captured step samples
+SAMPLE_LOGPROBS = 1     # log-probabilities of the captured step's logits, read back with the tokens
+SAMPLE_HOST = 2         # per-request state of the host (penalties, biases, grammars, plug-ins): the sampler runs on the step's logits
+SAMPLE_EAGER = 3        # more of the forward pass than its logits (pooling, log-probabilities of prompts)
 
 
 class _Staging:
@@ -83,6 +90,12 @@ class _Staging:
         self.diff_hdr = [mk(8 * R, dtype=torch.int32) for _ in range(G)] if pin else []
         self.diff_ids = [mk(min(R * MB, max(1 << 20, 4 * R + MB)), dtype=torch.int32) for _ in range(G)] if pin else []
         self.event = torch.cuda.Event() if pin else None
+        self.logprobs: Optional[torch.Tensor] = None         # packed log-probabilities, allocated with the first request for them
+
+    def logprobs_buf(self, rows: int, cols: int) -> torch.Tensor:
+        if self.logprobs is None or self.logprobs.numel() < rows * cols:
+            self.logprobs = torch.zeros(max(rows, self.rows.numel()) * cols, dtype=torch.int32).pin_memory()
+        return self.logprobs[:rows * cols].view(rows, cols)
 
     def wait(self) -> None:
         if self.event is not None:
@@ -126,6 +139,10 @@ class AsyncStepOutput:
             r.token_ids_cpu[row, n] = t
             r.num_tokens_cpu[row] = n + 1
             r.states[rid].output_token_ids.append(t)
+        lp = self.lp_out
+        if isinstance(lp, torch.Tensor):            # packed [nb, 2 k + 3] (ops/cuda.py ``logprobs``) of the rows that produced a token
+            a, k = lp.numpy()[np.nonzero(self.produces)[0]], (lp.shape[1] - 3) // 2
+            lp = LogprobsTensors(a[:, :k + 1], a[:, k + 1:2 * k + 2].copy().view(np.float32), a[:, -1])
         spec_ids = None
         if r.drafter is not None:
             rows = [r.req_index[rid] for rid in self.req_ids if rid in r.req_index]
@@ -135,7 +152,7 @@ class AsyncStepOutput:
             r._pending = None
         self._out = ModelRunnerOutput(
             req_ids=self.req_ids, req_id_to_index={x: i for i, x in enumerate(self.req_ids)},
-            sampled_token_ids=out_ids, logprobs=self.lp_out, prompt_logprobs_dict=self.plp,
+            sampled_token_ids=out_ids, logprobs=lp, prompt_logprobs_dict=self.plp,
             spec_token_ids=spec_ids, forward_ms=(time.perf_counter() - self.t0) * 1e3,
             kv_connector_output=r.kv_connector.get_finished() if r.kv_connector is not None else None)
         return self._out
@@ -219,7 +236,8 @@ class ModelRunner:
         self.num_computed_cpu = np.zeros(R, dtype=np.int32)
         self.temp_cpu = np.zeros(R, dtype=np.float32)
         self.seed_cpu = np.zeros(R, dtype=np.int64)
-        self.complex_cpu = np.zeros(R, dtype=bool)
+        self.mode_cpu = np.zeros(R, dtype=np.int8)               # SAMPLE_ constants
+        self.lp_cpu = np.full(R, -1, dtype=np.int32)             # log-probabilities wanted (-1: none)
         self.filter_cpu = np.zeros(R, dtype=bool)                # top-k / top-p / min-p
         self.block_tables_cpu: list[np.ndarray] = []
         self.num_blocks_cpu: list[np.ndarray] = []
@@ -390,7 +408,7 @@ class ModelRunner:
         n = self.num_tokens_cpu[src]
         self.token_ids_cpu[dst, :n] = self.token_ids_cpu[src, :n]
         for a in (self.num_tokens_cpu, self.num_logical_cpu, self.num_prompt_cpu, self.num_computed_cpu,
-                  self.temp_cpu, self.seed_cpu, self.complex_cpu, self.filter_cpu):
+                  self.temp_cpu, self.seed_cpu, self.mode_cpu, self.lp_cpu, self.filter_cpu):
             a[dst] = a[src]
         for g in range(self.num_kv_groups):
             nb = self.num_blocks_cpu[g][src]
@@ -442,23 +460,35 @@ class ModelRunner:
             self.seed_cpu[row] = (sp.seed if sp.seed is not None
                                   else zlib.crc32(st.req_id.encode()) * 2654435761 + self.mc.seed) & 0x7FFFFFFFFFFF
             self.filter_cpu[row] = sp.temperature >= 1e-5 and (sp.top_k > 0 or sp.top_p < 1.0 or sp.min_p > 0)
-            st.complex_sampling = bool(
-                sp.needs_penalties or sp.logprobs is not None or sp.prompt_logprobs is not None or sp.logit_bias
-                or sp.allowed_token_ids or sp.bad_words_token_ids or sp.min_tokens > 0
-                or sp.structured_outputs is not None
-                or (self.sampler.custom and any(k != "kv_transfer_params" for k in (sp.extra_args or {}))))
+            if sp.prompt_logprobs is not None:
+                st.sampling_mode = SAMPLE_EAGER
+            elif (sp.needs_penalties or sp.logit_bias or sp.allowed_token_ids or sp.bad_words_token_ids or sp.min_tokens > 0
+                    or sp.structured_outputs is not None or (sp.logprobs is not None and not self._logprobs_ok(sp.logprobs))
+                    or (self.sampler.custom and any(k != "kv_transfer_params" for k in (sp.extra_args or {})))):
+                st.sampling_mode = SAMPLE_HOST
+            else:
+                st.sampling_mode = SAMPLE_PLAIN if sp.logprobs is None else SAMPLE_LOGPROBS
+            self.lp_cpu[row] = -1 if sp.logprobs is None or sp.logprobs < 0 else sp.logprobs
         else:
             self.temp_cpu[row] = 0.0
             self.seed_cpu[row] = 0
             self.filter_cpu[row] = False
-            st.complex_sampling = True
-        self.complex_cpu[row] = st.complex_sampling
+            self.lp_cpu[row] = -1
+            st.sampling_mode = SAMPLE_EAGER
+        self.mode_cpu[row] = st.sampling_mode
         for g in range(self.num_kv_groups):
             ids = block_ids[g]
             self.block_tables_cpu[g][row, :len(ids)] = ids
             self.num_blocks_cpu[g][row] = len(ids)
         if self.gpu_prep:       # admission: the whole row travels once, with this step's uploads (_flush_gpu_state)
             self._new_tokens.append((st.req_id, 0))
+
+    def _logprobs_ok(self, k: int) -> bool:
+        """Does one launch read them off (ops/cuda.py ``logprobs``)?"""
+        if not self.is_cuda:
+            return False
+        from vllm_b200.ops import cuda_ops
+        return cuda_ops().logprobs_ok(self.vocab_size, k)
 
     def _add(self, nr) -> None:
         sp = nr.sampling_params
@@ -1002,7 +1032,7 @@ class ModelRunner:
             return ModelRunnerOutput()
         B_all = len(self.req_ids)
         # features that need the previous step's tokens on the host force a drain of the pipeline
-        if self._pending is not None and (bool(self.complex_cpu[:B_all].any()) or so.scheduled_spec_decode_tokens
+        if self._pending is not None and (bool((self.mode_cpu[:B_all] >= SAMPLE_HOST).any()) or so.scheduled_spec_decode_tokens
                                           or self.drafter is not None or so.grammar_bitmask is not None):
             self._pending.get()
         stg = self._next_staging()
@@ -1014,19 +1044,22 @@ class ModelRunner:
         decode_only = max_q == 1 and not has_spec
         pad_b = nb
         graph = None
-        simple = not bool(self.complex_cpu[rows].any()) and so.grammar_bitmask is None and so.logits_positions is None
+        mode = int(self.mode_cpu[rows].max()) if so.logits_positions is None else SAMPLE_EAGER
+        if so.grammar_bitmask is not None:
+            mode = max(mode, SAMPLE_HOST)
+        simple = mode == SAMPLE_PLAIN
         no_filter = not bool(self.filter_cpu[rows].any())
         kv_meta = so.kv_connector_metadata if self.kv_connector is not None else None
         lora_batch = None
         if getattr(self, "lora_manager", None) is not None:
             lreqs = [self.states[self.req_ids[r]].lora_request for r in rows]
             lora_batch = self.lora_manager.make_batch(lreqs, [int(x) for x in ns])
-        if (decode_only and self.use_cuda_graph and self.graphs and simple and no_filter and not kv_meta
-                and lora_batch is None):
+        if (decode_only and self.use_cuda_graph and self.graphs and mode < SAMPLE_EAGER and not kv_meta and lora_batch is None
+                and (simple and no_filter or self.drafter is None and self.spec_hidden is None)):
             pad_b = self._bucket(nb)
             graph = self.graphs.get(pad_b)
-            if graph is None:
-                pad_b = nb
+            if graph is None or not (simple and no_filter) and graph.logits is None:
+                pad_b, graph = nb, None
         pad_t = pad_b if graph is not None else T
         mixed = None
         if (graph is None and not decode_only and self.mixed_graphs and gpu_prep and simple and no_filter and not kv_meta
@@ -1066,6 +1099,17 @@ class ModelRunner:
             sampled = graph.replay_from_staging(stg, pad_b)[:nb]
             self.launch_count += graph.num_launches
             self.h2d_bytes += pad_b * 16
+            if mode <= SAMPLE_LOGPROBS and no_filter:
+                if mode == SAMPLE_LOGPROBS:
+                    lp_out = self._cu_ops().logprobs(graph.logits[:nb], sampled, int(self.lp_cpu[rows].max()))
+                    self.launch_count += 1
+            else:                                   # the sampler's own choice from the captured step's logits
+                l0 = self._launches()
+                states = [self.states[r] for r in req_ids]
+                bitmask = self._gather_bitmask(so, states) if so.grammar_bitmask is not None else None
+                so_out = self.sampler(graph.logits[:nb], self._sampling_metadata(states, rows, nb, simple), bitmask)
+                sampled, lp_out = so_out.sampled_token_ids, self._step_logprobs(so_out, produces)
+                self.launch_count += self._launches() - l0
         else:
             l0 = self._launches()
             states = [self.states[r] for r in req_ids]
@@ -1131,10 +1175,7 @@ class ModelRunner:
             bitmask = self._gather_bitmask(so, states) if so.grammar_bitmask is not None else None
             so_out = self.sampler(logits, smd, bitmask)
             sampled = so_out.sampled_token_ids
-            if so_out.logprobs is not None:
-                keep = torch.from_numpy(np.nonzero(produces)[0]).to(self.device)
-                ids, vals, ranks = so_out.logprobs
-                lp_out = LogprobsTensors(ids[keep].cpu(), vals[keep].cpu(), ranks[keep].cpu())
+            lp_out = self._step_logprobs(so_out, produces)
             if not simple and any(s.sampling_params is not None and s.sampling_params.prompt_logprobs is not None
                                   for s in states):
                 plp = self._prompt_logprobs(hidden, states, rows, ns, cu)
@@ -1148,6 +1189,8 @@ class ModelRunner:
             if gpu_prep:        # the new ids become next step's inputs on the device (no D2H → H2D round trip)
                 self._cu.append_sampled(self.dev_tokens, self.step_meta[:nb], self.step_meta[3 * nb:4 * nb], sampled)
             stg.sampled[:nb].copy_(sampled, non_blocking=True)
+            if isinstance(lp_out, torch.Tensor):
+                lp_out = stg.logprobs_buf(*lp_out.shape).copy_(lp_out, non_blocking=True)
             stg.event.record()
             ev = stg.event
         else:
@@ -1163,6 +1206,19 @@ class ModelRunner:
         return out.get()
 
     # ------------------------------------------------------------- helpers
+    @staticmethod
+    def _cu_ops():
+        from vllm_b200.ops import cuda_ops
+        return cuda_ops()
+
+    def _step_logprobs(self, so_out, produces):
+        """Packed log-probabilities of all rows on the device, or those of the rows that produced a token on the host, or None."""
+        if so_out.packed_logprobs is not None or so_out.logprobs is None:
+            return so_out.packed_logprobs
+        keep = torch.from_numpy(np.nonzero(produces)[0]).to(self.device)
+        ids, vals, ranks = so_out.logprobs
+        return LogprobsTensors(ids[keep].cpu(), vals[keep].cpu(), ranks[keep].cpu())
+
     def _launches(self) -> int:
         if not self.is_cuda:
             return 0
