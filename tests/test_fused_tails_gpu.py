@@ -1,0 +1,50 @@
+"""Block tails in one pass (norm + add + norm; expert combine + shared expert + add + norm)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+
+
+def _rel(x, y):
+    return float((x.double() - y).norm() / y.norm())
+
+
+def _norm(x, w, gemma, eps):
+    return x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps) * (w + 1 if gemma else w)
+
+
+@pytest.mark.parametrize("T,H", [(1, 64), (3, 2048), (700, 1032), (5, 16384)])
+@pytest.mark.parametrize("gemma", [False, True])
+@pytest.mark.parametrize("dtype", [BF, torch.float16])
+def test_norm_add_norm(T, H, gemma, dtype):
+    from vllm_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x, r = (torch.randn(T, H, device="cuda", generator=g).to(dtype) for _ in range(2))
+    w1, w2 = ((torch.randn(H, device="cuda", generator=g) * 0.1 + (0 if gemma else 1)).to(dtype) for _ in range(2))
+    s = r.double() + _norm(x.double(), w1.double(), gemma, 1e-6)
+    y, r2 = ops.norm_add_norm(x, r, w1, 1e-6, w2, 1e-5, gemma)
+    ulp = 2 ** -9 if dtype == BF else 2 ** -12
+    assert r2 is r and _rel(r, s) < ulp                      # one rounding
+    assert _rel(y, _norm(s, w2.double(), gemma, 1e-5)) < 2 * ulp          # of the stream, and its own
+
+
+@pytest.mark.parametrize("T,H,k", [(1, 64, 1), (37, 2048, 6), (300, 1032, 3), (2, 9000, 2)])
+@pytest.mark.parametrize("shared", [None, "plain", "gated"])
+def test_combine_norm(T, H, k, shared):
+    from vllm_b200.ops import cuda as cu
+    g = torch.Generator(device="cuda").manual_seed(2)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    rows, r, nw = rnd(T * k, H).to(BF), rnd(T, H).to(BF), (1 + 0.1 * rnd(H)).to(BF)
+    inv = torch.randperm(T * k, device="cuda", generator=g).int()
+    inv[torch.rand(T * k, device="cuda", generator=g) < 0.2] = -1          # pairs of other ranks
+    w = torch.rand(T, k, device="cuda", generator=g)
+    extra = None if shared is None else rnd(T, H).to(BF)
+    gate = rnd(T, 1).to(BF) if shared == "gated" else None
+    picked = rows.double()[inv.clamp_min(0).long()] * (inv >= 0)[:, None]
+    s = r.double() + (picked.view(T, k, H) * w.double()[..., None]).sum(1)
+    if extra is not None:
+        s = s + extra.double() * (1 if gate is None else gate.double().sigmoid())
+    y, r2 = cu.moe_combine_norm(rows, inv, w, r, nw, 1e-6, False, extra, gate)
+    assert r2 is r and _rel(r, s) < 2 ** -9
+    assert _rel(y, _norm(s, nw.double(), False, 1e-6)) < 2 ** -8

@@ -58,6 +58,61 @@ __global__ void __launch_bounds__(1024) rms_norm_kernel(T* __restrict__ out, T* 
   }
 }
 
+// Norm of a block's output, residual add and the next block's norm in one pass over the row:
+//   r += x * rsqrt(mean(x^2) + eps) * w1;  out = r * rsqrt(mean(r^2) + eps) * w2      (one rounding of r, one of out)
+template <typename T, bool GEMMA>
+__global__ void __launch_bounds__(1024) norm_add_norm_kernel(T* __restrict__ out, const T* __restrict__ x, T* __restrict__ residual,
+                                                              const T* __restrict__ w1, const T* __restrict__ w2, int H, float eps1, float eps2) {
+  constexpr int N = Vec16<T>::N;
+  __shared__ float red[32];
+  pdl_trigger();
+  pdl_wait();
+  const int64_t row = blockIdx.x;
+  const T* xr = x + row * (int64_t)H;
+  T* rr = residual + row * (int64_t)H;
+  const int nvec = H / N;
+  Vec16<T> v[MAXV], r[MAXV];
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < MAXV; ++i) {
+    const int vi = threadIdx.x + i * blockDim.x;
+    if (vi < nvec) {
+      v[i] = ld16(xr + vi * N);
+      r[i] = ld16(rr + vi * N);
+#pragma unroll
+      for (int j = 0; j < N; ++j) { const float f = to_f32(v[i].e[j]); ss += f * f; }
+    }
+  }
+  const float i1 = rsqrtf(block_sum(ss, red) / (float)H + eps1);
+  ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < MAXV; ++i) {
+    const int vi = threadIdx.x + i * blockDim.x;
+    if (vi < nvec) {
+      const Vec16<T> g = ld16(w1 + vi * N);
+#pragma unroll
+      for (int j = 0; j < N; ++j) {
+        const float w = to_f32(g.e[j]) + (GEMMA ? 1.f : 0.f);
+        r[i].e[j] = from_f32<T>(to_f32(r[i].e[j]) + to_f32(v[i].e[j]) * i1 * w);
+        const float f = to_f32(r[i].e[j]);
+        ss += f * f;
+      }
+      st16(rr + vi * N, r[i]);
+    }
+  }
+  const float i2 = rsqrtf(block_sum(ss, red) / (float)H + eps2);
+#pragma unroll
+  for (int i = 0; i < MAXV; ++i) {
+    const int vi = threadIdx.x + i * blockDim.x;
+    if (vi < nvec) {
+      const Vec16<T> g = ld16(w2 + vi * N);
+#pragma unroll
+      for (int j = 0; j < N; ++j) v[i].e[j] = from_f32<T>(to_f32(r[i].e[j]) * i2 * (to_f32(g.e[j]) + (GEMMA ? 1.f : 0.f)));
+      st16(out + row * (int64_t)H + vi * N, v[i]);
+    }
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(1024) layer_norm_kernel(T* __restrict__ out, const T* __restrict__ x,
                                                            const T* __restrict__ w, const T* __restrict__ b, int H,
@@ -229,6 +284,20 @@ EXPORT int vb_rms_norm(void* out, void* x, void* residual, const void* w, int T,
       if (gemma) vb_launch(rms_norm_kernel<TT, false, true>, T, thr, 0, st, (TT*)out, (TT*)x, (TT*)nullptr, (const TT*)w, H, eps, x_stride);
       else vb_launch(rms_norm_kernel<TT, false, false>, T, thr, 0, st, (TT*)out, (TT*)x, (TT*)nullptr, (const TT*)w, H, eps, x_stride);
     }
+  });
+  return (int)cudaGetLastError();
+}
+
+// x, residual, out [T, H] contiguous
+EXPORT int vb_norm_add_norm(void* out, const void* x, void* residual, const void* w1, const void* w2, int T, int H, float eps1, float eps2, int gemma,
+                            int dtype, cudaStream_t st) {
+  if (T == 0) return 0;
+  DISPATCH_DTYPE(dtype, TT, {
+    constexpr int N = Vec16<TT>::N;
+    if (H % N != 0 || H / N > 1024 * MAXV) return -1;
+    const int thr = norm_threads(H, N);
+    if (gemma) vb_launch(norm_add_norm_kernel<TT, true>, T, thr, 0, st, (TT*)out, (const TT*)x, (TT*)residual, (const TT*)w1, (const TT*)w2, H, eps1, eps2);
+    else vb_launch(norm_add_norm_kernel<TT, false>, T, thr, 0, st, (TT*)out, (const TT*)x, (TT*)residual, (const TT*)w1, (const TT*)w2, H, eps1, eps2);
   });
   return (int)cudaGetLastError();
 }

@@ -211,6 +211,25 @@ class FusedMoE(nn.Module):
             return None
         return out[0].view(x.shape), residual
 
+    def rows_reduce_norm(self, x: torch.Tensor, router_logits: torch.Tensor, residual: torch.Tensor, norm, shared, shared_gate=None):
+        """(normed, residual) = norm(moe(x) + sigmoid(shared_gate) * shared + residual) on one rank, everything behind the expert GEMMs in one
+        kernel (``residual`` in place).  ``shared`` [T, H] and ``shared_gate`` [T, 1] may be None.  None = not covered."""
+        if (not x.is_cuda or self.tp_size > 1 or self.ep or self.wide_ep or self.eplb or self.fp8_block or not self.gated or self.identity_experts
+                or norm is None or not isinstance(getattr(norm, "gemma", None), bool)):
+            return None
+        from vllm_b200 import envs
+        from vllm_b200.ops import moe
+        x2 = x.reshape(-1, x.shape[-1])
+        T, H = x2.shape
+        if (envs.VLLM_B200_FORCE_REF_OPS or not envs.VLLM_B200_FUSED_MOE or T == 0 or H % 8 or H > 32768 or residual.dtype != x.dtype
+                or norm.weight.dtype != x.dtype or not residual.is_contiguous() or (shared is not None and not shared.is_contiguous())
+                or not moe.rows_ok(x2, self.w13_weight, self.w2_weight, T * self.top_k)):
+            return None
+        w, ids = self.select_experts(router_logits.reshape(-1, router_logits.shape[-1]))
+        rows, inv = moe.moe_rows(x2, self.w13_weight, self.w2_weight, ids, self.act, self.expert_map)
+        return ops.cuda_ops().moe_combine_norm(rows, inv, w.to(torch.float32).contiguous(), residual.view(T, H), norm.weight, norm.eps, norm.gemma, shared,
+                                               None if shared_gate is None else shared_gate.contiguous())
+
     # ------------------------------------------------------------ EPLB
     def _set_placement(self, phy2log: torch.Tensor) -> None:
         """(Re)builds the routing tables IN PLACE — captured CUDA graphs keep pointing at the same buffers."""

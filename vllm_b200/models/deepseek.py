@@ -145,6 +145,16 @@ class DeepseekMoE(nn.Module):
             out = out + self.shared_experts(x)
         return out          # per-rank partial sum
 
+    def forward_reduce_norm(self, x: torch.Tensor, residual: torch.Tensor, norm) -> tuple[torch.Tensor, torch.Tensor]:
+        """(normed, residual) = norm(all_reduce(block(x)) + residual)."""
+        shared = self.shared_experts(x) if self.shared_experts is not None else None
+        logits = self.gate(x).float()
+        got = self.experts.rows_reduce_norm(x, logits, residual, norm, shared)
+        if got is not None:
+            return got
+        out = self.experts(x, logits)
+        return tp_reduce_residual_norm(out if shared is None else out + shared, residual, norm)
+
 
 class DeepseekDecoderLayer(nn.Module):
     def __init__(self, cfg, mc, dtype, quant_config, prefix: str, layer_idx: int, enable_ep: bool) -> None:
@@ -167,11 +177,11 @@ class DeepseekDecoderLayer(nn.Module):
         hidden, residual = self.self_attn.o_proj.forward_reduce_norm(a, residual, self.post_attention_layernorm)
         if not self.sparse:
             return self.mlp.forward_reduce_norm(hidden, residual, next_norm)
-        partial = self.mlp(hidden)
         if next_norm is None:
+            partial = self.mlp(hidden)
             tp = get_tp_group()
             return (tp.all_reduce(partial) if tp.world_size > 1 else partial), residual
-        return tp_reduce_residual_norm(partial, residual, next_norm)
+        return self.mlp.forward_reduce_norm(hidden, residual, next_norm)
 
 
 class DeepseekModel(LlamaModel):

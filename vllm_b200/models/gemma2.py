@@ -7,6 +7,7 @@ from typing import Optional
 import torch
 import torch.nn as nn
 
+from vllm_b200 import ops
 from vllm_b200.config import VllmConfig
 from vllm_b200.layers.attention import Attention
 from vllm_b200.layers.common import RMSNorm
@@ -53,11 +54,13 @@ class Gemma2DecoderLayer(nn.Module):
 
     def forward(self, positions, hidden, residual, next_norm: Optional[nn.Module]):
         """Same calling convention as the Llama layer: ``hidden`` = normalised block input, ``residual`` = stream."""
-        a = self.post_attention_layernorm(self.self_attn(positions, hidden))
-        stream = residual + a
-        m = self.post_feedforward_layernorm(self.mlp(self.pre_feedforward_layernorm(stream)))
-        stream = stream + m
-        return (next_norm(stream) if next_norm is not None else stream), stream
+        n1, n2, n3 = self.post_attention_layernorm, self.pre_feedforward_layernorm, self.post_feedforward_layernorm
+        hidden, residual = ops.norm_add_norm(self.self_attn(positions, hidden), residual, n1.weight, n1.eps, n2.weight, n2.eps, True)
+        m = self.mlp(hidden)
+        if next_norm is None:
+            stream = residual + n3(m)
+            return stream, stream
+        return ops.norm_add_norm(m, residual, n3.weight, n3.eps, next_norm.weight, next_norm.eps, True)
 
 
 class Gemma2Model(LlamaModel):

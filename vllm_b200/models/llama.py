@@ -238,7 +238,7 @@ class LlamaModel(nn.Module):
                 residual = residual + deep[:, (self.start + i) * H:(self.start + i + 1) * H].to(residual.dtype)
                 hidden = nxt(residual)
             if aux is not None and (self.start + i) in taps:
-                aux.append(residual)
+                aux.append(residual.clone())          # (the next layer adds to it in place)
         if aux:
             fctx.extra["aux_hidden"] = torch.cat(aux, dim=-1)
         if hidden.is_cuda:

@@ -53,6 +53,20 @@ class SparseMoeBlock(nn.Module):
         return out
 
 
+    def forward_reduce_norm(self, x: torch.Tensor, residual: torch.Tensor, norm) -> tuple[torch.Tensor, torch.Tensor]:
+        """(normed, residual) = norm(all_reduce(block(x)) + residual)."""
+        shared = self.shared_expert(x) if self.shared_expert is not None else None
+        gate = self.shared_expert_gate(x) if self.shared_expert_gate is not None else None
+        logits = self.gate(x)
+        got = self.experts.rows_reduce_norm(x, logits, residual, norm, shared, gate)
+        if got is not None:
+            return got
+        out = self.experts(x, logits)
+        if shared is not None:
+            out = out + (shared if gate is None else torch.sigmoid(gate) * shared)
+        return tp_reduce_residual_norm(out, residual, norm)
+
+
 class MoeDecoderLayer(nn.Module):
     def __init__(self, cfg, mc, dtype, quant_config, prefix: str, layer_idx: int, enable_ep: bool,
                  flavour: str) -> None:
@@ -92,11 +106,11 @@ class MoeDecoderLayer(nn.Module):
             fused = self.moe.experts.forward_reduce_norm(hidden, self.moe.gate(hidden), residual, next_norm)
             if fused is not None:
                 return fused
-        partial = self.moe(hidden)
         if next_norm is None:
+            partial = self.moe(hidden)
             tp = get_tp_group()
             return (tp.all_reduce(partial) if tp.world_size > 1 else partial), residual
-        return tp_reduce_residual_norm(partial, residual, next_norm)
+        return self.moe.forward_reduce_norm(hidden, residual, next_norm)
 
 
 class MoeModel(LlamaModel):

@@ -195,11 +195,9 @@ class GatedAttention(nn.Module):
     def forward(self, positions, hidden):
         T = hidden.shape[0]
         qg = self.q_proj(hidden).view(T, self.nh, 2 * self.hd)
-        q, gate = qg[..., :self.hd], qg[..., self.hd:].reshape(T, -1)
-        q = self.q_norm(q.reshape(-1, self.hd)).view(T, -1)
-        k = self.k_norm(self.k_proj(hidden).view(-1, self.hd)).view(T, -1)
-        o = self.attn(q, k, self.v_proj(hidden), positions)
-        return self.o_proj(o * torch.sigmoid(gate))
+        q, gate = qg[..., :self.hd].reshape(T, -1), qg[..., self.hd:].reshape(T, -1)
+        # norms, rotation and cache write are one launch; the gate is applied in place
+        return self.o_proj(self.attn(q, self.k_proj(hidden), self.v_proj(hidden), positions, qk_norm=(self.q_norm, self.k_norm), gate=gate))
 
 
 class Qwen3NextDecoderLayer(nn.Module):
@@ -227,9 +225,11 @@ class Qwen3NextDecoderLayer(nn.Module):
         self.post_attention_layernorm = RMSNorm(H, eps, dtype, True)
 
     def forward(self, positions, hidden, residual, next_norm: Optional[nn.Module]):
-        stream = residual + (self.self_attn(positions, hidden) if self.is_attn else self.linear_attn(hidden))
-        stream = stream + self.mlp(self.post_attention_layernorm(stream))
-        return (next_norm(stream) if next_norm is not None else stream), stream
+        hidden, residual = self.post_attention_layernorm(self.self_attn(positions, hidden) if self.is_attn else self.linear_attn(hidden), residual)
+        if next_norm is None:
+            stream = residual + self.mlp(hidden)
+            return stream, stream
+        return self.mlp.forward_reduce_norm(hidden, residual, next_norm)
 
 
 class Qwen3NextModel(Qwen2MoeModel):

@@ -50,6 +50,15 @@ def fused_add_rms_norm(x: torch.Tensor, residual: torch.Tensor, weight: torch.Te
     return ref.fused_add_rms_norm(x, residual, weight, eps, gemma)
 
 
+def norm_add_norm(x: torch.Tensor, residual: torch.Tensor, w1: torch.Tensor, eps1: float, w2: torch.Tensor, eps2: float, gemma: bool = False
+                  ) -> tuple[torch.Tensor, torch.Tensor]:
+    """(norm(s) * w2, s) with s = residual + norm(x) * w1.  The CUDA path updates ``residual`` in place."""
+    if _use_cuda(x) and _vec_ok(x) and x.is_contiguous() and residual.is_contiguous():
+        return cuda_ops().norm_add_norm(x, residual, w1, eps1, w2, eps2, gemma)
+    s = residual + ref.rms_norm(x, w1, eps1, gemma)
+    return ref.rms_norm(s, w2, eps2, gemma), s
+
+
 def layer_norm(x, weight, bias, eps):
     if _use_cuda(x):
         return cuda_ops().layer_norm(x, weight, bias, eps)

@@ -175,6 +175,19 @@ def fused_add_rms_norm(x, residual, weight, eps, gemma=False):
     return x, residual
 
 
+_norm_add_norm = _sig("vb_norm_add_norm", _vp, _vp, _vp, _vp, _vp, _i, _i, _f, _f, _i, _i, _vp)
+
+
+def norm_add_norm(x, residual, w1, eps1, w2, eps2, gemma=False):
+    """In place: residual += norm(x) * w1.  Returns (norm(residual) * w2, residual)."""
+    H = x.shape[-1]
+    out = torch.empty_like(x)
+    assert x.is_contiguous() and residual.is_contiguous() and residual.shape == x.shape and residual.dtype == w1.dtype == w2.dtype == x.dtype
+    _check(_norm_add_norm(out.data_ptr(), x.data_ptr(), residual.data_ptr(), w1.data_ptr(), w2.data_ptr(), x.numel() // H, H, eps1, eps2, int(gemma),
+                          _DT[x.dtype], _st()), "norm_add_norm")
+    return out, residual
+
+
 def layer_norm(x, weight, bias, eps):
     H = x.shape[-1]
     xc = _rows(x)
@@ -1177,6 +1190,21 @@ def moe_combine(y: torch.Tensor, inv: torch.Tensor, w: torch.Tensor, T: int) -> 
         _check(_post_norm(y.data_ptr(), y.stride(0), inv.data_ptr(), w.data_ptr(), k, None, 0, None, None, 0, out.data_ptr(), T, H,
                           0.0, _DT[y.dtype], _st()), "moe_combine")
     return out
+
+
+_moe_combine_norm = _sig("vb_moe_combine_norm", _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _f, _i, _i, _vp)
+
+
+def moe_combine_norm(rows, inv, w, residual, norm_w, eps: float, gemma: bool, extra=None, gate=None):
+    """In place: residual [T, H] += sum_j w[t, j] rows[inv[t k + j]] + sigmoid(gate[t]) extra[t].  Returns (norm of it, residual)."""
+    T, H = residual.shape
+    out = torch.empty_like(residual)
+    for t in (rows, residual, norm_w, extra, gate):
+        assert t is None or (t.dtype == rows.dtype and t.is_contiguous())
+    assert w.dtype == torch.float32 and w.is_contiguous() and inv.dtype == torch.int32 and inv.numel() == w.numel()
+    _check(_moe_combine_norm(rows.data_ptr(), inv.data_ptr(), w.data_ptr(), inv.numel() // max(T, 1), _p(extra), _p(gate), residual.data_ptr(),
+                             norm_w.data_ptr(), out.data_ptr(), T, H, eps, int(gemma), _DT[rows.dtype], _st()), "moe_combine_norm")
+    return out, residual
 
 
 def gemm_tc_grouped(xs: torch.Tensor, w: torch.Tensor, offs: torch.Tensor, bn: int, act: Optional[str] = None,

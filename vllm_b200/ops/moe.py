@@ -25,30 +25,38 @@ def _grouped_ok(x, w13, w2, R: int) -> bool:
             and w13.is_contiguous() and w2.is_contiguous() and envs.VLLM_B200_GEMM != "cublas")
 
 
+def grouped_rows(x, w13, w2, topk_ids, act, expert_map):
+    """(rows, inv) of ``expert_rows`` for decode-sized batches."""
+    from vllm_b200.ops import cuda as cu
+    R, E = topk_ids.numel(), w13.shape[0]
+    ids = topk_ids if topk_ids.dtype == torch.int32 else topk_ids.to(torch.int32)
+    sorted_tok, inv, offs = cu.moe_align(ids.contiguous(), E, expert_map)
+    bn = _tile_width(R, E)
+    h = cu.gemm_tc_grouped(cu.moe_gather(x, sorted_tok), w13, offs, bn)
+    return cu.gemm_tc_grouped(cu.act_and_mul(h, act), w2, offs, bn), inv
+
+
 def fused_moe_grouped(x, w13, w2, topk_w, topk_ids, act, expert_map):
     """Decode-sized MoE, fully on the device (no host sync → CUDA-graph capturable):
     align (counting sort by expert) → gather → grouped tcgen05 GEMM (w13) → act·mul → grouped GEMM (w2) →
     weighted combine.  Empty (expert, chunk) CTAs exit before touching their weights, so the weight traffic is
     exactly that of the experts that were actually routed to."""
-    from vllm_b200.ops import cuda as cu
-    T, k = topk_ids.shape
-    R = T * k
-    E = w13.shape[0]
-    ids = topk_ids if topk_ids.dtype == torch.int32 else topk_ids.to(torch.int32)
-    sorted_tok, inv, offs = cu.moe_align(ids.contiguous(), E, expert_map)
-    xs = cu.moe_gather(x, sorted_tok)
-    # token-tile width: average rows per expert rounded up, so that most experts need one chunk
-    avg = max(R // max(E, 1), 1)
-    bn = 16
-    while bn < 128 and bn < 2 * avg:
-        bn += 16
-    h = cu.gemm_tc_grouped(xs, w13, offs, bn)
-    a = cu.act_and_mul(h, act) if hasattr(cu, "act_and_mul") else None
-    if a is None:
-        from vllm_b200 import ops
-        a = ops.silu_and_mul(h) if act == "silu" else ops.gelu_and_mul(h)
-    y = cu.gemm_tc_grouped(a, w2, offs, bn)
-    return cu.moe_combine(y, inv, topk_w.to(torch.float32).contiguous(), T)
+    return combine_rows(*grouped_rows(x, w13, w2, topk_ids, act, expert_map), topk_w, x.shape[0])
+
+
+def rows_ok(x, w13, w2, R: int) -> bool:
+    """Are the expert outputs of R pairs computed as sorted rows on the device?"""
+    from vllm_b200 import envs
+    return _grouped_ok(x, w13, w2, R) or (
+        _rows_ok(x, w13) and w2.dtype == x.dtype and w13.is_contiguous() and w2.is_contiguous() and w13.shape[0] <= 512
+        and R > GROUPED_MAX_ROWS and envs.VLLM_B200_GEMM != "cublas")
+
+
+def moe_rows(x, w13, w2, topk_ids, act, expert_map):
+    """(rows, inv) of ``expert_rows`` where ``rows_ok``."""
+    if _grouped_ok(x, w13, w2, topk_ids.numel()):
+        return grouped_rows(x, w13, w2, topk_ids, act, expert_map)
+    return expert_rows_gated(x, w13, w2, topk_ids, act, expert_map)
 
 
 def _tile_width(R: int, E: int) -> int:
@@ -210,14 +218,11 @@ def fused_moe_reduce_norm(x, w13, w2, topk_w, topk_ids, act, expert_map, residua
 
 
 def fused_moe_cuda(x, w13, w2, topk_w, topk_ids, act="silu", expert_map: Optional[torch.Tensor] = None):
-    from vllm_b200 import envs, ops
-    if _grouped_ok(x, w13, w2, topk_ids.numel()):
-        return fused_moe_grouped(x, w13, w2, topk_w, topk_ids, act, expert_map)
+    from vllm_b200 import ops
+    if rows_ok(x, w13, w2, topk_ids.numel()):
+        return combine_rows(*moe_rows(x, w13, w2, topk_ids, act, expert_map), topk_w, x.shape[0])
     T, H = x.shape
     E = w13.shape[0]
-    if (_rows_ok(x, w13) and w2.dtype == x.dtype and w13.is_contiguous() and w2.is_contiguous() and E <= 512
-            and topk_ids.numel() > GROUPED_MAX_ROWS and envs.VLLM_B200_GEMM != "cublas"):
-        return fused_moe_rows(x, w13, w2, topk_w, topk_ids, act, expert_map, True)
     k = topk_ids.shape[1]
     ids = topk_ids.long()
     if expert_map is not None:
