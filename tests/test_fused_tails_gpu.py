@@ -1,4 +1,4 @@
-"""Block tails in one pass (norm + add + norm; expert combine + shared expert + add + norm)."""
+"""Block tails in one pass (norm + add + norm; expert combine + shared expert + add + norm) and values turned into transposed pages."""
 import pytest
 import torch
 
@@ -48,3 +48,30 @@ def test_combine_norm(T, H, k, shared):
     y, r2 = cu.moe_combine_norm(rows, inv, w, r, nw, 1e-6, False, extra, gate)
     assert r2 is r and _rel(r, s) < 2 ** -9
     assert _rel(y, _norm(s, nw.double(), False, 1e-6)) < 2 ** -8
+
+
+@pytest.mark.parametrize("Hkv,D,BS", [(2, 128, 64), (1, 64, 16), (3, 128, 32), (1, 256, 64), (2, 128, 4)])
+def test_values_turned(Hkv, D, BS):
+    """Slots that follow one another from any place, gaps, padding, shuffled ones; both kernels that use it."""
+    from vllm_b200.ops import cuda as cu
+    g = torch.Generator(device="cuda").manual_seed(3)
+    runs = [list(range(3, 70)), list(range(BS * 20, BS * 20 + 130)), [-1] * 5, list(range(1000, 1007)), list(range(1016, 1024)), list(range(2001, 2100))]
+    shuffled = (3000 + torch.randperm(60, generator=torch.Generator().manual_seed(1))).tolist()
+    slots = torch.tensor(sum(runs, []) + shuffled, device="cuda")
+    T = len(slots)
+    assert T > 257
+    qkv = torch.randn(T, (2 + 2 * Hkv) * D, device="cuda", generator=g).to(BF)
+    q, k, v = qkv.split([2 * D, Hkv * D, Hkv * D], -1)
+    cache = torch.zeros(-(-3100 // BS), 2, Hkv, BS, D, device="cuda", dtype=BF)
+    pos, cs = torch.arange(T, device="cuda") % 50, torch.randn(50, D, device="cuda", generator=g)
+    want = torch.zeros_like(cache[:, 1]).view(-1, Hkv, D, BS)
+    for t, s in enumerate(slots.tolist()):
+        if s >= 0:
+            want[s // BS, :, :, s % BS] = v[t].view(Hkv, D)
+    cu.rope_and_cache(pos, q, k, v, cs, D, True, cache, slots, vt=True)
+    assert torch.equal(cache[:, 1].reshape(want.shape), want)
+    if cu.qknorm_rope_ok(D, D, True):
+        cache.zero_()
+        w = torch.ones(D, device="cuda", dtype=BF)
+        cu.fused_qk_norm_rope(pos, q, k, w, w, cs, D, 1e-6, True, v=v, kv_cache=cache, slot_mapping=slots, vt=True)
+        assert torch.equal(cache[:, 1].reshape(want.shape), want)

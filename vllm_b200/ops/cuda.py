@@ -1550,6 +1550,10 @@ _qknorm_rope_row = _sig("vb_qknorm_rope_row", _vp, _vp, _vp, _vp, _vp, _vp, _vp,
                         _vp, _i, _i, _i, _i, _f, _i, _vp)
 
 
+_values_turned = _sig("vb_cache_values_turned", _vp, _i64, _vp, _vp, _i, _i, _i, _i, _i, _vp)
+TURN_MIN_TOKENS = 257       # as in csrc/rope_cache.cu
+
+
 def fused_qk_norm_rope(positions, q, k, q_weight, k_weight, cos_sin_cache, head_dim, eps, is_neox=True, *, v=None,
                        kv_cache=None, slot_mapping=None, gemma: bool = False, k_scale: float = 1.0, v_scale: float = 1.0,
                        vt: bool = False, v_head_dim: Optional[int] = None, keep32: bool = False, whole: bool = False, v_cos_sin=None):
@@ -1592,6 +1596,11 @@ def fused_qk_norm_rope(positions, q, k, q_weight, k_weight, cos_sin_cache, head_
                                 _p(kv_cache), _p(slot_mapping), BS, int(is_neox), int(gemma), int(vt), eps, _DT[q.dtype], _st()),
                "qknorm_rope_any")
         return q, k
+    if (vt and v is not None and kv_cache is not None and v_cos_sin is None and T >= TURN_MIN_TOKENS and kv_cache.dtype == q.dtype
+            and head_dim % 8 == 0 and head_dim <= 512 and v.stride(0) % 8 == 0 and v.data_ptr() % 16 == 0):
+        _check(_values_turned(v.data_ptr(), v.stride(0), kv_cache.data_ptr(), slot_mapping.data_ptr(), T, Hkv, head_dim, BS, _DT[q.dtype], _st()),
+               "cache_values_turned")
+        v = None
     _check(_qknorm_rope(_p(positions), q.data_ptr(), k.data_ptr(), _p(v), _p(q_weight), _p(k_weight), _p(cos_sin_cache),
                         _p(v_cos_sin), rot, T, Hq, Hkv, head_dim, q.stride(0), k.stride(0), v.stride(0) if v is not None else 0,
                         _p(kv_cache), _p(slot_mapping), BS, int(is_neox), int(gemma), flags, eps, k_scale, v_scale,
