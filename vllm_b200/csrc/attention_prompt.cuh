@@ -6,16 +6,17 @@
 //
 // A thread owns a query row (a lane of tensor memory): it reads all 128 scores of a key tile at once and keeps them in registers, so maximum,
 // exponentials and row sum take one pass and no exchange.  With two tiles the tensor core works on one tile's products while the
-// other tile's warpgroup is at its exponentials; with one tile per CTA the two take turns.  The products of a tile are issued in the order
-// P V of key tile j, Q K of tile j + 1 by one thread and run in that order, so a full S_t also says that O_t is complete: the
-// rescaling of O needs no barrier of its own, and P may lie over S.
+// other tile's warpgroup is at its exponentials; with one tile per CTA the two warpgroups share it, one takes the even, the other the odd key
+// tiles, and their results are merged at the end.  The products of a warpgroup are issued in the order P V of its key tile j, Q K of its
+// tile j + 1 by one thread and run in that order, so a full S_t also says that O_t is complete: the rescaling of O needs no barrier of
+// its own, and P may lie over S.
 //
 // CAP: scores are capped, c tanh(s / c).  SPLIT: the weights keep 16 more bits (P = hi + lo, two products): for paths whose weights are held
 // in 32 bits, at half as much tensor work again.  Tensor memory: S_0, S_1 (128 columns each), O_0, O_1 (up to 128 each).
 //
 // Bound by the special-function and issue rate of the softmax (a key tile takes the tensor core 2048 cycles for two query tiles, their 32768
 // exponentials as long).  Measured: 32 / 8 heads, two prompts of 3800 tokens 576 us with one tile of rows, scores read twice and weights
-// through shared memory, 360 us so; capped, 16 / 4 heads, eight prompts of 860 tokens 2536 us on the CUDA cores, 182 us so.
+// through shared memory, 347 us so; capped, 16 / 4 heads, eight prompts of 860 tokens 2536 us on the CUDA cores, 182 us so.
 #pragma once
 #include "common.cuh"
 
@@ -77,35 +78,41 @@ template <int KS, int VS> struct Bars {
   }
 };
 
-// MMA issuer (one warp).  qk(t, stage) issues S_t, pv(t, stage, first) issues O_t; `tiles` (1 or 2) query tiles over n >= 1 key tiles.
+// MMA issuer (one warp).  qk(t, stage) issues S_t, pv(t, stage, first) issues O_t.  n >= 1 key tiles, each for both of two query tiles
+// (`pair`), or the even ones for t = 0 and the odd ones for t = 1.
 template <int KS, int VS, class QK, class PV>
-VB_DEVICE void mma_role(Bars<KS, VS>& b, int n, int tiles, int lane, int& budget, QK qk, PV pv) {
+VB_DEVICE void mma_role(Bars<KS, VS>& b, int n, bool pair, int lane, int& budget, QK qk, PV pv) {
   mbar_wait_lim(&b.q_full, 0, budget);
-  mbar_wait_lim(&b.k_full[0], 0, budget);
-  tc_fence_after();
-  if (lane == 0) {
-    for (int t = 0; t < tiles; ++t) { qk(t, 0); umma_commit(&b.s_full[t]); }
-    umma_commit(&b.k_empty[0]);
+  const int ahead = pair ? 1 : 2;                          // key tiles between a product Q K of a warpgroup and its next
+  for (int j = 0; j < min(ahead, n); ++j) {
+    mbar_wait_lim(&b.k_full[j % KS], 0, budget);           // (ahead <= KS)
+    tc_fence_after();
+    if (lane == 0) {
+      for (int t = pair ? 0 : j; t < (pair ? 2 : j + 1); ++t) { qk(t, j % KS); umma_commit(&b.s_full[t]); }
+      umma_commit(&b.k_empty[j % KS]);
+    }
+    __syncwarp();
   }
-  __syncwarp();
   for (int j = 0; j < n; ++j) {
-    const int vs = j % VS, ks = (j + 1) % KS;
+    const int vs = j % VS, nx = j + ahead, ks = nx % KS;
     mbar_wait_lim(&b.v_full[vs], (j / VS) & 1, budget);
-    for (int t = 0; t < tiles; ++t) {
-      mbar_wait_lim(&b.p_full[t], j & 1, budget);
+    const int t0 = pair ? 0 : j & 1, t1 = pair ? 1 : t0;
+    const int phase = (pair ? j : j >> 1) & 1;
+    for (int t = t0; t <= t1; ++t) {
+      mbar_wait_lim(&b.p_full[t], phase, budget);
       tc_fence_after();
       if (lane == 0) {
-        pv(t, vs, j == 0);
-        if (t == tiles - 1) umma_commit(&b.v_empty[vs]);
-        if (j + 1 == n) umma_commit(&b.o_done[t]);
+        pv(t, vs, pair ? j == 0 : j < 2);
+        if (t == t1) umma_commit(&b.v_empty[vs]);
+        if (nx >= n) umma_commit(&b.o_done[t]);
       }
       __syncwarp();
-      if (j + 1 < n) {
-        if (t == 0) { mbar_wait_lim(&b.k_full[ks], ((j + 1) / KS) & 1, budget); tc_fence_after(); }
+      if (nx < n) {
+        if (t == t0) { mbar_wait_lim(&b.k_full[ks], (nx / KS) & 1, budget); tc_fence_after(); }
         if (lane == 0) {
           qk(t, ks);
           umma_commit(&b.s_full[t]);
-          if (t == tiles - 1) umma_commit(&b.k_empty[ks]);
+          if (t == t1) umma_commit(&b.k_empty[ks]);
         }
         __syncwarp();
       }
@@ -138,13 +145,14 @@ struct Softmax {
 };
 
 // Softmax of one query tile: thread = row.  The row sees the keys [lo, hi) of its request (lo >= hi: none); `first`: the first key of the first
-// key tile.  Leaves O_t complete; returns the row's reference maximum (powers of two) and its sum.
+// of the warpgroup's n key tiles, which are `step` keys apart.  Leaves O_t complete; returns the row's reference maximum (powers of two) and
+// its sum.
 template <typename T, int OC, bool CAP, int KS, int VS>
-VB_DEVICE void softmax_role(Bars<KS, VS>& b, int t, uint32_t t_s, uint32_t t_o, int n, int first, int lo, int hi, const Softmax& sm, bool split,
+VB_DEVICE void softmax_role(Bars<KS, VS>& b, int t, uint32_t t_s, uint32_t t_o, int n, int first, int step, int lo, int hi, const Softmax& sm, bool split,
                             int& budget, float& m_used, float& l_run) {
   m_used = -INFINITY;
   l_run = 0.f;
-  for (int j = 0; j < n; ++j, first += KEYS) {
+  for (int j = 0; j < n; ++j, first += step) {
     mbar_wait_lim(&b.s_full[t], j & 1, budget);
     __syncwarp();
     tc_fence_after();
@@ -253,6 +261,37 @@ VB_DEVICE void softmax_role(Bars<KS, VS>& b, int t, uint32_t t_s, uint32_t t_o, 
   mbar_wait_lim(&b.o_done[t], 0, budget);
   __syncwarp();
   tc_fence_after();
+}
+
+// One query tile shared by both warpgroups: the second hands its row's maximum and sum over (`ml`, one per row) when its O is complete; the
+// first waits for it and gets the factors of both O, those of the whole softmax.
+VB_DEVICE void hand_over(float2* ml, int row, float m, float l) {
+  ml[row] = make_float2(m, l);
+  tc_fence_before();
+  asm volatile("bar.sync 1, 256;" ::: "memory");
+}
+VB_DEVICE void take_over(const float2* ml, int row, float& m, float& l, float& f0, float& f1) {
+  asm volatile("bar.sync 1, 256;" ::: "memory");
+  tc_fence_after();
+  const float2 o = ml[row];
+  const float top = fmaxf(m, o.x);
+  f0 = m == -INFINITY ? 0.f : ex2(m - top);
+  f1 = o.x == -INFINITY ? 0.f : ex2(o.x - top);
+  l = l * f0 + o.y * f1;
+  m = top;
+}
+// columns c .. c + 31 of O, of a shared tile O_0 f0 + O_1 f1
+VB_DEVICE void load_o(uint32_t t_o, int c, bool shared, float f0, float f1, uint32_t (&v)[32]) {
+  tmem_ld_32x32(t_o + c, v);
+  if (shared) {
+    uint32_t u[32];
+    tmem_ld_32x32(t_o + 128 + c, u);
+    tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * f0 + __uint_as_float(u[i]) * f1);
+  } else {
+    tmem_ld_wait();
+  }
 }
 
 // O_t += P_t V: db(kk) is the descriptor of 16 keys of the values

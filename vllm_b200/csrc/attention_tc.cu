@@ -62,7 +62,8 @@ fmha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
   unsigned char* k_smem = q_smem + 2 * Q_BYTES;             // KV_STAGES x K_BYTES
   unsigned char* v_smem = k_smem + KV_STAGES * K_BYTES;     // KV_STAGES x V_BYTES
   Bars& bars = *reinterpret_cast<Bars*>(v_smem + KV_STAGES * V_BYTES);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(&bars + 1);
+  float2* ml = reinterpret_cast<float2*>(&bars + 1);        // [TILE_M]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ml + TILE_M);
   int* blk_ids = reinterpret_cast<int*>(tmem_slot + 2);   // [2 * MAX_TILES_SMEM]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -203,13 +204,14 @@ fmha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
     const uint32_t idesc = umma_idesc_f16(TILE_M, TILE_N, DTypeOf<T>::v == DT_BF16);
     const uint64_t d_q = umma_desc_sw128(q_smem), d_k = umma_desc_sw128(k_smem), d_v = umma_desc_sw128(v_smem);
     prompt::mma_role(
-        bars, n_tiles, tiles, lane, budget,
+        bars, n_tiles, tiles == 2, lane, budget,
         [&](int t, int s) {
+          const int qt = tiles == 2 ? t : 0;
 #pragma unroll
           for (int kb = 0; kb < 2; ++kb)
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-              umma_f16(tmem_base + t * 128, d_q + (uint64_t)((t * Q_BYTES + kb * BLK + k * 32) >> 4),
+              umma_f16(tmem_base + t * 128, d_q + (uint64_t)((qt * Q_BYTES + kb * BLK + k * 32) >> 4),
                        d_k + (uint64_t)((s * K_BYTES + kb * BLK + k * 32) >> 4), idesc, (kb | k) != 0);
         },
         [&](int t, int s, bool first) {
@@ -219,19 +221,25 @@ fmha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
     }
   } else {
     prompt::regs_inc<prompt::REGS_SOFTMAX>();
-    if (warp < 4 + 4 * tiles) {
     // ===== softmax / correction / epilogue: thread = query row = TMEM lane
     const int t = (warp >> 2) - 1, qd = warp & 3;
+    const bool shared = tiles == 1 && n_tiles > 1;   // both warpgroups at one tile
     const int r = qd * 32 + lane;
-    const uint32_t t_lane = (uint32_t)(qd * 32) << 16, t_o = tmem_base + 256 + t * 128 + t_lane;
-    const int tq = t * p.TQ + r / p.G, g = r % p.G;
+    const uint32_t t_lane = (uint32_t)(qd * 32) << 16, t_o = tmem_base + 256 + (tiles == 2 ? t : 0) * 128 + t_lane;
+    const int tq = (tiles == 2 ? t : 0) * p.TQ + r / p.G, g = r % p.G;
     const bool row_valid = tq < n_tok && r < p.G * p.TQ;
     const int qpos = row_valid ? pos0 + tq : -1;
     const int row_lo = max(max(p.window > 0 ? qpos - p.window + 1 : 0, p.chunk > 0 ? max(qpos, 0) / p.chunk * p.chunk : 0), kv_begin);
     const int row_hi = row_valid ? min(kv_end, p.causal ? qpos + 1 : kv_end) : -1;
-    float m_used, l_run;
-    prompt::softmax_role<T, D, CAP>(bars, t, tmem_base + t * 128 + t_lane, t_o, n_tiles, tile_lo * TILE_N, row_lo, row_hi, p.sm, CAP, budget,
-                                    m_used, l_run);
+    const int n_mine = tiles == 2 ? n_tiles : (n_tiles + 1 - t) / 2;
+    float m_used, l_run, f0 = 1.f, f1 = 0.f;
+    if (n_mine > 0)
+      prompt::softmax_role<T, D, CAP>(bars, t, tmem_base + t * 128 + t_lane, tmem_base + 256 + t * 128 + t_lane, n_mine,
+                                      (tile_lo + (tiles == 2 ? 0 : t)) * TILE_N, tiles == 2 ? TILE_N : 2 * TILE_N, row_lo, row_hi, p.sm, CAP, budget,
+                                      m_used, l_run);
+    if (shared && t == 1) prompt::hand_over(ml, r, m_used, l_run);
+    if (tiles == 2 || t == 0) {
+    if (shared) prompt::take_over(ml, r, m_used, l_run, f0, f1);
     // ---- epilogue
     const int64_t tok = q0 + tok0 + tq;
     const int hq = h * p.G + g;
@@ -249,8 +257,7 @@ fmha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
 #pragma unroll
       for (int c = 0; c < D; c += 32) {
         uint32_t v[32];
-        tmem_ld_32x32(t_o + c, v);
-        tmem_ld_wait();
+        prompt::load_o(t_o, c, shared, f0, f1, v);
         if (row_valid) {
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {
@@ -271,8 +278,7 @@ fmha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
 #pragma unroll
       for (int c = 0; c < D; c += 32) {
         uint32_t v[32];
-        tmem_ld_32x32(t_o + c, v);
-        tmem_ld_wait();
+        prompt::load_o(t_o, c, shared, f0, f1, v);
         if (row_valid) {
 #pragma unroll
           for (int i = 0; i < 32; i += 4)
@@ -325,12 +331,15 @@ static EncodeTiledFn get_encode() {
   return fn;
 }
 
-// Query tiles (of all requests and KV heads) from which a CTA takes two of them: below, the second tile would leave SMs without one.
+// Query tiles (of all requests and KV heads) from which a CTA takes two of them: below, SMs would be left without any, and the two
+// warpgroups of a CTA share one.  One prompt of 2000 tokens, 8 / 2 heads (125 tiles): 42 us shared, 57 us with one warpgroup at work; 2 x 1000,
+// 16 / 4 heads (250): 40 against 49; from 300 tiles on two per CTA: 8 x 300, 16 / 4 heads (300) 34 us, 2 x 2000, 32 / 8 (1000) 124 us, where one
+// tile of rows per CTA took 182.
 constexpr int PAIR_MIN_TILES = 2 * 148;
 
 template <typename T, bool CAP>
 static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const Params& p, dim3 grid, cudaStream_t st) {
-  const int smem = 2 * Q_BYTES + KV_STAGES * (K_BYTES + V_BYTES) + (int)sizeof(Bars) + 16 + 2 * MAX_TILES_SMEM * 4 + 1024;
+  const int smem = 2 * Q_BYTES + KV_STAGES * (K_BYTES + V_BYTES) + (int)sizeof(Bars) + TILE_M * 8 + 16 + 2 * MAX_TILES_SMEM * 4 + 1024;
   auto k = fmha_kernel<T, CAP>;
   static bool a = false;
   if (!a) { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); a = true; }

@@ -71,7 +71,8 @@ mla_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   unsigned char* v_smem = k_smem + KS * NQ * BLK;           // VS x NV blocks
   typedef prompt::Bars<KS, VS> Bars;
   Bars& bars = *reinterpret_cast<Bars*>(v_smem + VS * NV * BLK);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(&bars + 1);
+  float2* ml = reinterpret_cast<float2*>(&bars + 1);        // [TM]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ml + TM);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int budget = MBAR_BUDGET;                    // failed polls left (mbar_wait_lim)
@@ -137,13 +138,14 @@ mla_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       const uint64_t d_q = umma_desc_sw128(q_smem), d_k = umma_desc_sw128(k_smem), d_v = desc_mn(v_smem);
       const bool split = p.split != 0;
       prompt::mma_role(
-          bars, n_tiles, tiles, lane, budget,
+          bars, n_tiles, tiles == 2, lane, budget,
           [&](int t, int s) {
+            const int qt = tiles == 2 ? t : 0;
 #pragma unroll
             for (int kb = 0; kb < NQ; ++kb)
 #pragma unroll
               for (int k = 0; k < 4; ++k)
-                umma_f16(tmem_base + t * 128, d_q + (uint64_t)(((t * NQ + kb) * BLK + k * 32) >> 4),
+                umma_f16(tmem_base + t * 128, d_q + (uint64_t)(((qt * NQ + kb) * BLK + k * 32) >> 4),
                          d_k + (uint64_t)(((s * NQ + kb) * BLK + k * 32) >> 4), idesc_s, (kb | k) != 0);
           },
           [&](int t, int s, bool first) {                   // 16 keys per MMA: 16 rows of 128 bytes of V
@@ -153,24 +155,29 @@ mla_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     }
   } else {
     prompt::regs_inc<prompt::REGS_SOFTMAX>();
-    if (warp < 4 + 4 * tiles) {
-      // ===== softmax / rescale / epilogue: thread = query row = TMEM lane
-      const int t = (warp >> 2) - 1, qd = warp & 3;
-      const int r = t * TM + qd * 32 + lane;
-      const uint32_t t_lane = (uint32_t)(qd * 32) << 16, t_o = tmem_base + 256 + t * 128 + t_lane;
-      const bool row_valid = r < n_tok;
-      const int hi = row_valid ? pos0 + r + 1 : -1;
-      const int lo = p.window > 0 ? max(hi - p.window, 0) : 0;
-      float m_used, l_run;
-      prompt::softmax_role<T, NV * 64, false>(bars, t, tmem_base + t * 128 + t_lane, t_o, n_tiles, tile_lo * TN, lo, hi, p.sm, p.split != 0,
-                                              budget, m_used, l_run);
+    // ===== softmax / rescale / epilogue: thread = query row = TMEM lane
+    const int t = (warp >> 2) - 1, qd = warp & 3, row = qd * 32 + lane;
+    const bool shared = tiles == 1 && n_tiles > 1;          // both warpgroups at one tile
+    const int r = (tiles == 2 ? t : 0) * TM + row;
+    const uint32_t t_lane = (uint32_t)(qd * 32) << 16, t_o = tmem_base + 256 + (tiles == 2 ? t : 0) * 128 + t_lane;
+    const bool row_valid = r < n_tok;
+    const int hi = row_valid ? pos0 + r + 1 : -1;
+    const int lo = p.window > 0 ? max(hi - p.window, 0) : 0;
+    const int n_mine = tiles == 2 ? n_tiles : (n_tiles + 1 - t) / 2;
+    float m_used, l_run, f0 = 1.f, f1 = 0.f;
+    if (n_mine > 0)
+      prompt::softmax_role<T, NV * 64, false>(bars, t, tmem_base + t * 128 + t_lane, tmem_base + 256 + t * 128 + t_lane, n_mine,
+                                              (tile_lo + (tiles == 2 ? 0 : t)) * TN, tiles == 2 ? TN : 2 * TN, lo, hi, p.sm, p.split != 0, budget, m_used,
+                                              l_run);
+    if (shared && t == 1) prompt::hand_over(ml, row, m_used, l_run);
+    if (tiles == 2 || t == 0) {
+      if (shared) prompt::take_over(ml, row, m_used, l_run, f0, f1);
       const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
       T* orow = reinterpret_cast<T*>(p.out) + (int64_t)(q0 + r) * p.out_st + (int64_t)(p.h0 + h) * p.out_sh;
 #pragma unroll
       for (int c = 0; c < NV * 64; c += 32) {
         uint32_t v[32];
-        tmem_ld_32x32(t_o + c, v);
-        tmem_ld_wait();
+        prompt::load_o(t_o, c, shared, f0, f1, v);
         if (row_valid) {
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {
@@ -228,7 +235,7 @@ template <typename T, int NN, int NR, int NV>
 static int launch(const Maps& m, const Params& p, dim3 grid, cudaStream_t st) {
   constexpr int NQ = NN + NR;
   constexpr int VS = (2 + KS) * NQ + 2 * NV <= 14 ? 2 : 1;                    // what fits into shared memory
-  const int smem = ((2 + KS) * NQ + VS * NV) * BLK + (int)sizeof(prompt::Bars<KS, VS>) + 16 + 1024;
+  const int smem = ((2 + KS) * NQ + VS * NV) * BLK + (int)sizeof(prompt::Bars<KS, VS>) + TM * 8 + 16 + 1024;
   auto k = mla_prefill_kernel<T, NN, NR, NV, VS>;
   static bool a = false;
   if (!a) { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); a = true; }
