@@ -9,16 +9,17 @@
 // CTA = four warps of one (request, head); a warp owns 4 CW columns of S, a lane 4 NI rows (rg) x CW columns (cg) of them in registers, as
 // pairs of rows for packed products.  The decay is kept aside (S = A S', A the running product, folded in before it gets small) instead of
 // being multiplied through.  The 2 CW sums of a column group are reduced over the eight row groups by halving what a lane keeps at
-// each exchange (7 shuffles for CW = 4 instead of 24).  q and k rows of eight tokens at a time are copied to shared memory ahead of
+// each exchange (7 shuffles for CW = 4 instead of 24).  q, k and v rows of sixteen tokens at a time are copied to shared memory ahead of
 // their use; norms, k . q and the gates of a token are evaluated once per CTA.
 //
-// Measured against a warp per column with strided loads and two full reductions: 8 heads of 128 x 256, 8 prompts of 860 tokens 3408 → 560 us,
-// one of 4000 5747 → 2313 us, 24 decode steps 65 → 20 us; 32 heads of 128 x 128, 8 prompts 5910 → 1096 us, 64 decode steps 310 → 56 us.
+// Measured against a warp per column with strided loads and two full reductions: 8 heads of 128 x 256, 8 prompts of 860 tokens 3408 → 456 us,
+// one of 4000 5747 → 1459 us, 24 decode steps 65 → 19 us; 32 heads of 128 x 128, 8 prompts 5910 → 851 us, 64 decode steps 310 → 52 us.  (With v
+// read from global memory token by token and eight tokens at a time, 560, 2313, 20, 1096 and 56 us: the loads of v were on the chain.)
 #include "common.cuh"
 
 namespace gdn {
 
-constexpr int WARPS = 4, CHUNK = 8;
+constexpr int WARPS = 4, CHUNK = 16;
 
 struct Params {
   const float* q; const float* k; const float* v;    // heads of a token next to each other, rows `stride` apart
@@ -47,7 +48,10 @@ VB_DEVICE void cp16(void* dst, const void* src) {
 template <typename T, int NI, int CW, bool VEC>
 __global__ void __launch_bounds__(WARPS * 32) gdn_kernel(const Params p) {
   constexpr int DK = 32 * NI, LC = 4 * CW;                     // columns of a warp
-  __shared__ __align__(16) float kq[2][CHUNK][2][DK];
+  constexpr int BC = WARPS * LC;                               // columns of the CTA
+  extern __shared__ __align__(16) float gdn_smem[];
+  float (*kq)[CHUNK][2][DK] = reinterpret_cast<float (*)[CHUNK][2][DK]>(gdn_smem);                 // [2 buffers]
+  float (*vs)[CHUNK][BC] = reinterpret_cast<float (*)[CHUNK][BC]>(gdn_smem + 2 * CHUNK * 2 * DK);  // [2 buffers]
   __shared__ float4 scal[2][CHUNK];                            // a, b, 1 / |k|, dk^-1/2 / |q|
   __shared__ float kdot_s[2][CHUNK];                           // k . q, normalised
   pdl_trigger();
@@ -55,7 +59,7 @@ __global__ void __launch_bounds__(WARPS * 32) gdn_kernel(const Params p) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rg = lane >> 2, cg = lane & 3;
   const int blocks = (p.dv + WARPS * LC - 1) / (WARPS * LC);
   const int h = blockIdx.x / blocks, r = blockIdx.y;
-  const int col0 = ((blockIdx.x % blocks) * WARPS + warp) * LC + cg * CW;
+  const int bcol0 = (blockIdx.x % blocks) * BC, col0 = bcol0 + warp * LC + cg * CW;
   const int t0 = p.qsl[r], n = p.qsl[r + 1] - t0;
   if (n <= 0) return;
   const int per = p.nv / p.nk, kh = h / per;
@@ -74,10 +78,23 @@ __global__ void __launch_bounds__(WARPS * 32) gdn_kernel(const Params p) {
       const int t = i / (2 * (DK / 4)), w = i % (2 * (DK / 4)), part = w / (DK / 4), x = (w % (DK / 4)) * 4;     // part 0: k, 1: q
       cp16(&kq[buf][t][part][x], (part ? qp : kp) + (int64_t)(c + t) * p.q_stride + x);
     }
+    const int left = min(BC, p.dv - bcol0);                    // columns that exist
+    if constexpr (VEC) {
+      for (int i = threadIdx.x; i < m * (BC / 4); i += WARPS * 32) {
+        const int t = i / (BC / 4), x = (i % (BC / 4)) * 4;
+        if (x < left) cp16(&vs[buf][t][x], vp + (int64_t)(c + t) * p.v_stride + bcol0 + x);
+      }
+    } else {
+      for (int i = threadIdx.x; i < m * BC; i += WARPS * 32) {
+        const int t = i / BC, x = i % BC;
+        if (x < left) vs[buf][t][x] = vp[(int64_t)(c + t) * p.v_stride + bcol0 + x];
+      }
+    }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  // 16 threads per token: its norms and k . q; the raw gates were loaded a chunk before
-  const int st_t = threadIdx.x >> 4, st_l = threadIdx.x & 15;
+  // eight threads per token: its norms and k . q; the raw gates were loaded a chunk before
+  constexpr int PT = WARPS * 32 / CHUNK;
+  const int st_t = threadIdx.x / PT, st_l = threadIdx.x % PT;
   float raw_b = 0.f, raw_a = 0.f;
   auto raw = [&](int c) {
     if (st_l == 0 && c + st_t < n) {
@@ -122,7 +139,7 @@ __global__ void __launch_bounds__(WARPS * 32) gdn_kernel(const Params p) {
   // what a lane holds after the reduction: of column own (of its group) the product with k (lower half of the warp) or with q
   const int own = CW == 4 ? rg & 3 : (rg >> 1) & 1, my_col = col0 + own;
   const bool has_q = rg >= 4;
-  float A = 1.f, v_next = my_col < p.dv ? vp[my_col] : 0.f;
+  float A = 1.f;
   for (int c = 0; c < n; c += CHUNK) {
     const int buf = (c / CHUNK) & 1, m = min(CHUNK, n - c);
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -132,13 +149,13 @@ __global__ void __launch_bounds__(WARPS * 32) gdn_kernel(const Params p) {
       float kk = 0.f, qq = 0.f, kd = 0.f;
       if (st_t < m) {
 #pragma unroll
-        for (int i = 0; i < DK / 16; ++i) {
-          const float a = kq[buf][st_t][0][st_l + 16 * i], b = kq[buf][st_t][1][st_l + 16 * i];
+        for (int i = 0; i < DK / PT; ++i) {
+          const float a = kq[buf][st_t][0][st_l + PT * i], b = kq[buf][st_t][1][st_l + PT * i];
           kk += a * a; qq += b * b; kd += a * b;
         }
       }
 #pragma unroll
-      for (int o = 8; o > 0; o >>= 1) {
+      for (int o = PT / 2; o > 0; o >>= 1) {
         kk += __shfl_xor_sync(0xffffffffu, kk, o);
         qq += __shfl_xor_sync(0xffffffffu, qq, o);
         kd += __shfl_xor_sync(0xffffffffu, kd, o);
@@ -159,8 +176,7 @@ __global__ void __launch_bounds__(WARPS * 32) gdn_kernel(const Params p) {
 #pragma unroll 1
     for (int t = 0; t < m; ++t) {
       const float4 s = scal[buf][t];
-      const float kdot = kdot_s[buf][t], v = v_next;
-      if (c + t + 1 < n && my_col < p.dv) v_next = vp[(int64_t)(c + t + 1) * p.v_stride + my_col];
+      const float kdot = kdot_s[buf][t], v = my_col < p.dv ? vs[buf][t][my_col - bcol0] : 0.f;
       A *= s.x;
       uint64_t kv[2 * NI], a1[CW], a2[CW];
 #pragma unroll
@@ -216,7 +232,7 @@ __global__ void __launch_bounds__(WARPS * 32) gdn_kernel(const Params p) {
           for (int i = 0; i < 2 * NI; ++i) S[j][i] = mul2(S[j][i], aa);
         A = 1.f;
       }
-      const float f = s.z / A;
+      const float f = __fdividef(s.z, A);
 #pragma unroll
       for (int j = 0; j < CW; ++j) {
         const uint64_t dd = pk(dc[j] * f, dc[j] * f);
@@ -255,8 +271,10 @@ template <typename T, int NI, int CW>
 static int launch(const Params& p, bool vec, int num_reqs, cudaStream_t st) {
   const int blocks = (p.dv + WARPS * 4 * CW - 1) / (WARPS * 4 * CW);
   const dim3 grid(p.nv * blocks, num_reqs);
-  if (vec) vb_launch(gdn_kernel<T, NI, CW, true>, grid, dim3(WARPS * 32), 0, st, p);
-  else vb_launch(gdn_kernel<T, NI, CW, false>, grid, dim3(WARPS * 32), 0, st, p);
+  const size_t smem = (size_t)2 * CHUNK * (2 * 32 * NI + WARPS * 4 * CW) * sizeof(float);
+  auto k = vec ? gdn_kernel<T, NI, CW, true> : gdn_kernel<T, NI, CW, false>;
+  if (smem > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -5;
+  vb_launch(k, grid, dim3(WARPS * 32), smem, st, p);
   return (int)cudaGetLastError();
 }
 
@@ -276,7 +294,7 @@ EXPORT int vb_gated_delta(const float* q, const float* k, int64_t q_stride, cons
   p.q = q; p.k = k; p.v = v; p.ba = ba; p.A_log = A_log; p.dt_bias = dt_bias; p.g = g; p.beta = beta; p.o = o; p.state = state; p.qsl = qsl;
   p.seq_lens = seq_lens; p.rows = rows; p.q_stride = q_stride; p.v_stride = v_stride; p.ba_stride = ba_stride; p.state_stride = state_stride;
   p.state_off = state_off; p.rows_stride = rows_stride; p.nk = nk; p.nv = nv; p.dv = dv; p.q_scale = q_scale; p.beta_scale = beta_scale; p.eps = eps;
-  const bool vec = dv % 4 == 0 && state_stride % 4 == 0 && state_off % 4 == 0 && (reinterpret_cast<uintptr_t>(state) & 15) == 0;
+  const bool vec = dv % 4 == 0 && v_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(v) & 15) == 0 && state_stride % 4 == 0 && state_off % 4 == 0 && (reinterpret_cast<uintptr_t>(state) & 15) == 0;
 #define GO(NI, CW) launch<T, NI, CW>(p, vec, num_reqs, st)
   DISPATCH_DTYPE(dtype, T, {
     switch (dk / 32) {
