@@ -93,3 +93,22 @@ def test_gathered_rows_end_in_zeros(lens):
     for i, n in enumerate(lens or [5, 130, 64]):
         want[starts[i]:starts[i] + n] = cache[bt[i].long()].view(-1, 72)[:n]
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("H,R,P", [(16, 512, 64), (32, 512, 64), (5, 136, 16), (128, 512, 64)])
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_latent_rows(H, R, P, wide, splits):
+    lens = [1, 63, 64, 65, 200, 1030]
+    g = torch.Generator(device="cuda").manual_seed(8)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)  # noqa: E731
+    cache, q, qp = rnd(60, 64, R + P), rnd(len(lens), H, R), rnd(len(lens), H, P)
+    bt = torch.randperm(60, device="cuda", generator=g)[:17].int()[None].repeat(len(lens), 1).contiguous()
+    got = cu().mla_decode_tc(q, qp, cache, bt, torch.tensor(lens, dtype=torch.int32, device="cuda"), 0.06, max(lens), splits, wide=wide)
+    cu().check_kernel_error(q.device)
+    want = []
+    for i, n in enumerate(lens):
+        kv = cache[bt[i].long()].view(-1, R + P)[:n].double()
+        w = (torch.cat([q[i], qp[i]], -1).double() @ kv.t() * 0.06).softmax(-1)
+        want.append(w @ kv[:, :R])
+    assert _rel(got, torch.stack(want)) < LIMIT[wide], _rel(got, torch.stack(want))

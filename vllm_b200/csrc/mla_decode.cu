@@ -24,6 +24,9 @@
 // never looks at, and cost nothing that matters — at 16-32 heads per CTA the kernel is bound by the latent stream
 // (1152 B per token), not by tensor-core time.
 //
+// wide: the rows of short portions in steps that are not decode steps alone, whose weights were held in 32 bits on the CUDA cores: the second product
+// of the weights' low parts costs 1 to 3 us of 40; the rows of a step of 24 requests took 660 us there.
+//
 // Reference kernels for the op: csrc/libtorch_stable/attention/mla/sm100_cutlass_mla_kernel.cu (+ cutlass_sm100_mla/),
 // FlashMLA; algorithm: vllm/model_executor/layers/attention/mla_attention.py:1-200 (absorbed-weight decode).
 #include "common.cuh"
@@ -54,6 +57,7 @@ struct Params {
   int bt_stride;
   int H, BS, num_splits, R;
   int window;           // > 0: a query sees its last `window` keys
+  int wide;             // weights keep 16 more bits: P = hi + lo, two products (rows of mixed steps, whose weights are held in 32 bits)
   int* error;           // raised when a wait ran into its limit
   float scale_log2;
 };
@@ -96,7 +100,9 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_cons
   constexpr int NKB = Geo<NL, ROPE>::NKB, STAGE_BYTES = Geo<NL, ROPE>::STAGE_BYTES, STAGES = Geo<NL, ROPE>::STAGES;
   constexpr int NC = Geo<NL, ROPE>::NC;
   constexpr int Q_BYTES = NKB * N * 128;     // k-blocks of [N x 64]
-  constexpr int P_BYTES = N * 128;           // [N x 64 tok]
+  constexpr int P_BYTES = N * 128;           // [N x 64 tok]; low parts P_LOW further
+  constexpr int P_LOW = 4096;
+  static_assert(P_BYTES <= P_LOW, "both parts share 8 KB");
   constexpr int CH = 16;                     // TMEM columns moved per tcgen05.ld/st
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -266,10 +272,13 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_cons
         if (lane == 0) {
 #pragma unroll
           for (int c = 0; c < NC; ++c) {
+#pragma unroll 1
+            for (int low = 0; low <= p.wide; ++low) {
 #pragma unroll
-            for (int kk = 0; kk < TILE / 16; ++kk) {
-              const uint64_t da = d_kv_mn + (uint64_t)((st * STAGE_BYTES + (2 * c) * KB_BYTES + kk * 2048) >> 4);
-              umma_f16(tmem_o + c * N, da, d_p + (uint64_t)(kk * 2), idesc_o, (jj | kk) != 0);
+              for (int kk = 0; kk < TILE / 16; ++kk) {
+                const uint64_t da = d_kv_mn + (uint64_t)((st * STAGE_BYTES + (2 * c) * KB_BYTES + kk * 2048) >> 4);
+                umma_f16(tmem_o + c * N, da, d_p + (uint64_t)(low * (P_LOW / 16) + kk * 2), idesc_o, (jj | kk | low) != 0);
+              }
             }
             umma_commit(&kv_empty[st * NKB + 2 * c]);
             if (2 * c + 1 < NL) umma_commit(&kv_empty[st * NKB + 2 * c + 1]);
@@ -347,7 +356,11 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_cons
         const float m_ref = (m_used[g] == -INFINITY) ? 0.f : m_used[g];
         const float pe = ok ? ex2(s[g] - m_ref) : 0.f;
         l_thr[g] += pe;
-        if (t < TILE) *reinterpret_cast<T*>(pcol + g * 128 + ((chunk ^ (g & 7)) << 4)) = from_f32<T>(pe);
+        if (t < TILE) {
+          const T hi = from_f32<T>(pe);
+          *reinterpret_cast<T*>(pcol + g * 128 + ((chunk ^ (g & 7)) << 4)) = hi;
+          if (p.wide) *reinterpret_cast<T*>(pcol + P_LOW + g * 128 + ((chunk ^ (g & 7)) << 4)) = from_f32<T>(pe - to_f32(hi));
+        }
       }
       tc_fence_before();
       fence_proxy_async();
@@ -466,10 +479,10 @@ static int launch(const CUtensorMap& tqn, const CUtensorMap& tqr, const CUtensor
 // bf16 covers every R (a multiple of 8 up to 512) and rope part (none, or a multiple of 8 up to 64); fp16 R = 512 with 64 only.
 // window > 0: row b sees keys seq_lens[b] - window .. seq_lens[b] - 1.
 // `error` (device int, may be null) becomes 1 when a wait inside the kernel ran into its limit.
-EXPORT int vb_mla_decode(const void* q_nope, const void* q_pe, const void* cache, int64_t num_blocks, const int* block_table,
+EXPORT int vb_mla_decode2(const void* q_nope, const void* q_pe, const void* cache, int64_t num_blocks, const int* block_table,
                          const int* seq_lens, void* out, float* part_out, float* part_lse, float* lse_out, int* error, int B,
                          int H, int R, int rope, int BS, int64_t qn_stride_b, int64_t qn_stride_h, int64_t qr_stride_b,
-                         int64_t qr_stride_h, int64_t out_stride, int bt_stride, int num_splits, int window, float scale, int dtype,
+                         int64_t qr_stride_h, int64_t out_stride, int bt_stride, int num_splits, int window, int wide, float scale, int dtype,
                          cudaStream_t st) {
   using namespace mla;
   if (B == 0) return 0;
@@ -485,7 +498,7 @@ EXPORT int vb_mla_decode(const void* q_nope, const void* q_pe, const void* cache
   Params p;
   p.block_table = block_table; p.seq_lens = seq_lens; p.out = out; p.part_out = part_out; p.part_lse = part_lse;
   p.lse_out = lse_out; p.out_stride = out_stride; p.bt_stride = bt_stride; p.H = H; p.BS = BS; p.num_splits = num_splits;
-  p.R = R; p.error = error; p.window = window;
+  p.R = R; p.error = error; p.window = window; p.wide = wide;
   p.scale_log2 = scale * 1.4426950408889634f;
   CUtensorMap tqn, tqr, tkv;
   const int gbox = H < N ? H : N;

@@ -114,7 +114,7 @@ class LatentForms:
     ``window``, and ``_up()``, ``_expand(c, h0, h1)``."""
     # keys of a request start on a boundary of the prompt kernel's key tiles, zeros fill the gap: no tile holds two requests' values
     kv_apart = 1
-    # softmax weights of prompts keep 16 more bits; rows in the latent space keep 32 in steps that are not decode steps alone
+    # softmax weights keep 16 more bits in steps that are not decode steps alone
     wide_weights = False
 
     def _attend(self, q: torch.Tensor, md: AttentionMetadata, cache: torch.Tensor) -> torch.Tensor:
@@ -126,10 +126,8 @@ class LatentForms:
         plan = LatentPlan.of(md, q.device, self.window, self.kv_apart)
         if plan.num_rows:
             def attend(q_abs, q_pe):
-                if self.wide_weights:
-                    return ops.cuda_ops().mla_simt(q_abs, q_pe, cache, plan.row_block_table, plan.row_seq_lens, None, self.scale, window)
                 return ops.mla_attention_rows(q_abs, q_pe, cache, plan.row_block_table, plan.row_seq_lens, plan.max_row_len,
-                                              self.scale, window)
+                                              self.scale, window, self.wide_weights)
             if plan.rows is None:
                 return self._absorbed(q, out, attend)
             part = torch.empty(plan.num_rows, self.heads, self.v_dim, dtype=q.dtype, device=q.device)

@@ -228,12 +228,13 @@ def mla_attention(q_nope_abs, q_pe, kv_cache, md, scale, kv_lora_rank, sliding_w
     return ref.mla_decode_attention(q_nope_abs, q_pe, kv_cache, md.block_table, sl, qsl, scale, kv_lora_rank, sliding_window)
 
 
-def mla_attention_rows(q_abs, q_pe, kv_cache, block_table, seq_lens, max_len: int, scale, sliding_window: Optional[int] = None):
+def mla_attention_rows(q_abs, q_pe, kv_cache, block_table, seq_lens, max_len: int, scale, sliding_window: Optional[int] = None,
+                       wide: bool = False):
     """Attention over the latent cache for rows with a block table and a number of visible keys each (CUDA); with a window, of its last
-    ones."""
+    ones.  ``wide``: the softmax weights keep 16 more bits."""
     cu = cuda_ops()
     if cu._mla_tc_ok(q_abs, q_pe, kv_cache):
-        return cu.mla_decode_tc(q_abs, q_pe, kv_cache, block_table, seq_lens, scale, max_len, sliding_window=sliding_window)
+        return cu.mla_decode_tc(q_abs, q_pe, kv_cache, block_table, seq_lens, scale, max_len, sliding_window=sliding_window, wide=wide)
     return cu.mla_simt(q_abs, q_pe, kv_cache, block_table, seq_lens, None, scale, sliding_window)
 
 

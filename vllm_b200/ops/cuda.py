@@ -531,8 +531,8 @@ def merge_attn_states(o1, lse1, o2, lse2):
     return out, lse
 
 
-_mla_decode = _sig("vb_mla_decode", _vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i64, _i64,
-                   _i64, _i64, _i64, _i, _i, _i, _f, _i, _vp)
+_mla_decode = _sig("vb_mla_decode2", _vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i64, _i64,
+                   _i64, _i64, _i64, _i, _i, _i, _i, _f, _i, _vp)
 _mla_prefill = _sig("vb_mla_prefill2", _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i64, _i, _i, _i, _i, _i, _i, _i64, _i64,
                     _i64, _i64, _i64, _i64, _i64, _i, _i, _f, _i, _i, _vp)
 _mla_simt = _sig("vb_mla_simt", _vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _i, _i, _i, _i, _i, _i, _i64, _i64, _i64, _i64, _i64,
@@ -575,8 +575,9 @@ def mla_decode_splits(B: int, H: int, max_seq_len: int, least: int = 512) -> int
 
 
 def mla_decode_tc(q_nope_abs, q_pe, kv_cache, block_table, seq_lens, scale, max_seq_len: int, num_splits: int = 0,
-                  return_lse: bool = False, sliding_window: Optional[int] = None):
-    """tcgen05 MLA decode (csrc/mla_decode.cu): q_nope_abs [B, H, R], q_pe [B, H, P] or None, cache [blocks, BS, R + P]."""
+                  return_lse: bool = False, sliding_window: Optional[int] = None, wide: bool = False):
+    """tcgen05 MLA decode (csrc/mla_decode.cu): q_nope_abs [B, H, R], q_pe [B, H, P] or None, cache [blocks, BS, R + P].  ``wide``: the
+    softmax weights keep 16 more bits."""
     B, H, R = q_nope_abs.shape
     P = 0 if q_pe is None else q_pe.shape[-1]
     assert kv_cache.shape[-1] == R + P and q_nope_abs.stride(-1) == 1 and (q_pe is None or q_pe.stride(-1) == 1)
@@ -602,7 +603,7 @@ def mla_decode_tc(q_nope_abs, q_pe, kv_cache, block_table, seq_lens, scale, max_
                        block_table.data_ptr(), seq_lens.data_ptr(), out.data_ptr(), _p(po), _p(pl), _p(lse), err.data_ptr(), B,
                        H, R, P, kv_cache.shape[1], q_nope_abs.stride(0), q_nope_abs.stride(1),
                        q_pe.stride(0) if P else 0, q_pe.stride(1) if P else 0,
-                       out.stride(0), block_table.stride(0), splits, sliding_window or 0, scale, _DT[q_nope_abs.dtype], _st()),
+                       out.stride(0), block_table.stride(0), splits, sliding_window or 0, int(wide), scale, _DT[q_nope_abs.dtype], _st()),
            f"mla_decode(B={B},H={H},R={R})", 2 if splits > 1 else 1)
     return (out, lse) if return_lse else out
 
