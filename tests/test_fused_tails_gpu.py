@@ -14,7 +14,7 @@ def _norm(x, w, gemma, eps):
     return x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps) * (w + 1 if gemma else w)
 
 
-@pytest.mark.parametrize("T,H", [(1, 64), (3, 2048), (700, 1032), (5, 16384)])
+@pytest.mark.parametrize("T,H", [(1, 64), (3, 2048), (700, 1032), (5, 16384), (1025, 2056), (1024, 8192)])
 @pytest.mark.parametrize("gemma", [False, True])
 @pytest.mark.parametrize("dtype", [BF, torch.float16])
 def test_norm_add_norm(T, H, gemma, dtype):
@@ -29,7 +29,7 @@ def test_norm_add_norm(T, H, gemma, dtype):
     assert _rel(y, _norm(s, w2.double(), gemma, 1e-5)) < 2 * ulp          # of the stream, and its own
 
 
-@pytest.mark.parametrize("T,H,k", [(1, 64, 1), (37, 2048, 6), (300, 1032, 3), (2, 9000, 2)])
+@pytest.mark.parametrize("T,H,k", [(1, 64, 1), (37, 2048, 6), (300, 1032, 3), (2, 9000, 2), (9, 2048, 9)])
 @pytest.mark.parametrize("shared", [None, "plain", "gated"])
 def test_combine_norm(T, H, k, shared):
     from vllm_b200.ops import cuda as cu
@@ -75,3 +75,16 @@ def test_values_turned(Hkv, D, BS):
         w = torch.ones(D, device="cuda", dtype=BF)
         cu.fused_qk_norm_rope(pos, q, k, w, w, cs, D, 1e-6, True, v=v, kv_cache=cache, slot_mapping=slots, vt=True)
         assert torch.equal(cache[:, 1].reshape(want.shape), want)
+
+
+@pytest.mark.parametrize("T,H", [(1024, 2048), (1030, 2056), (1024, 16384), (1023, 2048)])
+@pytest.mark.parametrize("add", [False, True])
+def test_norms_of_prompts(T, H, add):
+    """Rows whose threads take several vectors, and the last batch that takes one."""
+    from vllm_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x, r, w = (torch.randn(*s, device="cuda", generator=g).to(BF) for s in ((T, H), (T, H), (H,)))
+    s = (x.float() + r.float()).to(BF) if add else x.clone()
+    y = ops.fused_add_rms_norm(x, r, w, 1e-6)[0] if add else ops.rms_norm(x, w, 1e-6)
+    assert not add or torch.equal(r, s)
+    assert _rel(y, _norm(s.double(), w.double(), False, 1e-6)) < 2 ** -9

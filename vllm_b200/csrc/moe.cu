@@ -377,7 +377,7 @@ __global__ void combine_kernel(const T* __restrict__ y, const int* __restrict__ 
 // Tail of a sparse block, one CTA per token:  r += sum_j w[t, j] y[inv[t k + j], :] + sigmoid(gate[t]) extra[t, :];  out = norm(r) * nw
 // (extra: a shared expert's output, or null; gate null: 1).  32-bit until r is rounded; a combine, a gating product, two additions and a
 // norm were six launches and as many passes over [T, H].
-template <typename T, bool GEMMA>
+template <typename T, bool GEMMA, int MAXV>
 __global__ void __launch_bounds__(1024) combine_norm_kernel(const T* __restrict__ y, const int* __restrict__ inv, const float* __restrict__ w, int k,
                                                             const T* __restrict__ extra, const T* __restrict__ gate, T* __restrict__ residual,
                                                             const T* __restrict__ nw, T* __restrict__ out, int H, float eps) {
@@ -385,7 +385,6 @@ __global__ void __launch_bounds__(1024) combine_norm_kernel(const T* __restrict_
   pdl_trigger();
   pdl_wait();
   const int64_t t = blockIdx.x;
-  constexpr int MAXV = 4;                      // vectors of a thread kept in registers (H <= 1024 * 8 * 4)
   const int nvec = H / 8;
   const float g = extra && gate ? 1.f / (1.f + expf(-to_f32(gate[t]))) : 1.f;
   Vec16<T> r[MAXV];
@@ -404,13 +403,21 @@ __global__ void __launch_bounds__(1024) combine_norm_kernel(const T* __restrict_
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] = 0.f;
     }
-    for (int u = 0; u < k; ++u) {
-      const int p = inv[t * k + u];
-      if (p < 0) continue;
-      const float wu = w[t * k + u];
-      const Vec16<T> v = ld16(y + (size_t)p * H + vi * 8);
+    for (int u0 = 0; u0 < k; u0 += 4) {          // four rows on their way at a time
+      int p[4];
+      float wu[4];
+      Vec16<T> v[4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] += wu * to_f32(v.e[j]);
+      for (int u = 0; u < 4; ++u) {
+        p[u] = u0 + u < k ? inv[t * k + u0 + u] : -1;
+        if (p[u] >= 0) { wu[u] = w[t * k + u0 + u]; v[u] = ld16(y + (size_t)p[u] * H + vi * 8); }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (p[u] < 0) continue;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] += wu[u] * to_f32(v[u].e[j]);
+      }
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -418,13 +425,13 @@ __global__ void __launch_bounds__(1024) combine_norm_kernel(const T* __restrict_
       const float f = to_f32(r[i].e[j]);
       ss += f * f;
     }
-    st16(residual + t * H + vi * 8, r[i]);
   }
   const float s = rsqrtf(block_sum(ss, red) / (float)H + eps);
 #pragma unroll
   for (int i = 0; i < MAXV; ++i) {
     const int vi = threadIdx.x + i * blockDim.x;
     if (vi >= nvec) continue;
+    st16(residual + t * H + vi * 8, r[i]);
     const Vec16<T> n = ld16(nw + vi * 8);
 #pragma unroll
     for (int j = 0; j < 8; ++j) r[i].e[j] = from_f32<T>(to_f32(r[i].e[j]) * s * (to_f32(n.e[j]) + (GEMMA ? 1.f : 0.f)));
@@ -534,9 +541,11 @@ EXPORT int vb_moe_combine_norm(const void* y, const int* inv, const float* w, in
                                const void* nw, void* out, int T_, int H, float eps, int gemma, int dtype, cudaStream_t st) {
   if (T_ == 0) return 0;
   if (dtype == DT_F32 || H % 8 || H / 8 > 4096 || k < 1) return -1;
-  int thr = (H / 8 + 31) / 32 * 32;
+  const int nvec = H / 8, quarter = ((nvec + 3) / 4 + 31) / 32 * 32;   // vectors of a row, threads with four each
+  int thr = (nvec + 31) / 32 * 32;
+  if (T_ >= 1024 && nvec >= 256) thr = quarter < 128 ? 128 : quarter;      // as norm_threads
   if (thr > 1024) thr = 1024;
-#define GO(G) vb_launch(moe::combine_norm_kernel<T, G>, dim3(T_), dim3(thr), 0, st, (const T*)y, inv, w, k, (const T*)extra, (const T*)gate, (T*)residual, (const T*)nw, (T*)out, H, eps)
+#define GO(G) vb_launch(thr >= nvec ? moe::combine_norm_kernel<T, G, 1> : moe::combine_norm_kernel<T, G, 4>, dim3(T_), dim3(thr), 0, st, (const T*)y, inv, w, k, (const T*)extra, (const T*)gate, (T*)residual, (const T*)nw, (T*)out, H, eps)
   DISPATCH_HALF(dtype, T, { if (gemma) GO(true); else GO(false); });
 #undef GO
   return (int)cudaGetLastError();

@@ -10,7 +10,8 @@ namespace {
 
 constexpr int MAXV = 4;  // 16B vectors per thread kept in registers
 
-template <typename T, bool ADD, bool GEMMA>
+// MV vectors of 16 bytes per thread: one where a CTA of a thread per vector exists (few rows: latency), up to four for prompts (norm_threads)
+template <typename T, bool ADD, bool GEMMA, int MV>
 __global__ void __launch_bounds__(1024) rms_norm_kernel(T* __restrict__ out, T* __restrict__ x,
                                                          T* __restrict__ residual, const T* __restrict__ w,
                                                          int H, float eps, int64_t x_stride) {
@@ -23,13 +24,14 @@ __global__ void __launch_bounds__(1024) rms_norm_kernel(T* __restrict__ out, T* 
   T* rr = ADD ? residual + row * (int64_t)H : nullptr;
   T* orow = out + row * (ADD ? x_stride : (int64_t)H);
   const int nvec = H / N;
-  Vec16<T> v[MAXV];
+  Vec16<T> v[MV], wv[MV];
   float ss = 0.f;
 #pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
+  for (int i = 0; i < MV; ++i) {
     const int vi = threadIdx.x + i * blockDim.x;
     if (vi < nvec) {
       v[i] = ld16(xr + vi * N);
+      wv[i] = ld16(w + vi * N);
       if (ADD) {
         Vec16<T> r = ld16(rr + vi * N);
 #pragma unroll
@@ -43,13 +45,13 @@ __global__ void __launch_bounds__(1024) rms_norm_kernel(T* __restrict__ out, T* 
   ss = block_sum(ss, red);
   const float inv = rsqrtf(ss / (float)H + eps);
 #pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
+  for (int i = 0; i < MV; ++i) {
     const int vi = threadIdx.x + i * blockDim.x;
     if (vi < nvec) {
-      Vec16<T> wv = ld16(w + vi * N), o;
+      Vec16<T> o;
 #pragma unroll
       for (int j = 0; j < N; ++j) {
-        float g = to_f32(wv.e[j]);
+        float g = to_f32(wv[i].e[j]);
         if (GEMMA) g += 1.f;
         o.e[j] = from_f32<T>(to_f32(v[i].e[j]) * inv * g);
       }
@@ -60,7 +62,7 @@ __global__ void __launch_bounds__(1024) rms_norm_kernel(T* __restrict__ out, T* 
 
 // Norm of a block's output, residual add and the next block's norm in one pass over the row:
 //   r += x * rsqrt(mean(x^2) + eps) * w1;  out = r * rsqrt(mean(r^2) + eps) * w2      (one rounding of r, one of out)
-template <typename T, bool GEMMA>
+template <typename T, bool GEMMA, int MV>
 __global__ void __launch_bounds__(1024) norm_add_norm_kernel(T* __restrict__ out, const T* __restrict__ x, T* __restrict__ residual,
                                                               const T* __restrict__ w1, const T* __restrict__ w2, int H, float eps1, float eps2) {
   constexpr int N = Vec16<T>::N;
@@ -71,10 +73,10 @@ __global__ void __launch_bounds__(1024) norm_add_norm_kernel(T* __restrict__ out
   const T* xr = x + row * (int64_t)H;
   T* rr = residual + row * (int64_t)H;
   const int nvec = H / N;
-  Vec16<T> v[MAXV], r[MAXV];
+  Vec16<T> v[MV], r[MV];
   float ss = 0.f;
 #pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
+  for (int i = 0; i < MV; ++i) {
     const int vi = threadIdx.x + i * blockDim.x;
     if (vi < nvec) {
       v[i] = ld16(xr + vi * N);
@@ -86,7 +88,7 @@ __global__ void __launch_bounds__(1024) norm_add_norm_kernel(T* __restrict__ out
   const float i1 = rsqrtf(block_sum(ss, red) / (float)H + eps1);
   ss = 0.f;
 #pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
+  for (int i = 0; i < MV; ++i) {
     const int vi = threadIdx.x + i * blockDim.x;
     if (vi < nvec) {
       const Vec16<T> g = ld16(w1 + vi * N);
@@ -102,7 +104,7 @@ __global__ void __launch_bounds__(1024) norm_add_norm_kernel(T* __restrict__ out
   }
   const float i2 = rsqrtf(block_sum(ss, red) / (float)H + eps2);
 #pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
+  for (int i = 0; i < MV; ++i) {
     const int vi = threadIdx.x + i * blockDim.x;
     if (vi < nvec) {
       const Vec16<T> g = ld16(w2 + vi * N);
@@ -256,10 +258,14 @@ __global__ void soft_cap_kernel(T* __restrict__ x, int64_t stride, int n, int64_
   }
 }
 
-int norm_threads(int H, int vecN) {
+// Prompts (enough rows to fill the SMs several times over) give a thread two to four vectors: fewer threads to hold up at the reduction, as many
+// loads in flight.  Add and norm of 7600 rows: 4096 wide 59 → 41 us (6.1 TB/s), 8192 wide 125 → 80; 1024 rows of 4096 14 → 10; below
+// and for rows of less than 256 vectors no difference.
+int norm_threads(int H, int vecN, int T = 0) {
   int nvec = H / vecN;
   int t = (nvec + MAXV - 1) / MAXV;
   t = ((t + 31) / 32) * 32;
+  if (T >= 1024 && nvec >= 256) return t > 1024 ? 1024 : (t < 128 ? 128 : t);
   if (t < 32) t = 32;
   // prefer more threads (1 vector each) while the row fits
   int t1 = ((nvec + 31) / 32) * 32;
@@ -270,19 +276,22 @@ int norm_threads(int H, int vecN) {
 }  // namespace
 
 // x: [T, H] (row stride x_stride elements), w: [H]. ADD: residual [T, H] contiguous updated in place, normed → x.
+#define NORM(A, G) (one ? rms_norm_kernel<TT, A, G, 1> : rms_norm_kernel<TT, A, G, MAXV>)
+#define TAIL(G) (one ? norm_add_norm_kernel<TT, G, 1> : norm_add_norm_kernel<TT, G, MAXV>)
 EXPORT int vb_rms_norm(void* out, void* x, void* residual, const void* w, int T, int H, int64_t x_stride, float eps,
                        int gemma, int dtype, cudaStream_t st) {
   if (T == 0) return 0;
   DISPATCH_DTYPE(dtype, TT, {
     constexpr int N = Vec16<TT>::N;
     if (H % N != 0 || H / N > 1024 * MAXV) return -1;
-    const int thr = norm_threads(H, N);
+    const int thr = norm_threads(H, N, T);
+    const bool one = thr * N >= H;
     if (residual) {
-      if (gemma) vb_launch(rms_norm_kernel<TT, true, true>, T, thr, 0, st, (TT*)x, (TT*)x, (TT*)residual, (const TT*)w, H, eps, x_stride);
-      else vb_launch(rms_norm_kernel<TT, true, false>, T, thr, 0, st, (TT*)x, (TT*)x, (TT*)residual, (const TT*)w, H, eps, x_stride);
+      if (gemma) vb_launch(NORM(true, true), T, thr, 0, st, (TT*)x, (TT*)x, (TT*)residual, (const TT*)w, H, eps, x_stride);
+      else vb_launch(NORM(true, false), T, thr, 0, st, (TT*)x, (TT*)x, (TT*)residual, (const TT*)w, H, eps, x_stride);
     } else {
-      if (gemma) vb_launch(rms_norm_kernel<TT, false, true>, T, thr, 0, st, (TT*)out, (TT*)x, (TT*)nullptr, (const TT*)w, H, eps, x_stride);
-      else vb_launch(rms_norm_kernel<TT, false, false>, T, thr, 0, st, (TT*)out, (TT*)x, (TT*)nullptr, (const TT*)w, H, eps, x_stride);
+      if (gemma) vb_launch(NORM(false, true), T, thr, 0, st, (TT*)out, (TT*)x, (TT*)nullptr, (const TT*)w, H, eps, x_stride);
+      else vb_launch(NORM(false, false), T, thr, 0, st, (TT*)out, (TT*)x, (TT*)nullptr, (const TT*)w, H, eps, x_stride);
     }
   });
   return (int)cudaGetLastError();
@@ -295,12 +304,16 @@ EXPORT int vb_norm_add_norm(void* out, const void* x, void* residual, const void
   DISPATCH_DTYPE(dtype, TT, {
     constexpr int N = Vec16<TT>::N;
     if (H % N != 0 || H / N > 1024 * MAXV) return -1;
-    const int thr = norm_threads(H, N);
-    if (gemma) vb_launch(norm_add_norm_kernel<TT, true>, T, thr, 0, st, (TT*)out, (const TT*)x, (TT*)residual, (const TT*)w1, (const TT*)w2, H, eps1, eps2);
-    else vb_launch(norm_add_norm_kernel<TT, false>, T, thr, 0, st, (TT*)out, (const TT*)x, (TT*)residual, (const TT*)w1, (const TT*)w2, H, eps1, eps2);
+    const int thr = norm_threads(H, N, T);
+    const bool one = thr * N >= H;
+    if (gemma) vb_launch(TAIL(true), T, thr, 0, st, (TT*)out, (const TT*)x, (TT*)residual, (const TT*)w1, (const TT*)w2, H, eps1, eps2);
+    else vb_launch(TAIL(false), T, thr, 0, st, (TT*)out, (const TT*)x, (TT*)residual, (const TT*)w1, (const TT*)w2, H, eps1, eps2);
   });
   return (int)cudaGetLastError();
 }
+
+#undef NORM
+#undef TAIL
 
 EXPORT int vb_layer_norm(void* out, const void* x, const void* w, const void* b, int T, int H, float eps, int dtype,
                          cudaStream_t st) {
@@ -427,7 +440,6 @@ EXPORT int vb_sigmoid_mul(const void* x, int64_t x_stride, const void* g, int64_
     if (n % N == 0 && x_stride % N == 0 && g_stride % N == 0 && y_stride % N == 0 && al(x) && al(g) && al(y)) GO(N);
     else GO(1);
   });
-#undef GO
   return (int)cudaGetLastError();
 }
 
