@@ -52,3 +52,20 @@ def test_prompt_experts_match_decode_experts(T, E, k, mapped):
     n = moe.GROUPED_MAX_ROWS // k
     want = torch.cat([moe.fused_moe_cuda(x[i:i + n], w13, w2, w[i:i + n], ids[i:i + n], "silu", emap) for i in range(0, T, n)])
     assert _rel(got, want) < 2 ** -7            # hidden rows rounded to bf16 on one side only, and both results
+
+
+@pytest.mark.parametrize("R,E,bn", [(6, 32, 16), (144, 32, 16), (384, 32, 32), (256, 16, 32), (513, 64, 32), (1000, 128, 16), (40, 8, 16)])
+def test_both_grids_of_decode_experts(R, E, bn):
+    """Grid by rows and grid by possible chunks: the same products, also where most experts have no row and rows are missing at the end."""
+    from vllm_b200.ops import cuda as cu, moe
+    assert moe.flat_grid(R, E, bn) == (bn == 16 or E * -(-R // bn) > 128)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(R, 128, device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn(E, 136, 128, device="cuda", generator=g).to(torch.bfloat16)
+    for spread in (E, max(E // 8, 1)):
+        n = torch.bincount(torch.randint(0, spread, (R - R // 10,), device="cuda", generator=g) * (E // spread), minlength=E)
+        offs = torch.cat([n.new_zeros(1), n.cumsum(0)]).int()
+        a, b = (cu.gemm_tc_grouped(x, w, offs, bn, flat=f)[:R - R // 10] for f in (False, True))
+        assert torch.equal(a, b)
+        want = torch.cat([xe.double() @ we.double().t() for xe, we in zip(x[:R - R // 10].split(n.tolist()), w)])
+        assert _rel(a, want) < 2 ** -9
