@@ -31,9 +31,9 @@ template <int N> VB_DEVICE void regs_inc() { asm volatile("setmaxnreg.inc.sync.a
 constexpr int BLK = 128 * 128;              // one [128 rows x 64 values] block of 16-bit values, 16 KB
 
 // D[tmem] (+)= A[tmem] * B[smem desc]: A holds two 16-bit values of a row in a column
-VB_DEVICE void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+VB_DEVICE void warp_umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
                ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
 }
 VB_DEVICE void tma_load_3d(void* dst, const void* tmap, int c0, int c1, int c2, uint64_t* bar) {
@@ -81,15 +81,16 @@ template <int KS, int VS> struct Bars {
 // MMA issuer (one warp).  qk(t, stage) issues S_t, pv(t, stage, first) issues O_t.  n >= 1 key tiles, each for both of two query tiles
 // (`pair`), or the even ones for t = 0 and the odd ones for t = 1.
 template <int KS, int VS, class QK, class PV>
-VB_DEVICE void mma_role(Bars<KS, VS>& b, int n, bool pair, int lane, int& budget, QK qk, PV pv) {
+VB_DEVICE void mma_role(Bars<KS, VS>& b, int n, bool pair, int& budget, QK qk, PV pv) {
   mbar_wait_lim(&b.q_full, 0, budget);
   const int ahead = pair ? 1 : 2;                          // key tiles between a product Q K of a warpgroup and its next
   for (int j = 0; j < min(ahead, n); ++j) {
     mbar_wait_lim(&b.k_full[j % KS], 0, budget);           // (ahead <= KS)
     tc_fence_after();
-    if (lane == 0) {
-      for (int t = pair ? 0 : j; t < (pair ? 2 : j + 1); ++t) { qk(t, j % KS); umma_commit(&b.s_full[t]); }
-      umma_commit(&b.k_empty[j % KS]);
+    __syncwarp();
+    {
+      for (int t = pair ? 0 : j; t < (pair ? 2 : j + 1); ++t) { qk(t, j % KS); warp_umma_commit(&b.s_full[t]); }
+      warp_umma_commit(&b.k_empty[j % KS]);
     }
     __syncwarp();
   }
@@ -101,18 +102,20 @@ VB_DEVICE void mma_role(Bars<KS, VS>& b, int n, bool pair, int lane, int& budget
     for (int t = t0; t <= t1; ++t) {
       mbar_wait_lim(&b.p_full[t], phase, budget);
       tc_fence_after();
-      if (lane == 0) {
+      __syncwarp();
+      {
         pv(t, vs, pair ? j == 0 : j < 2);
-        if (t == t1) umma_commit(&b.v_empty[vs]);
-        if (nx >= n) umma_commit(&b.o_done[t]);
+        if (t == t1) warp_umma_commit(&b.v_empty[vs]);
+        if (nx >= n) warp_umma_commit(&b.o_done[t]);
       }
       __syncwarp();
       if (nx < n) {
         if (t == t0) { mbar_wait_lim(&b.k_full[ks], (nx / KS) & 1, budget); tc_fence_after(); }
-        if (lane == 0) {
+        __syncwarp();
+        {
           qk(t, ks);
-          umma_commit(&b.s_full[t]);
-          if (t == t1) umma_commit(&b.k_empty[ks]);
+          warp_umma_commit(&b.s_full[t]);
+          if (t == t1) warp_umma_commit(&b.k_empty[ks]);
         }
         __syncwarp();
       }
@@ -297,10 +300,10 @@ VB_DEVICE void load_o(uint32_t t_o, int c, bool shared, float f0, float f1, uint
 // O_t += P_t V: db(kk) is the descriptor of 16 keys of the values
 template <class DB> VB_DEVICE void issue_pv(uint32_t tmem_o, uint32_t tmem_p, uint32_t idesc, bool first, bool split, DB db) {
 #pragma unroll
-  for (int kk = 0; kk < KEYS / 16; ++kk) umma_f16_ta(tmem_o, tmem_p + kk * 8, db(kk), idesc, !first || kk != 0);
+  for (int kk = 0; kk < KEYS / 16; ++kk) warp_umma_f16_ta(tmem_o, tmem_p + kk * 8, db(kk), idesc, !first || kk != 0);
   if (split) {
 #pragma unroll
-    for (int kk = 0; kk < KEYS / 16; ++kk) umma_f16_ta(tmem_o, tmem_p + KEYS / 2 + kk * 8, db(kk), idesc, 1);
+    for (int kk = 0; kk < KEYS / 16; ++kk) warp_umma_f16_ta(tmem_o, tmem_p + KEYS / 2 + kk * 8, db(kk), idesc, 1);
   }
 }
 

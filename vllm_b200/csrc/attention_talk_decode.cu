@@ -155,15 +155,16 @@ talk_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
           const int s = n % SLOTS;
           mbar_wait_lim(&full[s], (n / SLOTS) & 1, budget);
           tc_fence_after();
-          if (lane == 0) {
+          __syncwarp();
+          {
 #pragma unroll
             for (int kb = 0; kb < 2; ++kb)
 #pragma unroll
               for (int k = 0; k < 4; ++k)
-                umma_f16(tmem_base + ((j & 1) * G + a) * NQ, d_r + (uint64_t)(((s * TILE_BYTES + kb * TILE * 128) >> 4) + k * 2),
+                warp_umma_f16(tmem_base + ((j & 1) * G + a) * NQ, d_r + (uint64_t)(((s * TILE_BYTES + kb * TILE * 128) >> 4) + k * 2),
                          d_q + (uint64_t)(((a * Q_BYTES + kb * NQ * 128) >> 4) + k * 2), idesc_s, (kb | k) != 0);
-            umma_commit(&empty[s]);
-            if (a == G - 1) umma_commit(&s_full[j & 1]);
+            warp_umma_commit(&empty[s]);
+            if (a == G - 1) warp_umma_commit(&s_full[j & 1]);
           }
           __syncwarp();
         }
@@ -175,15 +176,16 @@ talk_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
           const int s = n % SLOTS;
           mbar_wait_lim(&full[s], (n / SLOTS) & 1, budget);
           tc_fence_after();
-          if (lane == 0) {
+          __syncwarp();
+          {
 #pragma unroll
             for (int kb = 0; kb < 2; ++kb)
 #pragma unroll
               for (int k = 0; k < 4; ++k)
-                umma_f16(tmem_o + c * HP, d_r + (uint64_t)(((s * TILE_BYTES + kb * D * 128) >> 4) + k * 2),
+                warp_umma_f16(tmem_o + c * HP, d_r + (uint64_t)(((s * TILE_BYTES + kb * D * 128) >> 4) + k * 2),
                          d_p + (uint64_t)(((pb * P_BYTES + kb * HP * 128) >> 4) + k * 2), idesc_o, (jj | kb | k) != 0);
-            umma_commit(&empty[s]);
-            if (c == G - 1) umma_commit(&pv_done[pb]);
+            warp_umma_commit(&empty[s]);
+            if (c == G - 1) warp_umma_commit(&pv_done[pb]);
           }
           __syncwarp();
         }

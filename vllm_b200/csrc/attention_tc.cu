@@ -204,14 +204,14 @@ fmha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
     const uint32_t idesc = umma_idesc_f16(TILE_M, TILE_N, DTypeOf<T>::v == DT_BF16);
     const uint64_t d_q = umma_desc_sw128(q_smem), d_k = umma_desc_sw128(k_smem), d_v = umma_desc_sw128(v_smem);
     prompt::mma_role(
-        bars, n_tiles, tiles == 2, lane, budget,
+        bars, n_tiles, tiles == 2, budget,
         [&](int t, int s) {
           const int qt = tiles == 2 ? t : 0;
 #pragma unroll
           for (int kb = 0; kb < 2; ++kb)
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-              umma_f16(tmem_base + t * 128, d_q + (uint64_t)((qt * Q_BYTES + kb * BLK + k * 32) >> 4),
+              warp_umma_f16(tmem_base + t * 128, d_q + (uint64_t)((qt * Q_BYTES + kb * BLK + k * 32) >> 4),
                        d_k + (uint64_t)((s * K_BYTES + kb * BLK + k * 32) >> 4), idesc, (kb | k) != 0);
         },
         [&](int t, int s, bool first) {

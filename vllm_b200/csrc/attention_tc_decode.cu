@@ -193,7 +193,8 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
           mbar_wait(&k_full[s], (g / STAGES) & 1);
           mbar_wait(&s_empty[sb], ((g >> 1) & 1) ^ 1);
           tc_fence_after();
-          if (lane == 0) {
+          __syncwarp();
+          {
             const unsigned char* ks = k_smem + s * K_BYTES;
 #pragma unroll
             for (int kb = 0; kb < 2; ++kb) {
@@ -201,10 +202,10 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
               const uint64_t db = umma_desc_sw128(qs + kb * (NQ * 128));
 #pragma unroll
               for (int k = 0; k < 4; ++k)
-                umma_f16(tmem_base + sb * NQ, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) != 0);
+                warp_umma_f16(tmem_base + sb * NQ, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) != 0);
             }
-            umma_commit(&s_full[sb]);
-            if (j == n_tiles - 1) umma_commit(&q_empty[qb]);      // every QK of this item has read Q
+            warp_umma_commit(&s_full[sb]);
+            if (j == n_tiles - 1) warp_umma_commit(&q_empty[qb]);      // every QK of this item has read Q
           }
           __syncwarp();
         }
@@ -213,7 +214,8 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
           mbar_wait(&v_full[s], (g / STAGES) & 1);
           mbar_wait(p_full, g & 1);
           tc_fence_after();
-          if (lane == 0) {
+          __syncwarp();
+          {
             const unsigned char* vs = v_smem + s * V_BYTES;
 #pragma unroll
             for (int kb = 0; kb < 2; ++kb) {
@@ -221,14 +223,14 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
               const uint64_t db = umma_desc_sw128(p_smem + kb * (NQ * 128));
 #pragma unroll
               for (int k = 0; k < 4; ++k)
-                umma_f16(tmem_o, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (jj | kb | k) != 0);
+                warp_umma_f16(tmem_o, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (jj | kb | k) != 0);
               if (CAP) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) umma_f16(tmem_o, da + (uint64_t)(k * 2), db + (uint64_t)(P_BYTES / 16 + k * 2), idesc, 1);
+                for (int k = 0; k < 4; ++k) warp_umma_f16(tmem_o, da + (uint64_t)(k * 2), db + (uint64_t)(P_BYTES / 16 + k * 2), idesc, 1);
               }
             }
-            umma_commit(&kv_empty[s]);
-            umma_commit(pv_done);
+            warp_umma_commit(&kv_empty[s]);
+            warp_umma_commit(pv_done);
           }
           __syncwarp();
         }

@@ -211,6 +211,23 @@ VB_DEVICE void umma_f8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32
 VB_DEVICE void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// The same for a whole converged warp with the same arguments in every lane; one lane, always the same, issues.  The operands stay in uniform
+// registers: behind a test of the lane an MMA took 115 cycles to issue, 60 to 75 so.  us before and after: decode GEMM 16 x 10752 x 2048 20.5
+// and 16.4, 16 x 6144 x 4096 22.5 and 18.5; fp8 blocks 1000 x 28672 x 4096 with 128 x 128 tiles 248 and 199.
+VB_DEVICE void warp_umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+               ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+VB_DEVICE void warp_umma_f8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+               "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
+               ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+VB_DEVICE void warp_umma_commit(uint64_t* bar) {
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+               "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)) : "memory");
+}
 // 32 lanes x 32 consecutive fp32 columns → 32 registers per thread (warp w reads lanes 32*(w%4)..+31)
 VB_DEVICE void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(

@@ -143,15 +143,16 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       }
       mbar_wait(&full[s], (kb / STAGES) & 1);
       tc_fence_after();
-      if (lane == 0) {
+      __syncwarp();
+      {
         const unsigned char* a_src = stage_base + s * L::STAGE_BYTES;
         const uint64_t da = umma_desc_sw128(a_src), db = umma_desc_sw128(a_src + L::A_BYTES);
         const uint32_t d = tmem_base + (uint32_t)(buf * BN);
 #pragma unroll
         for (int k = 0; k < BK / 32; ++k)     // UMMA_K = 32 fp8 = 32 B inside the swizzle span
-          umma_f8(d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, BLOCK ? (uint32_t)(k != 0) : (uint32_t)((kb | k) != 0));
-        umma_commit(&empty[s]);
-        if (BLOCK || kb == nkb - 1) umma_commit(&acc_full[buf]);
+          warp_umma_f8(d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, BLOCK ? (uint32_t)(k != 0) : (uint32_t)((kb | k) != 0));
+        warp_umma_commit(&empty[s]);
+        if (BLOCK || kb == nkb - 1) warp_umma_commit(&acc_full[buf]);
       }
       __syncwarp();
     }

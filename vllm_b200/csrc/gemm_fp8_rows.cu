@@ -7,8 +7,8 @@
 // and its first two blocks run beside a tile's stores.  Tiles are taken down M in bands of BAND row tiles, so that a wave's operands stay in L2.
 // Bound by the promotion's way out of tensor memory: 0.55 to 0.6 us per 128-deep block on a CTA alone as on all, the products take 0.27; with 32
 // columns fetched at a time 0.65, whether or not the next were on their way, scales staged ahead made no difference.
-// Measured against the tile kernel: 1000 x 28672 x 4096 248 → 136 us, 1000 x 4096 x 14336 130 → 73, 2000 x 6144 x 4096 118 → 66, 8192 x 4096 x
-// 14336 898 → 458 (2.1 PFLOP/s).
+// Measured against the tile kernel: 1000 x 28672 x 4096 199 → 139 us, 1000 x 4096 x 14336 109 → 70, 512 x 6144 x 4096 40 → 28, 8192 x 4096 x
+// 14336 915 → 457 (2.1 PFLOP/s).
 // Warps: 0 TMA producer, 1 MMA issuer, 4..7 and 8..11 promotion and stores of columns 0..127 and 128..255 (thread = token).
 #include "attention_prompt.cuh"
 
@@ -97,12 +97,13 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
           mbar_wait_lim(&acc_empty[buf], ((it >> 1) & 1) ^ 1, budget);
           mbar_wait_lim(&full[s], (it / STAGES) & 1, budget);
           tc_fence_after();
-          if (lane == 0) {
+          __syncwarp();
+          {
             const uint64_t da = d0 + (uint64_t)((s * STAGE) >> 4), db = da + (uint64_t)(A_BYTES >> 4);
 #pragma unroll
-            for (int k = 0; k < BK / 32; ++k) umma_f8(tmem_base + buf * TN, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, k != 0);
-            umma_commit(&empty[s]);
-            umma_commit(&acc_full[buf]);
+            for (int k = 0; k < BK / 32; ++k) warp_umma_f8(tmem_base + buf * TN, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, k != 0);
+            warp_umma_commit(&empty[s]);
+            warp_umma_commit(&acc_full[buf]);
           }
           __syncwarp();
         }

@@ -119,12 +119,13 @@ grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         const int s = it % STAGES;
         mbar_wait_lim(&full[s], (it / STAGES) & 1, budget);
         tc_fence_after();
-        if (lane == 0) {
+        __syncwarp();
+        {
           const uint64_t da = d0 + (uint64_t)((s * STAGE) >> 4), db = da + (uint64_t)(A_BYTES >> 4);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) umma_f16(tmem_base + buf * TN, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) != 0);
-          umma_commit(&empty[s]);
-          if (kb == nkb - 1) umma_commit(&acc_full[buf]);
+          for (int k = 0; k < BK / 16; ++k) warp_umma_f16(tmem_base + buf * TN, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) != 0);
+          warp_umma_commit(&empty[s]);
+          if (kb == nkb - 1) warp_umma_commit(&acc_full[buf]);
         }
         __syncwarp();
       }

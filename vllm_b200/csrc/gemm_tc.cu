@@ -188,15 +188,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const int s = kb % STAGES;
       mbar_wait(&full[s], (kb / STAGES) & 1);
       tc_fence_after();
-      if (lane == 0) {
-        if (kb == 0) VB_TRACE(3);
+      __syncwarp();
+      {
+        if (kb == 0 && lane == 0) VB_TRACE(3);
         const unsigned char* a_src = stage_base + s * L::STAGE_BYTES;
         const uint64_t da = umma_desc_sw128(a_src), db = umma_desc_sw128(a_src + L::A_BYTES);
 #pragma unroll
         for (int k = 0; k < BK / 16; ++k)   // UMMA_K = 16 → advance 32 B inside the swizzle span
-          umma_f16(tmem_base, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) != 0);
-        umma_commit(&empty[s]);                 // frees the smem slot once these MMAs retire
-        if (kb == nkb - 1) { umma_commit(tmem_full); VB_TRACE(4); }
+          warp_umma_f16(tmem_base, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) != 0);
+        warp_umma_commit(&empty[s]);                 // frees the smem slot once these MMAs retire
+        if (kb == nkb - 1) { warp_umma_commit(tmem_full); if (lane == 0) VB_TRACE(4); }
       }
       __syncwarp();
     }

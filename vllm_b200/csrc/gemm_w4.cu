@@ -158,15 +158,16 @@ gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_b, const Params p) {
       mbar_wait(&full_p[s], (kb / PSTAGES) & 1);             // activation tile (async proxy) landed
       mbar_wait(&conv_full[c], (kb / CSTAGES) & 1);          // converted weights written + fenced
       tc_fence_after();
-      if (lane == 0) {
-        if (p.trace && blockIdx.x == 0 && kb < 256) p.trace[kb * 8 + 5] = clock64();
+      __syncwarp();
+      {
+        if (lane == 0 && p.trace && blockIdx.x == 0 && kb < 256) p.trace[kb * 8 + 5] = clock64();
         const uint64_t da = umma_desc_sw128(conv + c * CONV_BYTES), db = umma_desc_sw128(bsm + s * B_BYTES);
 #pragma unroll
         for (int k = 0; k < BK / 16; ++k)
-          umma_f16(tmem_base, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) != 0);
-        umma_commit(&conv_empty[c]);
-        umma_commit(&empty_p[s]);
-        if (kb == nkb - 1) umma_commit(tmem_full);
+          warp_umma_f16(tmem_base, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) != 0);
+        warp_umma_commit(&conv_empty[c]);
+        warp_umma_commit(&empty_p[s]);
+        if (kb == nkb - 1) warp_umma_commit(tmem_full);
       }
       __syncwarp();
     }

@@ -248,18 +248,19 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_cons
           const int slot = st * NKB + kb;
           mbar_wait_lim(&kv_full[slot], par, budget);
           tc_fence_after();
-          if (lane == 0) {
+          __syncwarp();
+          {
             const uint64_t da = d_kv + (uint64_t)((st * STAGE_BYTES + kb * KB_BYTES) >> 4);
             const uint64_t db = d_q + (uint64_t)((kb * (N * 128)) >> 4);
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-              umma_f16(tmem_base + sb * N, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc_s, (i | k) != 0);
+              warp_umma_f16(tmem_base + sb * N, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc_s, (i | k) != 0);
           }
           __syncwarp();
         }
-        if (lane == 0) {
-          umma_commit(&s_full[sb]);
-          if (ROPE) umma_commit(&kv_empty[st * NKB + NKB - 1]);   // the rope block is only read by QK
+        {
+          warp_umma_commit(&s_full[sb]);
+          if (ROPE) warp_umma_commit(&kv_empty[st * NKB + NKB - 1]);   // the rope block is only read by QK
         }
         __syncwarp();
       }
@@ -269,7 +270,8 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_cons
         const int jj = j - 1, st = jj % STAGES;
         mbar_wait_lim(p_full, jj & 1, budget);
         tc_fence_after();
-        if (lane == 0) {
+        __syncwarp();
+        {
 #pragma unroll
           for (int c = 0; c < NC; ++c) {
 #pragma unroll 1
@@ -277,13 +279,13 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_cons
 #pragma unroll
               for (int kk = 0; kk < TILE / 16; ++kk) {
                 const uint64_t da = d_kv_mn + (uint64_t)((st * STAGE_BYTES + (2 * c) * KB_BYTES + kk * 2048) >> 4);
-                umma_f16(tmem_o + c * N, da, d_p + (uint64_t)(low * (P_LOW / 16) + kk * 2), idesc_o, (jj | kk | low) != 0);
+                warp_umma_f16(tmem_o + c * N, da, d_p + (uint64_t)(low * (P_LOW / 16) + kk * 2), idesc_o, (jj | kk | low) != 0);
               }
             }
-            umma_commit(&kv_empty[st * NKB + 2 * c]);
-            if (2 * c + 1 < NL) umma_commit(&kv_empty[st * NKB + 2 * c + 1]);
+            warp_umma_commit(&kv_empty[st * NKB + 2 * c]);
+            if (2 * c + 1 < NL) warp_umma_commit(&kv_empty[st * NKB + 2 * c + 1]);
           }
-          umma_commit(pv_done);
+          warp_umma_commit(pv_done);
         }
         __syncwarp();
       }

@@ -138,14 +138,14 @@ mla_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       const uint64_t d_q = umma_desc_sw128(q_smem), d_k = umma_desc_sw128(k_smem), d_v = desc_mn(v_smem);
       const bool split = p.split != 0;
       prompt::mma_role(
-          bars, n_tiles, tiles == 2, lane, budget,
+          bars, n_tiles, tiles == 2, budget,
           [&](int t, int s) {
             const int qt = tiles == 2 ? t : 0;
 #pragma unroll
             for (int kb = 0; kb < NQ; ++kb)
 #pragma unroll
               for (int k = 0; k < 4; ++k)
-                umma_f16(tmem_base + t * 128, d_q + (uint64_t)(((qt * NQ + kb) * BLK + k * 32) >> 4),
+                warp_umma_f16(tmem_base + t * 128, d_q + (uint64_t)(((qt * NQ + kb) * BLK + k * 32) >> 4),
                          d_k + (uint64_t)(((s * NQ + kb) * BLK + k * 32) >> 4), idesc_s, (kb | k) != 0);
           },
           [&](int t, int s, bool first) {                   // 16 keys per MMA: 16 rows of 128 bytes of V

@@ -1314,8 +1314,8 @@ def _fp8_plan(M: int, N: int, K: int) -> tuple:
 
 def fp8_rows(M: int, N: int, K: int) -> bool:
     """Do prompts take the 128 x 256 tiles?  They do one in up to 7 / 6 of the time of a 128 x 128 tile, so where that saves waves:
-    us, 512 x 6144 x 4096 (two waves against one) 44 → 28, 1000 x 4096 x 4096 45 → 27; one wave either way: 512 x 4096 x 14336 63.5 with the
-    smaller, 64 with the larger tiles, 1000 x 2112 x 7168 38 and 40."""
+    us, 512 x 6144 x 4096 (two waves against one) 40 → 28, 1000 x 4096 x 4096 41 → 27; one wave either way: 512 x 4096 x 14336 66 with the
+    smaller, 68 with the larger tiles, 1000 x 1536 x 7168 38 and 40."""
     if M <= 128 or K % 128 or N % 8:
         return False
     m, sms = -(-M // 128), num_sms()
