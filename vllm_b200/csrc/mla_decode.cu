@@ -24,8 +24,13 @@
 // never looks at, and cost nothing that matters — at 16-32 heads per CTA the kernel is bound by the latent stream
 // (1152 B per token), not by tensor-core time.
 //
+// Bound at these sizes by latency: about 14 us of set-up, first copies, last product and stores, and 3 us per tile of a split, two thirds of it the 36
+// products of Q K (90 cycles each, whatever their order or accumulator; a wait and a fence per k-block beside them), the rest the softmax.  24
+// requests of 600 tokens in 6 splits 42 → 28 us and 1200 tokens 44 → 34 since the sums' reductions, the rescaling rule and the stores are branch-free, with
+// their addresses formed once, and shared memory is cleared only where pages smaller than a tile need it.
+//
 // wide: the rows of short portions in steps that are not decode steps alone, whose weights were held in 32 bits on the CUDA cores: the second product
-// of the weights' low parts costs 1 to 3 us of 40; the rows of a step of 24 requests took 660 us there.
+// of the weights' low parts costs 1 to 3 us; the rows of a step of 24 requests took 660 us there.
 //
 // Reference kernels for the op: csrc/libtorch_stable/attention/mla/sm100_cutlass_mla_kernel.cu (+ cutlass_sm100_mla/),
 // FlashMLA; algorithm: vllm/model_executor/layers/attention/mla_attention.py:1-200 (absorbed-weight decode).
@@ -92,6 +97,12 @@ VB_HOST_DEVICE uint32_t idesc_f16_a_mn(int M, int N, bool bf16) {
   return umma_idesc_f16(M, N, bf16) | (1u << 15);     // bit 15: A operand is MN-major
 }
 
+VB_DEVICE float warp_max_f32(float x) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // FULL: the latent fills its blocks (R = 64 NL is a compile-time constant)
 template <typename T, int N, int NL, int ROPE, bool FULL>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
@@ -109,7 +120,8 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_cons
   unsigned char* kv_smem = smem;                                // STAGES tiles
   unsigned char* q_smem = kv_smem + STAGES * STAGE_BYTES;       // (also what QK's padding rows of the last k-block read)
   unsigned char* p_smem = q_smem + Q_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(p_smem + (P_BYTES < 8192 ? 8192 : P_BYTES));
+  float* wred = reinterpret_cast<float*>(p_smem + 8192);        // [2][N], of the warps that have tokens
+  uint64_t* bars = reinterpret_cast<uint64_t*>(wred + 4 * N);
   uint64_t* q_full = bars;
   uint64_t* kv_full = bars + 1;              // [STAGES * NKB] one per k-block buffer
   uint64_t* kv_empty = kv_full + STAGES * NKB;
@@ -118,8 +130,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_cons
   uint64_t* p_full = s_empty + 2;
   uint64_t* pv_done = p_full + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 1);
-  float* wred = reinterpret_cast<float*>(tmem_slot + 2);        // [4][N]
-  int* blk_ids = reinterpret_cast<int*>(wred + 4 * N);          // [MAX_IDS_SMEM]
+  int* blk_ids = reinterpret_cast<int*>(tmem_slot + 2);         // [MAX_IDS_SMEM]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int budget = MBAR_BUDGET;                  // failed polls left (mbar_wait_lim)
@@ -155,11 +166,11 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_cons
   }
   if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
   {
-    // padded Q / P rows and the not-yet-loaded part of the last tile must be finite: zero everything once
+    // padded Q and P rows must be finite, and the part of the last tile that pages smaller than a tile leave out: zeros once
     uint4 z = make_uint4(0, 0, 0, 0);
     uint4* s4 = reinterpret_cast<uint4*>(smem);
-    const int n16 = (STAGES * STAGE_BYTES + Q_BYTES + (P_BYTES < 8192 ? 8192 : P_BYTES)) / 16;
-    for (int i = threadIdx.x; i < n16; i += NUM_THREADS) s4[i] = z;
+    const int n16 = (STAGES * STAGE_BYTES + Q_BYTES + 8192) / 16;
+    for (int i = (ppt > 1 ? 0 : STAGES * STAGE_BYTES / 16) + threadIdx.x; i < n16; i += NUM_THREADS) s4[i] = z;
   }
   // token row (in the [num_blocks * BS, row] view of the cache) of every TMA box of this split, -1 = past the sequence
   auto box_row = [&](int i) -> int {
@@ -245,10 +256,13 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_cons
 #pragma unroll
         for (int i = 0; i < NKB; ++i) {
           const int kb = ROPE ? (i == 0 ? NKB - 1 : i - 1) : i;
-          const int slot = st * NKB + kb;
-          mbar_wait_lim(&kv_full[slot], par, budget);
-          tc_fence_after();
-          __syncwarp();
+          if (i % 3 == 0) {                  // three blocks at a time: a wait and its fence take as long as a block's products
+#pragma unroll
+            for (int u = i; u < (i + 3 < NKB ? i + 3 : NKB); ++u)
+              mbar_wait_lim(&kv_full[st * NKB + (ROPE ? (u == 0 ? NKB - 1 : u - 1) : u)], par, budget);
+            tc_fence_after();
+            __syncwarp();
+          }
           {
             const uint64_t da = d_kv + (uint64_t)((st * STAGE_BYTES + kb * KB_BYTES) >> 4);
             const uint64_t db = d_q + (uint64_t)((kb * (N * 128)) >> 4);
@@ -315,22 +329,28 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_cons
       mbar_arrive(&s_empty[sb]);
       const int kpos = (tile_lo + j) * TILE + t;
       const bool ok = t < TILE && kpos < seq_len && kpos >= kv_begin;        // TMEM lanes 64..127 are the QK padding rows
+      if (qd < 2) {
 #pragma unroll
-      for (int g = 0; g < N; ++g) {
-        s[g] = ok ? s[g] * p.scale_log2 : -INFINITY;
-        const float cm = warp_max(s[g]);
-        if (lane == 0) wred[qd * N + g] = cm;
+        for (int g = 0; g < N; ++g) {
+          s[g] = ok ? s[g] * p.scale_log2 : -INFINITY;
+          const float cm = warp_max_f32(s[g]);
+          if (lane == 0) wred[qd * N + g] = cm;
+        }
       }
       bar_sync_softmax();
       float alpha[N];
       bool rescale = false;
 #pragma unroll
-      for (int g = 0; g < N; ++g) {
-        const float mx = fmaxf(fmaxf(wred[g], wred[N + g]), fmaxf(wred[2 * N + g], wred[3 * N + g]));
-        alpha[g] = 1.f;
-        if (mx > m_used[g] + 8.f || (m_used[g] == -INFINITY && mx > -INFINITY)) {
-          if (m_used[g] != -INFINITY) { alpha[g] = ex2(m_used[g] - mx); rescale = true; }
-          m_used[g] = mx;
+      for (int g = 0; g < N; g += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(wred + g), c = *reinterpret_cast<const float4*>(wred + N + g);
+        const float mx[4] = {fmaxf(a.x, c.x), fmaxf(a.y, c.y), fmaxf(a.z, c.z), fmaxf(a.w, c.w)};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float was = m_used[g + e];
+          const bool up = mx[e] > was + 8.f, had = was != -INFINITY;       // (of the first key: had is false)
+          alpha[g + e] = up && had ? ex2(was - mx[e]) : 1.f;
+          rescale |= up && had;
+          m_used[g + e] = up ? mx[e] : was;
         }
       }
       if (j > 0) { mbar_wait_lim(pv_done, (j - 1) & 1, budget); tc_fence_after(); }   // P and O^T are free again
@@ -351,17 +371,21 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_cons
 #pragma unroll
         for (int g = 0; g < N; ++g) l_thr[g] *= alpha[g];
       }
-      unsigned char* pcol = p_smem + ((t & 63) & 7) * 2;
-      const int chunk = (t & 63) >> 3;
+      if (qd < 2) {
+        unsigned char* pcol = p_smem + (t & 7) * 2;
+        const int chunk = t >> 3;
 #pragma unroll
-      for (int g = 0; g < N; ++g) {
-        const float m_ref = (m_used[g] == -INFINITY) ? 0.f : m_used[g];
-        const float pe = ok ? ex2(s[g] - m_ref) : 0.f;
-        l_thr[g] += pe;
-        if (t < TILE) {
+        for (int g = 0; g < N; ++g) {
+          const float m_ref = (m_used[g] == -INFINITY) ? 0.f : m_used[g];
+          const float pe = ok ? ex2(s[g] - m_ref) : 0.f;
+          l_thr[g] += pe;
           const T hi = from_f32<T>(pe);
           *reinterpret_cast<T*>(pcol + g * 128 + ((chunk ^ (g & 7)) << 4)) = hi;
-          if (p.wide) *reinterpret_cast<T*>(pcol + P_LOW + g * 128 + ((chunk ^ (g & 7)) << 4)) = from_f32<T>(pe - to_f32(hi));
+          s[g] = pe - to_f32(hi);
+        }
+        if (p.wide) {
+#pragma unroll
+          for (int g = 0; g < N; ++g) *reinterpret_cast<T*>(pcol + P_LOW + g * 128 + ((chunk ^ (g & 7)) << 4)) = from_f32<T>(s[g]);
         }
       }
       tc_fence_before();
@@ -370,57 +394,54 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_cons
       bar_sync_softmax();                         // wred is reused by the next tile
     }
     // ---- epilogue
+    if (qd < 2) {
 #pragma unroll
-    for (int g = 0; g < N; ++g) {
-      const float lt = warp_sum(l_thr[g]);
-      if (lane == 0) wred[qd * N + g] = lt;
+      for (int g = 0; g < N; ++g) {
+        const float lt = warp_sum(l_thr[g]);
+        if (lane == 0) wred[qd * N + g] = lt;
+      }
     }
     bar_sync_softmax();
     mbar_wait_lim(pv_done, (n_tiles - 1) & 1, budget);
     tc_fence_after();
-    float inv[N], lsum[N];
+    float inv[N], my_l = 0.f, my_m = 0.f;                      // of head t: one thread each writes the sums' logarithms
 #pragma unroll
     for (int g = 0; g < N; ++g) {
-      lsum[g] = wred[g] + wred[N + g] + wred[2 * N + g] + wred[3 * N + g];
-      inv[g] = lsum[g] > 0.f ? 1.f / lsum[g] : 0.f;
+      const float l = wred[g] + wred[N + g];
+      inv[g] = l > 0.f ? 1.f / l : 0.f;
+      if (t == g) { my_l = l; my_m = m_used[g]; }
     }
+    const bool whole = p.num_splits == 1;
+    T* out = reinterpret_cast<T*>(p.out) + (int64_t)b * p.out_stride + (int64_t)h0 * R + t;
+    const int64_t first = ((int64_t)b * p.H + h0) * p.num_splits + split, step = (int64_t)p.num_splits * R;     // parts of a head lie together
+    float* part = whole ? nullptr : p.part_out + first * R + t;
 #pragma unroll
     for (int c4 = 0; c4 < NC; ++c4) {
-      const int d = c4 * 128 + t;
-      const bool d_ok = d < R;
+      const bool d_ok = c4 * 128 + t < R;
 #pragma unroll
       for (int c = 0; c < N; c += CH) {
         uint32_t ov[CH];
         tmem_ld_32x16(tmem_o + c4 * N + c + t_lane, ov);
         tmem_ld_wait();
 #pragma unroll
-        for (int g = 0; g < CH; ++g) {
-          if (c + g < G && d_ok) {
-            const float o = __uint_as_float(ov[g]) * inv[c + g];
-            const int hq = h0 + c + g;
-            if (p.num_splits == 1) {
-              reinterpret_cast<T*>(p.out)[(int64_t)b * p.out_stride + (int64_t)hq * R + d] = from_f32<T>(o);
-            } else {
-              const int64_t pi = ((int64_t)b * p.H + hq) * p.num_splits + split;
-              p.part_out[pi * R + d] = o;
-            }
-          }
+        for (int g = 0; g < CH; ++g) ov[g] = __float_as_uint(__uint_as_float(ov[g]) * inv[c + g]);
+        if (d_ok && whole) {
+#pragma unroll
+          for (int g = 0; g < CH; ++g)
+            if (c + g < G) out[(c + g) * R + c4 * 128] = from_f32<T>(__uint_as_float(ov[g]));
+        } else if (d_ok) {
+          float* to = part + c * step + c4 * 128;
+#pragma unroll
+          for (int g = 0; g < CH; ++g, to += step)
+            if (c + g < G) *to = __uint_as_float(ov[g]);
         }
+        __syncwarp();
       }
     }
-    if (t == 0) {
-#pragma unroll
-      for (int g = 0; g < N; ++g) {
-        if (g < G) {
-          const int hq = h0 + g;
-          const float lse2 = lsum[g] > 0.f ? m_used[g] + log2f(lsum[g]) : -INFINITY;
-          if (p.num_splits == 1) {
-            if (p.lse_out) p.lse_out[(int64_t)b * p.H + hq] = lse2 * 0.6931471805599453f;
-          } else {
-            p.part_lse[((int64_t)b * p.H + hq) * p.num_splits + split] = lse2;
-          }
-        }
-      }
+    if (t < G) {
+      const float lse2 = my_l > 0.f ? my_m + log2f(my_l) : -INFINITY;
+      if (!whole) p.part_lse[first + (int64_t)t * p.num_splits] = lse2;
+      else if (p.lse_out) p.lse_out[(int64_t)b * p.H + h0 + t] = lse2 * 0.6931471805599453f;
     }
     tc_fence_before();
   }
