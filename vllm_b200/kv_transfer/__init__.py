@@ -151,6 +151,10 @@ class FileBlockStore(BlockStore):
             return False
 
 
+def _capped(cfg) -> bool:
+    return isinstance(cfg, dict) and (bool(cfg.get("attn_logit_softcapping")) or any(_capped(v) for v in cfg.values()))
+
+
 class BlockConnector(KVConnectorBase):
     """Block-granular connector over a ``BlockStore``; keys are the prefix-cache block hashes, so any engine with
     the same model / block size / hash seed can reuse what another one stored."""
@@ -178,6 +182,8 @@ class BlockConnector(KVConnectorBase):
                  "tp": getattr(pc, "tensor_parallel_size", 1), "pp": getattr(pc, "pipeline_parallel_size", 1),
                  "dcp": getattr(pc, "decode_context_parallel_size", 1),
                  "hf": getattr(mc, "hf_config", None)}
+        if self.block_size == 64 and _capped(ident["hf"]):
+            ident["values"] = "transposed"     # pages of capped models held values token by token before the tensor-core kernels took them
         self._ns = hashlib.sha256(json.dumps(ident, sort_keys=True, default=str).encode()).hexdigest()[:12]
         self._tp, self._pp = ident["tp"] or 1, ident["pp"] or 1
         self._shard: Optional[str] = None      # resolved lazily on the worker (parallel groups exist by then)
