@@ -406,7 +406,7 @@ def paged_attention(q, kv_cache, md, scale, sliding_window=None, logits_soft_cap
             return (out, lse) if return_lse else out
         rc = _fmha_tc(q.data_ptr(), kv_cache.data_ptr(), kv_cache.shape[0], bt.data_ptr(), md.seq_lens.data_ptr(),
                       None if decode else md.query_start_loc.data_ptr(), out.data_ptr(),
-                      _p(ws.part_out) if ws else None, _p(ws.part_lse) if ws else None, _p(lse), kernel_error_flag(q.device).data_ptr(),
+                      _p(ws.part_out) if ws else None, _p(ws.part_lse) if ws else None, _p(lse), _error_flag(q.device),
                       md.num_reqs, T, md.max_query_len, Hq, Hkv, q.stride(0), out.stride(0), bt.stride(0), splits,
                       sliding_window or 0, scale, logits_soft_cap, int(causal), int(md.flat and not decode), chunk_size, _p(sinks), out_scale,
                       _DT[q.dtype], _st())
@@ -552,6 +552,13 @@ def kernel_error_flag(device: torch.device) -> torch.Tensor:
             raise RuntimeError("the kernel error flag must be allocated before CUDA-graph capture")
         t = _kernel_error[key] = torch.zeros(1, dtype=torch.int32, device=device)
     return t
+
+
+def _error_flag(device: torch.device) -> Optional[int]:
+    """Address of the flag, or None (which such kernels take) in a capture that nothing has run before: calls that may be captured so."""
+    if (device.index or 0) not in _kernel_error and torch.cuda.is_current_stream_capturing():
+        return None
+    return kernel_error_flag(device).data_ptr()
 
 
 def check_kernel_error(device: torch.device) -> None:
@@ -1230,7 +1237,7 @@ def gemm_grouped(xs: torch.Tensor, w: torch.Tensor, offs: torch.Tensor, act: Opt
     E, N, _ = w.shape
     assert xs.is_contiguous() and w.is_contiguous() and xs.dtype == w.dtype and w.shape[2] == K
     y = torch.empty((R, N if act is None else N // 2), dtype=xs.dtype, device=xs.device)
-    _check(_gemm_grouped_rows(xs.data_ptr(), w.data_ptr(), y.data_ptr(), offs.data_ptr(), kernel_error_flag(xs.device).data_ptr(), R, N, K, E,
+    _check(_gemm_grouped_rows(xs.data_ptr(), w.data_ptr(), y.data_ptr(), offs.data_ptr(), _error_flag(xs.device), R, N, K, E,
                               _GATED_ACT[act], num_sms(), _DT[xs.dtype], _st()), f"gemm_grouped(R={R},N={N},K={K},E={E})")
     return y
 
@@ -1327,7 +1334,7 @@ def gemm_fp8_rows(xq, xs, wq, ws, bias, y):
     M, K = xq.shape
     N = wq.shape[0]
     _check(_gemm_fp8_rows(xq.data_ptr(), xs.data_ptr(), xs.stride(1), wq.data_ptr(), ws.data_ptr(), _p(bias), y.data_ptr(),
-                          kernel_error_flag(xq.device).data_ptr(), M, N, K, num_sms(), _DT[y.dtype], _st()),
+                          _error_flag(xq.device), M, N, K, num_sms(), _DT[y.dtype], _st()),
            f"gemm_fp8_rows(M={M},N={N},K={K})")
     return y
 
