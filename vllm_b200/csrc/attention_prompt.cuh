@@ -23,7 +23,7 @@
 namespace prompt {
 
 constexpr int ROWS = 128, KEYS = 128;
-constexpr int NUM_THREADS = 384;            // warp 0 TMA producer, 1 MMA issuer (2, 3 idle), 4..7 and 8..11 softmax of the two tiles
+constexpr int NUM_THREADS = 384;            // warp 0 TMA producer, 1 MMA issuer, 2 and 3 clear values, 4..7 and 8..11 softmax of the two tiles
 // registers a thread: launched with 168; 384 x 168 = 128 x 72 + 256 x 216
 constexpr int REGS_AUX = 72, REGS_SOFTMAX = 216;
 template <int N> VB_DEVICE void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
@@ -59,14 +59,14 @@ VB_DEVICE void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
 }
 VB_DEVICE void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// KS stages of keys, VS of values
+// KS stages of keys, VS of values.  edge: values of the first and the last key tile, where they are cleared before the product
 template <int KS, int VS> struct Bars {
-  uint64_t q_full, k_full[KS], k_empty[KS], v_full[VS], v_empty[VS], s_full[2], p_full[2], o_done[2];
+  uint64_t q_full, k_full[KS], k_empty[KS], v_full[VS], v_empty[VS], s_full[2], p_full[2], o_done[2], edge[2];
   VB_DEVICE void init() {
     mbar_init(&q_full, 1);
     for (int s = 0; s < KS; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
     for (int s = 0; s < VS; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
-    for (int t = 0; t < 2; ++t) { mbar_init(&s_full[t], 1); mbar_init(&p_full[t], ROWS); mbar_init(&o_done[t], 1); }
+    for (int t = 0; t < 2; ++t) { mbar_init(&s_full[t], 1); mbar_init(&p_full[t], ROWS); mbar_init(&o_done[t], 1); mbar_init(&edge[t], 1); }
     mbar_fence_init();
   }
   // a producer that gave up: let its copies in flight land before the block gives up its memory
@@ -75,8 +75,35 @@ template <int KS, int VS> struct Bars {
       for (int n = 0; n < 4096 && !(mbar_try_wait(&k_full[s], 0) || mbar_try_wait(&k_full[s], 1)); ++n) {}
     for (int s = 0; s < VS; ++s)
       for (int n = 0; n < 4096 && !(mbar_try_wait(&v_full[s], 0) || mbar_try_wait(&v_full[s], 1)); ++n) {}
+    for (int t = 0; t < 2; ++t)
+      for (int n = 0; n < 4096 && !(mbar_try_wait(&edge[t], 0) || mbar_try_wait(&edge[t], 1)); ++n) {}
   }
 };
+
+// A tile of keys is multiplied whole, and a weight of 0 keeps neither an infinity nor a NaN out of a sum, but slots that no row sees (behind a
+// sequence's end, in front of a window) may hold values of another request.  Where a tile has such slots its values arrive at a barrier of
+// their own, 64 threads that have nothing else to do overwrite the slots with zeros and pass the tile on.  (In the softmax threads
+// the same took 549 → 594 us for 32 / 8 heads, 4 x 3800 tokens, by the registers it needs.)
+// Row r of a block of 64 tokens per 128-byte swizzled row: tokens [lo, hi) stay.
+VB_DEVICE void clear_tokens(unsigned char* block, int r, int lo, int hi) {
+#pragma unroll 1
+  for (int c = 0; c < 8; ++c) {
+    const int a = lo - c * 8, b = hi - c * 8;
+    if (a <= 0 && b >= 8) continue;
+    uint4* p = reinterpret_cast<uint4*>(block + r * 128 + ((c ^ (r & 7)) << 4));
+    if (a >= 8 || b <= 0) {
+      *p = make_uint4(0, 0, 0, 0);
+    } else {
+      for (int i = 0; i < 8; ++i)
+        if (i < a || i >= b) reinterpret_cast<uint16_t*>(p)[i] = 0;
+    }
+  }
+}
+VB_DEVICE void pass_on(uint64_t* v_full) {
+  fence_proxy_async();
+  asm volatile("bar.sync 2, 64;" ::: "memory");
+  if ((threadIdx.x & 63) == 0) mbar_arrive(v_full);
+}
 
 // MMA issuer (one warp).  qk(t, stage) issues S_t, pv(t, stage, first) issues O_t.  n >= 1 key tiles, each for both of two query tiles
 // (`pair`), or the even ones for t = 0 and the odd ones for t = 1.

@@ -9,7 +9,7 @@
 // (page-table driven: the block id of each page becomes the TMA row coordinate), with no transposes.
 //
 // CTA = one (request, kv head) x one or two tiles of 128 query rows (rows = q tokens x GQA group; decode uses G rows) x a KV
-// range (split-KV for decode); warps: 0 TMA producer, 1 MMA issuer + TMEM owner, 4..7 and 8..11 softmax and epilogue of the two tiles
+// range (split-KV for decode); warps: 0 TMA producer, 1 MMA issuer + TMEM owner, 2 and 3 clear values, 4..7 and 8..11 softmax and epilogue of the two tiles
 // (attention_prompt.cuh).
 #include "attention_prompt.cuh"
 
@@ -142,21 +142,16 @@ fmha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
     bars.init();
   }
   if (warp == 1) tmem_alloc(tmem_slot, 512);
-  // a last tile of one page leaves half of the values' stage as it was: it must not hold NaN bit patterns
-  if (n_pages_total < 2 * tile_hi) {
-    const uint4 z = make_uint4(0, 0, 0, 0);
-    uint4* s4 = reinterpret_cast<uint4*>(v_smem);
-    for (int i = threadIdx.x; i < KV_STAGES * V_BYTES / 16; i += NUM_THREADS) s4[i] = z;
-  }
   for (int i = threadIdx.x; i < 2 * n_tiles && i < 2 * MAX_TILES_SMEM; i += NUM_THREADS) {
     const int page = tile_lo * 2 + i;
     blk_ids[i] = page < n_pages_total ? p.block_table[(int64_t)b * p.bt_stride + page] : -1;
   }
-  fence_proxy_async();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // does key tile j (the first or the last) hold slots that are not this sequence's, or that no row sees?
+  auto edge = [&](int j) { return kv_begin > (tile_lo + j) * TILE_N || kv_end < (tile_lo + j + 1) * TILE_N; };
 
   if (warp < 4) {
     prompt::regs_dec<prompt::REGS_AUX>();
@@ -190,12 +185,13 @@ fmha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
         }
         mbar_wait_lim(&bars.v_empty[s], par, budget);
         if (budget < 0) break;
-        mbar_expect_tx(&bars.v_full[s], n_valid * BS * D * 2);
+        uint64_t* v_bar = edge(j) ? &bars.edge[j != 0] : &bars.v_full[s];
+        mbar_expect_tx(v_bar, n_valid * BS * D * 2);
         for (int u = 0; u < 2; ++u) {
           if (blk[u] < 0) continue;
           const int chunk = (blk[u] * 2 + 1) * p.Hkv + h;       // V chunk index
           // V view: [chunks*D rows, BS cols]; page u is k-block u of the PV product: [128 dims x 64 tokens]
-          tma_load_2d(vs + u * BLK, &tmap_v, 0, chunk * D, &bars.v_full[s]);
+          tma_load_2d(vs + u * BLK, &tmap_v, 0, chunk * D, v_bar);
         }
       }
       if (budget < 0) bars.drain();
@@ -218,6 +214,17 @@ fmha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
           prompt::issue_pv(tmem_base + 256 + t * 128, tmem_base + t * 128, idesc, first, CAP,
                            [&](int kk) { return d_v + (uint64_t)((s * V_BYTES + (kk / 4) * BLK + (kk & 3) * 32) >> 4); });
         });
+    } else if (warp >= 2) {
+      // ===== zeros into the values' slots that no row sees
+      for (int e = 0; e < 2; ++e) {
+        const int j = e ? n_tiles - 1 : 0, s = j % KV_STAGES, k0 = (tile_lo + j) * TILE_N;
+        if ((e && n_tiles == 1) || !edge(j)) continue;
+        mbar_wait_lim(&bars.edge[e], 0, budget);
+        for (int i = 0; i < 4; ++i)                // two pages, two rows of 64 threads each
+          prompt::clear_tokens(v_smem + s * V_BYTES + (i & 1) * BLK, (threadIdx.x & 63) + (i >> 1) * 64, kv_begin - k0 - (i & 1) * BS,
+                               kv_end - k0 - (i & 1) * BS);
+        prompt::pass_on(&bars.v_full[s]);
+      }
     }
   } else {
     prompt::regs_inc<prompt::REGS_SOFTMAX>();

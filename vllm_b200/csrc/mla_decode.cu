@@ -27,7 +27,7 @@
 // Bound at these sizes by latency: about 14 us of set-up, first copies, last product and stores, and 3 us per tile of a split, two thirds of it the 36
 // products of Q K (90 cycles each, whatever their order or accumulator; a wait and a fence per k-block beside them), the rest the softmax.  24
 // requests of 600 tokens in 6 splits 42 → 28 us and 1200 tokens 44 → 34 since the sums' reductions, the rescaling rule and the stores are branch-free, with
-// their addresses formed once, and shared memory is cleared only where pages smaller than a tile need it.
+// their addresses formed once, and of shared memory only the rows of Q and P are cleared at the start.
 //
 // wide: the rows of short portions in steps that are not decode steps alone, whose weights were held in 32 bits on the CUDA cores: the second product
 // of the weights' low parts costs 1 to 3 us; the rows of a step of 24 requests took 660 us there.
@@ -166,11 +166,10 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_cons
   }
   if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
   {
-    // padded Q and P rows must be finite, and the part of the last tile that pages smaller than a tile leave out: zeros once
+    // padded Q and P rows must be finite: zeros once
     uint4 z = make_uint4(0, 0, 0, 0);
-    uint4* s4 = reinterpret_cast<uint4*>(smem);
-    const int n16 = (STAGES * STAGE_BYTES + Q_BYTES + 8192) / 16;
-    for (int i = (ppt > 1 ? 0 : STAGES * STAGE_BYTES / 16) + threadIdx.x; i < n16; i += NUM_THREADS) s4[i] = z;
+    uint4* s4 = reinterpret_cast<uint4*>(q_smem);
+    for (int i = threadIdx.x; i < (Q_BYTES + 8192) / 16; i += NUM_THREADS) s4[i] = z;
   }
   // token row (in the [num_blocks * BS, row] view of the cache) of every TMA box of this split, -1 = past the sequence
   auto box_row = [&](int i) -> int {
@@ -327,14 +326,22 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_cons
       }
       tc_fence_before();
       mbar_arrive(&s_empty[sb]);
-      const int kpos = (tile_lo + j) * TILE + t;
-      const bool ok = t < TILE && kpos < seq_len && kpos >= kv_begin;        // TMEM lanes 64..127 are the QK padding rows
+      const int lo = kv_begin - (tile_lo + j) * TILE, hi = min(seq_len - (tile_lo + j) * TILE, TILE);     // tokens [lo, hi) of the tile are seen
+      const bool ok = t < hi && t >= lo;                       // TMEM lanes 64..127 are the QK padding rows
       if (qd < 2) {
 #pragma unroll
         for (int g = 0; g < N; ++g) {
           s[g] = ok ? s[g] * p.scale_log2 : -INFINITY;
           const float cm = warp_max_f32(s[g]);
           if (lane == 0) wred[qd * N + g] = cm;
+        }
+      } else if (t - TILE < lo || t - TILE >= hi) {
+        // slots that are not the sequence's may hold what a weight of 0 does not cancel (attention_prompt.cuh): the lanes without a token clear them
+#pragma unroll 1
+        for (int kb = 0; kb < NL; ++kb) {
+          uint4* to = reinterpret_cast<uint4*>(kv_smem + (j % STAGES) * STAGE_BYTES + kb * KB_BYTES + (t - TILE) * 128);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) to[(i + t) & 7] = make_uint4(0, 0, 0, 0);       // (neighbours on other banks)
         }
       }
       bar_sync_softmax();
