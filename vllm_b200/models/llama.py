@@ -223,7 +223,7 @@ class LlamaModel(nn.Module):
                 li = self.start + i
                 for k, src in enumerate(skip["save"]):
                     if li in src:
-                        saved[k] = residual
+                        saved[k] = residual.clone()       # (the next layer adds to it in place)
                 for k, dst in enumerate(skip["mix"]):
                     if li in dst and k in saved:
                         residual = saved[k] * skip["tv"] + residual * (1.0 - skip["tv"])
