@@ -536,17 +536,17 @@ EXPORT int vb_moe_gather(const void* x, const int* sorted_tok, void* xs, int R, 
   return (int)cudaGetLastError();
 }
 
-// all of [T, H] contiguous (y [R, H]); H a multiple of 8 up to 32768
+// all of [T, H] contiguous (y [R, H]); H a multiple of 8 up to 32768; flags as vb_rms_norm's
 EXPORT int vb_moe_combine_norm(const void* y, const int* inv, const float* w, int k, const void* extra, const void* gate, void* residual,
-                               const void* nw, void* out, int T_, int H, float eps, int gemma, int dtype, cudaStream_t st) {
+                               const void* nw, void* out, int T_, int H, float eps, int flags, int dtype, cudaStream_t st) {
   if (T_ == 0) return 0;
   if (dtype == DT_F32 || H % 8 || H / 8 > 4096 || k < 1) return -1;
   const int nvec = H / 8, quarter = ((nvec + 3) / 4 + 31) / 32 * 32;   // vectors of a row, threads with four each
   int thr = (nvec + 31) / 32 * 32;
-  if (T_ >= 1024 && nvec >= 256) thr = quarter < 128 ? 128 : quarter;      // as norm_threads
+  if (T_ >= 1024 && nvec >= 256 && !(flags & 2)) thr = quarter < 128 ? 128 : quarter;      // as norm_threads
   if (thr > 1024) thr = 1024;
 #define GO(G) vb_launch(thr >= nvec ? moe::combine_norm_kernel<T, G, 1> : moe::combine_norm_kernel<T, G, 4>, dim3(T_), dim3(thr), 0, st, (const T*)y, inv, w, k, (const T*)extra, (const T*)gate, (T*)residual, (const T*)nw, (T*)out, H, eps)
-  DISPATCH_HALF(dtype, T, { if (gemma) GO(true); else GO(false); });
+  DISPATCH_HALF(dtype, T, { if (flags & 1) GO(true); else GO(false); });
 #undef GO
   return (int)cudaGetLastError();
 }

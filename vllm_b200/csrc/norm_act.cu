@@ -260,7 +260,8 @@ __global__ void soft_cap_kernel(T* __restrict__ x, int64_t stride, int n, int64_
 
 // Prompts (enough rows to fill the SMs several times over) give a thread two to four vectors: fewer threads to hold up at the reduction, as many
 // loads in flight.  Add and norm of 7600 rows: 4096 wide 59 → 41 us (6.1 TB/s), 8192 wide 125 → 80; 1024 rows of 4096 14 → 10; below
-// and for rows of less than 256 vectors no difference.
+// and for rows of less than 256 vectors no difference.  The order of a row's sum goes by the threads: T = 0 (batch-invariant mode) leaves the
+// number of rows out.
 int norm_threads(int H, int vecN, int T = 0) {
   int nvec = H / vecN;
   int t = (nvec + MAXV - 1) / MAXV;
@@ -275,16 +276,18 @@ int norm_threads(int H, int vecN, int T = 0) {
 
 }  // namespace
 
+// flags of the norms: 1 weights are differences from 1 (gemma), 2 the order of a row's sum does not depend on T
 // x: [T, H] (row stride x_stride elements), w: [H]. ADD: residual [T, H] contiguous updated in place, normed → x.
 #define NORM(A, G) (one ? rms_norm_kernel<TT, A, G, 1> : rms_norm_kernel<TT, A, G, MAXV>)
 #define TAIL(G) (one ? norm_add_norm_kernel<TT, G, 1> : norm_add_norm_kernel<TT, G, MAXV>)
 EXPORT int vb_rms_norm(void* out, void* x, void* residual, const void* w, int T, int H, int64_t x_stride, float eps,
-                       int gemma, int dtype, cudaStream_t st) {
+                       int flags, int dtype, cudaStream_t st) {
   if (T == 0) return 0;
+  const bool gemma = flags & 1;
   DISPATCH_DTYPE(dtype, TT, {
     constexpr int N = Vec16<TT>::N;
     if (H % N != 0 || H / N > 1024 * MAXV) return -1;
-    const int thr = norm_threads(H, N, T);
+    const int thr = norm_threads(H, N, flags & 2 ? 0 : T);
     const bool one = thr * N >= H;
     if (residual) {
       if (gemma) vb_launch(NORM(true, true), T, thr, 0, st, (TT*)x, (TT*)x, (TT*)residual, (const TT*)w, H, eps, x_stride);
@@ -298,13 +301,14 @@ EXPORT int vb_rms_norm(void* out, void* x, void* residual, const void* w, int T,
 }
 
 // x, residual, out [T, H] contiguous
-EXPORT int vb_norm_add_norm(void* out, const void* x, void* residual, const void* w1, const void* w2, int T, int H, float eps1, float eps2, int gemma,
+EXPORT int vb_norm_add_norm(void* out, const void* x, void* residual, const void* w1, const void* w2, int T, int H, float eps1, float eps2, int flags,
                             int dtype, cudaStream_t st) {
   if (T == 0) return 0;
+  const bool gemma = flags & 1;
   DISPATCH_DTYPE(dtype, TT, {
     constexpr int N = Vec16<TT>::N;
     if (H % N != 0 || H / N > 1024 * MAXV) return -1;
-    const int thr = norm_threads(H, N, T);
+    const int thr = norm_threads(H, N, flags & 2 ? 0 : T);
     const bool one = thr * N >= H;
     if (gemma) vb_launch(TAIL(true), T, thr, 0, st, (TT*)out, (const TT*)x, (TT*)residual, (const TT*)w1, (const TT*)w2, H, eps1, eps2);
     else vb_launch(TAIL(false), T, thr, 0, st, (TT*)out, (const TT*)x, (TT*)residual, (const TT*)w1, (const TT*)w2, H, eps1, eps2);
@@ -440,6 +444,7 @@ EXPORT int vb_sigmoid_mul(const void* x, int64_t x_stride, const void* g, int64_
     if (n % N == 0 && x_stride % N == 0 && g_stride % N == 0 && y_stride % N == 0 && al(x) && al(g) && al(y)) GO(N);
     else GO(1);
   });
+#undef GO
   return (int)cudaGetLastError();
 }
 

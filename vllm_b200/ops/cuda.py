@@ -154,6 +154,11 @@ def _heads(x: torch.Tensor) -> torch.Tensor:
     return x if x.data_ptr() % 16 == 0 and (x.stride(0) * x.element_size()) % 16 == 0 else x.clone(memory_format=torch.contiguous_format)
 
 
+def _norm_flags(gemma: bool) -> int:
+    """Flags of the norm kernels (csrc/norm_act.cu)."""
+    return int(gemma) | 2 * int(batch_invariant())
+
+
 def rms_norm(x, weight, eps, gemma=False):
     H = x.shape[-1]
     x2 = x.reshape(-1, H)
@@ -161,7 +166,7 @@ def rms_norm(x, weight, eps, gemma=False):
         x2 = x2.clone(memory_format=torch.contiguous_format)
     out = torch.empty((x2.shape[0], H), dtype=x.dtype, device=x.device)
     _check(_rms_norm(out.data_ptr(), x2.data_ptr(), None, weight.data_ptr(), x2.shape[0], H, x2.stride(0), eps,
-                     int(gemma), _DT[x.dtype], _st()), "rms_norm")
+                     _norm_flags(gemma), _DT[x.dtype], _st()), "rms_norm")
     return out.view(x.shape)
 
 
@@ -170,7 +175,7 @@ def fused_add_rms_norm(x, residual, weight, eps, gemma=False):
     H = x.shape[-1]
     assert x.is_contiguous() and residual.is_contiguous()
     T = x.numel() // H
-    _check(_rms_norm(x.data_ptr(), x.data_ptr(), residual.data_ptr(), weight.data_ptr(), T, H, H, eps, int(gemma),
+    _check(_rms_norm(x.data_ptr(), x.data_ptr(), residual.data_ptr(), weight.data_ptr(), T, H, H, eps, _norm_flags(gemma),
                      _DT[x.dtype], _st()), "fused_add_rms_norm")
     return x, residual
 
@@ -183,7 +188,7 @@ def norm_add_norm(x, residual, w1, eps1, w2, eps2, gemma=False):
     H = x.shape[-1]
     out = torch.empty_like(x)
     assert x.is_contiguous() and residual.is_contiguous() and residual.shape == x.shape and residual.dtype == w1.dtype == w2.dtype == x.dtype
-    _check(_norm_add_norm(out.data_ptr(), x.data_ptr(), residual.data_ptr(), w1.data_ptr(), w2.data_ptr(), x.numel() // H, H, eps1, eps2, int(gemma),
+    _check(_norm_add_norm(out.data_ptr(), x.data_ptr(), residual.data_ptr(), w1.data_ptr(), w2.data_ptr(), x.numel() // H, H, eps1, eps2, _norm_flags(gemma),
                           _DT[x.dtype], _st()), "norm_add_norm")
     return out, residual
 
@@ -1211,7 +1216,7 @@ def moe_combine_norm(rows, inv, w, residual, norm_w, eps: float, gemma: bool, ex
         assert t is None or (t.dtype == rows.dtype and t.is_contiguous())
     assert w.dtype == torch.float32 and w.is_contiguous() and inv.dtype == torch.int32 and inv.numel() == w.numel()
     _check(_moe_combine_norm(rows.data_ptr(), inv.data_ptr(), w.data_ptr(), inv.numel() // max(T, 1), _p(extra), _p(gate), residual.data_ptr(),
-                             norm_w.data_ptr(), out.data_ptr(), T, H, eps, int(gemma), _DT[rows.dtype], _st()), "moe_combine_norm")
+                             norm_w.data_ptr(), out.data_ptr(), T, H, eps, _norm_flags(gemma), _DT[rows.dtype], _st()), "moe_combine_norm")
     return out, residual
 
 
