@@ -41,3 +41,41 @@ def test_norms(H, gemma):
     for name, run in runs.items():
         for a, b in zip(run(n), run(big)):
             assert torch.equal(a, b[:n]), name
+
+
+@pytest.mark.parametrize("Hq,Hkv,window,cap", [(32, 8, None, 0.0), (32, 8, 100, 0.0), (16, 4, None, 50.0), (8, 2, None, 1.0), (32, 8, 129, 50.0)])
+def test_prompt_attention(Hq, Hkv, window, cap):
+    """A prompt of 300 tokens alone, in portions, in a captured step's form, and in front of 12000 other tokens."""
+    import dataclasses
+    from tests.test_kernels_gpu import _mk_attn_case, _to_tc_layout
+    from vllm_b200.ops import cuda as cu
+    lens = [300] + [3000] * 4
+    q, cache, md = _mk_attn_case(len(lens), Hq, Hkv, 128, 64, lens, lens)
+    q, cache, md.kv_vt = q * 2, _to_tc_layout(cache), True
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+
+    def portion(a, b, **kw):
+        one = dataclasses.replace(md, num_reqs=1, num_actual_tokens=b - a, max_query_len=b - a, max_seq_len=b, query_start_loc=i32(0, b - a),
+                                  seq_lens=i32(b), block_table=md.block_table[:1], **kw)
+        return cu.paged_attention(q[a:b], cache, one, 0.1, window, cap)
+    want = cu.paged_attention(q, cache, md, 0.1, window, cap)[:300]
+    assert torch.equal(portion(0, 300), want)
+    assert torch.equal(portion(0, 300, flat=True), want)
+    assert torch.equal(torch.cat([portion(0, 77), portion(77, 205), portion(205, 206), portion(206, 300)]), want)
+
+
+@pytest.mark.parametrize("window", [0, 100])
+@pytest.mark.parametrize("split", [False, True])
+def test_expanded_prompts(window, split):
+    from vllm_b200.ops import cuda as cu
+    lens, H, D, V = [300] + [3000] * 4, 16, 64, 64
+    T = sum(lens)
+    q, k, v = _rnd(T, H, D, seed=5), _rnd(T, H, D, seed=6), _rnd(T, H, V, seed=7)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+
+    def run(n):
+        m, out = sum(lens[:n]), torch.zeros(sum(lens[:n]), H, V, dtype=q.dtype, device="cuda")
+        start = i32([sum(lens[:i]) for i in range(n)])
+        cu.mla_prefill(q[:m], k[:m], v[:m], out, start, i32(lens[:n]), i32(lens[:n]), start, 0, max(lens[:n]), 0.1, window=window, split=split)
+        return out[:300]
+    assert torch.equal(run(1), run(5))

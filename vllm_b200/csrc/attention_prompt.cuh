@@ -22,6 +22,13 @@
 
 namespace prompt {
 
+// Query tiles (of all requests and heads) for each SM from which a CTA takes two of them: below, SMs would be left without any, and the two
+// warpgroups of a CTA share one.  One prompt of 2000 tokens, 8 / 2 heads (125 tiles): 42 us shared, 57 us with one warpgroup at work; 2 x 1000,
+// 16 / 4 heads (250): 40 against 49; from 300 tiles on two per CTA: 8 x 300, 16 / 4 heads (300) 34 us, 2 x 2000, 32 / 8 (1000) 124 us, where one
+// tile of rows per CTA took 182.  The two forms add a row's keys in different orders, so batch-invariant mode (in_order) has one: always two
+// tiles, the second one empty where a portion ends within the first.
+constexpr int PAIR_MIN_TILES = 2;
+
 constexpr int ROWS = 128, KEYS = 128;
 constexpr int NUM_THREADS = 384;            // warp 0 TMA producer, 1 MMA issuer, 2 and 3 clear values, 4..7 and 8..11 softmax of the two tiles
 // registers a thread: launched with 168; 384 x 168 = 128 x 72 + 256 x 216
@@ -161,7 +168,7 @@ VB_DEVICE float cap_small(float x, float c2) {
   r = fmaf(r, z, 0.13325075805187225f);
   r = fmaf(r, z, -0.3333282768726349f);
   r = fmaf(r, z, 0.9999999403953552f);
-  return r * (x * c2);
+  return r * x * c2;                          // (as cap_any rounds it: a score's value does not depend on its warp's others)
 }
 VB_DEVICE float cap_any(float x, float c2) {
   const float e = ex2(fabsf(x) * 2.8853900817779268f);          // e^(2 |x|), at worst infinite: 1 - 0

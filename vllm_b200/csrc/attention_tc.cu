@@ -42,6 +42,7 @@ struct Params {
   int bt_stride;
   int Hq, Hkv, G, TQ, num_splits;
   int tiles;               // query tiles per CTA: 1 or 2
+  int in_order;            // a row's keys are added in their order, whatever else is in the batch
   int window, causal;
   prompt::Softmax sm;
   int flat_B;              // > 0: grid.x enumerates the (request, query tile) pairs of `flat_B` requests (device-side
@@ -111,7 +112,7 @@ fmha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
   const int tok0 = qt * TC;
   if (tok0 >= q_len) return;                       // uniform across the CTA
   const int n_tok = min(TC, q_len - tok0);
-  const int tiles = n_tok > p.TQ ? 2 : 1;
+  const int tiles = n_tok > p.TQ || p.in_order ? 2 : 1;
   const int pos0 = seq_len - q_len + tok0;
   const int pos_last = pos0 + n_tok - 1;
   const int kv_end = p.causal ? pos_last + 1 : seq_len;
@@ -338,12 +339,6 @@ static EncodeTiledFn get_encode() {
   return fn;
 }
 
-// Query tiles (of all requests and KV heads) from which a CTA takes two of them: below, SMs would be left without any, and the two
-// warpgroups of a CTA share one.  One prompt of 2000 tokens, 8 / 2 heads (125 tiles): 42 us shared, 57 us with one warpgroup at work; 2 x 1000,
-// 16 / 4 heads (250): 40 against 49; from 300 tiles on two per CTA: 8 x 300, 16 / 4 heads (300) 34 us, 2 x 2000, 32 / 8 (1000) 124 us, where one
-// tile of rows per CTA took 182.
-constexpr int PAIR_MIN_TILES = 2 * 148;
-
 template <typename T, bool CAP>
 static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const Params& p, dim3 grid, cudaStream_t st) {
   const int smem = 2 * Q_BYTES + KV_STAGES * (K_BYTES + V_BYTES) + (int)sizeof(Bars) + TILE_M * 8 + 16 + 2 * MAX_TILES_SMEM * 4 + 1024;
@@ -359,11 +354,12 @@ static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
 // kv_cache: [nb, 2, Hkv, BS*D] with K pages [BS, D] and V pages stored transposed [D, BS].
 // flat != 0 (varlen only): the grid is sized from (T_total, B) alone — T_total / TQ + B tiles bound every split of
 // T_total tokens over B requests — so one captured launch serves any mixed batch of that bucket.
-EXPORT int vb_fmha_tc3(const void* q, const void* kv_cache, int64_t num_blocks, const int* block_table,
+// in_order != 0: a row's result does not depend on the size of the batch or on where its portion begins.
+EXPORT int vb_fmha_tc4(const void* q, const void* kv_cache, int64_t num_blocks, const int* block_table,
                        const int* seq_lens, const int* qsl, void* out, float* part_out, float* part_lse,
                        float* lse_out, int* error, int B, int T_total, int max_q_len, int Hq, int Hkv, int64_t q_stride,
                        int64_t out_stride, int bt_stride, int num_splits, int window, float scale, float soft_cap, int causal,
-                       int flat, int chunk, const float* sinks, float out_scale, int dtype, cudaStream_t st) {
+                       int flat, int chunk, const float* sinks, float out_scale, int in_order, int num_sms, int dtype, cudaStream_t st) {
   using namespace fmha;
   if (B == 0) return 0;
   if (dtype == DT_F32) return -1;
@@ -381,7 +377,8 @@ EXPORT int vb_fmha_tc3(const void* q, const void* kv_cache, int64_t num_blocks, 
   p.sm.ku = soft_cap > 0.f ? scale / soft_cap : 0.f; p.sm.c2 = soft_cap * 1.4426950408889634f;
   p.flat_B = (flat && qsl) ? B : 0;
   p.chunk = chunk; p.sinks = sinks; p.out_scale = out_scale; p.error = error;
-  p.tiles = qsl && (int64_t)T_total * Hq / TILE_M >= PAIR_MIN_TILES ? 2 : 1;
+  p.in_order = in_order && qsl;
+  p.tiles = p.in_order || (qsl && (int64_t)T_total * Hq / TILE_M >= prompt::PAIR_MIN_TILES * num_sms) ? 2 : 1;
   CUtensorMap tq, tk, tv;
   {  // q: [T, Hq, D] with token stride q_stride; box {64, G, TQ}
     cuuint64_t dims[3] = {(cuuint64_t)D, (cuuint64_t)Hq, (cuuint64_t)T_total};

@@ -39,6 +39,7 @@ struct Params {
   int vdim;
   int window;              // > 0: a query sees its last `window` keys
   int tiles;               // query tiles per CTA: 1 or 2
+  int in_order;            // a row's keys are added in their order, whatever else is in the batch
   int split;               // weights keep 16 more bits
   prompt::Softmax sm;
   int* error;
@@ -84,7 +85,7 @@ mla_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   const int tok0 = qt * TM * p.tiles;
   if (tok0 >= q_len) return;                                // uniform over the CTA
   const int n_tok = min(TM * p.tiles, q_len - tok0);
-  const int tiles = n_tok > TM ? 2 : 1;
+  const int tiles = n_tok > TM || p.in_order ? 2 : 1;
   const int q0 = p.q_start[b] + tok0;
   const int kv0 = p.kv_start[b];
   const int pos0 = p.seq_len[b] - q_len + tok0;             // position of the first tile's first query
@@ -228,9 +229,6 @@ static int tmap(CUtensorMap* m, const void* ptr, int width, int heads, int64_t r
 
 struct Maps { CUtensorMap q, k, v, qr, kr; };
 
-// Query tiles (of all requests and heads) from which a CTA takes two of them (attention_tc.cu)
-constexpr int PAIR_MIN_TILES = 2 * 148;
-
 template <typename T, int NN, int NR, int NV>
 static int launch(const Maps& m, const Params& p, dim3 grid, cudaStream_t st) {
   constexpr int NQ = NN + NR;
@@ -248,10 +246,11 @@ static int launch(const Maps& m, const Params& p, dim3 grid, cudaStream_t st) {
 // q [T, H, dim + rot] and out [T, H, vdim] (row strides q_st / out_st); k [KV, hl, dim], v [KV, hl, vdim] (row and head strides free) hold
 // the heads h0 .. h0 + hl - 1; k_pe [KV, rot] (row stride kr_st; rot = 0: none) is the rotated key part of all heads.  Request b owns query rows
 // q_start[b] .. + q_len[b] and key rows kv_start[b] .. + seq_len[b], of which its portion is the tail.
-EXPORT int vb_mla_prefill2(const void* q, const void* k, const void* v, const void* k_pe, void* out, const int* q_start, const int* q_len,
+EXPORT int vb_mla_prefill3(const void* q, const void* k, const void* v, const void* k_pe, void* out, const int* q_start, const int* q_len,
                           const int* seq_len, const int* kv_start, int* error, int B, int T_, int64_t KV, int H, int h0, int hl,
                           int dim, int rot, int vdim, int64_t q_st, int64_t k_st, int64_t k_sh, int64_t v_st, int64_t v_sh, int64_t kr_st,
-                          int64_t out_st, int max_q, int window, float scale, int split, int dtype, cudaStream_t st) {
+                          int64_t out_st, int max_q, int window, float scale, int split, int in_order, int num_sms,
+                          int dtype, cudaStream_t st) {
   using namespace mlap;
   if (B == 0 || T_ == 0 || max_q <= 0) return 0;
   if (dtype == DT_F32 || dim < 8 || dim > 128 || dim % 8 || vdim < 8 || vdim > 128 || vdim % 8 || rot < 0 || rot > 64 || rot % 8) return -1;
@@ -270,7 +269,8 @@ EXPORT int vb_mla_prefill2(const void* q, const void* k, const void* v, const vo
   Params p;
   p.q_start = q_start; p.q_len = q_len; p.seq_len = seq_len; p.kv_start = kv_start; p.out = out; p.out_st = out_st;
   p.out_sh = vdim; p.h0 = h0; p.vdim = vdim; p.window = window; p.sm.scale_log2 = scale * 1.4426950408889634f; p.sm.ku = p.sm.c2 = 0.f; p.split = split; p.error = error;
-  p.tiles = (int64_t)(T_ / TM) * hl >= PAIR_MIN_TILES ? 2 : 1;
+  p.in_order = in_order;
+  p.tiles = in_order || (int64_t)(T_ / TM) * hl >= prompt::PAIR_MIN_TILES * num_sms ? 2 : 1;
   const dim3 grid((max_q + TM * p.tiles - 1) / (TM * p.tiles), hl, B);
   const int nq = (dim + 63) / 64, nv = (vdim + 63) / 64;
 #define GV(TT, N, R) (nv == 1 ? launch<TT, N, R, 1>(m, p, grid, st) : launch<TT, N, R, 2>(m, p, grid, st))

@@ -91,8 +91,8 @@ _paged_attention = _sig("vb_paged_attention", _vp, _vp, _vp, _vp, _vp, _vp, _vp,
                         _i64, _i64, _i, _i, _i, _f, _f, _f, _i, _i, _i, _vp)
 _paged_attention_ex = _sig("vb_paged_attention_ex", _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,
                            _i64, _i64, _i, _i, _i, _f, _f, _f, _i, _i, _i, _vp, _vp, _i, _vp)
-_fmha_tc = _sig("vb_fmha_tc3", _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i64, _i64, _i,
-                _i, _i, _f, _f, _i, _i, _i, _vp, _f, _i, _vp)
+_fmha_tc = _sig("vb_fmha_tc4", _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i64, _i64, _i,
+                _i, _i, _f, _f, _i, _i, _i, _vp, _f, _i, _i, _i, _vp)
 _fmha_tc_decode = _sig("vb_fmha_tc_decode2", _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i64, _i,
                        _i, _i, _f, _f, _i, _vp, _f, _i, _vp)
 _any_attention = _sig("vb_any_attention", _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i64, _i64, _i, _i, _i,
@@ -414,7 +414,7 @@ def paged_attention(q, kv_cache, md, scale, sliding_window=None, logits_soft_cap
                       _p(ws.part_out) if ws else None, _p(ws.part_lse) if ws else None, _p(lse), _error_flag(q.device),
                       md.num_reqs, T, md.max_query_len, Hq, Hkv, q.stride(0), out.stride(0), bt.stride(0), splits,
                       sliding_window or 0, scale, logits_soft_cap, int(causal), int(md.flat and not decode), chunk_size, _p(sinks), out_scale,
-                      _DT[q.dtype], _st())
+                      int(batch_invariant()), num_sms(), _DT[q.dtype], _st())
         _check(rc, f"fmha_tc(G={Hq // Hkv})", 2 if splits > 1 else 1)
         return (out, lse) if return_lse else out
     if not _simt_attention_ok(D, DV, BS, G, q.dtype) or out_scale != 1.0:
@@ -538,8 +538,8 @@ def merge_attn_states(o1, lse1, o2, lse2):
 
 _mla_decode = _sig("vb_mla_decode2", _vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i64, _i64,
                    _i64, _i64, _i64, _i, _i, _i, _i, _f, _i, _vp)
-_mla_prefill = _sig("vb_mla_prefill2", _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i64, _i, _i, _i, _i, _i, _i, _i64, _i64,
-                    _i64, _i64, _i64, _i64, _i64, _i, _i, _f, _i, _i, _vp)
+_mla_prefill = _sig("vb_mla_prefill3", _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i64, _i, _i, _i, _i, _i, _i, _i64, _i64,
+                    _i64, _i64, _i64, _i64, _i64, _i, _i, _f, _i, _i, _i, _i, _vp)
 _mla_simt = _sig("vb_mla_simt", _vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _i, _i, _i, _i, _i, _i, _i64, _i64, _i64, _i64, _i64,
                  _i64, _i, _f, _i, _vp)
 _latent_rope = _sig("vb_latent_rope_cache2", _vp, _vp, _i64, _i64, _i, _i, _i, _i, _vp, _f, _vp, _vp, _i, _vp, _i64, _vp, _i, _i, _vp)
@@ -675,7 +675,8 @@ def mla_prefill(q, k, v, out, q_start, q_len, seq_len, kv_start, h0: int, max_q:
     _check(_mla_prefill(q.data_ptr(), k.data_ptr(), v.data_ptr(), _p(k_pe), out.data_ptr(), q_start.data_ptr(), q_len.data_ptr(),
                         seq_len.data_ptr(), kv_start.data_ptr(), kernel_error_flag(q.device).data_ptr(), q_len.numel(), T, KV, H,
                         h0, hl, D, P, VD, q.stride(0), k.stride(0), k.stride(1), v.stride(0), v.stride(1),
-                        0 if k_pe is None else k_pe.stride(0), out.stride(0), max_q, window, scale, int(split), _DT[q.dtype], _st()),
+                        0 if k_pe is None else k_pe.stride(0), out.stride(0), max_q, window, scale, int(split),
+                        int(batch_invariant()), num_sms(), _DT[q.dtype], _st()),
            f"mla_prefill(T={T},KV={KV},H={H})")
 
 
