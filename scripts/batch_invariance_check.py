@@ -1,6 +1,6 @@
 """Bitwise batch-invariance check on a GPU (VLLM_BATCH_INVARIANT=1).
 
-    VLLM_BATCH_INVARIANT=1 python scripts/batch_invariance_check.py [--model llama-3-8b-4l] [--tp 1]
+    VLLM_BATCH_INVARIANT=1 python scripts/batch_invariance_check.py [--model llama-3-8b] [--tp 1]
 
 Generates from one prompt (a) alone, (b) first in a batch of 48 unrelated prompts of mixed length, (c) last in that batch,
 (d) arriving while the others are mid-decode, and compares the sampled-token logprobs bit for bit.  Prints one JSON
@@ -19,14 +19,14 @@ os.environ.setdefault("VLLM_LOGGING_LEVEL", "WARNING")
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("--model", default="llama-3-8b-4l")
+    ap.add_argument("--model", default="llama-3-8b")
     ap.add_argument("--tp", type=int, default=1)
     ap.add_argument("--tokens", type=int, default=32)
     a = ap.parse_args()
     from vllm_b200 import LLM, SamplingParams
     llm = LLM(a.model, load_format="dummy", tensor_parallel_size=a.tp, max_model_len=4096, max_num_seqs=64,
               gpu_memory_utilization=0.5)
-    V = llm.llm_engine.vllm_config.model_config.get_vocab_size()
+    V = llm.llm_engine.vllm_config.model_config.vocab_size
     sp = SamplingParams(max_tokens=a.tokens, temperature=0.0, ignore_eos=True, logprobs=1)
     needle = {"prompt_token_ids": [(17 * i + 3) % (V - 10) + 5 for i in range(301)]}
     others = [{"prompt_token_ids": [(31 * i + 7 * j) % (V - 10) + 5 for j in range(16 + 61 * (i % 9))]} for i in range(48)]

@@ -79,3 +79,27 @@ def test_expanded_prompts(window, split):
         cu.mla_prefill(q[:m], k[:m], v[:m], out, start, i32(lens[:n]), i32(lens[:n]), start, 0, max(lens[:n]), 0.1, window=window, split=split)
         return out[:300]
     assert torch.equal(run(1), run(5))
+
+
+@pytest.mark.parametrize("T,E,k", [(1200, 8, 4), (2100, 64, 8), (600, 4, 2)])
+def test_experts(T, E, k):
+    """A few tokens alone and in a batch above 1024 pairs and above 64 pairs for each expert."""
+    from vllm_b200.ops import moe
+    H, inter = 2048, 192
+    x, w13, w2 = _rnd(T, H), _rnd(E, 2 * inter, H, seed=1, scale=H ** -0.5), _rnd(E, H, inter, seed=2, scale=inter ** -0.5)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    ids = torch.rand(T, E, device="cuda", generator=g).topk(k, -1).indices.int()
+    w = torch.rand(T, k, device="cuda", generator=g)
+    whole = moe.fused_moe_cuda(x, w13, w2, w, ids)
+    for n in (1, 30, 250):
+        assert torch.equal(moe.fused_moe_cuda(x[:n].contiguous(), w13, w2, w[:n].contiguous(), ids[:n].contiguous()), whole[:n])
+
+
+def test_block_scaled_products():
+    from vllm_b200.ops import cuda as cu, ref
+    x = _rnd(2000, 512)
+    wq, ws = ref.block_quant_weight_fp8(torch.randn(8192, 512, device="cuda") * 0.05, 128)
+    xq, xs = cu.per_token_group_quant_fp8(x, 128, col_major=True)
+    whole = cu.gemm_fp8_block(xq, xs, wq, ws.contiguous())
+    xq, xs = cu.per_token_group_quant_fp8(x[:200].contiguous(), 128, col_major=True)
+    assert torch.equal(cu.gemm_fp8_block(xq, xs, wq, ws.contiguous()), whole[:200])

@@ -333,7 +333,8 @@ def batch_invariant() -> bool:
     made from that row's own shape only — never from how many other rows share the launch.  Concretely: no split-K in
     the decode GEMMs (the split factor is otherwise chosen per (N, K) but switches off above 256 rows), no split-KV in
     decode attention (the split count depends on batch × heads), decode-only batches run the same varlen attention
-    kernel as mixed batches, collectives reduce in rank order at every size (no in-switch multimem reduction, no
+    kernel as mixed batches, prompts attend in one form of it, experts keep to one form of their products, the norms' thread count
+    goes by the width alone, collectives reduce in rank order at every size (no in-switch multimem reduction, no
     Lamport fused GEMM + all-reduce), and the MoE combine does not use ``red.add`` epilogues (atomic arrival order).
     Reference: vllm/model_executor/layers/batch_invariant.py (``VLLM_BATCH_INVARIANT`` swaps in fixed-reduction-order
     matmul / softmax / rms-norm kernels, fixes the attention split size and pins NCCL to one algorithm :1105-1180),

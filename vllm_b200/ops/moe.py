@@ -56,6 +56,9 @@ def fused_moe_grouped(x, w13, w2, topk_w, topk_ids, act, expert_map):
 def rows_ok(x, w13, w2, R: int) -> bool:
     """Are the expert outputs of R pairs computed as sorted rows on the device?"""
     from vllm_b200 import envs
+    from vllm_b200.ops import cuda as cu
+    if cu.batch_invariant():          # the shapes decide, at every R
+        return _grouped_ok(x, w13, w2, 0)
     return _grouped_ok(x, w13, w2, R) or (
         _rows_ok(x, w13) and w2.dtype == x.dtype and w13.is_contiguous() and w2.is_contiguous() and w13.shape[0] <= 512
         and R > GROUPED_MAX_ROWS and envs.VLLM_B200_GEMM != "cublas")
@@ -95,7 +98,8 @@ def expert_rows_gated(x, w13, w2, topk_ids, act, expert_map):
     sorted_tok, inv, offs = cu.moe_align(ids.contiguous(), E, expert_map)
     x = x.contiguous()
     if _rows_ok(x, w13):
-        if R >= PROMPT_ROWS * E and R > GROUPED_MAX_ROWS and act in cu._GATED_ACT:
+        # (batch-invariant mode keeps to the decode tiles, which round the hidden rows before the activation)
+        if R >= PROMPT_ROWS * E and R > GROUPED_MAX_ROWS and act in cu._GATED_ACT and not cu.batch_invariant():
             return cu.gemm_grouped(cu.gemm_grouped(cu.moe_gather(x, sorted_tok), w13, offs, act), w2, offs), inv
         bn = _tile_width(R, E)
         h = cu.gemm_tc_grouped(cu.moe_gather(x, sorted_tok), w13, offs, bn, flat=True)

@@ -10,16 +10,20 @@ decode GEMM (M ≤ 256)  cluster split-K chosen per (N, K); none above 256 rows 
 fp8 GEMM               split-K per (N, K)                                          no split-K
 decode attention       split-KV count from batch × kv heads × context              one CTA per (sequence, kv head), pages in order
 decode-only batches    swap-AB decode kernel                                       the varlen kernel a mixed batch would use
+prompt attention       one or two query tiles per CTA by the batch's tokens        two per CTA, a row's keys in their order
 MLA decode             split-KV from batch × heads                                 no split
+DeepSeek prompts       expanded or latent form by the portion's length              latent form
+experts                decode tiles, 128 x 256 tiles from 64 pairs per expert       decode tiles
+norms                  a quarter of the threads per row from 1024 rows              threads by the width
 TP all-reduce          one-shot ≤ 512 rows, NVLS two-shot above, Lamport fused     rank-ordered one-shot at every size
                        GEMM + all-reduce for decode
 MoE combine            ``red.add.f32`` epilogue into per-token accumulators        sorted combine kernel (fixed k order)
 NCCL fallbacks         library's size-dependent algorithm / protocol               tree + Simple, one channel, no NVLS / CollNet
 =====================  =========================================================  ==========================================
 
-Per-row kernels (RMSNorm / LayerNorm: one CTA per row with a thread count that depends on H only; RoPE; activation;
-sampling: one row per CTA) are already invariant.  Not covered: MLA decode rows inside a mixed batch (they take the
-prefill path), FP4 weight-only GEMMs, LoRA shrink/expand split over slots.
+Per-row kernels (LayerNorm; RoPE; activation; sampling: one row per CTA) are already invariant.  Not covered: products of
+more than 256 rows in 16 bits, whose kernel the library picks by the rows; MLA decode rows inside a mixed batch (they take
+the prefill path), FP4 weight-only GEMMs, LoRA shrink/expand split over slots.
 
 Reference: vllm/model_executor/layers/batch_invariant.py (``init_batch_invariance`` /
 ``override_envs_for_invariance``), vllm/distributed/device_communicators/cuda_communicator.py:61-64 (custom all-reduce
