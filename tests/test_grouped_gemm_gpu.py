@@ -69,3 +69,19 @@ def test_both_grids_of_decode_experts(R, E, bn):
         assert torch.equal(a, b)
         want = torch.cat([xe.double() @ we.double().t() for xe, we in zip(x[:R - R // 10].split(n.tolist()), w)])
         assert _rel(a, want) < 2 ** -9
+
+
+@pytest.mark.parametrize("E,act", [(1024, "silu"), (600, "gelu_tanh"), (512, "silu")])
+def test_more_experts_than_the_prompt_tiles_take(E, act):
+    """64 pairs for each of more than 512 experts: the decode tiles go on with them."""
+    from vllm_b200.ops import moe
+    g = torch.Generator(device="cuda").manual_seed(4)
+    rnd = lambda *s, scale=1.0: (torch.randn(*s, device="cuda", generator=g) * scale).to(torch.bfloat16)  # noqa: E731
+    T, k, H, inter = 8 * E, 8, 64, 64
+    x, w13, w2 = rnd(T, H), rnd(E, 2 * inter, H, scale=H ** -0.5), rnd(E, H, inter, scale=inter ** -0.5)
+    ids = (torch.arange(T * k, device="cuda").view(T, k) * 7 % E).int()
+    w = torch.rand(T, k, device="cuda", generator=g)
+    got = moe.fused_moe_rows(x, w13, w2, w, ids, act, None, True)
+    n = 100
+    want = moe.fused_moe_rows(x[:n], w13, w2, w[:n], ids[:n], act, None, True)
+    assert _rel(got[:n], want) < 2 ** -7            # hidden rows rounded to bf16 on one side only, and both results

@@ -1235,6 +1235,7 @@ def gemm_tc_grouped(xs: torch.Tensor, w: torch.Tensor, offs: torch.Tensor, bn: i
 
 
 _GATED_ACT = {None: -1, "silu": 0, "swish": 0, "gelu": 1, "gelu_tanh": 2, "gelu_pytorch_tanh": 2}
+GROUPED_MAX_EXPERTS = 512       # MAX_E of csrc/gemm_grouped.cu
 
 
 def gemm_grouped(xs: torch.Tensor, w: torch.Tensor, offs: torch.Tensor, act: Optional[str] = None) -> torch.Tensor:

@@ -60,7 +60,8 @@ def rows_ok(x, w13, w2, R: int) -> bool:
     if cu.batch_invariant():          # the shapes decide, at every R
         return _grouped_ok(x, w13, w2, 0)
     return _grouped_ok(x, w13, w2, R) or (
-        _rows_ok(x, w13) and w2.dtype == x.dtype and w13.is_contiguous() and w2.is_contiguous() and w13.shape[0] <= 512
+        _rows_ok(x, w13) and w2.dtype == x.dtype and w13.is_contiguous() and w2.is_contiguous()
+        and w13.shape[0] <= cu.GROUPED_MAX_EXPERTS
         and R > GROUPED_MAX_ROWS and envs.VLLM_B200_GEMM != "cublas")
 
 
@@ -99,7 +100,8 @@ def expert_rows_gated(x, w13, w2, topk_ids, act, expert_map):
     x = x.contiguous()
     if _rows_ok(x, w13):
         # (batch-invariant mode keeps to the decode tiles, which round the hidden rows before the activation)
-        if R >= PROMPT_ROWS * E and R > GROUPED_MAX_ROWS and act in cu._GATED_ACT and not cu.batch_invariant():
+        if (R >= PROMPT_ROWS * E and R > GROUPED_MAX_ROWS and act in cu._GATED_ACT and E <= cu.GROUPED_MAX_EXPERTS
+                and not cu.batch_invariant()):
             return cu.gemm_grouped(cu.gemm_grouped(cu.moe_gather(x, sorted_tok), w13, offs, act), w2, offs), inv
         bn = _tile_width(R, E)
         h = cu.gemm_tc_grouped(cu.moe_gather(x, sorted_tok), w13, offs, bn, flat=True)
