@@ -85,3 +85,13 @@ def test_more_experts_than_the_prompt_tiles_take(E, act):
     n = 100
     want = moe.fused_moe_rows(x[:n], w13, w2, w[:n], ids[:n], act, None, True)
     assert _rel(got[:n], want) < 2 ** -7            # hidden rows rounded to bf16 on one side only, and both results
+
+
+def test_refused_activations_are_refused_at_every_size():
+    from vllm_b200.ops import moe
+    x = torch.zeros(300, 64, device="cuda", dtype=torch.bfloat16)
+    w13, w2 = torch.zeros(4, 128, 64, device="cuda", dtype=torch.bfloat16), torch.zeros(4, 64, 64, device="cuda", dtype=torch.bfloat16)
+    ids, w = torch.arange(1200, device="cuda").view(300, 4).int() % 4, torch.ones(300, 4, device="cuda")
+    for n in (10, 300):
+        with pytest.raises(KeyError):
+            moe.fused_moe_cuda(x[:n], w13, w2, w[:n], ids[:n], "swish")

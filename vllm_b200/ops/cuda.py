@@ -1234,7 +1234,7 @@ def gemm_tc_grouped(xs: torch.Tensor, w: torch.Tensor, offs: torch.Tensor, bn: i
     return y
 
 
-_GATED_ACT = {None: -1, "silu": 0, "swish": 0, "gelu": 1, "gelu_tanh": 2, "gelu_pytorch_tanh": 2}
+_GATED_ACT = {None: -1, "silu": 0, "gelu": 1, "gelu_tanh": 2, "gelu_pytorch_tanh": 2}
 GROUPED_MAX_EXPERTS = 512       # MAX_E of csrc/gemm_grouped.cu
 
 
