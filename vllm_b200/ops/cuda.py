@@ -549,14 +549,18 @@ _mla_ws: dict[int, tuple] = {}
 _kernel_error: dict[int, torch.Tensor] = {}
 
 
+KERNEL_GAVE_UP = "a kernel gave up waiting for a copy or a matrix product; its outputs are not valid"
+
+
 def kernel_error_flag(device: torch.device) -> torch.Tensor:
-    """Device int that a kernel with bounded waits raises when one of them ran into its limit."""
+    """Int that a kernel with bounded waits raises when one of them ran into its limit.  It lies in pinned host memory, which the kernel
+    stores to (in that case only): behind an event of the step the host reads it like any other of its own."""
     key = device.index or 0
     t = _kernel_error.get(key)
     if t is None:
         if torch.cuda.is_current_stream_capturing():
             raise RuntimeError("the kernel error flag must be allocated before CUDA-graph capture")
-        t = _kernel_error[key] = torch.zeros(1, dtype=torch.int32, device=device)
+        t = _kernel_error[key] = torch.zeros(1, dtype=torch.int32, pin_memory=True)
     return t
 
 
@@ -570,9 +574,11 @@ def _error_flag(device: torch.device) -> Optional[int]:
 def check_kernel_error(device: torch.device) -> None:
     """Raise if a kernel gave up on a wait since the last check (synchronises)."""
     t = _kernel_error.get(device.index or 0)
-    if t is not None and int(t.item()):
-        t.zero_()
-        raise RuntimeError("a kernel gave up waiting for a copy or a matrix product; its outputs are not valid")
+    if t is not None:
+        torch.cuda.synchronize(device)
+        if int(t):
+            t.zero_()
+            raise RuntimeError(KERNEL_GAVE_UP)
 
 
 def mla_decode_splits(B: int, H: int, max_seq_len: int, least: int = 512) -> int:

@@ -123,6 +123,7 @@ class AsyncStepOutput:
             t_w = time.perf_counter()
             self.event.synchronize()
             r.wait_s += time.perf_counter() - t_w
+        r.check_kernels()
         toks = self.staging.sampled[:self.nb].tolist()
         r.d2h_bytes += self.nb * 8
         out_ids: list[list[int]] = []
@@ -166,6 +167,11 @@ class ModelRunner:
         self.cc = vllm_config.cache_config
         self.device = device
         self.is_cuda = device.type == "cuda"
+        # raised by a kernel that gave up on a wait; made before anything is captured, so every captured launch has it
+        self.kernel_error: Optional[np.ndarray] = None
+        if self.is_cuda:
+            from vllm_b200.ops import cuda_ops
+            self.kernel_error = cuda_ops().kernel_error_flag(device).numpy()
         self.dtype = self.mc.torch_dtype
         self.max_num_reqs = self.sc.max_num_seqs
         self.max_num_tokens = self.sc.max_num_batched_tokens
@@ -1022,6 +1028,7 @@ class ModelRunner:
     def execute_model(self, so: SchedulerOutput, intermediate=None, non_block: bool = False):
         """Launch one step. Returns a ModelRunnerOutput, or (non_block) an AsyncStepOutput."""
         t0 = time.perf_counter()
+        self.check_kernels()            # of steps whose results this rank does not read back
         self._step += 1
         self._update_states(so)
         if so.total_num_scheduled_tokens == 0:
@@ -1157,11 +1164,11 @@ class ModelRunner:
             if isinstance(hidden, dict):  # non-last PP stage
                 return ModelRunnerOutput(kv_connector_output=hidden)
             if so.logits_positions is not None:
-                return self._wanted_logits(so, hidden, req_ids, rows, ns, cu, stg, t0)
+                return self._checked(self._wanted_logits(so, hidden, req_ids, rows, ns, cu, stg, t0))
             if any(s.pooling_params is not None for s in states):
-                return self._pool(hidden, states, rows, cu, produces, t0)
+                return self._checked(self._pool(hidden, states, rows, cu, produces, t0))
             if has_spec:
-                return self._verify_spec(so, hidden, states, rows, ns, cu, t0)
+                return self._checked(self._verify_spec(so, hidden, states, rows, ns, cu, t0))
             last_idx = torch.from_numpy(cu[1:].astype(np.int64) - 1).to(self.device, non_blocking=True)
             if getattr(self.drafter, "needs_step_hidden", False):
                 # EAGLE / MTP heads consume the target hidden state of every position computed this step
@@ -1206,6 +1213,18 @@ class ModelRunner:
         return out.get()
 
     # ------------------------------------------------------------- helpers
+    def check_kernels(self) -> None:
+        """Raise if a kernel gave up on a wait; complete for steps whose results are on the host."""
+        if self.kernel_error is not None and self.kernel_error[0]:
+            from vllm_b200.ops.cuda import KERNEL_GAVE_UP
+            self.kernel_error[0] = 0
+            raise RuntimeError(KERNEL_GAVE_UP)
+
+    def _checked(self, out):
+        """``out``, which holds results that were read back."""
+        self.check_kernels()
+        return out
+
     @staticmethod
     def _cu_ops():
         from vllm_b200.ops import cuda_ops
