@@ -31,6 +31,7 @@ import torch
 import torch.nn as nn
 
 from vllm_b200 import ops
+from vllm_b200.config import get_current_vllm_config_or_none
 from vllm_b200.forward_context import AttentionMetadata, get_forward_context
 from vllm_b200.layers.attention import MLAAttentionCore
 from vllm_b200.layers.common import RMSNorm
@@ -42,8 +43,23 @@ from vllm_b200.parallel.utils import divide
 # portions of at most this many tokens attend in the latent space, one row per token: re-reading the context that often is
 # still cheaper than writing its keys and values out
 ABSORB_MAX_TOKENS = 16
-# bytes of expanded keys and values held at a time; a longer context is done a few heads at a time
+# bytes of expanded keys and values held at a time (a longer context is done a few heads at a time), and of the latent rows that they come
+# from (more contexts are done a few requests at a time)
 EXPAND_BYTES = 1 << 30
+
+
+@dataclass
+class Contexts:
+    """Contexts of some requests of a step, expanded together: one entry per request."""
+    block_table: torch.Tensor
+    q_start: torch.Tensor
+    q_len: torch.Tensor
+    seq_len: torch.Tensor      # keys of each request that some row of its portion sees
+    kv_first: Optional[torch.Tensor]    # position of the first of them (None: all start at 0)
+    cu_kv: torch.Tensor        # [n + 1] key rows before each request
+    num_kv: int
+    max_q: int
+    max_kv: int
 
 
 @dataclass
@@ -54,26 +70,20 @@ class LatentPlan:
     row_seq_lens: Optional[torch.Tensor] = None
     num_rows: int = 0
     max_row_len: int = 0
-    block_table: Optional[torch.Tensor] = None  # expanded: one entry per request
-    q_start: Optional[torch.Tensor] = None
-    q_len: Optional[torch.Tensor] = None
-    seq_len: Optional[torch.Tensor] = None     # keys of each request that some row of its portion sees
-    kv_first: Optional[torch.Tensor] = None    # position of the first of them (None: all start at 0)
-    cu_kv: Optional[torch.Tensor] = None       # [n + 1] key rows before each request
-    num_kv: int = 0
-    max_q: int = 0
-    max_kv: int = 0
+    contexts: tuple[Contexts, ...] = ()        # expanded
 
     @classmethod
-    def of(cls, md: AttentionMetadata, device: torch.device, window: int, apart: int = 1) -> "LatentPlan":
+    def of(cls, md: AttentionMetadata, device: torch.device, window: int, apart: int, most: int) -> "LatentPlan":
         plans = md.latent_plan = md.latent_plan if md.latent_plan is not None else {}
-        if (window, apart) not in plans:
-            plans[window, apart] = cls.build(md, device, window, apart)
-        return plans[window, apart]
+        key = window, apart, most
+        if key not in plans:
+            plans[key] = cls.build(md, device, *key)
+        return plans[key]
 
     @classmethod
-    def build(cls, md: AttentionMetadata, device: torch.device, window: int = 0, apart: int = 1) -> "LatentPlan":
-        """``apart``: key rows of a request start at multiples of it."""
+    def build(cls, md: AttentionMetadata, device: torch.device, window: int = 0, apart: int = 1, most: int = 1 << 62) -> "LatentPlan":
+        """``apart``: key rows of a request start at multiples of it.  ``most``: key rows of requests that are expanded together (one request
+        may have more)."""
         if md.host_lens is not None:
             cu, sl = md.host_lens
         else:
@@ -91,27 +101,48 @@ class LatentPlan:
         vis = sl[req] - ql[req] + off + 1
         kv_first = np.maximum(sl[long] - ql[long] + 1 - window, 0) if window else np.zeros(n, dtype=np.int64)
         kl = sl[long] - kv_first
-        cu_kv = np.concatenate([[0], np.cumsum(-(-kl // apart) * apart)])
-        parts = [cu[req] + off, req, vis, long, cu[long], ql[long], kl, kv_first, cu_kv]
+        rows_kv = -(-kl // apart) * apart
+        parts = [cu[req] + off, req, vis]
+        groups = grouped(rows_kv, most)
+        for i, j in groups:
+            parts += [long[i:j], cu[long[i:j]], ql[long[i:j]], kl[i:j], kv_first[i:j], np.concatenate([[0], np.cumsum(rows_kv[i:j])])]
         packed = torch.from_numpy(np.concatenate(parts).astype(np.int32)).to(device, non_blocking=True)
-        rows, req_t, vis_t, long_t, q_start, q_len, seq_len, first_t, cu_t = packed.split([len(p) for p in parts])
+        rows, req_t, vis_t, *rest = packed.split([len(p) for p in parts])
         plan = cls(num_rows=n_rows)
         if n_rows:
             plan.rows = rows.long() if n else None
             plan.row_block_table = md.block_table.index_select(0, req_t)
             plan.row_seq_lens = vis_t
             plan.max_row_len = int(vis.max())
-        if n:
-            plan.block_table = md.block_table.index_select(0, long_t)
-            plan.q_start, plan.q_len, plan.seq_len, plan.cu_kv = q_start, q_len, seq_len, cu_t
-            plan.kv_first = first_t if kv_first.any() else None
-            plan.num_kv, plan.max_q, plan.max_kv = int(cu_kv[-1]), int(ql[long].max()), int((cu_kv[1:] - cu_kv[:-1]).max())
+        contexts = []
+        for g, (i, j) in enumerate(groups):
+            long_t, q_start, q_len, seq_len, first_t, cu_t = rest[6 * g:6 * g + 6]
+            contexts.append(Contexts(md.block_table.index_select(0, long_t), q_start, q_len, seq_len, first_t if kv_first[i:j].any() else None, cu_t,
+                                     int(rows_kv[i:j].sum()), int(ql[long[i:j]].max()), int(rows_kv[i:j].max())))
+        plan.contexts = tuple(contexts)
         return plan
+
+
+def grouped(sizes, most: int) -> list[tuple[int, int]]:
+    """Ranges of neighbours whose sizes add up to at most ``most``, or that are one."""
+    out, i, total = [], 0, 0
+    for j, n in enumerate(int(n) for n in sizes):
+        if j > i and total + n > most:
+            out.append((i, j))
+            i, total = j, 0
+        total += n
+    return out + [(i, len(sizes))] if len(sizes) else out
+
+
+def step_limits():
+    """The scheduler configuration of the model that is being built, if there is one."""
+    vc = get_current_vllm_config_or_none()
+    return None if vc is None else vc.scheduler_config
 
 
 class LatentForms:
     """The two forms over a layer's attributes ``attn`` (its ``MLAAttentionCore``), ``heads``, ``dim``, ``rot``, ``v_dim``, ``kv_rank``, ``scale``,
-    ``window``, and ``_up()``, ``_expand(c, h0, h1)``."""
+    ``window``, ``limits`` (``step_limits()``), and ``_up()``, ``_expand(c, h0, h1)``."""
     # keys of a request start on a boundary of the prompt kernel's key tiles, zeros fill the gap: no tile holds two requests' values
     kv_apart = 1
     # softmax weights keep 16 more bits in steps that are not decode steps alone
@@ -123,7 +154,7 @@ class LatentForms:
         window = self.window or None
         if md.decode_only or not ops.latent_expand_ok(q, self.dim, self.rot, self.v_dim, self.kv_rank):
             return self._absorbed(q, out, lambda q_abs, q_pe: ops.mla_attention(q_abs, q_pe, cache, md, self.scale, self.kv_rank, window))
-        plan = LatentPlan.of(md, q.device, self.window, self.kv_apart)
+        plan = LatentPlan.of(md, q.device, self.window, self.kv_apart, self._most_rows(q.element_size()))
         if plan.num_rows:
             def attend(q_abs, q_pe):
                 return ops.mla_attention_rows(q_abs, q_pe, cache, plan.row_block_table, plan.row_seq_lens, plan.max_row_len,
@@ -132,7 +163,8 @@ class LatentForms:
                 return self._absorbed(q, out, attend)
             part = torch.empty(plan.num_rows, self.heads, self.v_dim, dtype=q.dtype, device=q.device)
             out.index_copy_(0, plan.rows, self._absorbed(q.index_select(0, plan.rows), part, attend))
-        self._expanded(q, out, plan, cache)
+        for contexts in plan.contexts:
+            self._expanded(q, out, contexts, cache, self.shares_rows and len(plan.contexts) == 1)
         return out
 
     def _absorbed(self, q: torch.Tensor, out: torch.Tensor, attend) -> torch.Tensor:
@@ -142,23 +174,42 @@ class LatentForms:
         torch.bmm(o_lat.transpose(0, 1), w_uv.transpose(1, 2), out=out.transpose(0, 1))
         return out
 
-    def _expanded(self, q: torch.Tensor, out: torch.Tensor, plan: LatentPlan, cache: torch.Tensor) -> None:
+    def _expanded(self, q: torch.Tensor, out: torch.Tensor, c: Contexts, cache: torch.Tensor, share: bool) -> None:
         # layers that share a cache (and see as much of it) share the gathered rows too
-        gathered = get_forward_context().extra.setdefault("latent_rows", {})
+        gathered = get_forward_context().extra.setdefault("latent_rows", {}) if share else {}
         key = self.attn.cache_name, self.window
         rows = gathered.get(key)
         if rows is None:
-            rows = ops.gather_latents(cache, plan.block_table, plan.cu_kv, plan.num_kv, plan.max_kv, plan.kv_first,
-                                      plan.seq_len if self.kv_apart > 1 else None)
-            if self.shares_rows:
-                gathered[key] = rows
-        per_head = plan.num_kv * (self.dim + self.v_dim) * q.element_size()
-        step = max(1, min(self.heads, EXPAND_BYTES // max(per_head, 1)))
+            rows = gathered[key] = ops.gather_latents(cache, c.block_table, c.cu_kv, c.num_kv, c.max_kv, c.kv_first,
+                                                      c.seq_len if self.kv_apart > 1 else None)
+        step = self._heads_at_a_time(c.num_kv, q.element_size())
         for h0 in range(0, self.heads, step):
             h1 = min(self.heads, h0 + step)
             k, v = self._expand(rows[:, :self.kv_rank], h0, h1)
-            ops.mla_prefill(q, k, v, out, plan.q_start, plan.q_len, plan.seq_len, plan.cu_kv, h0, plan.max_q, self.scale,
+            ops.mla_prefill(q, k, v, out, c.q_start, c.q_len, c.seq_len, c.cu_kv, h0, c.max_q, self.scale,
                             rows[:, self.kv_rank:] if self.rot else None, self.window, self.wide_weights)
+
+    def _most_rows(self, itemsize: int) -> int:
+        return EXPAND_BYTES // ((self.kv_rank + self.rot) * itemsize)
+
+    def _heads_at_a_time(self, num_kv: int, itemsize: int) -> int:
+        return max(1, min(self.heads, EXPAND_BYTES // max(num_kv * (self.dim + self.v_dim) * itemsize, 1)))
+
+    def expanded_bytes(self, requests: int, tokens: int, length: int, itemsize: int) -> int:
+        """The most that a step of so many requests and tokens holds of latent rows, keys and values, its contexts ``length`` tokens long at
+        most."""
+        one = min(length, self.window + tokens) if self.window else length
+        one = -(-one // self.kv_apart) * self.kv_apart
+        rows = min(min(requests, tokens // (ABSORB_MAX_TOKENS + 1)) * one, max(self._most_rows(itemsize), one))
+        per_head = rows * (self.dim + self.v_dim) * itemsize
+        return rows * (self.kv_rank + self.rot) * itemsize + max(per_head, min(EXPAND_BYTES, self.heads * per_head))
+
+    def _hold_expanded(self, q: torch.Tensor) -> None:
+        """Memory-profiling run: holds for a moment what a step may take."""
+        sc = self.limits
+        if sc is not None and ops.latent_expand_ok(q, self.dim, self.rot, self.v_dim, self.kv_rank):
+            torch.empty(self.expanded_bytes(sc.max_num_seqs, sc.max_num_batched_tokens, sc.max_model_len, q.element_size()), dtype=torch.uint8,
+                        device=q.device)
 
 
 class LatentAttention(LatentForms, nn.Module):
@@ -177,7 +228,7 @@ class LatentAttention(LatentForms, nn.Module):
         self.heads = divide(num_heads, get_tp_group().world_size)
         self.dim, self.v_dim, self.q_rank, self.kv_rank = dim, v_dim, q_rank, kv_rank
         self.rope, self.rot, self.window = rope, 0 if rope is None else rope.rotary_dim, window
-        self.scale, self.eps = float(scale), eps
+        self.scale, self.eps, self.limits = float(scale), eps, step_limits()
         self.owns_latent = kv_sharing_target is None
         self.kv_norm = RMSNorm(kv_rank, eps, dtype) if self.owns_latent else None
         if q_rank:
@@ -237,9 +288,7 @@ class LatentAttention(LatentForms, nn.Module):
             gate = parts[self.part["g"]] if "g" in self.part else None
             c_kv = parts[self.part["kv"]][:, :self.kv_rank] if own else None
         if md is None:
-            # memory-profiling run: hold what expanding a batch of prompts would
-            if c_kv is not None:
-                self.ukv(c_kv)
+            self._hold_expanded(q)
             return self.o(q.new_zeros(T, self.heads * self.v_dim))
         o = self._attend(q, md, cache).view(T, self.heads * self.v_dim)
         return self.o(o if gate is None else ops.sigmoid_mul_(o, gate))

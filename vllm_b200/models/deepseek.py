@@ -20,7 +20,7 @@ from vllm_b200 import envs, ops
 from vllm_b200.config import VllmConfig
 from vllm_b200.layers.attention import MLAAttentionCore
 from vllm_b200.layers.common import RMSNorm
-from vllm_b200.layers.latent import LatentForms
+from vllm_b200.layers.latent import LatentForms, step_limits
 from vllm_b200.layers.linear import (ColumnParallelLinear, ReplicatedLinear, RowParallelLinear,
                                      tp_reduce_residual_norm)
 from vllm_b200.layers.moe import FusedMoE
@@ -71,7 +71,7 @@ class DeepseekMLA(LatentForms, nn.Module):
         self.attn = MLAAttentionCore(self.local_heads, self.kv_lora, self.rope_dim, scale, prefix=f"{prefix}.attn")
         # what the two forms of the attention read
         self.heads, self.dim, self.rot, self.kv_rank = self.local_heads, self.nope, self.rope_dim, self.kv_lora
-        self.scale, self.window = scale, 0
+        self.scale, self.window, self.limits = scale, 0, step_limits()
 
     def _up(self) -> tuple[torch.Tensor, torch.Tensor]:
         """(W_uk [h, nope, R], W_uv [h, v, R]): views of the stacked weight."""
@@ -109,8 +109,8 @@ class DeepseekMLA(LatentForms, nn.Module):
         k_pe = lat[:, self.kv_lora:].contiguous()
         q_pe, k_pe = self.rope(positions, q_pe.reshape(T, -1).contiguous(), k_pe)
         q_pe = q_pe.view(T, self.local_heads, self.rope_dim)
-        if md is None:
-            self._expand(kv_c, 0, self.local_heads)      # memory-profiling run: hold what expanding a batch of prompts would
+        if md is None and get_dcp_group().world_size == 1 and not (q.is_cuda and ops.cuda_ops().batch_invariant()):
+            self._hold_expanded(q)
         w_uk, w_uv = self._up()
         q_abs = torch.einsum("thn,hnr->thr", q_nope, w_uk)
         o_lat = self.attn(q_abs, q_pe, kv_c, k_pe)                           # [T, h, R]
