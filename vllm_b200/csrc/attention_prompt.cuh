@@ -87,24 +87,43 @@ template <int KS, int VS> struct Bars {
   }
 };
 
-// A tile of keys is multiplied whole, and a weight of 0 keeps neither an infinity nor a NaN out of a sum, but slots that no row sees (behind a
-// sequence's end, in front of a window) may hold values of another request.  Where a tile has such slots its values arrive at a barrier of
-// their own, 64 threads that have nothing else to do overwrite the slots with zeros and pass the tile on.  (In the softmax threads
-// the same took 549 → 594 us for 32 / 8 heads, 4 x 3800 tokens, by the registers it needs.)
-// Row r of a block of 64 tokens per 128-byte swizzled row: tokens [lo, hi) stay.
-VB_DEVICE void clear_tokens(unsigned char* block, int r, int lo, int hi) {
-#pragma unroll 1
-  for (int c = 0; c < 8; ++c) {
-    const int a = lo - c * 8, b = hi - c * 8;
-    if (a <= 0 && b >= 8) continue;
-    uint4* p = reinterpret_cast<uint4*>(block + r * 128 + ((c ^ (r & 7)) << 4));
-    if (a >= 8 || b <= 0) {
-      *p = make_uint4(0, 0, 0, 0);
-    } else {
-      for (int i = 0; i < 8; ++i)
-        if (i < a || i >= b) reinterpret_cast<uint16_t*>(p)[i] = 0;
+// A weight of 0 keeps neither an infinity nor a NaN out of a sum, but the slots of a key tile that no row sees (behind a sequence's end, in front
+// of a window) may hold values of another request.  The products leave out the groups of 16 slots (an MMA's depth) that nobody sees; where
+// a part of a group is seen, the rest of it is overwritten with zeros before the product.  In prompts such a tile's values arrive at a
+// barrier of their own and two idle warps clear and pass them on (in the softmax warps: 549 → 594 us for 32 / 8 heads, 4 x 3800 tokens, by the
+// registers); in decode steps the softmax warps do it last, where the product waits for the values as well.  us without and so: 32 / 8
+// heads, 4 x 3800 tokens 553 and 534 (no clearing of shared memory at the start), decode 24 x 500 11.6 and 11.6, 64 x 280 16.7 and
+// 17.9, 64 x 288 16.7 and 16.5, 64 x 1000 46.3 and 46.6.
+// Tokens [lo, hi) of the tile are seen, of `keys`.
+struct Seen {
+  int lo, hi;
+  VB_DEVICE Seen(int first, int begin, int end, int keys) : lo(max(begin - first, 0)), hi(min(end - first, keys)) {}
+  VB_DEVICE bool cut() const { return ((lo | hi) & 15) != 0; }
+  VB_DEVICE int k0() const { return lo >> 4; }
+  VB_DEVICE int k1() const { return (hi + 15) >> 4; }
+};
+// Row r of blocks of 64 tokens per 128-byte swizzled row, `stride` bytes apart: tokens [lo, hi), all of one group of 16, become zeros.
+VB_DEVICE void clear_group(unsigned char* blocks, int stride, int r, int lo, int hi) {
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int c = (lo >> 4) * 2 + e, a = lo - c * 8, b = hi - c * 8;        // 16 bytes: 8 tokens
+    if (a >= 8 || b <= 0) continue;
+    uint4* p = reinterpret_cast<uint4*>(blocks + (c >> 3) * stride + r * 128 + (((c & 7) ^ (r & 7)) << 4));
+    if (a <= 0 && b >= 8) { *p = make_uint4(0, 0, 0, 0); continue; }
+    uint4 v = *p;
+    uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (2 * i >= a && 2 * i < b) w[i] &= 0xffff0000u;
+      if (2 * i + 1 >= a && 2 * i + 1 < b) w[i] &= 0x0000ffffu;
     }
+    *p = make_uint4(w[0], w[1], w[2], w[3]);
   }
+}
+// what is not seen of the groups that are seen in part, in row r
+VB_DEVICE void clear_cut(unsigned char* blocks, int stride, int r, const Seen& s) {
+  if (s.lo & 15) clear_group(blocks, stride, r, s.lo & ~15, s.lo);
+  if (s.hi & 15) clear_group(blocks, stride, r, s.hi, (s.hi + 15) & ~15);
 }
 VB_DEVICE void pass_on(uint64_t* v_full) {
   fence_proxy_async();
@@ -112,7 +131,7 @@ VB_DEVICE void pass_on(uint64_t* v_full) {
   if ((threadIdx.x & 63) == 0) mbar_arrive(v_full);
 }
 
-// MMA issuer (one warp).  qk(t, stage) issues S_t, pv(t, stage, first) issues O_t.  n >= 1 key tiles, each for both of two query tiles
+// MMA issuer (one warp).  qk(t, stage) issues S_t, pv(t, stage, key tile, first) issues O_t.  n >= 1 key tiles, each for both of two query tiles
 // (`pair`), or the even ones for t = 0 and the odd ones for t = 1.
 template <int KS, int VS, class QK, class PV>
 VB_DEVICE void mma_role(Bars<KS, VS>& b, int n, bool pair, int& budget, QK qk, PV pv) {
@@ -138,7 +157,7 @@ VB_DEVICE void mma_role(Bars<KS, VS>& b, int n, bool pair, int& budget, QK qk, P
       tc_fence_after();
       __syncwarp();
       {
-        pv(t, vs, pair ? j == 0 : j < 2);
+        pv(t, vs, j, pair ? j == 0 : j < 2);
         if (t == t1) warp_umma_commit(&b.v_empty[vs]);
         if (nx >= n) warp_umma_commit(&b.o_done[t]);
       }
@@ -168,12 +187,11 @@ VB_DEVICE float cap_small(float x, float c2) {
   r = fmaf(r, z, 0.13325075805187225f);
   r = fmaf(r, z, -0.3333282768726349f);
   r = fmaf(r, z, 0.9999999403953552f);
-  return r * x * c2;                          // (as cap_any rounds it: a score's value does not depend on its warp's others)
+  return r * (x * c2);
 }
 VB_DEVICE float cap_any(float x, float c2) {
   const float e = ex2(fabsf(x) * 2.8853900817779268f);          // e^(2 |x|), at worst infinite: 1 - 0
-  const float y = fabsf(x) <= 1.f ? fabsf(cap_small(x, 1.f)) : 1.f - 2.f / (e + 1.f);
-  return copysignf(y, x) * c2;
+  return fabsf(x) <= 1.f ? cap_small(x, c2) : copysignf(1.f - 2.f / (e + 1.f), x) * c2;      // (no matter which of the two a warp takes)
 }
 
 struct Softmax {
@@ -331,13 +349,22 @@ VB_DEVICE void load_o(uint32_t t_o, int c, bool shared, float f0, float f1, uint
   }
 }
 
-// O_t += P_t V: db(kk) is the descriptor of 16 keys of the values
-template <class DB> VB_DEVICE void issue_pv(uint32_t tmem_o, uint32_t tmem_p, uint32_t idesc, bool first, bool split, DB db) {
+// O_t += P_t V: db(kk) is the descriptor of 16 keys of the values; groups k0 .. k1 - 1 of 16 keys
+template <class DB> VB_DEVICE void issue_pv(uint32_t tmem_o, uint32_t tmem_p, uint32_t idesc, bool first, bool split, int k0, int k1, DB db) {
+  if (k0 == 0 && k1 == KEYS / 16) {
 #pragma unroll
-  for (int kk = 0; kk < KEYS / 16; ++kk) warp_umma_f16_ta(tmem_o, tmem_p + kk * 8, db(kk), idesc, !first || kk != 0);
-  if (split) {
+    for (int kk = 0; kk < KEYS / 16; ++kk) warp_umma_f16_ta(tmem_o, tmem_p + kk * 8, db(kk), idesc, !first || kk != 0);
+    if (split) {
 #pragma unroll
-    for (int kk = 0; kk < KEYS / 16; ++kk) warp_umma_f16_ta(tmem_o, tmem_p + KEYS / 2 + kk * 8, db(kk), idesc, 1);
+      for (int kk = 0; kk < KEYS / 16; ++kk) warp_umma_f16_ta(tmem_o, tmem_p + KEYS / 2 + kk * 8, db(kk), idesc, 1);
+    }
+  } else {
+#pragma unroll 1
+    for (int kk = k0; kk < k1; ++kk) warp_umma_f16_ta(tmem_o, tmem_p + kk * 8, db(kk), idesc, !first || kk != k0);
+    if (split) {
+#pragma unroll 1
+      for (int kk = k0; kk < k1; ++kk) warp_umma_f16_ta(tmem_o, tmem_p + KEYS / 2 + kk * 8, db(kk), idesc, 1);
+    }
   }
 }
 

@@ -151,8 +151,7 @@ fmha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // does key tile j (the first or the last) hold slots that are not this sequence's, or that no row sees?
-  auto edge = [&](int j) { return kv_begin > (tile_lo + j) * TILE_N || kv_end < (tile_lo + j + 1) * TILE_N; };
+  auto seen = [&](int j) { return prompt::Seen((tile_lo + j) * TILE_N, kv_begin, kv_end, TILE_N); };   // cut: the first or the last key tile
 
   if (warp < 4) {
     prompt::regs_dec<prompt::REGS_AUX>();
@@ -186,7 +185,7 @@ fmha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
         }
         mbar_wait_lim(&bars.v_empty[s], par, budget);
         if (budget < 0) break;
-        uint64_t* v_bar = edge(j) ? &bars.edge[j != 0] : &bars.v_full[s];
+        uint64_t* v_bar = seen(j).cut() ? &bars.edge[j != 0] : &bars.v_full[s];
         mbar_expect_tx(v_bar, n_valid * BS * D * 2);
         for (int u = 0; u < 2; ++u) {
           if (blk[u] < 0) continue;
@@ -211,19 +210,18 @@ fmha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ 
               warp_umma_f16(tmem_base + t * 128, d_q + (uint64_t)((qt * Q_BYTES + kb * BLK + k * 32) >> 4),
                        d_k + (uint64_t)((s * K_BYTES + kb * BLK + k * 32) >> 4), idesc, (kb | k) != 0);
         },
-        [&](int t, int s, bool first) {
-          prompt::issue_pv(tmem_base + 256 + t * 128, tmem_base + t * 128, idesc, first, CAP,
+        [&](int t, int s, int j, bool first) {
+          const prompt::Seen k = seen(j);
+          prompt::issue_pv(tmem_base + 256 + t * 128, tmem_base + t * 128, idesc, first, CAP, k.k0(), k.k1(),
                            [&](int kk) { return d_v + (uint64_t)((s * V_BYTES + (kk / 4) * BLK + (kk & 3) * 32) >> 4); });
         });
     } else if (warp >= 2) {
       // ===== zeros into the values' slots that no row sees
       for (int e = 0; e < 2; ++e) {
-        const int j = e ? n_tiles - 1 : 0, s = j % KV_STAGES, k0 = (tile_lo + j) * TILE_N;
-        if ((e && n_tiles == 1) || !edge(j)) continue;
+        const int j = e ? n_tiles - 1 : 0, s = j % KV_STAGES;
+        if ((e && n_tiles == 1) || !seen(j).cut()) continue;
         mbar_wait_lim(&bars.edge[e], 0, budget);
-        for (int i = 0; i < 4; ++i)                // two pages, two rows of 64 threads each
-          prompt::clear_tokens(v_smem + s * V_BYTES + (i & 1) * BLK, (threadIdx.x & 63) + (i >> 1) * 64, kv_begin - k0 - (i & 1) * BS,
-                               kv_end - k0 - (i & 1) * BS);
+        for (int r = threadIdx.x & 63; r < 128; r += 64) prompt::clear_cut(v_smem + s * V_BYTES, BLK, r, seen(j));
         prompt::pass_on(&bars.v_full[s]);
       }
     }

@@ -18,7 +18,7 @@
 namespace fmha_dec {
 
 constexpr int D = 128, BS = 64, TILE = 128, NQ = 16;
-constexpr int NUM_THREADS = 256;   // warp 0 TMA producer, 1 MMA issuer, 2..5 softmax, 6 and 7 clear values
+constexpr int NUM_THREADS = 192;
 constexpr int STAGES = 3;
 constexpr int K_BYTES = TILE * D * 2;   // 32 KB: 2 k-blocks (dims 0-63 / 64-127) of [128 tokens x 64]
 constexpr int V_BYTES = D * TILE * 2;   // 32 KB: 2 pages of [128 dims x 64 tokens]
@@ -73,8 +73,7 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   uint64_t* s_empty = s_full + 2;          // [2]
   uint64_t* p_full = s_empty + 2;
   uint64_t* pv_done = p_full + 1;
-  uint64_t* edge_full = pv_done + 1;       // [STAGES] values of a tile that is cleared before the product (attention_prompt.cuh)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(edge_full + STAGES);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 1);
   float* wred = reinterpret_cast<float*>(tmem_slot + 2);        // [4 warps][NQ] column max / sum exchange
   int* blk_ids = reinterpret_cast<int*>(wred + 4 * NQ);         // [2 * MAX_TILES_SMEM] (producer warp only)
 
@@ -86,7 +85,7 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmap_q); tma_prefetch_desc(&tmap_k); tma_prefetch_desc(&tmap_v);
     for (int s = 0; s < 2; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1); }
-    for (int s = 0; s < STAGES; ++s) { mbar_init(&k_full[s], 1); mbar_init(&v_full[s], 1); mbar_init(&kv_empty[s], 1); mbar_init(&edge_full[s], 1); }
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&k_full[s], 1); mbar_init(&v_full[s], 1); mbar_init(&kv_empty[s], 1); }
     for (int s = 0; s < 2; ++s) { mbar_init(&s_full[s], 1); mbar_init(&s_empty[s], 128); }
     mbar_init(p_full, 128);
     mbar_init(pv_done, 1);
@@ -125,9 +124,6 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     return max(tile_hi - tile_lo, 0);
   };
 
-  // does key tile `tile` hold slots that are not the sequence's, or that its query does not see?
-  auto is_edge = [](int tile, int kv_begin, int kv_end) { return kv_begin > tile * TILE || kv_end < (tile + 1) * TILE; };
-
   if (warp == 0) {
     // ===== TMA producer (the whole warp stages the item's block ids, lane 0 issues the copies)
     int gt = 0, qi = 0;
@@ -164,8 +160,7 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
           unsigned char* ks = k_smem + s * K_BYTES;
           unsigned char* vs = v_smem + s * V_BYTES;
           mbar_expect_tx(&k_full[s], n_valid * BS * D * 2);
-          uint64_t* v_bar = is_edge(tile_lo + j, kv_begin, kv_end) ? &edge_full[s] : &v_full[s];
-          mbar_expect_tx(v_bar, n_valid * BS * D * 2);
+          mbar_expect_tx(&v_full[s], n_valid * BS * D * 2);
           for (int u = 0; u < 2; ++u) {
             if (blk[u] < 0) continue;
             const int chunk = (blk[u] * 2 + 0) * p.Hkv + h;
@@ -175,7 +170,7 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
           for (int u = 0; u < 2; ++u) {
             if (blk[u] < 0) continue;
             const int chunk = (blk[u] * 2 + 1) * p.Hkv + h;
-            tma_load_2d_hint(vs + u * (D * 128), &tmap_v, 0, chunk * D, v_bar, L2_EVICT_FIRST);
+            tma_load_2d_hint(vs + u * (D * 128), &tmap_v, 0, chunk * D, &v_full[s], L2_EVICT_FIRST);
           }
         }
       }
@@ -222,16 +217,27 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
           __syncwarp();
           {
             const unsigned char* vs = v_smem + s * V_BYTES;
+            const prompt::Seen k16((tile_lo + jj) * TILE, kv_begin, kv_end, TILE);
+            if (k16.k0() == 0 && k16.k1() == TILE / 16) {
 #pragma unroll
-            for (int kb = 0; kb < 2; ++kb) {
-              const uint64_t da = umma_desc_sw128(vs + kb * (D * 128));
-              const uint64_t db = umma_desc_sw128(p_smem + kb * (NQ * 128));
+              for (int kb = 0; kb < 2; ++kb) {
+                const uint64_t da = umma_desc_sw128(vs + kb * (D * 128));
+                const uint64_t db = umma_desc_sw128(p_smem + kb * (NQ * 128));
 #pragma unroll
-              for (int k = 0; k < 4; ++k)
-                warp_umma_f16(tmem_o, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (jj | kb | k) != 0);
-              if (CAP) {
+                for (int k = 0; k < 4; ++k)
+                  warp_umma_f16(tmem_o, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (jj | kb | k) != 0);
+                if (CAP) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) warp_umma_f16(tmem_o, da + (uint64_t)(k * 2), db + (uint64_t)(P_BYTES / 16 + k * 2), idesc, 1);
+                  for (int k = 0; k < 4; ++k) warp_umma_f16(tmem_o, da + (uint64_t)(k * 2), db + (uint64_t)(P_BYTES / 16 + k * 2), idesc, 1);
+                }
+              }
+            } else {
+#pragma unroll 1
+              for (int k = k16.k0(); k < k16.k1(); ++k) {
+                const uint64_t da = umma_desc_sw128(vs + (k >> 2) * (D * 128)) + (uint64_t)((k & 3) * 2);
+                const uint64_t db = umma_desc_sw128(p_smem + (k >> 2) * (NQ * 128)) + (uint64_t)((k & 3) * 2);
+                warp_umma_f16(tmem_o, da, db, idesc, jj > 0 || k > k16.k0());
+                if (CAP) warp_umma_f16(tmem_o, da, db + (uint64_t)(P_BYTES / 16), idesc, 1);
               }
             }
             warp_umma_commit(&kv_empty[s]);
@@ -242,25 +248,6 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       }
       gt += n_tiles;
       ++qi;
-    }
-  } else if (warp >= 6) {
-    // ===== zeros into the values' slots that are not the sequence's
-    int gt = 0;
-    uint32_t phase = 0;                      // bit s: parity of the barrier's next phase
-    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
-      int split, h, b, tile_lo, kv_begin, kv_end;
-      const int n_tiles = item_range(it, split, h, b, tile_lo, kv_begin, kv_end);
-      for (int e = 0; e < 2; ++e) {          // the first and the last tile
-        const int j = e ? n_tiles - 1 : 0, s = (gt + j) % STAGES, k0 = (tile_lo + j) * TILE;
-        if (n_tiles <= e || !is_edge(tile_lo + j, kv_begin, kv_end)) continue;
-        mbar_wait(&edge_full[s], (phase >> s) & 1);
-        phase ^= 1u << s;
-        for (int i = 0; i < 4; ++i)          // two pages, two rows of 64 threads each
-          prompt::clear_tokens(v_smem + s * V_BYTES + (i & 1) * (D * 128), (threadIdx.x & 63) + (i >> 1) * 64, kv_begin - k0 - (i & 1) * BS,
-                               kv_end - k0 - (i & 1) * BS);
-        prompt::pass_on(&v_full[s]);
-      }
-      gt += n_tiles;
     }
   } else {
     // ===== softmax: thread = kv token of the tile (TMEM lane); later thread = output dim
@@ -341,6 +328,11 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
           const T hi = from_f32<T>(pe);
           *reinterpret_cast<T*>(pcol + g * 128 + ((chunk ^ (g & 7)) << 4)) = hi;
           if (CAP) *reinterpret_cast<T*>(pcol + P_BYTES + g * 128 + ((chunk ^ (g & 7)) << 4)) = from_f32<T>(pe - to_f32(hi));
+        }
+        const prompt::Seen seen((tile_lo + j) * TILE, kv_begin, kv_end, TILE);
+        if (seen.cut()) {                           // (here, as the product waits for the values too; the scores are there, so the stage's barrier
+          mbar_wait(&v_full[gj % STAGES], (gj / STAGES) & 1);      // is at this tile's)
+          prompt::clear_cut(v_smem + (gj % STAGES) * V_BYTES, D * 128, t, seen);
         }
         tc_fence_before();
         fence_proxy_async();

@@ -149,8 +149,8 @@ mla_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 warp_umma_f16(tmem_base + t * 128, d_q + (uint64_t)(((qt * NQ + kb) * BLK + k * 32) >> 4),
                          d_k + (uint64_t)(((s * NQ + kb) * BLK + k * 32) >> 4), idesc_s, (kb | k) != 0);
           },
-          [&](int t, int s, bool first) {                   // 16 keys per MMA: 16 rows of 128 bytes of V
-            prompt::issue_pv(tmem_base + 256 + t * 128, tmem_base + t * 128, idesc_o, first, split,
+          [&](int t, int s, int, bool first) {              // 16 keys per MMA: 16 rows of 128 bytes of V
+            prompt::issue_pv(tmem_base + 256 + t * 128, tmem_base + t * 128, idesc_o, first, split, 0, TN / 16,
                              [&](int kk) { return d_v + (uint64_t)((s * NV * BLK + kk * 2048) >> 4); });
           });
     }
