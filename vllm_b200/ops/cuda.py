@@ -784,11 +784,14 @@ def select_candidates(cands: torch.Tensor, W: int, out: torch.Tensor) -> torch.T
 
 
 _logprobs = _sig("vb_logprobs", _vp, _i64, _i, _i, _vp, _i, _vp, _i, _vp)
-MAX_LOGPROBS = 64       # likeliest tokens that the one-launch kernel picks one by one; more are sorted
+# The one-launch kernel picks the k likeliest tokens of V one by one, each at the price of a part of a pass over the row; the library's sort does not
+# grow with k.  us for a row, kernel and library: V 32000, k 5: 21 and 136, k 64: 139 and 137; V 128256, k 20: 137 and 186, k 32: 207 and 186; V
+# 256000, k 5: 96 and 214, k 10: 162 and 211, k 20: 291 and 211 (more rows: the same kernel time up to 64, the library's grows).
+MAX_LOGPROBS, MAX_LOGPROBS_WORK = 64, 3_000_000
 
 
 def logprobs_ok(V: int, k: int) -> bool:
-    return 0 <= k <= min(MAX_LOGPROBS, V)
+    return 0 <= k <= min(MAX_LOGPROBS, V) and k * V <= MAX_LOGPROBS_WORK
 
 
 def logprobs(logits, sampled, k: int) -> torch.Tensor:
