@@ -240,6 +240,7 @@ __global__ void concat_cache_mla_kernel(const T* __restrict__ kv_c, const T* __r
 // Tokens from which values are turned in tiles: batches larger than any decode step, whose slots mostly follow one another.  32 / 8 heads of 128,
 // 7600 tokens: 100 us with 2-byte stores, 66 us so; decode steps, whose slots lie apart, gain nothing and keep the one pass.
 constexpr int TURN_MIN_TOKENS = 257;
+EXPORT int vb_turn_min_tokens() { return TURN_MIN_TOKENS; }
 
 // q may be null (cache write only, rot = 0); kv_cache may be null (rope only).  v_cos_sin [positions, D] (optional): values are rotated on
 // their way into the cache.

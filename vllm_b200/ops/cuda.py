@@ -10,6 +10,7 @@ that defines it is compiled then, by itself: a process compiles the kernels its 
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from typing import Optional
 
@@ -1599,7 +1600,13 @@ _qknorm_rope_row = _sig("vb_qknorm_rope_row", _vp, _vp, _vp, _vp, _vp, _vp, _vp,
 
 
 _values_turned = _sig("vb_cache_values_turned", _vp, _i64, _vp, _vp, _i, _i, _i, _i, _i, _vp)
-TURN_MIN_TOKENS = 257       # as in csrc/rope_cache.cu
+_turn_min_tokens = _sig("vb_turn_min_tokens")
+
+
+@functools.lru_cache(maxsize=None)
+def turn_min_tokens() -> int:
+    """Tokens from which values are turned in tiles (csrc/rope_cache.cu)."""
+    return _turn_min_tokens()
 
 
 def fused_qk_norm_rope(positions, q, k, q_weight, k_weight, cos_sin_cache, head_dim, eps, is_neox=True, *, v=None,
@@ -1644,7 +1651,7 @@ def fused_qk_norm_rope(positions, q, k, q_weight, k_weight, cos_sin_cache, head_
                                 _p(kv_cache), _p(slot_mapping), BS, int(is_neox), int(gemma), int(vt), eps, _DT[q.dtype], _st()),
                "qknorm_rope_any")
         return q, k
-    if (vt and v is not None and kv_cache is not None and v_cos_sin is None and T >= TURN_MIN_TOKENS and kv_cache.dtype == q.dtype
+    if (vt and v is not None and kv_cache is not None and v_cos_sin is None and T >= turn_min_tokens() and kv_cache.dtype == q.dtype
             and head_dim % 8 == 0 and head_dim <= 512 and v.stride(0) % 8 == 0 and v.data_ptr() % 16 == 0):
         _check(_values_turned(v.data_ptr(), v.stride(0), kv_cache.data_ptr(), slot_mapping.data_ptr(), T, Hkv, head_dim, BS, _DT[q.dtype], _st()),
                "cache_values_turned")
