@@ -150,7 +150,7 @@ def _sentinel_path() -> str:
 
 
 def run_reference(args) -> None:
-    install_note = ("pip install of /root/reference into baseline/_ref is not possible offline: the metadata step needs "
+    install_note = ("pip install of the reference's sources into baseline/_ref is not possible offline: the metadata step needs "
                     "setuptools_rust (no Rust toolchain) and it pins torch==2.13 / flashinfer 0.6.17 vs torch 2.11 in "
                     "this image; see DESIGN.md")
     rank, world = int(os.environ.get("RANK", 0)), int(os.environ.get("WORLD_SIZE", 1))

@@ -14,7 +14,9 @@ sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 
 
 def main() -> None:
-    path = sys.argv[1] if len(sys.argv) > 1 else "/root/reference/vllm/model_executor/models/registry.py"
+    if len(sys.argv) != 2:
+        sys.exit(__doc__)
+    path = sys.argv[1]
     ref = set(re.findall(r'^\s+"(\w+)":\s*\(', open(path).read(), re.M))
     from vllm_b200.models import registry as r
     from vllm_b200.spec_decode import DRAFT_ARCHS

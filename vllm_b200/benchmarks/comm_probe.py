@@ -11,7 +11,7 @@ inside a CUDA graph of ``iters`` back-to-back calls on the live TP communicator,
 max over ranks.  exposed = fused − local per call; × layers = exposed communication per decode step.  The
 roofline of the fused path is the slower of its weight bytes over the measured HBM bandwidth and the bytes it
 moves over NVLink (two-shot: every partial row travels to its owner, the reduced row is multicast back:
-2·T·H·2·(W−1)/W bytes per rank and direction) over the measured 770 GB/s per direction (B200_PROFILING.md).
+2·T·H·2·(W−1)/W bytes per rank and direction) over the measured 770 GB/s per direction.
 """
 from __future__ import annotations
 

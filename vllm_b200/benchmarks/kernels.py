@@ -1,8 +1,8 @@
 """Head-to-head kernel micro-benchmarks on one B200 (tracked; the table it prints lands in profiles/kernels_bench.md).
 
-    python -m vllm_b200.benchmarks.kernels [--out gpurun_out/kernels_bench.md] [--only gemm,fp8,attn,mla,quant]
+    python -m vllm_b200.benchmarks.kernels [--out kernels_bench.md] [--only gemm,fp8,attn,mla,quant]
 
-Method (B200_PROFILING.md): CUDA events on the launching stream, >= 5 warm-up calls, every timed call preceded by a
+Method: CUDA events on the launching stream, >= 5 warm-up calls, every timed call preceded by a
 write of a 256 MB buffer (flushes the 126 MB L2) on the same stream, median of the timed calls; library baselines
 (cuBLASLt through torch, FlashInfer / the stock vLLM wheel's ops when importable) are timed the same way.  Achieved
 bandwidth = algorithmic bytes / time against the measured copy bandwidth of MEASURED_PEAKS.json.
@@ -257,7 +257,7 @@ def bench_quant(rows: list) -> None:
 
 def main() -> None:
     ap = argparse.ArgumentParser()
-    ap.add_argument("--out", default="gpurun_out/kernels_bench.md")
+    ap.add_argument("--out", default="kernels_bench.md")
     ap.add_argument("--only", default="gemm,w4,fp8,attn,mla,quant")
     args = ap.parse_args()
     rows = [f"# Kernel micro-benchmarks on {torch.cuda.get_device_name()} (measured HBM copy {hbm_gbs():.0f} GB/s)"]
