@@ -24,7 +24,7 @@ def test_norm_add_norm(T, H, gemma, dtype):
     w1, w2 = ((torch.randn(H, device="cuda", generator=g) * 0.1 + (0 if gemma else 1)).to(dtype) for _ in range(2))
     s = r.double() + _norm(x.double(), w1.double(), gemma, 1e-6)
     y, r2 = ops.norm_add_norm(x, r, w1, 1e-6, w2, 1e-5, gemma)
-    ulp = 2 ** -9 if dtype == BF else 2 ** -12
+    ulp = 2 ** -9 if dtype == BF else 2 ** -12               # above the 2^-9.35 and 2^-12.35 of a rounding in the 2-norm (test_prompt_attention_gpu.py)
     assert r2 is r and _rel(r, s) < ulp                      # one rounding
     assert _rel(y, _norm(s, w2.double(), gemma, 1e-5)) < 2 * ulp          # of the stream, and its own
 

@@ -28,8 +28,8 @@ def test_grouped_rows(rows, N, K, act, dtype):
     for xe, we in zip(x.split(rows), w):
         h = xe.double() @ we.double().t()
         want.append(h if act is None else fn[act](h[:, :N // 2]) * h[:, N // 2:])
-    # one rounding of the result: at most 2^-9 (bf16) or 2^-12 (fp16) of each value
-    assert _rel(got, torch.cat(want)) < (2 ** -9 if dtype == torch.bfloat16 else 2 ** -11)
+    # one rounding of the result: at most 2^-8 (bf16) or 2^-11 (fp16) of each value, 2^-9.35 or 2^-12.35 in the 2-norm (test_prompt_attention_gpu.py)
+    assert _rel(got, torch.cat(want)) < (2 ** -9 if dtype == torch.bfloat16 else 2 ** -12)
 
 
 @pytest.mark.parametrize("T,E,k", [(300, 8, 4), (600, 4, 2), (2100, 64, 8)])
