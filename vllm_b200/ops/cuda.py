@@ -340,7 +340,7 @@ def batch_invariant() -> bool:
     Reference: vllm/model_executor/layers/batch_invariant.py (``VLLM_BATCH_INVARIANT`` swaps in fixed-reduction-order
     matmul / softmax / rms-norm kernels, fixes the attention split size and pins NCCL to one algorithm :1105-1180),
     tests/v1/determinism/test_batch_invariance.py."""
-    return bool(envs.VLLM_BATCH_INVARIANT)
+    return "VLLM_BATCH_INVARIANT" in os.environ and bool(envs.VLLM_BATCH_INVARIANT)      # (asked for by every norm, seldom set)
 
 
 def decode_splits(B: int, Hkv: int, max_seq_len: int, block_size: int) -> int:
