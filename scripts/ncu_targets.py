@@ -148,3 +148,35 @@ if which in ("talk", "all"):
     lat, out = (torch.randn(8192, 576, device="cuda") * 0.3).to(dt), torch.empty(8192, H, 128, device="cuda", dtype=dt)
     start, lens = torch.arange(0, 8192, 4096, **i32), torch.full((2,), 4096, **i32)
     rep(lambda: cu.mla_prefill(q, k, v, out, start, lens, lens, start, 0, 4096, 0.07, lat[:, 512:], 2048))
+if which in ("prompts", "all"):
+    # prompts of Llama, Gemma-2, DeepSeek, Mixtral and Qwen3-Next layers: attention (capped too), expanded latents, experts, block-scaled fp8, gated delta rule
+    from vllm_b200.benchmarks.kernels import _mk_paged
+    from vllm_b200.forward_context import AttentionMetadata
+    i32 = dict(dtype=torch.int32, device="cuda")
+
+    def prompts(n, q, table):
+        return AttentionMetadata(num_reqs=n, num_actual_tokens=n * q, max_query_len=q, max_seq_len=q, query_start_loc=torch.arange(0, n * q + 1, q, **i32),
+                                 seq_lens=torch.full((n,), q, **i32), block_table=table, slot_mapping=None, decode_only=False)
+    for n, q, Hq, Hkv, cap in ((2, 3800, 32, 8, 0.0), (8, 860, 16, 4, 50.0)):
+        NB, bt, _ = _mk_paged(n, Hkv, 128, 64, q)
+        kv = (torch.randn(NB, 2, Hkv, 64, 128, device="cuda") * 0.3).to(dt)
+        md, x = prompts(n, q, bt), torch.randn(n * q, Hq, 128, device="cuda").to(dt)
+        md.kv_vt = True
+        rep(lambda: cu.paged_attention(x, kv, md, 128 ** -0.5, None, cap))
+    n, q, H = 8, 860, 16
+    x, start, lens = torch.randn(n * q, H, 192, device="cuda").to(dt), torch.arange(0, n * q, q, **i32), torch.full((n,), q, **i32)
+    at, rows = torch.arange(0, n * 896 + 1, 896, **i32), torch.randn(n * 896, 576, device="cuda").to(dt)
+    kv, out = torch.randn(n * 896, H, 256, device="cuda").to(dt), torch.empty(n * q, H, 128, device="cuda", dtype=dt)
+    rep(lambda: cu.mla_prefill(x, kv[..., :128], kv[..., 128:], out, start, lens, lens, at, 0, q, 192 ** -0.5, rows[:, 512:], 0, True))
+    xs, w = torch.randn(13760, 2048, device="cuda", dtype=dt) * 0.1, torch.randn(8, 4096, 2048, device="cuda", dtype=dt) * 0.02
+    offs = torch.arange(0, 13761, 1720, **i32)
+    rep(lambda: cu.gemm_grouped(xs, w, offs, "silu"))
+    wq, ws = ref.block_quant_weight_fp8(torch.randn(28672, 4096, device="cuda") * 0.02, 128)
+    xq, sc = cu.per_token_group_quant_fp8(torch.randn(1000, 4096, device="cuda", dtype=dt) * 0.1, 128, col_major=True)
+    ws = ws.contiguous()
+    rep(lambda: cu.gemm_fp8_block(xq, sc, wq, ws))
+    nh, dk, dv = 8, 128, 256
+    qkv, ba = torch.randn(n * q, nh * (2 * dk + dv), device="cuda"), torch.randn(n * q, 2 * nh, device="cuda").to(dt)
+    pool, A, b = torch.zeros(n + 1, nh * dk * dv, device="cuda"), torch.zeros(nh, device="cuda"), torch.zeros(nh, device="cuda")
+    rep(lambda: cu.gated_delta(qkv, ba, A, b, pool, 0, prompts(n, q, (torch.arange(n, **i32) + 1).view(-1, 1)), nh, nh, dk, dv, 1.0, 1e-6))
+    cu.check_kernel_error(torch.device("cuda", 0))

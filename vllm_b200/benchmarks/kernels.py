@@ -3,7 +3,7 @@
     python -m vllm_b200.benchmarks.kernels [--out kernels_bench.md] [--only gemm,fp8,attn,mla,quant]
 
 Method: CUDA events on the launching stream, >= 5 warm-up calls, every timed call preceded by a
-write of a 256 MB buffer (flushes the 126 MB L2) on the same stream, median of the timed calls; library baselines
+read of a 256 MB buffer (replaces what the 126 MB L2 holds) on the same stream, median of the timed calls; library baselines
 (cuBLASLt through torch, FlashInfer / the stock vLLM wheel's ops when importable) are timed the same way.  Achieved
 bandwidth = algorithmic bytes / time against the measured copy bandwidth of MEASURED_PEAKS.json.
 """

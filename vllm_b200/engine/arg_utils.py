@@ -41,7 +41,7 @@ class EngineArgs:
     model_loader_extra_config: Optional[dict[str, Any]] = None
     device: str = "auto"
     # cache
-    block_size: Optional[int] = None      # default: 64 (tcgen05 attention page) when head_dim is 128, else 32
+    block_size: Optional[int] = None      # tokens of a KV page (prefix-cache hits are whole pages); default: 64 where the tcgen05 attention kernels run, else 32
     gpu_memory_utilization: float = 0.92
     swap_space: float = 4.0
     kv_cache_dtype: str = "auto"
