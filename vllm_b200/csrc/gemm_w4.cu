@@ -248,20 +248,6 @@ gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_b, const Params p) {
   if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn get_encode() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) != cudaSuccess || !ptr) return nullptr;
-    fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
-  return fn;
-}
-
 template <typename T, int BN>
 static int launch(const CUtensorMap& tb, const Params& p, dim3 grid, cudaStream_t st) {
   const int smem = CSTAGES * CONV_BYTES + PSTAGES * (BN * BK * 2) + PSTAGES * PK_STRIDE + (2 * PSTAGES + 2 * CSTAGES + 1) * 8 +

@@ -200,20 +200,6 @@ mla_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   if (budget < 0 && p.error) *p.error = 1;
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn get_encode() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) != cudaSuccess || !ptr) return nullptr;
-    fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
-  return fn;
-}
-
 // [rows, heads, width] with row stride `rs` and head stride `hs` elements; box = 128 rows of 64 values of one head
 static int tmap(CUtensorMap* m, const void* ptr, int width, int heads, int64_t rows, int64_t rs, int64_t hs, bool bf16) {
   auto enc = get_encode();
