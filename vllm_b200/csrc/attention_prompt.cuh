@@ -12,11 +12,15 @@
 // its own, and P may lie over S.
 //
 // CAP: scores are capped, c tanh(s / c).  SPLIT: the weights keep 16 more bits (P = hi + lo, two products): for paths whose weights are held
-// in 32 bits, at half as much tensor work again.  Tensor memory: S_0, S_1 (128 columns each), O_0, O_1 (up to 128 each).
+// in 32 bits elsewhere, at half as much tensor work again.  Results of capped prompts and decode steps are then as far from 64 bits as with
+// 32-bit weights on the CUDA cores, to three digits (8 / 2 and 16 / 4 heads, 16 to 4100 tokens: bf16 0.00139 to 0.00170, fp16 0.00017 to 0.00021).
+// Tensor memory: S_0, S_1 (128 columns each), O_0, O_1 (up to 128 each).
 //
-// Bound by the special-function and issue rate of the softmax (a key tile takes the tensor core 2048 cycles for two query tiles, their 32768
-// exponentials as long).  Measured: 32 / 8 heads, two prompts of 3800 tokens 576 us with one tile of rows, scores read twice and weights
-// through shared memory, 347 us so; capped, 16 / 4 heads, eight prompts of 860 tokens 2536 us on the CUDA cores, 182 us so.
+// Bound by the length of a turn (scores out of tensor memory, maximum, exponentials, weights back) and not by a unit: 32 / 8 heads, two prompts
+// of 3800 tokens keep the tensor core busy for 44 % of the cycles, the special-function unit for 44 %, and instructions issue in 37 %;
+// capped, 16 / 4 heads, eight prompts of 860 tokens 13, 9 and 32 % (instruction fetches and barriers are what warps wait for most).  Measured:
+// the former 576 us with one tile of rows, scores read twice and weights through shared memory, 347 us so; the latter 2536 us on the CUDA
+// cores, 182 us so.
 #pragma once
 #include "common.cuh"
 

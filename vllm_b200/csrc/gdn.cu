@@ -4,7 +4,8 @@
 //   a = exp(-exp(A_log) softplus(x_a + dt_bias)),  b = sigmoid(x_b) beta_scale
 //
 // all in 32 bits on the CUDA cores, the recurrence itself: a token costs two dot products of the OLD state (o = a S^T q + d (k . q)) and one
-// rank-1 update, a chain that no other token of the request can start before it ends, so its latency is the cost.
+// rank-1 update, a chain that no other token of the request can start before it ends, so its latency is the cost (8 prompts of 860 tokens:
+// instructions issue in 42 % of the cycles, most stalls are for the instruction before; DRAM at 4 %).
 //
 // CTA = four warps of one (request, head); a warp owns 4 CW columns of S, a lane 4 NI rows (rg) x CW columns (cg) of them in registers, as
 // pairs of rows for packed products.  The decay is kept aside (S = A S', A the running product, folded in before it gets small) instead of

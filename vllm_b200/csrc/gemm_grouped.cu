@@ -6,6 +6,8 @@
 // takes tiles of 128 rows x 256 columns (two accumulators of 256 columns fill tensor memory): 48 KB of operands per 64-deep step feed
 // twice the products, rows are stored 16 bytes at a time, and the epilogue of a tile runs while the next tile's products do.  Persistent:
 // every CTA walks the (expert, 128 rows, 256 columns) tiles with a stride of the grid, columns first, so that neighbours share rows.
+// Bound by the operands' way from L2: 13760 rows of 2048 into 8 experts of 4096 columns (gated) take 186 us (1.24 PFLOP/s); the counters show 2.7 GB out of
+// L2, 59 bytes per cycle and SM, and the tensor core busy for 64 % of the cycles.
 // Warps: 0 TMA producer, 1 MMA issuer, 2..5 epilogue (thread = row).
 #include "act.cuh"
 
