@@ -114,7 +114,15 @@ _talk_mix = _sig("vb_talk_mix", _vp, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp, _i64,
 
 
 def _st() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_device())           # torch.cuda.current_stream() builds an object of 2 us around it
+
+
+def _stream_of_device():
+    raw, dev = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+    return (raw, dev) if raw and dev else (lambda d: torch.cuda.current_stream(d).cuda_stream, torch.cuda.current_device)
+
+
+_raw_stream, _device = _stream_of_device()
 
 
 def _p(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -1897,10 +1905,15 @@ def gated_delta(qkv, ba, A_log, dt_bias, cache, state_off: int, md, nk: int, nv:
 
 
 # ------------------------------------------------------------------ GPU-side input preparation (csrc/input_prep.cu)
-_prep_step = _sig("vb_prep_step3", _vp, _vp, _vp, _i, _i, _i, _vp, _i64, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _vp,
+_prep_step = _sig("vb_prep_step4", _vp, _vp, _vp, _i, _i, _i, _vp, _i64, _i, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _vp,
                   _i, _vp)
-_bt_diff = _sig("vb_block_table_diff", _vp, _i64, _vp, _vp, _vp, _vp, _vp, _i, _vp)
-_append_sampled = _sig("vb_append_sampled", _vp, _i64, _vp, _vp, _vp, _i, _vp)
+_row_update = _sig("vb_row_update", _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp)
+_publish = _sig("vb_publish", _vp, _i64, _vp, _vp, _vp, _i, _vp, _vp, _vp, _i64, _vp)
+
+
+def pointers(tensors):
+    """Host array of the tensors' addresses; the caller keeps the tensors."""
+    return (ctypes.c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
 
 
 def prep_step(rows, num_computed, num_sched, token_table, block_rows, input_ids, positions, qsl, seq_lens, slot_mapping,
@@ -1909,22 +1922,49 @@ def prep_step(rows, num_computed, num_sched, token_table, block_rows, input_ids,
     """Expand per-request (row, computed, scheduled) triples into the per-token step inputs on the device.  Entries
     [nb, pad_b) are CUDA-graph bucket padding: one-token requests on the null block (decode buckets, ``pad_t`` = 0) or
     empty requests plus padding tokens up to ``pad_t`` (mixed-batch buckets)."""
-    nb = rows.numel()
-    _check(_prep_step(rows.data_ptr(), num_computed.data_ptr(), num_sched.data_ptr(), nb, max(pad_b, nb), pad_t,
-                      token_table.data_ptr(), token_table.stride(0), block_rows.data_ptr(), block_rows.stride(0),
-                      input_ids.data_ptr(), positions.data_ptr(), qsl.data_ptr(), seq_lens.data_ptr(),
-                      slot_mapping.data_ptr(), block_table.data_ptr(), block_table.stride(0), nblk, block_size,
-                      _p(pos_delta), int(write_tokens), _st()), "prep_step")
+    prep_step_groups(rows.data_ptr(), num_computed.data_ptr(), num_sched.data_ptr(), rows.numel(), token_table, 1, pointers([block_rows]),
+                     block_rows.stride(0), input_ids, positions, qsl, seq_lens, None, pointers([slot_mapping]), pointers([block_table]),
+                     block_table.stride(0), nblk, block_size, pad_b, pad_t, pos_delta, write_tokens)
+
+
+def prep_step_groups(rows: int, num_computed: int, num_sched: int, nb: int, token_table, groups: int, block_rows, br_stride: int, input_ids,
+                     positions, qsl, seq_lens, last, slot_mappings, block_tables, bt_stride: int, nblk: int, block_size: int, pad_b: int = 0,
+                     pad_t: int = 0, pos_delta=None, write_tokens: bool = True) -> None:
+    """``prep_step`` for all KV groups in one launch: the first three are addresses of int32 [nb], the groups' tables come as ``pointers``.
+    ``last`` (int64, optional) receives the place of every request's last scheduled token."""
+    _check(_prep_step(rows, num_computed, num_sched, nb, max(pad_b, nb), pad_t, token_table.data_ptr(), token_table.stride(0), groups, block_rows,
+                      br_stride, input_ids.data_ptr(), positions.data_ptr(), qsl.data_ptr(), seq_lens.data_ptr(), _p(last), slot_mappings,
+                      block_tables, bt_stride, nblk, block_size, _p(pos_delta), int(write_tokens), _st()), "prep_step", -(-groups // 8))
 
 
 def block_table_apply_diffs(block_rows, d_row, d_start, d_cnt, d_off, ids_flat) -> None:
-    _check(_bt_diff(block_rows.data_ptr(), block_rows.stride(0), d_row.data_ptr(), d_start.data_ptr(), d_cnt.data_ptr(),
-                    d_off.data_ptr(), ids_flat.data_ptr(), d_row.numel(), _st()), "block_table_diff")
+    row_update(pointers([block_rows]), (ctypes.c_int64 * 1)(block_rows.stride(0)), 1, None, d_row.data_ptr(), d_start.data_ptr(),
+               d_cnt.data_ptr(), d_off.data_ptr(), ids_flat.data_ptr(), d_row.numel())
+
+
+def row_update(tables, strides, n_tables: int, tbl, row: int, start: int, cnt: int, off: int, ids, n: int, moved: bool = False) -> None:
+    """Entry e: cnt[e] ints go into row row[e] of table tbl[e] (None: the only one) from start[e] on, out of ids[off[e]:] or (``moved``) out of
+    row off[e] of that table.  All but the first three are device addresses of int32 [n]."""
+    _check(_row_update(tables, strides, n_tables, tbl, row, start, cnt, off, ids, n, int(moved), _st()), "row_update")
 
 
 def append_sampled(token_table, rows, pos, sampled) -> None:
-    _check(_append_sampled(token_table.data_ptr(), token_table.stride(0), rows.data_ptr(), pos.data_ptr(),
-                           sampled.data_ptr(), rows.numel(), _st()), "append_sampled")
+    publish(token_table, rows.data_ptr(), pos.data_ptr(), sampled, rows.numel())
+
+
+def publish(token_table, rows: int, pos: int, sampled, nb: int, host_ids=None, lp=None, host_lp=None) -> None:
+    """token_table[rows[b], pos[b]] = sampled[b] where pos[b] >= 0; ``sampled`` also goes to the pinned ``host_ids`` and the contiguous int32
+    ``lp`` to the pinned ``host_lp``, both complete after an event behind this call."""
+    assert sampled.dtype == torch.int64 and sampled.is_contiguous() and sampled.numel() >= nb
+    if host_ids is not None:
+        assert host_ids.is_pinned() and host_ids.dtype == torch.int64 and host_ids.numel() >= nb and host_ids.is_contiguous()
+    n_lp = 0
+    if lp is not None:
+        n_lp = lp.numel()
+        assert lp.dtype == host_lp.dtype == torch.int32 and lp.is_contiguous() and host_lp.is_contiguous() and host_lp.is_pinned()
+        assert host_lp.numel() >= n_lp
+    _check(_publish(token_table.data_ptr(), token_table.stride(0), rows, pos, sampled.data_ptr(), nb, _p(host_ids), _p(lp), _p(host_lp), n_lp,
+                    _st()), "publish")
 
 
 # ------------------------------------------------------------------ weight-only FP4 decode GEMM (csrc/gemm_w4.cu)

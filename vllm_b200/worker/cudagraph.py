@@ -31,9 +31,7 @@ class DecodeGraph:
         self.runner = runner
         self.b = b
         dev = runner.device
-        self.temperature = torch.zeros(b, dtype=torch.float32, device=dev)
-        self.seeds = torch.zeros(b, dtype=torch.int64, device=dev)
-        self.steps = torch.zeros(b, dtype=torch.int32, device=dev)
+        self._sampling_inputs()
         self.out = torch.zeros(b, dtype=torch.int64, device=dev)
         # safe placeholder inputs for warm-up / capture: one token at position 0 of the null block
         runner.input_ids[:b].zero_()
@@ -65,6 +63,16 @@ class DecodeGraph:
             self._body()
         self.num_launches = cuda_ops().LAUNCHES - n0
 
+    def _sampling_inputs(self) -> None:
+        """Temperatures, noise counters, seeds [b]: of the runner's packed upload where there is one, else copied before each replay."""
+        r, b, dev = self.runner, self.b, self.runner.device
+        if r.gpu_prep:
+            self.temperature, self.steps, self.seeds = (x[:b] for x in r.sampling_vectors)
+        else:
+            self.temperature = torch.zeros(b, dtype=torch.float32, device=dev)
+            self.steps = torch.zeros(b, dtype=torch.int32, device=dev)
+            self.seeds = torch.zeros(b, dtype=torch.int64, device=dev)
+
     # logits of the captured step, [b, V]: a view that does not keep its memory from the pool's other graphs, so it holds them from a
     # replay of this graph to the next replay of any (None: the step samples without whole logits)
     logits: Optional[torch.Tensor] = None
@@ -84,9 +92,10 @@ class DecodeGraph:
 
     def replay_from_staging(self, stg, b: int) -> torch.Tensor:
         """Sampling vectors come from the pinned staging set (filled from the runner's per-row arrays)."""
-        self.temperature.copy_(stg.temperature[:b], non_blocking=True)
-        self.seeds.copy_(stg.seeds[:b], non_blocking=True)
-        self.steps.copy_(stg.steps[:b], non_blocking=True)
+        if not self.runner.gpu_prep:
+            self.temperature.copy_(stg.temperature[:b], non_blocking=True)
+            self.seeds.copy_(stg.seeds[:b], non_blocking=True)
+            self.steps.copy_(stg.steps[:b], non_blocking=True)
         self.graph.replay()
         self.replays = getattr(self, "replays", 0) + 1
         return self.out
@@ -107,9 +116,7 @@ class MixedGraph(DecodeGraph):
         self.runner = runner
         self.b = b
         dev = runner.device
-        self.temperature = torch.zeros(b, dtype=torch.float32, device=dev)
-        self.seeds = torch.zeros(b, dtype=torch.int64, device=dev)
-        self.steps = torch.zeros(b, dtype=torch.int32, device=dev)
+        self._sampling_inputs()
         self.out = torch.zeros(b, dtype=torch.int64, device=dev)
         # placeholder inputs for warm-up / capture: one request of t tokens at positions 0..t-1 writing nowhere
         runner.input_ids[:t].zero_()

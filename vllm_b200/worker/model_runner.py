@@ -63,6 +63,11 @@ SAMPLE_HOST = 2         # per-request state of the host (penalties, biases, gram
 SAMPLE_EAGER = 3        # more of the forward pass than its logits (pooling, log-probabilities of prompts)
 
 
+def _sampling_views(pack: torch.Tensor, R: int):
+    """Temperatures, noise counters and seeds, [R] each, at the beginning of a packed upload."""
+    return pack[:R].view(torch.float32), pack[R:2 * R], pack[2 * R:4 * R].view(torch.int64)
+
+
 class _Staging:
     """One set of pinned host buffers (inputs H2D, sampled ids D2H) + the event that guards their reuse."""
 
@@ -77,18 +82,17 @@ class _Staging:
         self.slots = [mk(T, dtype=torch.int64) for _ in range(G)]
         self.block_tables = [mk(R, MB, dtype=torch.int32) for _ in range(G)]
         self.sampled = mk(R, dtype=torch.int64)
-        self.temperature = mk(R, dtype=torch.float32)
-        self.seeds = mk(R, dtype=torch.int64)
-        self.steps = mk(R, dtype=torch.int32)
+        # GPU-side input prep: everything that a step uploads, one after the other, for ONE H2D copy: temperatures [R], noise counters [R], seeds
+        # [R] (64 bits), [rows | num_computed | num_scheduled | append_pos] of the step's requests (4 R reserved), row changes of the device
+        # tables [table | row | start | count | offset] and their ids
+        self.room = 5 * R * (4 + 6 * G) + T + G * min(R * MB, max(1 << 20, 4 * R + MB)) if pin else 0
+        self.pack = mk(8 * R + self.room, dtype=torch.int32)
+        self.temperature, self.steps, self.seeds = _sampling_views(self.pack, R)
+        self.np_pack, self.np_temperature = self.pack.numpy(), self.temperature.numpy()
+        self.np_steps, self.np_seeds = self.steps.numpy(), self.seeds.numpy()
         self.fix_idx = mk(R, dtype=torch.int64)
         self.fix_rows = mk(R, dtype=torch.int64)
         self.rows = mk(R, dtype=torch.int64)
-        # GPU-side input prep: [rows | num_computed | num_scheduled | append_pos] packed for ONE H2D copy per step, and
-        # the staged block-table appends [row | start | count | offset] + their ids
-        self.meta = mk(4 * R, dtype=torch.int32)
-        self.tok_hdr = mk(4 * R, dtype=torch.int32)
-        self.diff_hdr = [mk(8 * R, dtype=torch.int32) for _ in range(G)] if pin else []
-        self.diff_ids = [mk(min(R * MB, max(1 << 20, 4 * R + MB)), dtype=torch.int32) for _ in range(G)] if pin else []
         self.event = torch.cuda.Event() if pin else None
         self.logprobs: Optional[torch.Tensor] = None         # packed log-probabilities, allocated with the first request for them
 
@@ -275,6 +279,8 @@ class ModelRunner:
         self.dev_block_rows: list[torch.Tensor] = []
         self._bt_diffs: list[list[tuple[str, int, list[int]]]] = []
         self._new_tokens: list[tuple[str, int]] = []     # (request, first token the device table does not have)
+        self._late_rows: list[tuple[int, int]] = []      # (table, row) of changes that the packed upload had no room for
+        self._row_at: dict[int, int] = {}                # row → the row of the device tables that still holds its content
         self.prep_host_s = 0.0  # host seconds spent preparing + uploading step inputs (diagnostic)
         self.prep_decode_s, self.prep_decode_n = 0.0, 0
         self.wait_s = 0.0       # host seconds blocked on the device (D2H of sampled ids, staging reuse)
@@ -402,12 +408,17 @@ class ModelRunner:
         self.dev_tokens = torch.zeros(R, L, dtype=torch.int32, device=self.device)
         self.dev_block_rows = [torch.zeros(R, self.max_blocks_per_req, dtype=torch.int32, device=self.device)
                                for _ in range(self.num_kv_groups)]
-        self.step_meta = torch.zeros(4 * R, dtype=torch.int32, device=self.device)
-        self.tok_hdr_dev = torch.zeros(4 * R, dtype=torch.int32, device=self.device)
-        self.diff_hdr_dev = [torch.zeros(8 * R, dtype=torch.int32, device=self.device) for _ in range(self.num_kv_groups)]
-        self.diff_ids_dev = [torch.zeros(self.staging[0].diff_ids[g].numel(), dtype=torch.int32, device=self.device)
-                             for g in range(self.num_kv_groups)]
+        self.pack = torch.zeros(self.staging[0].pack.numel(), dtype=torch.int32, device=self.device)
+        self.step_meta = self.pack[4 * R:8 * R]
+        self.sampling_vectors = _sampling_views(self.pack, R)
+        self.last_token = torch.zeros(R, dtype=torch.int64, device=self.device)       # where a request's last token of the step is
         self._bt_diffs = [[] for _ in range(self.num_kv_groups)]
+        import ctypes
+        cu, tables = self._cu, [self.dev_tokens, *self.dev_block_rows]
+        # a launch takes the tables of eight groups; changes of further groups' rows go in launches of their own
+        self._row_tables = [tables[:9]] + [tables[i:i + 9] for i in range(9, len(tables), 9)]
+        self._row_args = [(cu.pointers(t), (ctypes.c_int64 * len(t))(*[x.stride(0) for x in t]), len(t)) for t in self._row_tables]
+        self._group_args = (cu.pointers(self.dev_block_rows), cu.pointers(self.slot_mappings), cu.pointers(self.block_tables))
 
     # ------------------------------------------------------- batch maintenance
     def _move_row(self, src: int, dst: int) -> None:
@@ -420,14 +431,10 @@ class ModelRunner:
             nb = self.num_blocks_cpu[g][src]
             self.block_tables_cpu[g][dst, :nb] = self.block_tables_cpu[g][src, :nb]
             self.num_blocks_cpu[g][dst] = nb
-        if self.is_cuda:
+        if self.gpu_prep:       # the device's rows follow in one launch (_flush_gpu_state)
+            self._row_at[dst] = self._row_at.pop(src, src)
+        elif self.is_cuda:
             self.last_sampled[dst:dst + 1].copy_(self.last_sampled[src:src + 1])
-        if self.gpu_prep:       # stream-ordered after the append of the step that is still in flight
-            nl = int(self.num_logical_cpu[src]) + 1
-            self.dev_tokens[dst, :nl].copy_(self.dev_tokens[src, :nl])
-            for g in range(self.num_kv_groups):
-                nb = int(self.num_blocks_cpu[g][src])
-                self.dev_block_rows[g][dst, :nb].copy_(self.dev_block_rows[g][src, :nb])
 
     def _remove(self, req_id: str, park: bool = False) -> None:
         row = self.req_index.pop(req_id, None)
@@ -446,6 +453,7 @@ class ModelRunner:
             self.states[mv].row = row
             self._move_row(last, row)
         self.req_ids.pop()
+        self._row_at.pop(last, None)
 
     def _add_row(self, st: ReqState, token_ids, block_ids, num_computed: int) -> None:
         row = len(self.req_ids)
@@ -487,6 +495,7 @@ class ModelRunner:
             self.block_tables_cpu[g][row, :len(ids)] = ids
             self.num_blocks_cpu[g][row] = len(ids)
         if self.gpu_prep:       # admission: the whole row travels once, with this step's uploads (_flush_gpu_state)
+            self._row_at.pop(row, None)
             self._new_tokens.append((st.req_id, 0))
 
     def _logprobs_ok(self, k: int) -> bool:
@@ -507,11 +516,12 @@ class ModelRunner:
         self._add_row(st, nr.prompt_token_ids, nr.block_ids, nr.num_computed_tokens)
 
     def _update_states(self, so: SchedulerOutput) -> None:
-        for rid in so.finished_req_ids:
-            self._remove(rid)
-            self._parked.pop(rid, None)
-        for rid in so.preempted_req_ids:
-            self._remove(rid, park=True)
+        # from the last row to the first: what then moves into a hole is a row that stays, and most often there is none
+        gone = so.finished_req_ids | so.preempted_req_ids
+        for rid in sorted(gone, key=lambda r: self.req_index.get(r, -1), reverse=True):
+            self._remove(rid, park=rid not in so.finished_req_ids)
+            if rid in so.finished_req_ids:
+                self._parked.pop(rid, None)
         for nr in so.scheduled_new_reqs:
             if nr.req_id in self.req_index:
                 self._remove(nr.req_id)
@@ -636,80 +646,68 @@ class ModelRunner:
                 torch.arange(T + 1, T + 1 + pad_b - nb, dtype=torch.int32, device=self.device))
 
     # ------------------------------------------------- device-side input prep
-    def _flush_gpu_state(self, stg: _Staging) -> None:
-        """Bring the device mirrors up to date with O(1) CUDA calls: the token rows of requests admitted this step and
-        the block ids appended since the last step are packed into pinned staging, shipped with one copy each, and
-        scattered into the tables by ``block_table_apply_diffs`` (row, start, count, offset) entries."""
-        cu = self._cu
-        R = self.max_num_reqs
-        if self._new_tokens:
-            fresh, self._new_tokens = self._new_tokens, []
-            pin, cap = stg.input_ids, stg.input_ids.numel()
-            pv = pin.numpy()
-            d_row, d_start, d_cnt, d_off = [], [], [], []
-            off = 0
-            for rid, first in fresh:
-                row = self.req_index.get(rid)
-                if row is None:
+    def _pack_gpu_state(self, stg: _Staging) -> tuple[int, list[tuple[int, int, int, bool]]]:
+        """Bring the device mirrors up to date: rows that moved, the token rows of requests admitted this step and the block ids appended
+        since the last step are listed in the step's packed upload.  Returns its length and the launches that apply it: (place of the list,
+        entries, which tables, moved)."""
+        R, v = self.max_num_reqs, stg.np_pack
+        at, end, launches = 8 * R, 8 * R + stg.room, []
+
+        def put(entries, which, moved):
+            nonlocal at
+            n = len(entries)
+            if n:
+                v[at:at + 5 * n] = np.asarray(entries, dtype=np.int32).T.reshape(-1)
+                launches.append((at, n, which, moved))
+                at += 5 * n
+        moves, self._row_at = self._row_at, {}
+        while moves:            # a row whose content another one still waits for is written after that one
+            held = set(moves.values())
+            now = [d for d in moves if d not in held or moves[d] == d]
+            lists: dict[int, list] = {}
+            for d in now:
+                o = moves.pop(d)
+                if o == d or d >= len(self.req_ids):
                     continue
-                n = int(self.num_tokens_cpu[row]) - first
-                for g in range(self.num_kv_groups if first == 0 else 0):
-                    k = int(self.num_blocks_cpu[g][row])  # the whole block list of the row goes through the diff path
+                lens = [int(self.num_logical_cpu[d]) + 1, *(int(self.num_blocks_cpu[g][d]) for g in range(self.num_kv_groups))]
+                for t, k in enumerate(lens):
                     if k:
-                        self._bt_diffs[g].append((rid, 0, self.block_tables_cpu[g][row, :k]))
-                if off + n <= cap and len(d_row) < R:
-                    pv[off:off + n] = self.token_ids_cpu[row, first:first + n]
-                    d_row.append(row)
-                    d_start.append(first)
-                    d_cnt.append(n)
-                    d_off.append(off)
-                    off += n
-                else:                       # does not fit the packed upload (very long prompts): pageable row copy
-                    self.dev_tokens[row, first:first + n].copy_(torch.from_numpy(self.token_ids_cpu[row, first:first + n].copy()))
-                self.h2d_bytes += n * 4
-            n_e = len(d_row)
-            if n_e:
-                hv = stg.tok_hdr.numpy()
-                hv[:n_e], hv[n_e:2 * n_e], hv[2 * n_e:3 * n_e], hv[3 * n_e:4 * n_e] = d_row, d_start, d_cnt, d_off
-                self.tok_hdr_dev[:4 * n_e].copy_(stg.tok_hdr[:4 * n_e], non_blocking=True)
-                # the step's own input_ids buffer doubles as device scratch: prep_step overwrites it afterwards
-                self.input_ids[:off].copy_(pin[:off], non_blocking=True)
-                th = self.tok_hdr_dev
-                cu.block_table_apply_diffs(self.dev_tokens, th[:n_e], th[n_e:2 * n_e], th[2 * n_e:3 * n_e],
-                                           th[3 * n_e:4 * n_e], self.input_ids)
-        for g in range(self.num_kv_groups):
-            diffs = self._bt_diffs[g]
-            if not diffs:
-                continue
-            iv = stg.diff_ids[g].numpy()
-            d_row, d_start, d_cnt, d_off = [], [], [], []
-            o = 0
-            for rid, start, new in diffs:
+                        lists.setdefault(t // 9, []).append((t % 9, d, 0, k, o))
+            for which, e in lists.items():
+                put(e, which, True)
+        fresh: list[tuple[int, int, int, Any]] = []          # (table, row, start, ids)
+        if self._new_tokens:
+            added, self._new_tokens = self._new_tokens, []
+            for rid, first in added:
                 row = self.req_index.get(rid)
                 if row is None:
                     continue
-                k = len(new)
-                if len(d_row) >= 2 * R or o + k > iv.shape[0]:   # staging full (pathological): upload the row
-                    tot = int(self.num_blocks_cpu[g][row])
-                    self.dev_block_rows[g][row, :tot].copy_(torch.from_numpy(self.block_tables_cpu[g][row, :tot].copy()))
-                    continue
-                d_row.append(row)
-                d_start.append(start)
-                d_cnt.append(k)
-                d_off.append(o)
-                iv[o:o + k] = new
-                o += k
-            diffs.clear()
-            n = len(d_row)
-            if n == 0:
+                n = int(self.num_tokens_cpu[row])
+                fresh.append((0, row, first, self.token_ids_cpu[row, first:n]))
+                for g in range(self.num_kv_groups if first == 0 else 0):
+                    k = int(self.num_blocks_cpu[g][row])  # the whole block list of the row goes the same way
+                    if k:
+                        fresh.append((1 + g, row, 0, self.block_tables_cpu[g][row, :k]))
+        for g in range(self.num_kv_groups):
+            for rid, start, new in self._bt_diffs[g]:
+                row = self.req_index.get(rid)
+                if row is not None:
+                    fresh.append((1 + g, row, start, new))
+            self._bt_diffs[g].clear()
+        lists = {}
+        reserve = 5 * len(fresh)
+        ids_at = at + reserve
+        for t, row, start, new in fresh:
+            k = len(new)
+            if ids_at + k > end or at + reserve > end:        # does not fit the packed upload (pathological): the row itself, behind the launches
+                self._late_rows.append((t, row))
                 continue
-            hv = stg.diff_hdr[g].numpy()
-            hv[:n], hv[n:2 * n], hv[2 * n:3 * n], hv[3 * n:4 * n] = d_row, d_start, d_cnt, d_off
-            dh, di = self.diff_hdr_dev[g], self.diff_ids_dev[g]
-            dh[:4 * n].copy_(stg.diff_hdr[g][:4 * n], non_blocking=True)
-            di[:o].copy_(stg.diff_ids[g][:o], non_blocking=True)
-            self.h2d_bytes += 16 * n + 4 * o
-            cu.block_table_apply_diffs(self.dev_block_rows[g], dh[:n], dh[n:2 * n], dh[2 * n:3 * n], dh[3 * n:4 * n], di)
+            v[ids_at:ids_at + k] = new
+            lists.setdefault(t // 9, []).append((t % 9, row, start, k, ids_at))
+            ids_at += k
+        for which, e in lists.items():
+            put(e, which, False)
+        return (ids_at if lists else at), launches
 
     def _prepare_gpu(self, so: SchedulerOutput, stg: _Staging):
         """O(requests) host work: which rows run, how many tokens each, and the scalars the device expansion needs."""
@@ -725,27 +723,44 @@ class ModelRunner:
         computed = self.num_computed_cpu[rows]
         seq_lens = computed + ns
         produces = seq_lens >= self.num_logical_cpu[rows]
-        m = stg.meta.numpy()
+        R = self.max_num_reqs
+        m = stg.np_pack[4 * R:]
         m[:nb] = rows
         m[nb:2 * nb] = computed
         m[2 * nb:3 * nb] = ns
         m[3 * nb:4 * nb] = np.where(produces, seq_lens, -1)     # where the sampled id goes in the device token table
-        stg.rows[:nb] = torch.from_numpy(rows)
+        self._stage_sampling(stg, rows, nb, R)
         max_q = int(ns.max()) if nb else 0
         max_s = int(seq_lens.max()) if nb else 0
         return rows, ns, cu, T, max_q, max_s, 0
 
+    def _stage_sampling(self, stg: _Staging, rows, nb: int, pad_b: int) -> None:
+        """Temperature / seed / noise counter of the step's rows; graph-bucket padding is greedy."""
+        stg.np_temperature[:nb] = self.temp_cpu[rows]
+        stg.np_seeds[:nb] = self.seed_cpu[rows]
+        stg.np_steps[:nb] = self.num_logical_cpu[rows] - self.num_prompt_cpu[rows]
+        stg.np_temperature[nb:pad_b] = 0.0
+
     def _h2d_gpu(self, stg: _Staging, nb, T, pad_b, max_s, pad_t: int = 0) -> None:
         cu = self._cu
-        self._flush_gpu_state(stg)
-        self.step_meta[:4 * nb].copy_(stg.meta[:4 * nb], non_blocking=True)
-        self.h2d_bytes += 16 * nb
+        n, launches = self._pack_gpu_state(stg)
+        self.pack[:n].copy_(stg.pack[:n], non_blocking=True)
+        self.h2d_bytes += 4 * n
+        base = self.pack.data_ptr()
+        for at, k, which, moved in launches:
+            p = base + 4 * at
+            cu.row_update(*self._row_args[which], p, p + 4 * k, p + 8 * k, p + 12 * k, p + 16 * k, base, k, moved)
+        if self._late_rows:
+            late, self._late_rows = self._late_rows, []
+            for t, row in late:
+                host = self.token_ids_cpu if t == 0 else self.block_tables_cpu[t - 1]
+                k = int(self.num_tokens_cpu[row] if t == 0 else self.num_blocks_cpu[t - 1][row])
+                (self.dev_tokens if t == 0 else self.dev_block_rows[t - 1])[row, :k].copy_(torch.from_numpy(host[row, :k].copy()))
         nbk = max(cdiv(max_s, self.vblock), 1)
-        sm = self.step_meta
-        for g in range(self.num_kv_groups):
-            cu.prep_step(sm[:nb], sm[nb:2 * nb], sm[2 * nb:3 * nb], self.dev_tokens, self.dev_block_rows[g], self.input_ids,
-                         self.positions, self.qsl, self.seq_lens, self.slot_mappings[g], self.block_tables[g], nbk,
-                         self.block_size, pad_b=pad_b, write_tokens=(g == 0), pad_t=pad_t)
+        m, (rows, slots, tables) = base + 16 * self.max_num_reqs, self._group_args
+        cu.prep_step_groups(m, m + 4 * nb, m + 8 * nb, nb, self.dev_tokens, self.num_kv_groups, rows, self.dev_block_rows[0].stride(0),
+                            self.input_ids, self.positions, self.qsl, self.seq_lens, self.last_token, slots, tables,
+                            self.block_tables[0].stride(0), nbk, self.block_size, pad_b, pad_t)
 
     def _make_metadata(self, nb, T, max_q, max_s, decode_only, cpu_qsl=None, cpu_sl=None, host_lens=None
                        ) -> dict[int, AttentionMetadata]:
@@ -1098,14 +1113,11 @@ class ModelRunner:
         req_ids = [self.req_ids[r] for r in rows]
         if graph is not None:
             # fast path: temperature / seed / step vectors straight from the per-row arrays
-            stg.temperature[:nb] = torch.from_numpy(self.temp_cpu[rows])
-            stg.seeds[:nb] = torch.from_numpy(self.seed_cpu[rows])
-            stg.steps[:nb] = torch.from_numpy(self.num_logical_cpu[rows] - self.num_prompt_cpu[rows])
-            if pad_b > nb:
-                stg.temperature[nb:pad_b] = 0.0
+            if not gpu_prep:
+                self._stage_sampling(stg, rows, nb, pad_b)
+                self.h2d_bytes += pad_b * 16
             sampled = graph.replay_from_staging(stg, pad_b)[:nb]
             self.launch_count += graph.num_launches
-            self.h2d_bytes += pad_b * 16
             if mode <= SAMPLE_LOGPROBS and no_filter:
                 if mode == SAMPLE_LOGPROBS:
                     lp_out = self._cu_ops().logprobs(graph.logits[:nb], sampled, int(self.lp_cpu[rows].max()))
@@ -1114,7 +1126,7 @@ class ModelRunner:
                 l0 = self._launches()
                 states = [self.states[r] for r in req_ids]
                 bitmask = self._gather_bitmask(so, states) if so.grammar_bitmask is not None else None
-                so_out = self.sampler(graph.logits[:nb], self._sampling_metadata(states, rows, nb, simple), bitmask)
+                so_out = self.sampler(graph.logits[:nb], self._sampling_metadata(states, rows, nb, simple, gpu_prep), bitmask)
                 sampled, lp_out = so_out.sampled_token_ids, self._step_logprobs(so_out, produces)
                 self.launch_count += self._launches() - l0
         else:
@@ -1169,7 +1181,8 @@ class ModelRunner:
                 return self._checked(self._pool(hidden, states, rows, cu, produces, t0))
             if has_spec:
                 return self._checked(self._verify_spec(so, hidden, states, rows, ns, cu, t0))
-            last_idx = torch.from_numpy(cu[1:].astype(np.int64) - 1).to(self.device, non_blocking=True)
+            last_idx = (self.last_token[:nb] if gpu_prep else
+                        torch.from_numpy(cu[1:].astype(np.int64) - 1).to(self.device, non_blocking=True))
             if getattr(self.drafter, "needs_step_hidden", False):
                 # EAGLE / MTP heads consume the target hidden state of every position computed this step
                 src = self._last_aux if getattr(self.drafter, "aux_layers", None) else hidden
@@ -1178,7 +1191,7 @@ class ModelRunner:
             if self.spec_hidden is not None:        # hidden-state proposers (Medusa) read the newest position's state
                 self.spec_hidden.index_copy_(0, torch.from_numpy(rows.astype(np.int64)).to(self.device), last_hidden)
             logits = self.model.compute_logits(last_hidden)
-            smd = self._sampling_metadata(states, rows, nb, simple)
+            smd = self._sampling_metadata(states, rows, nb, simple, gpu_prep)
             bitmask = self._gather_bitmask(so, states) if so.grammar_bitmask is not None else None
             so_out = self.sampler(logits, smd, bitmask)
             sampled = so_out.sampled_token_ids
@@ -1191,13 +1204,18 @@ class ModelRunner:
         # publish: device-side last_sampled (for the next step's input patch) + async D2H
         ev = None
         if self.is_cuda:
-            rows_dev = stg.rows[:nb].to(self.device, non_blocking=True)
-            self.last_sampled.index_copy_(0, rows_dev, sampled)
-            if gpu_prep:        # the new ids become next step's inputs on the device (no D2H → H2D round trip)
-                self._cu.append_sampled(self.dev_tokens, self.step_meta[:nb], self.step_meta[3 * nb:4 * nb], sampled)
-            stg.sampled[:nb].copy_(sampled, non_blocking=True)
-            if isinstance(lp_out, torch.Tensor):
-                lp_out = stg.logprobs_buf(*lp_out.shape).copy_(lp_out, non_blocking=True)
+            lp_dev = lp_out if isinstance(lp_out, torch.Tensor) else None
+            if lp_dev is not None:
+                lp_out = stg.logprobs_buf(*lp_dev.shape)
+            if gpu_prep:        # the new ids become next step's inputs on the device (no D2H → H2D round trip) and go to the host as well
+                meta = self.step_meta.data_ptr()
+                self._cu.publish(self.dev_tokens, meta, meta + 12 * nb, sampled, nb, stg.sampled, lp_dev, None if lp_dev is None else lp_out)
+            else:
+                rows_dev = stg.rows[:nb].to(self.device, non_blocking=True)
+                self.last_sampled.index_copy_(0, rows_dev, sampled)
+                stg.sampled[:nb].copy_(sampled, non_blocking=True)
+                if lp_dev is not None:
+                    lp_out.copy_(lp_dev, non_blocking=True)
             stg.event.record()
             ev = stg.event
         else:
@@ -1250,19 +1268,26 @@ class ModelRunner:
                 return s
         return -1
 
-    def _sampling_metadata(self, states: list[ReqState], rows, pad_b: int, simple: bool = False) -> SamplingMetadata:
+    def _sampling_metadata(self, states: list[ReqState], rows, pad_b: int, simple: bool = False, uploaded: bool = False
+                           ) -> SamplingMetadata:
+        """``uploaded``: temperatures, seeds and noise counters of ``rows`` came with the step's inputs."""
         B = len(states)
         dev = self.device
         rows = np.asarray(rows)
         temps = self.temp_cpu[rows].copy()
         all_greedy = bool((temps < 1e-5).all())
         all_random = bool((temps >= 1e-5).all())
-        t = torch.from_numpy(temps).to(dev, non_blocking=True)
+        if uploaded:
+            t, steps, seeds = (x[:B] for x in self.sampling_vectors)
+        else:
+            t, steps, seeds = torch.from_numpy(temps).to(dev, non_blocking=True), None, None
+        if not all_greedy and seeds is None:
+            seeds = torch.from_numpy(self.seed_cpu[rows]).to(dev)
+            steps = torch.from_numpy((self.num_logical_cpu[rows] - self.num_prompt_cpu[rows]).astype(np.int32)).to(dev)
         if simple and not bool(self.filter_cpu[rows].any()):
             md = SamplingMetadata(temperature=t, all_greedy=all_greedy, all_random=all_random)
             if not all_greedy:
-                md.seeds = torch.from_numpy(self.seed_cpu[rows]).to(dev)
-                md.steps = torch.from_numpy((self.num_logical_cpu[rows] - self.num_prompt_cpu[rows]).astype(np.int32)).to(dev)
+                md.seeds, md.steps = seeds, steps
                 if not self.is_cuda:  # the reference sampler draws from per-request torch generators
                     md.generators = {i: s.generator for i, s in enumerate(states) if s.generator is not None}
             return md
@@ -1313,8 +1338,7 @@ class ModelRunner:
                 md.top_p = torch.from_numpy(top_p).to(dev)
             if (min_p > 0).any():
                 md.min_p = torch.from_numpy(min_p).to(dev)
-            md.seeds = torch.from_numpy(self.seed_cpu[rows]).to(dev)
-            md.steps = torch.from_numpy((self.num_logical_cpu[rows] - self.num_prompt_cpu[rows]).astype(np.int32)).to(dev)
+            md.seeds, md.steps = seeds, steps
         if any_pen:
             md.no_penalties = False
             md.presence, md.frequency = torch.from_numpy(pres).to(dev), torch.from_numpy(freq).to(dev)
