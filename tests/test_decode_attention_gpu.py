@@ -76,3 +76,34 @@ def test_rules():
     for B, Hkv, k in ((1, 1, 1), (1, 8, 130), (64, 4, 4096), (1, 1, 1 << 17), (1000, 8, 4096)):
         p = c.decode_parts(B, Hkv, k)
         assert p in (1, 2, 4, 8) and (p == 1 or B * Hkv * p <= n)
+
+
+@pytest.mark.parametrize("R,P,dtype", [(512, 64, torch.bfloat16), (512, 64, torch.float16), (512, 0, torch.bfloat16), (384, 64, torch.bfloat16),
+                                       (72, 40, torch.bfloat16), (192, 16, torch.bfloat16)])
+@pytest.mark.parametrize("H,BS", [(1, 64), (16, 64), (17, 16), (40, 128)])
+@pytest.mark.parametrize("parts,window,wide", [(0, None, False), (1, 100, True), (3, None, True), (16, 16, False)])
+def test_latents_against_64_bits(R, P, dtype, H, BS, parts, window, wide):
+    g = torch.Generator(device="cuda").manual_seed(R + H)
+    B, mb = len(LENS), -(-max(LENS) // BS)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).to(dtype)                    # noqa: E731
+    q, qp, cache = rnd(B, H, R), rnd(B, H, P) if P else None, rnd(B * mb + 1, BS, R + P)
+    bt = (torch.randperm(B * mb, device="cuda", generator=g) + 1).int().view(B, mb)
+    scale = 3.0 / (R + P) ** 0.5
+    want, mass = (torch.zeros(B, H, R, dtype=torch.float64, device="cuda") for _ in range(2))
+    lse = torch.zeros(B, H, dtype=torch.float64, device="cuda")
+    bad = cache.clone()
+    for b, n in enumerate(LENS):
+        rows = cache[bt[b].long()].view(-1, R + P)[:n].double()
+        first = max(0, n - window) if window else 0
+        s = (torch.cat([q[b], qp[b]], -1) if P else q[b]).double() @ rows[first:].t() * scale
+        w, lse[b] = s.softmax(-1), torch.logsumexp(s, -1)
+        want[b], mass[b] = w @ rows[first:, :R], w @ rows[first:, :R].abs()
+        for t in [*range(first), *range(n, mb * BS)]:
+            bad[int(bt[b, t // BS]), t % BS] = float("nan")
+    got, got_lse = cu().mla_decode_tc(q, qp, bad, bt, torch.tensor(LENS, dtype=torch.int32, device="cuda"), scale, max(LENS), parts, return_lse=True,
+                                      sliding_window=window, wide=wide)
+    # weights of 16 bits or (wide) in two parts of 16, the result rounded once; 32-bit sums and exponentials of scores up to 16 beside them
+    u = 2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -11
+    bound = (u * u if wide else u) * mass + u * want.abs() + 4e-5 * mass + (6e-8 if dtype is torch.float16 else 0.0)
+    assert ((got.double() - want).abs() <= bound).all(), ((got.double() - want).abs() / bound).max()
+    assert (got_lse.double() - lse).abs().max() < 2e-4
