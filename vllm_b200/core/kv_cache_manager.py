@@ -225,6 +225,11 @@ class SingleTypeManager:
         self.req_to_blocks: dict[str, list[KVCacheBlock]] = {}
         self.num_cached: dict[str, int] = {}
 
+    def settled(self, request_id: str, num_computed_tokens: int, num_tokens: int) -> bool:
+        """Would ``num_tokens`` in all neither take a block nor give one back?"""
+        blocks = self.req_to_blocks.get(request_id)
+        return blocks is not None and num_tokens <= len(blocks) * self.block_size
+
     # number of *additional* blocks needed for ``num_tokens`` total tokens
     def blocks_needed(self, request_id: str, num_tokens: int, new_computed: Sequence[KVCacheBlock]) -> int:
         have = len(self.req_to_blocks.get(request_id, ())) + len(new_computed)
@@ -297,6 +302,13 @@ class SlidingWindowManager(SingleTypeManager):
         first_token = max(0, num_computed_tokens - sw + 1)
         return first_token // self.block_size
 
+    def settled(self, request_id: str, num_computed_tokens: int, num_tokens: int) -> bool:
+        blocks = self.req_to_blocks.get(request_id)
+        if blocks is None or num_tokens > len(blocks) * self.block_size:
+            return False
+        last = min(self._first_useful_block(num_computed_tokens), len(blocks)) - 1
+        return last < 0 or blocks[last].is_null
+
     def remove_skipped_blocks(self, request_id: str, num_computed_tokens: int) -> None:
         blocks = self.req_to_blocks.get(request_id)
         if not blocks:
@@ -333,6 +345,9 @@ class SlidingWindowManager(SingleTypeManager):
 
 class MambaManager(SingleTypeManager):
     """One state slot per request regardless of length (``pool`` holds slots, not token pages)."""
+
+    def settled(self, request_id, num_computed_tokens, num_tokens) -> bool:
+        return bool(self.req_to_blocks.get(request_id))
 
     def blocks_needed(self, request_id, num_tokens, new_computed) -> int:
         return 0 if self.req_to_blocks.get(request_id) else 1
@@ -491,6 +506,16 @@ class KVCacheManager:
                         if final // bs > m.num_cached.get(rid, 0):
                             m.cache_blocks(request, final)
                     return self._empty
+        elif new_computed_blocks is None and num_new_computed_tokens == 0:
+            # the same for several groups: no group takes a block or gives one back (two groups of 24 requests cost 0.3 ms a step)
+            nc = request.num_computed_tokens
+            total = min(nc + num_new_tokens + num_lookahead_tokens, self.max_model_len)
+            if all(m.settled(rid, nc, total) for m in self.managers):
+                if self.enable_caching and not delay_cache_blocks:
+                    final = min(nc + num_new_tokens, request.num_tokens)
+                    for m in self.managers:
+                        m.cache_blocks(request, final)
+                return self._empty
         new_computed = new_computed_blocks.blocks if new_computed_blocks is not None else \
             tuple([] for _ in self.managers)
         # reclaim out-of-window blocks first so they can serve this very allocation

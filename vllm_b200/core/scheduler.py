@@ -101,20 +101,20 @@ class PriorityQueue:
 
 def check_stop(request: Request, max_model_len: int) -> bool:
     """Length / EOS / stop-token checks after appending one token."""
-    sp = request.sampling_params
-    if request.num_tokens >= max_model_len or request.num_output_tokens >= request.max_tokens:
+    sp, out = request.sampling_params, request._output_token_ids
+    if len(request._all_token_ids) >= max_model_len or len(out) >= request.max_tokens:
         request.status = RequestStatus.FINISHED_LENGTH_CAPPED
         return True
     if request.pooling_params is not None:
         return False
     assert sp is not None
-    if request.num_output_tokens < sp.min_tokens:
+    if len(out) < sp.min_tokens:
         return False
-    last = request.output_token_ids[-1]
+    last = out[-1]
     if not sp.ignore_eos and last == request.eos_token_id:
         request.status = RequestStatus.FINISHED_STOPPED
         return True
-    if last in sp.all_stop_token_ids and not (sp.ignore_eos and last == request.eos_token_id):
+    if sp.all_stop_token_ids and last in sp.all_stop_token_ids and not (sp.ignore_eos and last == request.eos_token_id):
         request.status = RequestStatus.FINISHED_STOPPED
         request.stop_reason = last if last != request.eos_token_id else None
         return True
@@ -207,16 +207,16 @@ class Scheduler:
         structured_ids: list[str] = []
 
         # 1. running requests
-        i = 0
+        # (attributes instead of properties, here and below: a property costs as much as the line around it, 64 times a step)
+        i, ahead, max_len = 0, self.async_scheduling, self.max_model_len
         while i < len(self.running) and budget > 0:
             req = self.running[i]
-            n_new = req.num_tokens_with_spec + req.num_output_placeholders - req.num_computed_tokens
+            computed, coming, known = req.num_computed_tokens, req.num_output_placeholders, len(req._all_token_ids)
+            n_new = known + len(req.spec_token_ids) + coming - computed
             if 0 < thr < n_new:
                 n_new = thr
-            n_new = min(n_new, budget, self.max_model_len - 1 - req.num_computed_tokens)
-            if self.async_scheduling and req.num_output_placeholders > 0 and (
-                    req.num_output_tokens + req.num_output_placeholders >= req.max_tokens
-                    or req.num_tokens + req.num_output_placeholders >= self.max_model_len):
+            n_new = min(n_new, budget, max_len - 1 - computed)
+            if ahead and coming > 0 and (len(req._output_token_ids) + coming >= req.max_tokens or known + coming >= max_len):
                 n_new = 0  # the in-flight tokens already reach the length cap: wait for them
             if n_new <= 0:
                 i += 1
@@ -443,6 +443,14 @@ class Scheduler:
         c = CachedRequestData()
         pp = self.vllm_config.parallel_config.pipeline_parallel_size > 1
         empty = self.kv_cache_manager.empty_blocks()
+        if not resumed and not pp:
+            c.req_ids = [r.request_id for r in running]
+            c.resumed_from_preemption = [False] * len(running)
+            c.new_token_ids = [[]] * len(running)
+            c.new_block_ids = [None if b is None or b is empty else b.get_block_ids() for b in map(new_blocks_of.get, c.req_ids)]
+            c.num_computed_tokens = [r.num_computed_tokens for r in running]
+            c.num_output_tokens = [len(r._output_token_ids) for r in running]
+            return c
         for is_resumed, reqs in ((False, running), (True, resumed)):
             for r in reqs:
                 rid = r.request_id
@@ -496,9 +504,9 @@ class Scheduler:
             for g in sampled:
                 lp_offsets.append(acc)
                 acc += len(g)
-        # plain generation step (no speculation / logprobs / pooling / prompt logprobs / NaN report): the per-request
+        # plain generation step (no speculation / pooling / prompt logprobs / NaN report): the per-request
         # work below shrinks to "append the token, check the stop conditions, emit the delta"
-        plain = (not so.scheduled_spec_decode_tokens and lp_ids is None and not mo.pooler_output
+        plain = (not so.scheduled_spec_decode_tokens and not mo.pooler_output
                  and not mo.prompt_logprobs_dict and mo.spec_token_ids is None and not mo.num_nans_in_logits)
         requests, r2i, n_samp, mml = self.requests, mo.req_id_to_index, len(sampled), self.max_model_len
         for rid, n_sched in so.num_scheduled_tokens.items():
@@ -520,6 +528,10 @@ class Scheduler:
                     if check_stop(req, mml):
                         stopped, new_ids = True, gen[:k + 1]
                         break
+                new_lp = None
+                if lp_ids is not None and req.sampling_params is not None and req.sampling_params.logprobs is not None:
+                    sl = slice(lp_offsets[idx], lp_offsets[idx] + len(new_ids))
+                    new_lp = LogprobsLists(lp_ids[sl], lp_vals[sl], lp_ranks[sl])
                 kv_params = None
                 if stopped:
                     kv_params = self._free_request(req)
@@ -532,7 +544,7 @@ class Scheduler:
                     outs = outputs[req.client_index] = []
                 nct = req.num_cached_tokens
                 outs.append(EngineCoreOutput(
-                    request_id=rid, new_token_ids=list(new_ids),
+                    request_id=rid, new_token_ids=list(new_ids), new_logprobs=new_lp,
                     finish_reason=int(req.get_finished_reason()) if stopped else None, stop_reason=req.stop_reason,
                     num_cached_tokens=nct if nct > 0 else 0, kv_transfer_params=kv_params,
                     events=req.take_events() if req.events else None))

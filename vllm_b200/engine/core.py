@@ -60,6 +60,7 @@ class EngineCore:
         self.batch_queue_size = n_batches
         self.step_fn: Callable = self.step if self.batch_queue is None else self.step_with_batch_queue
         self._aborts_since_step: list[str] = []
+        self._ahead = False
 
     def _initialize_kv_caches(self):
         t0 = time.perf_counter()
@@ -96,6 +97,8 @@ class EngineCore:
         if sp is not None and sp.structured_outputs is not None:
             so_req = self.structured_output_manager.make_request(req.request_id, sp.structured_outputs)
         r = Request.from_engine_core_request(req, self.block_hasher, so_req)
+        if self._ahead and not self._steps_ahead(r):
+            raise RuntimeError("a request that is sampled with host state cannot join steps that run ahead")
         if len(r.prompt_token_ids) >= self.vllm_config.scheduler_config.max_model_len:
             raise ValueError(f"prompt of {len(r.prompt_token_ids)} tokens exceeds max_model_len")
         self.scheduler.add_request(r)
@@ -157,7 +160,11 @@ class EngineCore:
             so = self.scheduler.schedule()
             if so.total_num_scheduled_tokens > 0 or so.finished_req_ids:
                 so.grammar_bitmask = self.scheduler.get_grammar_bitmask(so)
-                fut = self.model_executor.execute_model(so, non_block=True)
+                try:
+                    fut = self.model_executor.execute_model(so, non_block=True)
+                except Exception:
+                    self._dump_failed_step(so)
+                    raise
                 bq.appendleft((fut, so))
                 scheduled = so.total_num_scheduled_tokens > 0
                 if scheduled and len(bq) < self.batch_queue_size and not bq[-1][0].done():
@@ -167,6 +174,45 @@ class EngineCore:
         fut, so = bq.pop()
         mo = fut.result()
         return self.scheduler.update_from_output(so, mo), scheduled
+
+    # ------------------------------------------------------- one step ahead
+    def start_ahead(self) -> bool:
+        """For a caller that steps until all its requests are done: the next step is scheduled and launched while the device works on this one,
+        as with ``async_scheduling``, until ``stop_ahead``.  Only where a step needs nothing from the host but its tokens: one worker in
+        this process, no speculation or connector, and requests without per-token host state.  False: steps stay synchronous."""
+        from vllm_b200.executor import UniProcExecutor
+        s = self.scheduler
+        if (self.batch_queue is not None or type(self.model_executor) is not UniProcExecutor or type(s) is not Scheduler
+                or self.vllm_config.speculative_config is not None or s.connector is not None
+                or self.vllm_config.lora_config is not None or not hasattr(self.model_executor.worker, "set_async") or not all(map(self._steps_ahead, s.requests.values()))):
+            return False
+        self._set_ahead(True)
+        return True
+
+    @staticmethod
+    def _steps_ahead(r: Request) -> bool:
+        sp = r.sampling_params
+        return (sp is not None and not r.use_structured_output and not r.mm_features and r.lora_request is None and not r.kv_transfer_params
+                and sp.prompt_logprobs is None and not sp.needs_penalties and not sp.logit_bias and not sp.allowed_token_ids and not sp.bad_words
+                and not sp.bad_words_token_ids and sp.min_tokens == 0 and not sp.stop and not sp.extra_args)
+
+    def _set_ahead(self, on: bool) -> None:
+        self._ahead = on
+        self.batch_queue, self.batch_queue_size = (deque(maxlen=2), 2) if on else (None, 1)
+        self.step_fn = self.step_with_batch_queue if on else self.step
+        self.scheduler.async_scheduling = on
+        self.model_executor.worker.set_async(on)
+
+    def stop_ahead(self) -> None:
+        """Back to synchronous steps.  What is in flight is waited for: a step of requests that ended, or were aborted, with the one before."""
+        if not self._ahead:
+            return
+        try:
+            while self.batch_queue:
+                fut, so = self.batch_queue.pop()
+                self.scheduler.update_from_output(so, fut.result())
+        finally:
+            self._set_ahead(False)
 
     # -------------------------------------------------------------- utility
     def profile(self, is_start: bool = True) -> None:

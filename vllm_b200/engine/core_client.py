@@ -50,6 +50,12 @@ class EngineCoreClient:
     def call_utility(self, method: str, *args) -> Any: raise NotImplementedError
     def dp_engines_running(self) -> bool: return False
 
+    def start_ahead(self) -> bool:
+        """Steps may run one ahead until ``stop_ahead`` (engines of their own process schedule by themselves)."""
+        return False
+
+    def stop_ahead(self) -> None: ...
+
     # convenience wrappers
     def profile(self, is_start=True): return self.call_utility("profile", is_start)
     def reset_prefix_cache(self): return self.call_utility("reset_prefix_cache")
@@ -80,6 +86,12 @@ class InprocClient(EngineCoreClient):
 
     def call_utility(self, method: str, *args) -> Any:
         return getattr(self.engine_core, method)(*args)
+
+    def start_ahead(self) -> bool:
+        return self.engine_core.start_ahead()
+
+    def stop_ahead(self) -> None:
+        self.engine_core.stop_ahead()
 
     def shutdown(self) -> None:
         self.engine_core.shutdown()

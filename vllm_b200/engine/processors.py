@@ -244,6 +244,11 @@ class LogprobsProcessor:
         self.cumulative_logprob: Optional[float] = 0.0 if sp.logprobs is not None else None
 
     def _entry(self, ids: list[int], vals: list[float], rank: int, k: Optional[int]) -> dict[int, Logprob]:
+        if self.tok is None and (k is None or k < 0 or len(ids) <= k + 1):
+            d = {i: Logprob(v, j, None) for j, (i, v) in enumerate(zip(ids, vals))}
+            if ids:                     # the sampled token: its own rank, also where it is among the likeliest
+                d[ids[0]] = Logprob(vals[0], rank, None)
+            return d
         d: dict[int, Logprob] = {}
         toks = self.tok.convert_ids_to_tokens(ids) if self.tok is not None else [None] * len(ids)
         for j, (i, v) in enumerate(zip(ids, vals)):

@@ -81,21 +81,32 @@ class LLM:
         if use_tqdm:
             from tqdm import tqdm
             pbar = tqdm(total=self.llm_engine.get_num_unfinished_requests(), desc="Processed prompts")
-        while self.llm_engine.has_unfinished_requests():
-            try:
-                step_outs = self.llm_engine.step()
-            except BaseException:
-                # leave the engine reusable: drop every request of this call (front-end state and scheduler)
+        core = self.llm_engine.engine_core
+        core.start_ahead()          # nobody else steps the engine or adds to it until all is done
+        failed = True
+        try:
+            while self.llm_engine.has_unfinished_requests():
                 try:
-                    self.llm_engine.abort_request(list(self.llm_engine.output_processor.request_states))
-                except Exception:
-                    pass
-                raise
-            for o in step_outs:
-                if o.finished:
-                    outs.append(o)
-                    if pbar:
-                        pbar.update(1)
+                    step_outs = self.llm_engine.step()
+                except BaseException:
+                    # leave the engine reusable: drop every request of this call (front-end state and scheduler)
+                    try:
+                        self.llm_engine.abort_request(list(self.llm_engine.output_processor.request_states))
+                    except Exception:
+                        pass
+                    raise
+                for o in step_outs:
+                    if o.finished:
+                        outs.append(o)
+                        if pbar:
+                            pbar.update(1)
+            failed = False
+        finally:
+            try:
+                core.stop_ahead()
+            except Exception:
+                if not failed:
+                    raise           # (else the error of before is the one to report)
         if pbar:
             pbar.close()
         return sorted(outs, key=lambda o: int(o.request_id) if str(o.request_id).isdigit() else 0)

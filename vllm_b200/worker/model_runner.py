@@ -131,19 +131,21 @@ class AsyncStepOutput:
         toks = self.staging.sampled[:self.nb].tolist()
         r.d2h_bytes += self.nb * 8
         out_ids: list[list[int]] = []
-        for j, rid in enumerate(self.req_ids):
-            if not self.produces[j]:
+        rows, kept, index = [], [], r.req_index
+        for rid, produced, t in zip(self.req_ids, self.produces.tolist(), toks):
+            if not produced:
                 out_ids.append([])
                 continue
-            t = toks[j]
             out_ids.append([t])
-            row = r.req_index.get(rid)
-            if row is None:  # aborted / finished while the step was in flight
-                continue
-            n = r.num_tokens_cpu[row]
-            r.token_ids_cpu[row, n] = t
-            r.num_tokens_cpu[row] = n + 1
-            r.states[rid].output_token_ids.append(t)
+            row = index.get(rid)
+            if row is not None:     # (else aborted / finished while the step was in flight)
+                rows.append(row)
+                kept.append(t)
+                r.states[rid].output_token_ids.append(t)
+        if rows:
+            n = r.num_tokens_cpu[rows]
+            r.token_ids_cpu[rows, n] = kept
+            r.num_tokens_cpu[rows] = n + 1
         lp = self.lp_out
         if isinstance(lp, torch.Tensor):            # packed [nb, 2 k + 3] (ops/cuda.py ``logprobs``) of the rows that produced a token
             a, k = lp.numpy()[np.nonzero(self.produces)[0]], (lp.shape[1] - 3) // 2
@@ -527,7 +529,13 @@ class ModelRunner:
                 self._remove(nr.req_id)
             self._add(nr)
         c = so.scheduled_cached_reqs
-        for i, rid in enumerate(c.req_ids):
+        todo = range(len(c.req_ids))
+        if c.req_ids and not any(c.resumed_from_preemption) and all(rid in self.req_index for rid in c.req_ids):
+            # no row comes back: one assignment for all, and only those that bring tokens or blocks are looked at
+            self.num_computed_cpu[[self.req_index[rid] for rid in c.req_ids]] = c.num_computed_tokens
+            todo = [i for i, (t, b) in enumerate(zip(c.new_token_ids, c.new_block_ids)) if t or b is not None]
+        for i in todo:
+            rid = c.req_ids[i]
             if c.resumed_from_preemption[i] or rid not in self.req_index:
                 # re-admit with its full token history (prompt + outputs so far)
                 st = self._parked.pop(rid, None) or self.states.get(rid)
@@ -1110,7 +1118,7 @@ class ModelRunner:
         total_after = self.num_computed_cpu[rows] + ns
         produces = total_after >= self.num_logical_cpu[rows]  # spec rows: logical count excludes drafts
         lp_out, plp = None, {}
-        req_ids = [self.req_ids[r] for r in rows]
+        req_ids = self.req_ids[:] if nb == B_all else [self.req_ids[r] for r in rows]
         if graph is not None:
             # fast path: temperature / seed / step vectors straight from the per-row arrays
             if not gpu_prep:

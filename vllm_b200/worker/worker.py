@@ -130,6 +130,10 @@ class Worker:
         gpu_sync_debug.arm()      # VLLM_GPU_SYNC_CHECK: from here on the step may not block on the device
 
     # -------------------------------------------------------------- execute
+    def set_async(self, on: bool) -> None:
+        """Whether ``execute_model(non_block=True)`` leaves a step in flight."""
+        self.runner.async_mode = on
+
     @torch.inference_mode()
     def execute_model(self, so: SchedulerOutput, non_block: bool = False):
         pp = pstate.get_pp_group()
