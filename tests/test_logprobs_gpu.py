@@ -52,3 +52,25 @@ def test_captured_steps_match_eager_ones(extra):
             assert {t: v.rank for t, v in x.items()} == {t: v.rank for t, v in y.items()}
             for t in x:
                 assert abs(x[t].logprob - y[t].logprob) < 1e-3
+
+
+@pytest.mark.parametrize("V,k", [(33, 33), (8191, 64), (8193, 5), (8192, 8), (65536, 3), (65537, 20), (131073, 64), (262144, 1), (262145, 11)])       # around the ends of a CTA's and of a cluster's share
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_kernel_takes_ties_in_order_of_their_places(V, k, dtype):
+    from vllm_b200.ops import cuda as cu
+    g = torch.Generator(device="cuda").manual_seed(V)
+    x = torch.randint(-3, 4, (3, V), device="cuda", generator=g).to(dtype)
+    x[0, torch.randperm(V, device="cuda", generator=g)[:V - k // 2]] = float("-inf")        # fewer finite values than the list is long
+    x[1, :V - 1] = -5                                                                       # the likeliest at the very end
+    sampled = torch.tensor([0, V - 1, V // 2], device="cuda")
+    p = cu.logprobs(x, sampled, k)
+    order = x.float().sort(dim=-1, descending=True, stable=True)
+    assert torch.equal(p[:, 1:k + 1].long(), order.indices[:, :k])
+    assert torch.equal(p[:, -1].long(), (x > x.gather(1, sampled[:, None])).sum(-1) + 1)
+    got = p[:, k + 1:2 * k + 2].contiguous().view(torch.float32).double()
+    want = x.double().log_softmax(-1)
+    want = torch.cat([want.gather(1, sampled[:, None]), want.gather(1, order.indices[:, :k])], 1)
+    fin = want.isfinite()
+    assert torch.equal(got.isfinite(), fin)
+    # at most 13 additions of the sum follow one another in a share's tree of roundings after 32 in a thread, each 2^-24 of it; expf and logf a few more
+    assert float((got - want).abs()[fin].max()) < 64 * 2.0 ** -24 * (1 + float(want[fin].abs().max()))

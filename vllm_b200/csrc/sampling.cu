@@ -6,7 +6,7 @@
 // One CTA per row; logits are read once with 16-byte loads straight from the LM-head output
 // dtype (no fp32 staging copy); the noise is a counter-based hash of (seed, step, token) so
 // the result is independent of launch geometry and reproducible per request seed.
-#include "common.cuh"
+#include "warp_mma.cuh"
 
 namespace {
 
@@ -172,6 +172,192 @@ __global__ void __launch_bounds__(1024) logprobs_kernel(const T* __restrict__ lo
     }
     t = top();
   }
+}
+
+// The same for vocabularies of up to 8 x 32 x THREADS tokens: a row is a cluster's, 32 x THREADS values of it a CTA's, 32 a thread's, which holds
+// them in registers for all passes.  The k likeliest are among the values that reach the k-th of the maxima of 2 k groups and more: hardly more than k
+// of them, which the CTAs list and the first one ranks by comparing each with each.  Where the lists are too short for that (equal
+// values, rows that are masked for the most part), a warp takes its k likeliest one by one, the CTA merges its warps' lists, the first CTA those of
+// the cluster.  What bounds it is the chain of exchanges, not the 1.5 MB
+// of 24 such rows: us for k = 5, here and with a CTA per row, 1 row of 32000 6.9 and 15.2, 24 rows 7.5 and 15.7, 24 rows of 102400 18 and 36, of
+// 256000 32 and 89; for k = 64, 1 row of 32000 11 and 136.  Rows of one value, which take the second way: 24 of 32000 24 and 17.
+template <typename T, int THREADS>
+__global__ void __launch_bounds__(THREADS) logprobs_cluster_kernel(const T* __restrict__ logits, int64_t row_stride, int V,
+                                                                   const int64_t* __restrict__ sampled, int k, int* __restrict__ out, int parts) {
+  constexpr int N = Vec16<T>::N, NV = 32 / N, WARPS = THREADS / 32, LIST = 512, ALL = 1024;
+  extern __shared__ float lp_smem[];                 // [WARPS + 1][k] values, then places: of the warps, then of the CTA
+  float* lv = lp_smem;
+  int* li = reinterpret_cast<int*>(lp_smem + (WARPS + 1) * k);
+  __shared__ float red[32];
+  __shared__ float part[2];                          // of the CTA: maximum, sum of exponentials
+  __shared__ float groups[128], row_groups[256];     // maxima of the CTA's groups, of the row's
+  __shared__ int count[2];                           // of the CTA: tokens above the sampled one, listed values
+  __shared__ __align__(8) float2 list[LIST], all[ALL];               // (value, place)
+  pdl_trigger();
+  pdl_wait();
+  const int row = blockIdx.x / parts, rank = blockIdx.x % parts, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const T* lr = logits + (int64_t)row * row_stride;
+  const int base = rank * THREADS * 32;
+  float v[32];                                       // place of v[j N + u]: at(j, u); behind the end -inf
+  auto at = [&](int j, int u) { return base + (j * THREADS + (int)threadIdx.x) * N + u; };
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    if (at(j, N - 1) < V) {
+      const Vec16<T> x = ld16(lr + at(j, 0));
+#pragma unroll
+      for (int u = 0; u < N; ++u) v[j * N + u] = to_f32(x.e[u]);
+    } else {
+#pragma unroll
+      for (int u = 0; u < N; ++u) v[j * N + u] = at(j, u) < V ? to_f32(lr[at(j, u)]) : -INFINITY;
+    }
+  }
+  const int64_t pick = sampled[row];
+  const int sidx = (int)(pick < 0 ? 0 : pick >= V ? V - 1 : pick);
+  const float picked = to_f32(lr[sidx]);
+  if (threadIdx.x < 2) count[threadIdx.x] = 0;
+  float mx = -INFINITY;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) mx = fmaxf(mx, v[j]);
+  int size = 32;                                     // threads of a group: a warp, or fewer where those are not twice the k that are looked for
+  while (parts * THREADS < 2 * k * size) size >>= 1;
+  float gm = mx;
+  for (int o = size >> 1; o > 0; o >>= 1) gm = fmaxf(gm, __shfl_xor_sync(0xffffffffu, gm, o));
+  const int ng = THREADS / size;
+  if (threadIdx.x % size == 0) groups[threadIdx.x / size] = gm;
+  mx = warp_max(gm);
+  if (lane == 0) red[w] = mx;
+  __syncthreads();
+  mx = warp_max(lane < WARPS ? red[lane] : -INFINITY);
+  float sum = 0.f;
+  if (mx != -INFINITY) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) sum += expf(v[j] - mx);             // 0 behind the end
+  }
+  __syncthreads();
+  sum = block_sum(sum, red);
+  if (threadIdx.x == 0) { part[0] = mx; part[1] = sum; }
+  cluster_sync();
+  const float pm = lane < parts ? ld_dsmem_f32(dsmem_addr(smem_u32(&part[0]), lane)) : -INFINITY;
+  const float ps = lane < parts ? ld_dsmem_f32(dsmem_addr(smem_u32(&part[1]), lane)) : 0.f;
+  if (k > 0) {                                       // the k-th of the maxima: no fewer than k values reach it
+    for (int i = threadIdx.x; i < parts * ng; i += THREADS) row_groups[i] = ld_dsmem_f32(dsmem_addr(smem_u32(&groups[i % ng]), i / ng));
+    __syncthreads();
+    for (int i = threadIdx.x; i < parts * ng; i += THREADS) {
+      const float x = row_groups[i];
+      int r = 0;
+      for (int q = 0; q < parts * ng; ++q) r += row_groups[q] > x || (row_groups[q] == x && q < i) ? 1 : 0;
+      if (r == k - 1) red[0] = x;
+    }
+    __syncthreads();
+  }
+  const float bound = red[0];
+  mx = warp_max(pm);
+  const float lsum = logf(warp_sum(pm == -INFINITY ? 0.f : ps * expf(pm - mx)));
+  const float slp = (picked - mx) - lsum;
+  int above = 0;
+#pragma unroll
+  for (int j = 0; j < NV; ++j)
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      const float x = v[j * N + u];
+      above += (x - mx) - lsum > slp ? 1 : 0;        // (nothing behind the end: -inf or NaN on the left)
+      if (k > 0 && x >= bound && at(j, u) < V) {
+        const int n = atomicAdd(&count[1], 1);
+        if (n < LIST) list[n] = make_float2(x, __int_as_float(at(j, u)));
+      }
+    }
+  above = __reduce_add_sync(0xffffffffu, above);
+  if (lane == 0 && above) atomicAdd(&count[0], above);
+  cluster_sync();
+  int* o = out + (int64_t)row * (2 * k + 3);
+  const int c0 = lane < parts ? __float_as_int(ld_dsmem_f32(dsmem_addr(smem_u32(&count[0]), lane))) : 0;
+  const int c1 = lane < parts ? __float_as_int(ld_dsmem_f32(dsmem_addr(smem_u32(&count[1]), lane))) : 0;
+  if (rank == 0 && threadIdx.x == 0) {
+    o[0] = (int)pick;
+    o[k + 1] = __float_as_int(slp);
+  }
+  above = __reduce_add_sync(0xffffffffu, c0);
+  if (rank == 0 && threadIdx.x == 0) o[2 * k + 2] = above + 1;
+  if (k == 0) { cluster_sync(); return; }
+  const int n = __reduce_add_sync(0xffffffffu, c1);
+  if (!__any_sync(0xffffffffu, c1 > LIST) && n <= ALL) {             // the same in all threads of the cluster
+    if (rank == 0) {
+      for (int q = w; q < parts; q += WARPS) {       // a warp copies a CTA's list
+        const int first = __reduce_add_sync(0xffffffffu, lane < q ? c1 : 0), len = __shfl_sync(0xffffffffu, c1, q);
+        for (int i = lane; i < len; i += 32) all[first + i] = ld_dsmem_f32x2(dsmem_addr(smem_u32(&list[i]), q));
+      }
+      __syncthreads();
+      for (int r = n + threadIdx.x; r < k; r += THREADS) {           // (fewer numbers than k: the rest is NaN)
+        o[1 + r] = 0;
+        o[k + 2 + r] = __float_as_int((-INFINITY - mx) - lsum);
+      }
+      for (int i = threadIdx.x; i < n; i += THREADS) {
+        const ArgMax me{all[i].x, __float_as_int(all[i].y)};
+        int r = 0;
+        for (int q = 0; q < n; ++q) r += all[q].x > me.v || (all[q].x == me.v && __float_as_int(all[q].y) < me.i) ? 1 : 0;
+        if (r < k) {
+          o[1 + r] = me.i;
+          o[k + 2 + r] = __float_as_int((me.v - mx) - lsum);
+        }
+      }
+    }
+    cluster_sync();                                  // the first CTA reads the others' lists until here
+    return;
+  }
+  // the likeliest of the thread's behind (value, place) in order
+  auto next = [&](float old, int old_i) {
+    ArgMax b{-INFINITY, 0x7fffffff};
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+#pragma unroll
+      for (int u = 0; u < N; ++u) {
+        const float x = v[j * N + u];
+        const int i = at(j, u);
+        if (i < V && (x < old || (x == old && i > old_i))) b = better(b, ArgMax{x, i});
+      }
+    return b;
+  };
+  auto warp_best = [&](ArgMax b) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) b = better(b, ArgMax{__shfl_xor_sync(0xffffffffu, b.v, o), __shfl_xor_sync(0xffffffffu, b.i, o)});
+    return b;
+  };
+  ArgMax best = next(INFINITY, -1);
+  for (int r = 0; r < k; ++r) {                      // the warp's k likeliest
+    const ArgMax t = warp_best(best);
+    if (lane == 0) { lv[w * k + r] = t.v; li[w * k + r] = t.i; }
+    if (t.i == 0x7fffffff) {                         // (no more than there are)
+      for (int q = r + 1 + lane; q < k; q += 32) { lv[w * k + q] = -INFINITY; li[w * k + q] = 0x7fffffff; }
+      break;
+    }
+    if (best.i == t.i) best = next(t.v, t.i);
+  }
+  // the k likeliest of n sorted lists, a list per lane
+  auto merge = [&](int n, auto value, auto place, auto put) {
+    int mine = 0;
+    ArgMax head = lane < n ? ArgMax{value(lane, 0), place(lane, 0)} : ArgMax{-INFINITY, 0x7fffffff};
+    for (int r = 0; r < k; ++r) {
+      const ArgMax t = warp_best(head);
+      if (lane == 0) put(r, t);
+      if (t.i != 0x7fffffff && head.i == t.i) {
+        ++mine;
+        head = mine < k ? ArgMax{value(lane, mine), place(lane, mine)} : ArgMax{-INFINITY, 0x7fffffff};
+      }
+    }
+  };
+  __syncthreads();
+  if (w == 0)
+    merge(WARPS, [&](int l, int r) { return lv[l * k + r]; }, [&](int l, int r) { return li[l * k + r]; },
+          [&](int r, ArgMax t) { lv[WARPS * k + r] = t.v; li[WARPS * k + r] = t.i; });
+  cluster_sync();
+  if (rank == 0 && w == 0)
+    merge(parts, [&](int l, int r) { return ld_dsmem_f32(dsmem_addr(smem_u32(lv + WARPS * k + r), l)); },
+          [&](int l, int r) { return __float_as_int(ld_dsmem_f32(dsmem_addr(smem_u32(li + WARPS * k + r), l))); },
+          [&](int r, ArgMax t) {
+            o[1 + r] = t.i == 0x7fffffff ? 0 : t.i;
+            o[k + 2 + r] = __float_as_int((t.v - mx) - lsum);
+          });
+  cluster_sync();
 }
 
 // In-place top-k / top-p / min-p masking of fp32 logits (already divided by temperature).
@@ -364,6 +550,18 @@ EXPORT int vb_row_lse(const void* logits, int64_t row_stride, int B, int V, floa
 EXPORT int vb_logprobs(const void* logits, int64_t row_stride, int B, int V, const int64_t* sampled, int k, int* out, int dtype, cudaStream_t st) {
   if (B == 0) return 0;
   if (k < 0 || k > V) return -1;
+  // Clusters for up to 7.5 M values: beyond that there are rows enough for all SMs, and a CTA per row has less to exchange, while k is small (its
+  // cost grows with k).  us for k = 5, clusters and CTAs: 128 rows of 32000 15 and 24, 256 29 and 24, 512 56 and 44; 64 rows of 102400 44 and 50, 128 79 and 58.
+  if (B <= INT32_MAX / 8 && V <= 8 * 32 * 1024 && k <= 64 && (k > 8 || (int64_t)B * V <= 7500000)) {
+    // the smallest CTAs of which eight hold a row
+    const int threads = V <= 8 * 32 * 256 ? 256 : V <= 8 * 32 * 512 ? 512 : 1024, parts = (V + threads * 32 - 1) / (threads * 32);
+    const size_t smem = (size_t)2 * (threads / 32 + 1) * k * 4;
+    DISPATCH_DTYPE(dtype, T, {
+      auto* kernel = threads == 256 ? logprobs_cluster_kernel<T, 256> : threads == 512 ? logprobs_cluster_kernel<T, 512> : logprobs_cluster_kernel<T, 1024>;
+      vb_launch_parts(kernel, dim3(B * parts), dim3(threads), smem, st, parts, reinterpret_cast<const T*>(logits), row_stride, V, sampled, k, out, parts);
+    });
+    return (int)cudaGetLastError();
+  }
   DISPATCH_DTYPE(dtype, T, vb_launch(logprobs_kernel<T>, dim3(B), dim3(1024), 0, st, reinterpret_cast<const T*>(logits), row_stride, V, sampled, k, out));
   return (int)cudaGetLastError();
 }

@@ -819,9 +819,9 @@ def select_candidates(cands: torch.Tensor, W: int, out: torch.Tensor) -> torch.T
 
 
 _logprobs = _sig("vb_logprobs", _vp, _i64, _i, _i, _vp, _i, _vp, _i, _vp)
-# The one-launch kernel picks the k likeliest tokens of V one by one, each at the price of a part of a pass over the row; the library's sort does not
-# grow with k.  us for a row, kernel and library: V 32000, k 5: 21 and 136, k 64: 139 and 137; V 128256, k 20: 137 and 186, k 32: 207 and 186; V
-# 256000, k 5: 96 and 214, k 10: 162 and 211, k 20: 291 and 211 (more rows: the same kernel time up to 64, the library's grows).
+# One launch for what a decode step asks for.  us for a row of 32000, kernel and the library's sort: k 5 7 and 136, k 64 11 and 137; of 128256, k 20: 10
+# and 186; of 256000, k 10: 15 and 211.  Longer lists stay with the sort, whose time depends neither on k nor on how many values are equal: the kernel
+# takes 15 for the 20 likeliest of 256000 normal numbers and 95 where all are one, one CTA per row (vocabularies above 262144, many rows) 278.
 MAX_LOGPROBS, MAX_LOGPROBS_WORK = 64, 3_000_000
 
 
