@@ -1,0 +1,61 @@
+"""Several linear layers of one input in one launch, and router logits read in 16 bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M", [1, 17, 24, 128])
+@pytest.mark.parametrize("K,parts", [(2048, [(1536, "silu", False), (32, None, False), (1, None, False)]), (1024, [(1024, 128, False), (256, None, True), (255, None, True)]),
+                                     (192, [(12, "silu", False), (129, None, True)]), (64, [(8, 4, True), (8, None, False), (1000, None, False), (16640, None, False)])])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_products_of_one_input(M, K, parts, dtype):
+    from vllm_b200.ops import cuda as cu
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    wide = torch.randn(M, K + 8, device="cuda", generator=g).to(dtype)
+    x = wide[:, :K]                                                    # rows at a stride of their own
+    ws = [(torch.randn(n, K, device="cuda", generator=g) * K ** -0.5).to(dtype) for n, _, _ in parts]
+    bs = [torch.randn(n, device="cuda", generator=g).to(dtype) if b else None for n, _, b in parts]
+    forms = [f for _, f, _ in parts]
+    got = cu.linear_parts(x, ws, bs, forms)
+    assert (got is None) == (sum(-(-n // 128) for n, _, _ in parts) > cu.PARTS_TILES)
+    if got is None:
+        return
+    u, tiny = (2.0 ** -8, 0.0) if dtype == torch.bfloat16 else (2.0 ** -11, 2.0 ** -25)
+    for y, w, b, f in zip(got, ws, bs, forms):
+        exact = x.double() @ w.double().T
+        bound = K * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)       # of the sums in 32 bits, in any order
+        if b is not None:
+            exact, bound = exact + b.double(), bound + 2.0 ** -24 * b.double().abs()
+        if f == "silu":
+            gate, up = exact[:, ::2], exact[:, 1::2]
+            want = gate * torch.sigmoid(gate) * up
+            # |silu'| <= 1.1, |silu(g)| <= |g|; a quick exponential and division: a few 2^-22
+            bound = 1.1 * bound[:, ::2] * up.abs() + gate.abs() * bound[:, 1::2] + 1.1 * bound[:, ::2] * bound[:, 1::2] + 2.0 ** -20 * (gate * up).abs()
+        elif f:
+            want, bound = (t.view(M, -1, 2, f).transpose(0, 2).transpose(1, 2).reshape(2, M, -1) for t in (exact, bound))
+        else:
+            want = exact
+        assert y.shape == want.shape and y.dtype == dtype and y.is_contiguous()
+        assert bool(((y.double() - want).abs() <= bound * (1 + u) + u * want.abs() + tiny).all())
+
+
+def test_rows_and_forms_that_are_not_covered():
+    from vllm_b200.ops import cuda as cu
+    x, w = torch.zeros(129, 64, device="cuda", dtype=torch.bfloat16), torch.zeros(128, 64, device="cuda", dtype=torch.bfloat16)
+    assert cu.linear_parts(x, [w, w], [None] * 2, [None] * 2) is None
+    assert cu.linear_parts(x[:4], [w], [None], [None]) is None and cu.linear_parts(x[:4], [w] * 5, [None] * 5, [None] * 5) is None
+    assert cu.linear_parts(x[:4].float(), [w, w], [None] * 2, [None] * 2) is None and cu.linear_parts(x[:4], [w, w.half()], [None] * 2, [None] * 2) is None
+    assert cu.linear_parts(x[:4], [w, w[:, :32]], [None] * 2, [None] * 2) is None and cu.linear_parts(x[:4], [w, w], [None] * 2, [None, 6]) is None
+    assert cu.linear_parts(x[:0], [w, w], [None] * 2, [None] * 2) is None
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("scoring", ["sigmoid", "softmax"])
+def test_router_logits_in_16_bits(dtype, scoring):
+    from vllm_b200.ops import cuda as cu
+    g = torch.Generator(device="cuda").manual_seed(3)
+    lg = torch.randn(37, 32, device="cuda", generator=g).to(dtype)
+    bias = torch.randn(32, device="cuda", generator=g)
+    a, b = (cu.grouped_topk(t, 6, 4, 2, True, scoring, bias, 2.5) for t in (lg, lg.float()))
+    assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])

@@ -54,6 +54,20 @@ struct Params {
   long long* trace;        // debug: per-CTA clock64 stamps [cta][16] (null in production)
 };
 
+// Several matrices of one K applied to the same rows (SWAP only): the tiles of part i are those from first[i] on along grid x.  A decode step's
+// small products cost 3.5 to 5 us each whatever they read (launch, first bytes, exchange of the splits), so those of one input go together.  Of a
+// captured step, for 24 rows of 2048: 1536 gated, 32 and 1 outputs 4.9 us (4.4, 3.9 and 3.6 in turn); 4096, 512 and 512, the first ones split into
+// queries and gates, 8.6 (8.2, 5.7 and 3.8, and 5.5 for the two copies).
+constexpr int MAX_PARTS = 4;
+struct Parts {
+  CUtensorMap map[MAX_PARTS];
+  int first[MAX_PARTS], N[MAX_PARTS], act[MAX_PARTS];
+  int run[MAX_PARTS];      // not 0: the outputs are pairs of runs of this many; the first runs of all rows lie before the second runs, [2, M, N / 2]
+  void* y[MAX_PARTS];
+  const void* bias[MAX_PARTS];
+};
+struct One { CUtensorMap map[1]; };
+
 VB_DEVICE void red_add_f32(float* p, float v) { asm volatile("red.relaxed.gpu.global.add.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory"); }
 VB_DEVICE void red_add_f32_sys(float* p, float v) {
   asm volatile("red.relaxed.sys.global.add.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
@@ -67,9 +81,10 @@ template <int BN> struct SmemLayout {
 
 // STAGES <= 4 is the two-CTAs-per-SM variant (smem <= 113 KB): used when the grid has more tiles than SMs, so the
 // prologue / epilogue of one tile overlaps the weight stream of its neighbour instead of leaving the SM idle.
-template <typename T, int BN, int STAGES, bool SWAP>
+template <typename T, int BN, int STAGES, bool SWAP, typename A = One>
 __global__ void __launch_bounds__(NUM_THREADS, STAGES <= 4 && BN <= 128 ? 2 : 1)
-gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const Params p) {
+gemm_kernel(const __grid_constant__ A a, const __grid_constant__ CUtensorMap tmap_b, const Params p) {
+  constexpr bool PARTS = !std::is_same<A, One>::value;
   using L = SmemLayout<BN>;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -81,7 +96,26 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // tile coordinates: A-operand tile index (x), B-operand tile index (y), K split (z)
-  const int a_tile = blockIdx.x, b_tile = blockIdx.y, split = blockIdx.z;
+  const int b_tile = blockIdx.y, split = blockIdx.z;
+  int a_tile = blockIdx.x, part = 0;
+  if constexpr (PARTS) {
+#pragma unroll
+    for (int i = 1; i < MAX_PARTS; ++i) part = (int)blockIdx.x >= a.first[i] ? i : part;
+    a_tile -= a.first[part];
+  }
+  const CUtensorMap& tmap_a = a.map[part];
+  int N = p.N, act = p.act;
+  void* out = p.y;
+  const void* bias_at = p.bias;
+  if constexpr (PARTS) { N = a.N[part]; act = a.act[part]; out = a.y[part]; bias_at = a.bias[part]; }
+  auto at = [&](T* y, int m, int n) -> T* {
+    if constexpr (PARTS)
+      if (const int run = a.run[part]) {
+        const int h = n / (2 * run), r = n - 2 * run * h, second = r >= run ? 1 : 0;
+        return y + ((size_t)second * p.M + m) * (N >> 1) + h * run + r - second * run;
+      }
+    return y + (size_t)m * N + n;
+  };
   const int kb0 = split * p.k_blocks_per_split;
   const int total_kb = (p.K + BK - 1) / BK;
   const int nkb = max(0, min(p.k_blocks_per_split, total_kb - kb0));
@@ -127,7 +161,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       b_row0 = p.expert_offs[e] + chunk * BN;
       m_lim = p.expert_offs[e + 1] - b_row0;
       if (m_lim <= 0) return;               // no token of this chunk routed to expert e: nothing to stream
-      a_row0 += e * p.N;
+      a_row0 += e * N;
     }
   }
   if (warp == 0 && lane == 0) {
@@ -250,7 +284,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       do_store = false;
     }
     if (do_store) {
-      T* y = reinterpret_cast<T*>(p.y);
+      T* y = reinterpret_cast<T*>(out);
       for (int c = 0; c < BN; c += CH) {
         float v[CH];
         load_chunk(c, v);
@@ -264,46 +298,46 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
               const float val = v[j] * p.pair_w[pair];
               const int tok = pair / p.red_k;
               const size_t off = (size_t)tok * p.red_H + n;
-              if (n < p.N) {
+              if (n < N) {
                 if (p.red_world > 1) red_add_f32_sys(p.red_peer[tok / p.red_per] + off, val);
                 else red_add_f32(p.red_acc + off, val);
               }
             }
           }
-        } else if (SWAP && p.act == 1) {
+        } else if (SWAP && act == 1) {
           // rows interleave (gate_i, up_i): even lane holds gate, odd lane up → y[tok, i] = silu(gate) * up
           const int n = a_tile * TM + row;
           const int m0 = b_row0 + c;
-          const int n_out = p.N >> 1;
+          const int n_out = N >> 1;
 #pragma unroll
           for (int j = 0; j < CH; ++j) {
             const float other = __shfl_xor_sync(0xffffffffu, v[j], 1);
             const float g = v[j];
             const float r = (g / (1.f + __expf(-g))) * other;
-            if ((lane & 1) == 0 && n < p.N && c + j < m_lim) y[(size_t)(m0 + j) * n_out + (n >> 1)] = from_f32<T>(r);
+            if ((lane & 1) == 0 && n < N && c + j < m_lim) y[(size_t)(m0 + j) * n_out + (n >> 1)] = from_f32<T>(r);
           }
         } else if (SWAP) {
           // accumulator is Y^T: row = output feature, column = token
           const int n = a_tile * TM + row;
-          if (n < p.N) {
-            const float bias = p.bias ? to_f32(reinterpret_cast<const T*>(p.bias)[n]) : 0.f;
+          if (n < N) {
+            const float bias = bias_at ? to_f32(reinterpret_cast<const T*>(bias_at)[n]) : 0.f;
             const int m0 = b_row0 + c;
 #pragma unroll
             for (int j = 0; j < CH; ++j)
               if (c + j < m_lim) {
                 float o = v[j] + bias;
-                if (p.act == 2) { o = fmaxf(o, 0.f); o *= o; }
-                if (p.act == 3) o = xielu16(o, p.act_coef[0], p.act_coef[1]);
-                y[(size_t)(m0 + j) * p.N + n] = from_f32<T>(o);
+                if (act == 2) { o = fmaxf(o, 0.f); o *= o; }
+                if (act == 3) o = xielu16(o, p.act_coef[0], p.act_coef[1]);
+                *at(y, m0 + j, n) = from_f32<T>(o);
               }
           }
         } else {
           const int m = a_tile * TM + row;
           if (m < p.M) {
             const int n0 = b_tile * BN + c;
-            T* yr = y + (size_t)m * p.N + n0;
-            const T* bp = p.bias ? reinterpret_cast<const T*>(p.bias) + n0 : nullptr;
-            if (n0 + CH <= p.N && (p.N % 8) == 0) {
+            T* yr = y + (size_t)m * N + n0;
+            const T* bp = bias_at ? reinterpret_cast<const T*>(bias_at) + n0 : nullptr;
+            if (n0 + CH <= N && (N % 8) == 0) {
 #pragma unroll
               for (int j = 0; j < CH; j += 8) {
                 Vec16<T> o;
@@ -314,7 +348,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             } else {
 #pragma unroll
               for (int j = 0; j < CH; ++j)
-                if (n0 + j < p.N) yr[j] = from_f32<T>(v[j] + (bp ? to_f32(bp[j]) : 0.f));
+                if (n0 + j < N) yr[j] = from_f32<T>(v[j] + (bp ? to_f32(bp[j]) : 0.f));
             }
           }
         }
@@ -333,7 +367,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       if (warp >= 2) {
         const int et = threadIdx.x - 64;
         if (et == 0) VB_TRACE(7);
-        T* y = reinterpret_cast<T*>(p.y);
+        T* y = reinterpret_cast<T*>(out);
         const int m_base = b_row0;
         const int cols = min(BN, m_lim);                           // real tokens in this tile
         const int units = cols * (TM / 4);                         // unit = 4 consecutive features of one token
@@ -364,30 +398,30 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
               if (r < p.splits) { acc.x += x[h][r].x; acc.y += x[h][r].y; acc.z += x[h][r].z; acc.w += x[h][r].w; }
             const int n = a_tile * TM + rq * 4;
             float o[4] = {acc.x, acc.y, acc.z, acc.w};
-            if (p.act == 1) {      // (gate, up) pairs are adjacent features: two outputs per unit
-              if (n + 4 <= p.N) {
-                T* ya = y + (size_t)(m_base + col) * (p.N >> 1) + (n >> 1);
+            if (act == 1) {      // (gate, up) pairs are adjacent features: two outputs per unit
+              if (n + 4 <= N) {
+                T* ya = y + (size_t)(m_base + col) * (N >> 1) + (n >> 1);
                 const uint32_t pk = pack2<T>((o[0] / (1.f + __expf(-o[0]))) * o[1], (o[2] / (1.f + __expf(-o[2]))) * o[3]);
                 *reinterpret_cast<uint32_t*>(ya) = pk;
               }
               continue;
             }
-            T* yr = y + (size_t)(m_base + col) * p.N + n;
-            if (p.bias) {
+            T* yr = at(y, m_base + col, n);
+            if (bias_at) {
 #pragma unroll
-              for (int e = 0; e < 4; ++e) if (n + e < p.N) o[e] += to_f32(reinterpret_cast<const T*>(p.bias)[n + e]);
+              for (int e = 0; e < 4; ++e) if (n + e < N) o[e] += to_f32(reinterpret_cast<const T*>(bias_at)[n + e]);
             }
-            if (p.act == 3) {
+            if (act == 3) {
 #pragma unroll
               for (int e = 0; e < 4; ++e) o[e] = xielu16(o[e], p.act_coef[0], p.act_coef[1]);
             }
-            if (n + 4 <= p.N && (p.N & 3) == 0) {
+            if (n + 4 <= N && (N & 3) == 0) {
               uint2 pk;
               pk.x = pack2<T>(o[0], o[1]); pk.y = pack2<T>(o[2], o[3]);
               *reinterpret_cast<uint2*>(yr) = pk;
             } else {
 #pragma unroll
-              for (int e = 0; e < 4; ++e) if (n + e < p.N) yr[e] = from_f32<T>(o[e]);
+              for (int e = 0; e < 4; ++e) if (n + e < N) yr[e] = from_f32<T>(o[e]);
             }
           }
         }
@@ -420,11 +454,11 @@ static int make_tmap(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t co
   return r == CUDA_SUCCESS ? 0 : -11;
 }
 
-template <typename T, int BN, int STAGES, bool SWAP>
-static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, dim3 grid, cudaStream_t st) {
+template <typename T, int BN, int STAGES, bool SWAP, typename A>
+static int launch(const A& ta, const CUtensorMap& tb, const Params& p, dim3 grid, cudaStream_t st) {
   using L = SmemLayout<BN>;
   const int smem = STAGES * L::STAGE_BYTES + (2 * STAGES + 1) * 8 + 16 + 1024;
-  auto k = gemm_kernel<T, BN, STAGES, SWAP>;
+  auto k = gemm_kernel<T, BN, STAGES, SWAP, A>;
   static bool attr = false;
   if (!attr) { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); attr = true; }
   if (grid.z > 1) vb_launch_cluster(k, grid, dim3(NUM_THREADS), (size_t)smem, st, grid.z, ta, tb, p);
@@ -509,7 +543,8 @@ EXPORT int vb_gemm_tc2(const void* x, const void* w, const void* bias, void* y, 
   if (dtype == DT_F32 || K % 8 != 0) return -1;
   if (act && (!swap || !(act == 1 ? !bias && !(N & 3) : act == 3 && act_coef))) return -1;
   const bool bf16 = dtype == DT_BF16;
-  CUtensorMap ta, tb;
+  One ta;
+  CUtensorMap tb;
   Params p;
   p.trace = g_trace;
   p.expert_offs = nullptr; p.n_experts = 0; p.flat = 0; p.red_acc = nullptr; p.row_pair = nullptr; p.pair_w = nullptr; p.red_k = 1; p.red_H = 0; p.red_world = 1; p.red_per = 1;
@@ -520,7 +555,7 @@ EXPORT int vb_gemm_tc2(const void* x, const void* w, const void* bias, void* y, 
   p.k_blocks_per_split = (kb + splits - 1) / splits;
   int rc;
   if (swap) {
-    if ((rc = make_tmap(&ta, w, N, K, K, TM, bf16))) return rc;
+    if ((rc = make_tmap(&ta.map[0], w, N, K, K, TM, bf16))) return rc;
     if ((rc = make_tmap(&tb, x, M, K, x_stride, bn, bf16))) return rc;
     dim3 grid((N + TM - 1) / TM, (M + bn - 1) / bn, splits);
     static int n_sms = 0;
@@ -551,7 +586,7 @@ EXPORT int vb_gemm_tc2(const void* x, const void* w, const void* bias, void* y, 
     }
 #undef GO
   } else {
-    if ((rc = make_tmap(&ta, x, M, K, x_stride, TM, bf16))) return rc;
+    if ((rc = make_tmap(&ta.map[0], x, M, K, x_stride, TM, bf16))) return rc;
     if ((rc = make_tmap(&tb, w, N, K, K, bn, bf16))) return rc;
     dim3 grid((M + TM - 1) / TM, (N + bn - 1) / bn, 1);
     if (bn != 128) return -2;
@@ -560,6 +595,46 @@ EXPORT int vb_gemm_tc2(const void* x, const void* w, const void* bias, void* y, 
   }
 }
 
+// y[i] = act(x w[i]^T + bias[i]) for n matrices [N[i], K] at once, M <= 128 rows; act as above (0 or 1), splits from the plan for all their tiles
+// run[i] (act 0, a multiple of 4): see Parts
+EXPORT int vb_gemm_tc_parts(const void* x, const void* const* w, const void* const* bias, void* const* y, const int* N, const int* act, const int* run, int n,
+                            int M, int K, int64_t x_stride, int bn, int splits, int dtype, cudaStream_t st) {
+  using namespace gemm;
+  if (dtype == DT_F32 || K % 8 != 0 || n < 1 || n > MAX_PARTS || M < 1 || M > bn || bn > 128 || bn % 16 || splits < 1 || splits > 8) return -1;
+  const bool bf16 = dtype == DT_BF16;
+  Parts ta = {};
+  CUtensorMap tb;
+  Params p = {};
+  p.M = M; p.K = K; p.splits = splits; p.red_k = 1; p.red_world = 1; p.red_per = 1;
+  p.k_blocks_per_split = ((K + BK - 1) / BK + splits - 1) / splits;
+  int rc, tiles = 0;
+  for (int i = 0; i < MAX_PARTS; ++i) {
+    ta.first[i] = i < n ? tiles : INT32_MAX;
+    if (i >= n) continue;
+    if (act[i] && (act[i] != 1 || bias[i] || (N[i] & 3) || run[i])) return -1;
+    if (run[i] < 0 || run[i] % 4 || (run[i] && N[i] % (2 * run[i]))) return -1;
+    if ((rc = make_tmap(&ta.map[i], w[i], N[i], K, K, TM, bf16))) return rc;
+    ta.N[i] = N[i]; ta.act[i] = act[i]; ta.run[i] = run[i]; ta.y[i] = y[i]; ta.bias[i] = bias[i];
+    tiles += (N[i] + TM - 1) / TM;
+  }
+  if ((rc = make_tmap(&tb, x, M, K, x_stride, bn, bf16))) return rc;
+  const dim3 grid(tiles, 1, splits);
+#define GOP(BNV, ST)                                                                     \
+    if (bf16) return launch<__nv_bfloat16, BNV, ST, true>(ta, tb, p, grid, st);          \
+    else return launch<__half, BNV, ST, true>(ta, tb, p, grid, st);
+  switch (bn) {
+    case 16: GOP(16, 8)
+    case 32: GOP(32, 8)
+    case 48: GOP(48, 8)
+    case 64: GOP(64, 8)
+    case 80: GOP(80, 6)
+    case 96: GOP(96, 6)
+    case 112: GOP(112, 6)
+    case 128: GOP(128, 6)
+    default: return -2;
+  }
+#undef GOP
+}
 
 // Grouped (MoE) GEMM: Y[r, :] = X[r, :] · W[e(r)]^T for rows sorted by expert; offs[e] .. offs[e+1] delimit expert e.
 // X: [R, K], W: [E, N, K] contiguous, Y: [R, N].  bn = token-tile width (16..128), every expert gets
@@ -597,7 +672,8 @@ static int grouped_impl(const void* x, const void* w, void* y, const int* offs, 
   using namespace gemm;
   if (dtype == DT_F32 || K % 8 != 0 || bn > 128 || bn % 16) return -1;
   const bool bf16 = dtype == DT_BF16;
-  CUtensorMap ta, tb;
+  One ta;
+  CUtensorMap tb;
   Params p;
   p.trace = nullptr; p.pf = 0;
   p.y = y; p.bias = nullptr; p.ws = nullptr; p.counters = nullptr; p.M = R; p.N = N; p.K = K; p.splits = 1; p.act = act; p.act_coef = nullptr;
@@ -609,7 +685,7 @@ static int grouped_impl(const void* x, const void* w, void* y, const int* offs, 
   const int kb = (K + BK - 1) / BK;
   p.k_blocks_per_split = kb;
   int rc;
-  if ((rc = make_tmap(&ta, w, (uint64_t)E * N, K, K, TM, bf16))) return rc;
+  if ((rc = make_tmap(&ta.map[0], w, (uint64_t)E * N, K, K, TM, bf16))) return rc;
   if ((rc = make_tmap(&tb, x, R, K, K, bn, bf16))) return rc;
   const int chunks = (R + bn - 1) / bn;
   dim3 grid((N + TM - 1) / TM, flat ? R / bn + (E < R ? E : R) : E * chunks, 1);

@@ -84,6 +84,27 @@ class ReplicatedLinear(LinearBase):
         param.data.copy_(w)
 
 
+def products(x: torch.Tensor, *parts) -> list:
+    """The results of several layers for one input, one launch for all in decode.  A part is (layer, form): form None is the layer's own result,
+    "silu" that of ``forward_gated_silu``, n the two results between which the layer's outputs alternate in runs of n."""
+    layers, forms = [p[0] for p in parts], [p[1] for p in parts]
+    if all(type(m.quant_method) is LinearMethod and not m.lora_table for m in layers):
+        got = ops.linear_parts(x, [m.weight for m in layers], [m.bias for m in layers], forms)
+        if got is not None:
+            return got
+    out = []
+    for m, form in parts:
+        if form == "silu":
+            out.append(m.forward_gated_silu(x))
+            continue
+        y = m(x)
+        if form is not None:
+            pairs = y.view(*y.shape[:-1], -1, 2, form)
+            y = [pairs[..., i, :].reshape(*y.shape[:-1], -1) for i in (0, 1)]
+        out.append(y)
+    return out
+
+
 class MergedReplicatedLinear(ReplicatedLinear):
     """Several replicated matrices over the same input, stacked along the output dim (one GEMM).  ``align``: every part starts
     at a multiple of this many outputs (zero rows between), so that its columns of the result can be read in vectors."""

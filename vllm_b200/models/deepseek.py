@@ -21,7 +21,7 @@ from vllm_b200.config import VllmConfig
 from vllm_b200.layers.attention import MLAAttentionCore
 from vllm_b200.layers.common import RMSNorm
 from vllm_b200.layers.latent import LatentForms, step_limits
-from vllm_b200.layers.linear import (ColumnParallelLinear, ReplicatedLinear, RowParallelLinear,
+from vllm_b200.layers.linear import (ColumnParallelLinear, ReplicatedLinear, RowParallelLinear, products,
                                      tp_reduce_residual_norm)
 from vllm_b200.layers.moe import FusedMoE
 from vllm_b200.layers.rotary import get_rope, yarn_mscale
@@ -93,10 +93,11 @@ class DeepseekMLA(LatentForms, nn.Module):
     def forward(self, positions: torch.Tensor, hidden: torch.Tensor) -> torch.Tensor:
         T = hidden.shape[0]
         if self.q_lora:
-            q = self.q_b_proj(self.q_a_layernorm(self.q_a_proj(hidden)))
+            q, lat = products(hidden, (self.q_a_proj, None), (self.kv_a_proj_with_mqa, None))
+            q = self.q_b_proj(self.q_a_layernorm(q))
         else:
             q = self.q_proj(hidden)
-        lat = self.kv_a_proj_with_mqa(hidden)
+            lat = self.kv_a_proj_with_mqa(hidden)
         md, cache = self.attn.bound_cache()
         if md is not None and self._fused(q, lat, md, cache):
             ops.cuda_ops().mla_rope_cache(q, lat, self.local_heads, self.nope, self.rope_dim, self.kv_lora, self.kv_a_layernorm.weight,
@@ -140,15 +141,18 @@ class DeepseekMoE(nn.Module):
             self.shared_experts.down_proj.reduce_results = False
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        out = self.experts(x, self.gate(x).float())
+        out = self.experts(x, self.gate(x))
         if self.shared_experts is not None:
             out = out + self.shared_experts(x)
         return out          # per-rank partial sum
 
     def forward_reduce_norm(self, x: torch.Tensor, residual: torch.Tensor, norm) -> tuple[torch.Tensor, torch.Tensor]:
         """(normed, residual) = norm(all_reduce(block(x)) + residual)."""
-        shared = self.shared_experts(x) if self.shared_experts is not None else None
-        logits = self.gate(x).float()
+        if self.shared_experts is None:
+            shared, logits = None, self.gate(x)
+        else:
+            h, logits = products(x, self.shared_experts.up_part(), (self.gate, None))
+            shared = self.shared_experts.down(h)
         got = self.experts.rows_reduce_norm(x, logits, residual, norm, shared)
         if got is not None:
             return got

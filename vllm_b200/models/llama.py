@@ -42,6 +42,13 @@ class LlamaMLP(nn.Module):
             return self.gate_up_proj.forward_gated_silu(x)
         return self.act(self.gate_up_proj(x))
 
+    def up_part(self) -> tuple:
+        """This block's first product as a part of ``layers.linear.products``; ``down`` takes its result."""
+        return self.gate_up_proj, "silu" if self.gate_up_proj.interleave else None
+
+    def down(self, h):
+        return self.down_proj(h if self.gate_up_proj.interleave else self.act(h))
+
     def forward(self, x):
         return self.down_proj(self._gated(x))
 

@@ -13,7 +13,7 @@ import torch.nn as nn
 
 from vllm_b200.config import VllmConfig
 from vllm_b200.layers.common import RMSNorm
-from vllm_b200.layers.linear import ReplicatedLinear, tp_reduce_residual_norm
+from vllm_b200.layers.linear import ReplicatedLinear, products, tp_reduce_residual_norm
 from vllm_b200.layers.moe import FusedMoE
 from vllm_b200.models.llama import LlamaAttention, LlamaForCausalLM, LlamaMLP, LlamaModel
 from vllm_b200.parallel.state import get_tp_group
@@ -55,9 +55,15 @@ class SparseMoeBlock(nn.Module):
 
     def forward_reduce_norm(self, x: torch.Tensor, residual: torch.Tensor, norm) -> tuple[torch.Tensor, torch.Tensor]:
         """(normed, residual) = norm(all_reduce(block(x)) + residual)."""
-        shared = self.shared_expert(x) if self.shared_expert is not None else None
-        gate = self.shared_expert_gate(x) if self.shared_expert_gate is not None else None
-        logits = self.gate(x)
+        shared = gate = None
+        if self.shared_expert is None:
+            logits = self.gate(x)
+        else:
+            parts = [self.shared_expert.up_part(), (self.gate, None)]
+            if self.shared_expert_gate is not None:
+                parts.append((self.shared_expert_gate, None))
+            h, logits, *rest = products(x, *parts)
+            shared, gate = self.shared_expert.down(h), rest[0] if rest else None
         got = self.experts.rows_reduce_norm(x, logits, residual, norm, shared, gate)
         if got is not None:
             return got

@@ -22,7 +22,7 @@ from vllm_b200.forward_context import get_forward_context
 from vllm_b200.layers import attention as _attn
 from vllm_b200.layers.attention import Attention
 from vllm_b200.layers.common import RMSNorm
-from vllm_b200.layers.linear import ReplicatedLinear
+from vllm_b200.layers.linear import ReplicatedLinear, products
 from vllm_b200.layers.rotary import get_rope
 from vllm_b200.models.llama import LlamaMLP
 from vllm_b200.models.mixtral import Qwen2MoeForCausalLM, Qwen2MoeModel, SparseMoeBlock
@@ -113,7 +113,7 @@ class GatedDeltaNet(nn.Module):
         ctx = get_forward_context()
         md = ctx.metadata_for(self.layer_name)
         cache = ctx.kv_caches.get(self.layer_name)
-        qkvz, ba = self.in_proj_qkvz(hidden), self.in_proj_ba(hidden)
+        qkvz, ba = products(hidden, (self.in_proj_qkvz, None), (self.in_proj_ba, None))
         T, dev = hidden.shape[0], hidden.device
         from vllm_b200.layers.mamba import _cuda_ssm
         if md is not None and cache is not None and _cuda_ssm(qkvz) and self.dk % 32 == 0 and self.dk <= 256 and 2 <= self.k <= 4:
@@ -193,11 +193,9 @@ class GatedAttention(nn.Module):
         self.attn = Attention(nh, self.hd, self.hd ** -0.5, self.nkv, prefix=f"{prefix}.attn", rope=rope)
 
     def forward(self, positions, hidden):
-        T = hidden.shape[0]
-        qg = self.q_proj(hidden).view(T, self.nh, 2 * self.hd)
-        q, gate = qg[..., :self.hd].reshape(T, -1), qg[..., self.hd:].reshape(T, -1)
+        (q, gate), k, v = products(hidden, (self.q_proj, self.hd), (self.k_proj, None), (self.v_proj, None))
         # norms, rotation and cache write are one launch; the gate is applied in place
-        return self.o_proj(self.attn(q, self.k_proj(hidden), self.v_proj(hidden), positions, qk_norm=(self.q_norm, self.k_norm), gate=gate))
+        return self.o_proj(self.attn(q, k, v, positions, qk_norm=(self.q_norm, self.k_norm), gate=gate))
 
 
 class Qwen3NextDecoderLayer(nn.Module):

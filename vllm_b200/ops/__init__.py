@@ -370,6 +370,11 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     return torch.nn.functional.linear(x, weight, bias)
 
 
+def linear_parts(x: torch.Tensor, weights, biases, forms) -> Optional[list]:
+    """Several linear layers of one input at once (csrc/gemm_tc.cu), or None where each is better off alone; ``forms`` as in ops/cuda.py."""
+    return cuda_ops().linear_parts(x, weights, biases, forms) if _use_cuda(x) else None
+
+
 def topk_softmax(gating, k, renormalize):
     if _use_cuda(gating):
         return cuda_ops().topk_softmax(gating, k, renormalize)

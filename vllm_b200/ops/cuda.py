@@ -1078,6 +1078,37 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     return torch.nn.functional.linear(x, weight, bias)
 
 
+_gemm_parts = _sig("vb_gemm_tc_parts", _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i, _i, _i, _vp)
+MAX_PARTS, PARTS_ROWS, PARTS_TILES = 4, 128, 132        # as many tiles as have a CTA each: beyond that two to an SM, which only the single product has
+
+
+def linear_parts(x: torch.Tensor, weights, biases, forms) -> Optional[list]:
+    """x W_i^T (+ b_i) for up to four matrices in one launch, for rows that ``linear`` would give to ``gemm_tc`` one product at a time.  ``forms``: None;
+    "silu" (W's rows interleave gate and up, the result is silu(gate) * up); or n (the outputs alternate between two results in runs of n: a tensor of
+    both).  None = not covered."""
+    x2 = x.reshape(-1, x.shape[-1])
+    M, K = x2.shape
+    tiles = sum(-(-w.shape[0] // 128) for w in weights)
+    if (not 0 < M <= PARTS_ROWS or not 1 < len(weights) <= MAX_PARTS or tiles > PARTS_TILES or envs.VLLM_B200_GEMM_SK or batch_invariant()
+            or not all(w.shape[1] == K and _tc_ok(x2, w) for w in weights)):
+        return None
+    outs = []
+    for w, b, f in zip(weights, biases, forms):
+        N = w.shape[0]
+        if (f == "silu" and (N % 4 or b is not None)) or (isinstance(f, int) and (f % 4 or N % (2 * f))) or (b is not None and b.dtype != x.dtype):
+            return None
+        outs.append(torch.empty((2, M, N // 2) if isinstance(f, int) else (M, N // 2 if f == "silu" else N), dtype=x.dtype, device=x.device))
+    _, bn, splits, _, _ = _plan(M, tiles * 128, K)
+    n = len(weights)
+    ptrs, ints = ctypes.c_void_p * n, _i * n
+    _check(_gemm_parts(x2.data_ptr(), ptrs(*[w.data_ptr() for w in weights]), ptrs(*[_p(b) for b in biases]), ptrs(*[y.data_ptr() for y in outs]),
+                       ints(*[w.shape[0] for w in weights]), ints(*[int(f == "silu") for f in forms]),
+                       ints(*[f if isinstance(f, int) else 0 for f in forms]), n, M, K, x2.stride(0), bn, splits, _DT[x.dtype], _st()),
+           f"linear_parts(M={M},N={[w.shape[0] for w in weights]},K={K})")
+    lead = x.shape[:-1]
+    return [y.view((2,) + lead + (-1,)) if isinstance(f, int) else y.view(lead + (-1,)) for y, f in zip(outs, forms)]
+
+
 # ------------------------------------------------------------------ symmetric-heap collectives
 _comm_ar_rows = _sig("vb_comm_allreduce_rows", _vp, _vp, _vp, _vp, _i, _i, _vp, _i64, _i64, _vp, _vp, _f, _i, _i, _i,
                      _i, _i, _vp)
@@ -1307,13 +1338,15 @@ def grouped_simt(x: torch.Tensor, w: torch.Tensor, offs: torch.Tensor, R: int, r
 
 def grouped_topk(scores, k, n_group, topk_group, renormalize, scoring="sigmoid", bias=None, routed_scaling_factor=1.0, group_score=None):
     T, E = scores.shape
-    lg = scores.float().contiguous()
+    lg = scores.contiguous()
+    half = lg.dtype in (torch.bfloat16, torch.float16)         # read as they are
+    lg = lg if half else lg.float()
     w = torch.empty((T, k), dtype=torch.float32, device=scores.device)
     ids = torch.empty((T, k), dtype=torch.int32, device=scores.device)
     b = None if bias is None else bias.float().contiguous()
-    _check(_grouped_topk(lg.data_ptr(), None, 0, None, 0, _p(b), w.data_ptr(), ids.data_ptr(), T, E, k, n_group,
+    _check(_grouped_topk(None if half else lg.data_ptr(), lg.data_ptr() if half else None, 0, None, 0, _p(b), w.data_ptr(), ids.data_ptr(), T, E, k, n_group,
                          topk_group if n_group > 1 else 1, _group_top2(group_score, bias), int(scoring != "sigmoid"), int(renormalize),
-                         float(routed_scaling_factor), 2, _st()), f"grouped_topk(E={E},k={k})")
+                         float(routed_scaling_factor), _DT[lg.dtype], _st()), f"grouped_topk(E={E},k={k})")
     return w, ids
 
 
