@@ -32,9 +32,29 @@ def grouped_rows(x, w13, w2, topk_ids, act, expert_map):
     ids = topk_ids if topk_ids.dtype == torch.int32 else topk_ids.to(torch.int32)
     sorted_tok, inv, offs = cu.moe_align(ids.contiguous(), E, expert_map)
     bn = _tile_width(R, E)
+    if streamed(R, w13, act):
+        bn = _stream_width(bn)
+        return cu.gemm_experts(cu.gemm_experts(cu.moe_gather(x, sorted_tok), w13, offs, bn, act), w2, offs, bn), inv
     flat = flat_grid(R, E, bn)
     h = cu.gemm_tc_grouped(cu.moe_gather(x, sorted_tok), w13, offs, bn, flat=flat)
     return cu.gemm_tc_grouped(cu.act_and_mul(h, act), w2, offs, bn, flat=flat), inv
+
+
+def streamed(R: int, w13, act) -> bool:
+    """Does csrc/gemm_experts.cu (a block per SM whose ring runs through all its tiles) take the products of R pairs rather than gemm_tc.cu (a block per
+    tile)?  From three pairs per expert on, and from one on where 16 experts and more spread over the SMs; with fewer, some SMs have one tile more than
+    the others and little else to read meanwhile.  us of both products, gemm_tc.cu (with the activation between them) → gemm_experts.cu: 2048 x 768, 32
+    experts, 6 of them for each of 4 tokens 35 → 35, 8 tokens 42 → 38, 24 58 → 49, 128 64 → 55 (the weights' bytes take 47); 8 of 2048 x 2048, 2 for each of 4
+    tokens 32 → 35, 8 38 → 37, 16 41 → 36, 128 48 → 41 (31); 16 of 1024 x 512, 4 for each of 4 tokens 17 → 14, 64 30 → 16 (8); 128 of 2048 x 768, 8
+    for each of 4 tokens 56 → 54, 16 134 → 121, 128 203 → 185 (187).  Not in batch-invariant mode, which rounds the hidden rows before the activation."""
+    from vllm_b200.ops import cuda as cu
+    E, N, _ = w13.shape
+    return act in cu._GATED_ACT and N % 128 == 0 and E <= cu.GROUPED_MAX_EXPERTS and (R >= 3 * E or R >= E >= 16) and not cu.batch_invariant()
+
+
+def _stream_width(bn: int) -> int:
+    """Rows of an expert at a time there: of its four widths the one for ``_tile_width``'s.  64 for up to 40 rows on average, which 58 seldom exceed."""
+    return 16 if bn <= 16 else 32 if bn <= 32 else 64 if bn <= 80 else 128
 
 
 def flat_grid(R: int, E: int, bn: int) -> bool:
@@ -211,8 +231,11 @@ def fused_moe_reduce_norm(x, w13, w2, topk_w, topk_ids, act, expert_map, residua
     bn = 16
     while bn < 128 and bn < 2 * avg:
         bn += 16
-    h = cu.gemm_tc_grouped(xs, w13, offs, bn)
-    a = cu.act_and_mul(h, act)
+    stream = streamed(R, w13, act)
+    if stream:
+        a = cu.gemm_experts(xs, w13, offs, _stream_width(bn), act)
+    else:
+        a = cu.act_and_mul(cu.gemm_tc_grouped(xs, w13, offs, bn), act)
     pw = topk_w.to(torch.float32).contiguous()
     if multi:
         acc_off = comm.next_moe_acc()
@@ -226,7 +249,10 @@ def fused_moe_reduce_norm(x, w13, w2, topk_w, topk_ids, act, expert_map, residua
         if torch.cuda.is_current_stream_capturing():
             raise RuntimeError("MoE accumulator must be allocated before CUDA-graph capture")
         acc = _local_acc[dev] = torch.zeros(MOE_T_CAP * LAM_H_MAX, dtype=torch.float32, device=x.device)
-    cu.gemm_tc_grouped_combine(a, w2, offs, bn, pairs, pw, k, H, acc_ptr=acc.data_ptr())
+    if stream:
+        cu.gemm_experts(a, w2, offs, _stream_width(bn), sums=(acc.data_ptr(), pairs, pw, k))
+    else:
+        cu.gemm_tc_grouped_combine(a, w2, offs, bn, pairs, pw, k, H, acc_ptr=acc.data_ptr())
     out = torch.empty((T, H), dtype=x.dtype, device=x.device)
     cu.moe_finish(acc.data_ptr(), residual, norm_w, out, T, H, eps, gemma)
     return out, residual
