@@ -4,7 +4,7 @@
 // Reference counterparts: csrc/moe/topk_softmax_kernels.cu, moe_align_sum_kernels.cu, moe_permute_unpermute_op.cu
 // (here: routing probabilities + top-k in one warp per token; counting sort of (token, slot) pairs by expert with
 // an inverse map; weighted un-permute that sums a token's k expert outputs in a fixed order → deterministic).
-#include "common.cuh"
+#include "warp_mma.cuh"
 
 namespace moe {
 
@@ -285,6 +285,84 @@ __global__ void align_kernel(const int* __restrict__ ids, const int* __restrict_
   for (int p = start[E] + threadIdx.x; p < R; p += blockDim.x) { sorted_tok[p] = 0; if (sorted_pair) sorted_pair[p] = 0; }
 }
 
+// The same for prompts, over a cluster: each CTA counts a share of the pairs, kept in registers, adds up what the CTAs before it have of every expert and
+// places its own.  One CTA spent its time on the counters' atomics: 41400 pairs, 32 experts 6.9 us (28 in one CTA).
+constexpr int ALIGN_CTAS = 8, ALIGN_THREADS = 1024, ALIGN_KEEP = 8;
+__global__ void __launch_bounds__(ALIGN_THREADS) align_cluster_kernel(const int* __restrict__ ids, const int* __restrict__ emap, int* __restrict__ sorted_tok,
+                                                                      int* __restrict__ inv, int* __restrict__ offs, int R, int k, int E,
+                                                                      int* __restrict__ sorted_pair) {
+  extern __shared__ int sm[];
+  int* cnt = sm;            // [E] of this CTA; then its cursor
+  int* next = sm + E;       // [E]
+  __shared__ int tot[32];
+  __shared__ int valid;
+  pdl_trigger();
+  pdl_wait();
+  const int rank = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int per = (R + ALIGN_CTAS - 1) / ALIGN_CTAS, lo = min(R, rank * per), hi = min(R, lo + per);
+  auto expert = [&](int i) { int e = ids[i]; return emap ? emap[e] : e; };
+  for (int e = threadIdx.x; e < E; e += ALIGN_THREADS) cnt[e] = 0;
+  __syncthreads();
+  int keep[ALIGN_KEEP];
+#pragma unroll
+  for (int u = 0; u < ALIGN_KEEP; ++u) {
+    const int i = lo + u * ALIGN_THREADS + (int)threadIdx.x;
+    keep[u] = i < hi ? expert(i) : -1;
+    if (keep[u] >= 0) atomicAdd(&cnt[keep[u]], 1);
+  }
+  for (int i = lo + ALIGN_KEEP * ALIGN_THREADS + (int)threadIdx.x; i < hi; i += ALIGN_THREADS) {
+    const int e = expert(i);
+    if (e >= 0) atomicAdd(&cnt[e], 1);
+  }
+  cluster_sync();
+  // experts in runs of 1024: how many pairs all CTAs have of each, and how many the ones before this
+  int base = 0;
+  for (int e0 = 0; e0 < E; e0 += ALIGN_THREADS) {
+    const int e = e0 + (int)threadIdx.x;
+    int all = 0, before = 0;
+    if (e < E) {
+#pragma unroll
+      for (int r = 0; r < ALIGN_CTAS; ++r) {
+        const int c = __float_as_int(ld_dsmem_f32(dsmem_addr(smem_u32(&cnt[e]), r)));
+        all += c;
+        if (r < rank) before += c;
+      }
+    }
+    int inc = all;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, inc, o); if (lane >= o) inc += v; }
+    if (lane == 31) tot[w] = inc;
+    __syncthreads();
+    int t = tot[lane], ti = t;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, ti, o); if (lane >= o) ti += v; }
+    const int first = base + __shfl_sync(0xffffffffu, ti - t, w) + inc - all;
+    if (e < E) {
+      next[e] = first + before;
+      if (rank == 0) offs[e] = first;
+    }
+    base += __shfl_sync(0xffffffffu, ti, 31);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) { valid = base; if (rank == 0) offs[E] = base; }
+  __syncthreads();
+  auto put = [&](int i, int e) {
+    if (e < 0) { inv[i] = -1; return; }
+    const int p = atomicAdd(&next[e], 1);
+    sorted_tok[p] = i / k;
+    if (sorted_pair) sorted_pair[p] = i;
+    inv[i] = p;
+  };
+#pragma unroll
+  for (int u = 0; u < ALIGN_KEEP; ++u) {
+    const int i = lo + u * ALIGN_THREADS + (int)threadIdx.x;
+    if (i < hi) put(i, keep[u]);
+  }
+  for (int i = lo + ALIGN_KEEP * ALIGN_THREADS + (int)threadIdx.x; i < hi; i += ALIGN_THREADS) put(i, expert(i));
+  for (int p = valid + rank * ALIGN_THREADS + (int)threadIdx.x; p < R; p += ALIGN_CTAS * ALIGN_THREADS) { sorted_tok[p] = 0; if (sorted_pair) sorted_pair[p] = 0; }
+  cluster_sync();           // the others read this CTA's counts until their placement
+}
+
 // Tail of the fused MoE combine: acc (fp32, every rank holds the complete sum after the multimem.red epilogue of the
 // w2 grouped GEMM) + residual → new residual, RMSNorm → out; acc is zeroed for its next use.  One CTA per token.
 template <typename T, bool GEMMA>
@@ -451,7 +529,30 @@ __global__ void gather_kernel(const T* __restrict__ x, const int* __restrict__ s
   for (int g = threadIdx.x; g < H / 8; g += blockDim.x) st16(xs + (size_t)p * H + g * 8, ld16(src + g * 8));
 }
 
+// The same from the tokens' side, one CTA each: a row is read once and written where its k pairs went (inv).  Places that no pair has are left alone.
+// 6900 rows of 2048, k = 6: 32 us, 6.1 TB/s (45 by places: a CTA per place, k reads of a row); 1365 rows 5.8 and 9.1
+template <typename T>
+__global__ void __launch_bounds__(256) spread_kernel(const T* __restrict__ x, const int* __restrict__ inv, T* __restrict__ xs, int H, int k) {
+  pdl_trigger();
+  pdl_wait();
+  const int64_t t = blockIdx.x;
+  for (int g = threadIdx.x; g < H / 8; g += blockDim.x) {
+    const Vec16<T> v = ld16(x + t * H + g * 8);
+    for (int j = 0; j < k; ++j) {
+      const int p = inv[t * k + j];
+      if (p >= 0) st16(xs + (size_t)p * H + g * 8, v);
+    }
+  }
+}
+
 }  // namespace moe
+
+EXPORT int vb_moe_spread(const void* x, const int* inv, void* xs, int T_, int H, int k, int dtype, cudaStream_t st) {
+  if (T_ == 0) return 0;
+  if (dtype == DT_F32 || H % 8 || k < 1) return -1;
+  DISPATCH_HALF(dtype, T, vb_launch(moe::spread_kernel<T>, dim3(T_), dim3(256), 0, st, (const T*)x, inv, (T*)xs, H, k));
+  return (int)cudaGetLastError();
+}
 
 EXPORT int vb_moe_topk_softmax(const void* logits, float* out_w, int* out_ids, int n_tokens, int E, int k, int renorm,
                                float scale, int dtype, cudaStream_t st) {
@@ -499,7 +600,12 @@ EXPORT int vb_moe_grouped_simt(const void* x, const void* w, void* y, const int*
 EXPORT int vb_moe_align2(const int* ids, const int* emap, int* sorted_tok, int* inv, int* offs, int R, int k, int E,
                          int* sorted_pair, cudaStream_t st) {
   if (E > 4096) return -1;
-  vb_launch(moe::align_kernel, dim3(1), dim3(R > 4096 ? 1024 : 256), (size_t)(2 * E + 1) * sizeof(int), st, ids, emap, sorted_tok, inv, offs,
+  if (R > 4096) {           // us for 4200, 8190 and 41400 pairs of 32 experts, one CTA of 1024 threads and eight: 5.0 and 3.7, 7.1 and 4.2, 28 and 6.9
+    vb_launch_parts(moe::align_cluster_kernel, dim3(moe::ALIGN_CTAS), dim3(moe::ALIGN_THREADS), (size_t)2 * E * sizeof(int), st, (unsigned)moe::ALIGN_CTAS, ids, emap,
+                    sorted_tok, inv, offs, R, k, E, sorted_pair);
+    return (int)cudaGetLastError();
+  }
+  vb_launch(moe::align_kernel, dim3(1), dim3(256), (size_t)(2 * E + 1) * sizeof(int), st, ids, emap, sorted_tok, inv, offs,
             R, k, E, sorted_pair);
   return (int)cudaGetLastError();
 }

@@ -246,6 +246,19 @@ __global__ void sigmoid_mul_kernel(const T* __restrict__ x, int64_t x_stride, co
   }
 }
 
+// y[0 or 1, t, h run + c] = x[t, (2 h + (0 or 1)) run + c]: the two halves of every pair of runs, apart (run a multiple of 8, rows of n)
+template <typename T>
+__global__ void unzip_kernel(const T* __restrict__ x, T* __restrict__ y, int n, int run, int64_t total, int64_t half) {
+  pdl_trigger();
+  pdl_wait();
+  const int per_row = n / 8;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t t = i / per_row;
+    const int c = (int)(i - t * per_row) * 8, h = c / (2 * run), r = c - 2 * run * h, second = r >= run;
+    st16(y + second * half + t * (n / 2) + h * run + r - second * run, ld16(x + i * 8));
+  }
+}
+
 // x[t, c] = cap tanh(x[t, c] / cap) in place, rows of n at any stride
 template <typename T>
 __global__ void soft_cap_kernel(T* __restrict__ x, int64_t stride, int n, int64_t total, float cap) {
@@ -445,6 +458,15 @@ EXPORT int vb_sigmoid_mul(const void* x, int64_t x_stride, const void* g, int64_
     else GO(1);
   });
 #undef GO
+  return (int)cudaGetLastError();
+}
+
+EXPORT int vb_unzip(const void* x, void* y, int64_t T, int n, int run, int dtype, cudaStream_t st) {
+  if (T == 0 || n == 0) return 0;
+  if (dtype == DT_F32 || run < 8 || run % 8 || n % (2 * run)) return -1;
+  const int64_t total = T * (n / 8);
+  const int blocks = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
+  DISPATCH_HALF(dtype, TT, { vb_launch(unzip_kernel<TT>, blocks, 256, 0, st, (const TT*)x, (TT*)y, n, run, total, T * (n / 2)); });
   return (int)cudaGetLastError();
 }
 

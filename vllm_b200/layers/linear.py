@@ -98,10 +98,7 @@ def products(x: torch.Tensor, *parts) -> list:
             out.append(m.forward_gated_silu(x))
             continue
         y = m(x)
-        if form is not None:
-            pairs = y.view(*y.shape[:-1], -1, 2, form)
-            y = [pairs[..., i, :].reshape(*y.shape[:-1], -1) for i in (0, 1)]
-        out.append(y)
+        out.append(y if form is None else ops.unzip(y, form))
     return out
 
 

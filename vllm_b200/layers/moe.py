@@ -201,8 +201,10 @@ class FusedMoE(nn.Module):
             comm = get_tp_group().device_comm
             if comm is None:
                 return None
-        from vllm_b200.ops.moe import fused_moe_reduce_norm
+        from vllm_b200.ops.moe import fused_moe_reduce_norm, reduce_norm_ok
         x2 = x.reshape(-1, x.shape[-1])
+        if not reduce_norm_ok(x2, self.w13_weight, self.w2_weight, self.top_k, self.act, residual.view(-1, x.shape[-1]), norm.weight, comm):
+            return None
         w, ids = self.select_experts(router_logits.reshape(-1, router_logits.shape[-1]))
         out = fused_moe_reduce_norm(x2, self.w13_weight, self.w2_weight, w.to(torch.float32), ids, self.act,
                                     self.expert_map, residual.view(-1, x.shape[-1]), norm.weight, norm.eps,

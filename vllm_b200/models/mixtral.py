@@ -53,11 +53,12 @@ class SparseMoeBlock(nn.Module):
         return out
 
 
-    def forward_reduce_norm(self, x: torch.Tensor, residual: torch.Tensor, norm) -> tuple[torch.Tensor, torch.Tensor]:
-        """(normed, residual) = norm(all_reduce(block(x)) + residual)."""
+    def forward_reduce_norm(self, x: torch.Tensor, residual: torch.Tensor, norm, logits: Optional[torch.Tensor] = None
+                            ) -> tuple[torch.Tensor, torch.Tensor]:
+        """(normed, residual) = norm(all_reduce(block(x)) + residual).  ``logits``: the router's, where they are there already."""
         shared = gate = None
         if self.shared_expert is None:
-            logits = self.gate(x)
+            logits = self.gate(x) if logits is None else logits
         else:
             parts = [self.shared_expert.up_part(), (self.gate, None)]
             if self.shared_expert_gate is not None:
@@ -108,15 +109,17 @@ class MoeDecoderLayer(nn.Module):
         hidden, residual = self.self_attn.o_proj.forward_reduce_norm(a, residual, self.post_attention_layernorm)
         if self.dense is not None:
             return self.dense.forward_reduce_norm(hidden, residual, next_norm)
+        logits = None
         if next_norm is not None and self.moe.shared_expert is None:
-            fused = self.moe.experts.forward_reduce_norm(hidden, self.moe.gate(hidden), residual, next_norm)
+            logits = self.moe.gate(hidden)
+            fused = self.moe.experts.forward_reduce_norm(hidden, logits, residual, next_norm)
             if fused is not None:
                 return fused
         if next_norm is None:
             partial = self.moe(hidden)
             tp = get_tp_group()
             return (tp.all_reduce(partial) if tp.world_size > 1 else partial), residual
-        return self.moe.forward_reduce_norm(hidden, residual, next_norm)
+        return self.moe.forward_reduce_norm(hidden, residual, next_norm, logits)
 
 
 class MoeModel(LlamaModel):

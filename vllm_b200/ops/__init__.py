@@ -370,6 +370,15 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     return torch.nn.functional.linear(x, weight, bias)
 
 
+def unzip(x: torch.Tensor, run: int) -> list:
+    """The two results between which the columns of x alternate in runs of ``run``."""
+    got = cuda_ops().unzip(x, run) if _use_cuda(x) else None
+    if got is None:
+        pairs = x.view(*x.shape[:-1], -1, 2, run)
+        got = [pairs[..., i, :].reshape(*x.shape[:-1], -1) for i in (0, 1)]
+    return got
+
+
 def linear_parts(x: torch.Tensor, weights, biases, forms) -> Optional[list]:
     """Several linear layers of one input at once (csrc/gemm_tc.cu), or None where each is better off alone; ``forms`` as in ops/cuda.py."""
     return cuda_ops().linear_parts(x, weights, biases, forms) if _use_cuda(x) else None

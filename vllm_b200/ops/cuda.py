@@ -244,6 +244,19 @@ def sigmoid_mul_(x, g):
     return x
 
 
+_unzip = _sig("vb_unzip", _vp, _vp, _i64, _i, _i, _i, _vp)
+
+
+def unzip(x: torch.Tensor, run: int) -> Optional[list]:
+    """The two results between which the columns of x alternate in runs of ``run``, or None where rows are not read in vectors."""
+    n = x.shape[-1]
+    if x.dtype not in _HALF_DTYPES or run % 8 or n % (2 * run) or not x.is_contiguous() or x.data_ptr() % 16:
+        return None
+    y = torch.empty((2,) + x.shape[:-1] + (n // 2,), dtype=x.dtype, device=x.device)
+    _check(_unzip(x.data_ptr(), y.data_ptr(), x.numel() // n, n, run, _DT[x.dtype], _st()), "unzip")
+    return list(y)
+
+
 def soft_cap_(x, cap: float):
     """x = cap tanh(x / cap) in place; rows of any stride."""
     assert x.dim() == 2 and x.stride(1) == 1
@@ -1266,6 +1279,17 @@ def moe_gather(x: torch.Tensor, sorted_tok: torch.Tensor) -> torch.Tensor:
     R, H = sorted_tok.numel(), x.shape[1]
     xs = torch.empty((R, H), dtype=x.dtype, device=x.device)
     _check(_moe_gather(x.data_ptr(), sorted_tok.data_ptr(), xs.data_ptr(), R, H, _DT[x.dtype], _st()), "moe_gather")
+    return xs
+
+
+_moe_spread = _sig("vb_moe_spread", _vp, _vp, _vp, _i, _i, _i, _i, _vp)
+
+
+def moe_spread(x: torch.Tensor, inv: torch.Tensor) -> torch.Tensor:
+    """``moe_gather`` from the tokens' side; rows that no pair went to are left as they are (``inv`` -1: a pair of another rank)."""
+    (T, H), R = x.shape, inv.numel()
+    xs = torch.empty((R, H), dtype=x.dtype, device=x.device)
+    _check(_moe_spread(x.data_ptr(), inv.data_ptr(), xs.data_ptr(), T, H, R // max(T, 1), _DT[x.dtype], _st()), "moe_spread")
     return xs
 
 

@@ -122,7 +122,7 @@ def expert_rows_gated(x, w13, w2, topk_ids, act, expert_map):
         # (batch-invariant mode keeps to the decode tiles, which round the hidden rows before the activation)
         if (R >= PROMPT_ROWS * E and R > GROUPED_MAX_ROWS and act in cu._GATED_ACT and E <= cu.GROUPED_MAX_EXPERTS
                 and not cu.batch_invariant()):
-            return cu.gemm_grouped(cu.gemm_grouped(cu.moe_gather(x, sorted_tok), w13, offs, act), w2, offs), inv
+            return cu.gemm_grouped(cu.gemm_grouped(cu.moe_spread(x, inv), w13, offs, act), w2, offs), inv
         bn = _tile_width(R, E)
         h = cu.gemm_tc_grouped(cu.moe_gather(x, sorted_tok), w13, offs, bn, flat=True)
         return cu.gemm_tc_grouped(cu.act_and_mul(h, act), w2, offs, bn, flat=True), inv
@@ -201,6 +201,18 @@ def fp8_grouped_ok(x, w13q, w2q, R: int, block: int) -> bool:
 _local_acc: dict[int, torch.Tensor] = {}
 
 
+def reduce_norm_ok(x, w13, w2, k: int, act, residual, norm_w, comm) -> bool:
+    """Does ``fused_moe_reduce_norm`` cover x's tokens, k experts each?"""
+    from vllm_b200.ops import cuda as cu
+    from vllm_b200.parallel.symm import LAM_H_MAX, MOE_T_CAP
+    T, H = x.shape
+    if cu.batch_invariant():          # red.add epilogues sum a token's k expert rows in arrival order
+        return False
+    return not (not _grouped_ok(x, w13, w2, T * k) or T > MOE_T_CAP or H > LAM_H_MAX or H % 8 or act not in ("silu", "gelu", "gelu_tanh")
+                or (residual is not None and (not residual.is_contiguous() or residual.dtype != x.dtype))
+                or (comm is not None and comm.world > 1 and (H // 8 > 1024 or norm_w is None)))
+
+
 def fused_moe_reduce_norm(x, w13, w2, topk_w, topk_ids, act, expert_map, residual, norm_w, eps, gemma=False, comm=None):
     """MoE block tail inside the GEMM: align → gather → grouped GEMM (w13) → act·mul → grouped GEMM (w2) whose epilogue
     scales every output row by its routing weight and ADDS it (red.add.f32) into the fp32 accumulator row of its token —
@@ -217,11 +229,7 @@ def fused_moe_reduce_norm(x, w13, w2, topk_w, topk_ids, act, expert_map, residua
     H = x.shape[1]
     R = T * k
     multi = comm is not None and comm.world > 1
-    if cu.batch_invariant():          # red.add epilogues sum a token's k expert rows in arrival order
-        return None
-    if (not _grouped_ok(x, w13, w2, R) or T > MOE_T_CAP or H > LAM_H_MAX or H % 8 or act not in ("silu", "gelu", "gelu_tanh")
-            or (residual is not None and (not residual.is_contiguous() or residual.dtype != x.dtype))
-            or (multi and (H // 8 > 1024 or norm_w is None))):
+    if not reduce_norm_ok(x, w13, w2, k, act, residual, norm_w, comm):
         return None
     E = w13.shape[0]
     ids = topk_ids if topk_ids.dtype == torch.int32 else topk_ids.to(torch.int32)
