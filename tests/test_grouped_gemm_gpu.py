@@ -32,6 +32,14 @@ def test_grouped_rows(rows, N, K, act, dtype):
     assert _rel(got, torch.cat(want)) < (2 ** -9 if dtype == torch.bfloat16 else 2 ** -12)
 
 
+@pytest.mark.parametrize("rows,N,K", [([0, 1, 255, 256, 257, 300, 129, 0], 512, 256), ([700], 208, 72), ([130] * 40, 96, 1032), ([2999, 1], 1040, 64)])
+@pytest.mark.parametrize("act", [None, "gelu_tanh"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_rows_of_pairs_of_blocks(rows, N, K, act, dtype):
+    """Sizes that go to pairs of blocks: edges of their 256 rows, a second block without rows, more tiles than pairs."""
+    test_grouped_rows(rows, N, K, act, dtype)
+
+
 @pytest.mark.parametrize("T,E,k", [(300, 8, 4), (600, 4, 2), (2100, 64, 8)])
 @pytest.mark.parametrize("mapped", [False, True])
 def test_prompt_experts_match_decode_experts(T, E, k, mapped):

@@ -14,6 +14,7 @@
 // Scores are capped, cap tanh(s / cap), with cap <= 60: e^s then fits into fp32 (and bf16) whatever the score is, and the softmax needs no
 // running maximum: one pass over S, no rescaling, and partial sums of different key ranges simply add up.
 #include "common.cuh"
+#include "pair_mma.cuh"
 #include "talk.cuh"
 
 namespace talk {
@@ -43,54 +44,6 @@ VB_DEVICE void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
         "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
 VB_DEVICE void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// ---- pairs of CTAs: one MMA over the rows of both, issued by the leader (rank 0).  Each CTA holds its own rows of A and D, and half of
-// the N rows of B.
-// D[tmem] (+)= A * B; A from shared memory, or from TMEM (row = lane, two 16-bit values per column).  The whole warp calls these and one
-// lane is elected inside: descriptors stay in uniform registers, an MMA behind a lane test takes a hundred cycles to issue.
-VB_DEVICE void umma2_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-               "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-               ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-}
-VB_DEVICE void umma2_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-               "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-               ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-}
-// arrives on the barrier at this offset in both CTAs once the MMAs issued before have completed
-VB_DEVICE void umma2_commit(uint64_t* bar) {
-  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
-               "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
-               ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
-}
-// loads into this CTA's shared memory and counts the bytes on a barrier of the pair (a shared::cluster address)
-VB_DEVICE void tma2_load_2d(void* dst, const void* tmap, int c0, int c1, uint32_t bar) {
-  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-               ::"r"(smem_u32(dst)), "l"(tmap), "r"(bar), "r"(c0), "r"(c1) : "memory");
-}
-VB_DEVICE void tma2_load_3d(void* dst, const void* tmap, int c0, int c1, int c2, uint32_t bar) {
-  asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-               ::"r"(smem_u32(dst)), "l"(tmap), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
-}
-VB_DEVICE void tmem2_alloc(uint32_t* smem_dst, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(ncols) : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-VB_DEVICE void tmem2_dealloc(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-VB_DEVICE void arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-VB_DEVICE void wait_cluster_lim(uint64_t* bar, uint32_t parity, int& budget) {      // what threads of the other CTA have arrived on
-  for (;;) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    if (ok || --budget < 0) break;
-  }
-}
-
 // Pair of CTAs = two query tiles in a row x KV head of the scores x some pairs of value heads (one after the other), one request.  Both
 // tiles read the same keys and values; each CTA fetches half of them (a page of the key tile; one value head, or half of a single one).
 // Warp roles: 0 TMA producer, 1 MMA issuer (leader) + TMEM owner, 2..17 softmax / epilogue (thread = query row = TMEM lane, a quarter of
