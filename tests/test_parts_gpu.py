@@ -59,3 +59,44 @@ def test_router_logits_in_16_bits(dtype, scoring):
     bias = torch.randn(32, device="cuda", generator=g)
     a, b = (cu.grouped_topk(t, 6, 4, 2, True, scoring, bias, 2.5) for t in (lg, lg.float()))
     assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+
+
+@pytest.mark.parametrize("E,groups,keep,k", [(32, 4, 2, 6), (33, 1, 1, 33 - 1), (64, 8, 3, 8), (96, 32, 32, 32), (160, 5, 2, 7), (256, 8, 4, 8), (256, 1, 1, 1), (24, 3, 1, 8)])
+@pytest.mark.parametrize("scoring,biased,top2", [("sigmoid", True, "top2"), ("softmax", False, "max"), ("sigmoid", True, "max")])
+def test_a_warp_per_token_chooses_as_a_block(E, groups, keep, k, scoring, biased, top2):
+    """Equal scores (the first expert wins), infinities and NaN among them; the block form takes the same numbers behind a router of its own: an identity."""
+    from vllm_b200.ops import cuda as cu
+    g = torch.Generator(device="cuda").manual_seed(E + k)
+    lg = torch.randint(-4, 5, (1101, E), device="cuda", generator=g).float() / 2
+    lg[::7] = torch.randn(lg[::7].shape, device="cuda", generator=g)
+    lg[3, ::3], lg[5, 1] = float("-inf"), float("inf") if scoring == "sigmoid" else 50.0
+    bias = torch.randint(-2, 3, (E,), device="cuda", generator=g).float() if biased else None
+    a = cu.grouped_topk(lg, k, groups, keep, True, scoring, bias, 2.5, top2)
+    s = lg.double().sigmoid() if scoring == "sigmoid" else lg.double().softmax(-1)
+    s32 = lg.sigmoid() if scoring == "sigmoid" else s.float()
+    for t in (0, 3, 5, 7, *range(100, 1101, 91)):
+        ch = (s32[t] + (bias if biased else 0)).view(groups, -1)
+        gs = ch.topk(2, -1).values.sum(-1) if top2 == "top2" and E // groups > 1 else ch.max(-1).values
+        ids = a[1][t].long()
+        n = min(k, keep * (E // groups))
+        assert len(set(ids[:n].tolist())) == n
+        kept = set((ids[:n] // (E // groups)).tolist())
+        eps = 4e-7 * (1 + float(ch.abs().max()))                  # scores in 32 bits on both sides
+        assert len(kept) <= keep
+        if groups > 1:
+            out = [i for i in range(groups) if i not in kept]
+            full = [i for i in kept]
+            if len(kept) == keep and out:
+                assert float(gs[full].min()) >= float(gs[out].max()) - 2 * eps
+        inside = torch.zeros(groups, device="cuda", dtype=torch.bool)
+        inside[list(kept)] = True
+        c = torch.where(inside[:, None].expand(ch.shape), ch, torch.full_like(ch, float("-inf"))).view(-1)
+        picked = c[ids[:n]]
+        assert bool((picked[:-1] >= picked[1:] - eps).all())
+        rest = c.clone()
+        rest[ids[:n]] = float("-inf")
+        if len(kept) == keep:
+            assert float(picked[-1]) >= float(rest.max()) - eps
+        w = s[t, ids[:n]]
+        want = w * 2.5 / s32[t, ids].sum().double()
+        assert torch.allclose(a[0][t, :n].double(), want, rtol=1e-5, atol=1e-12)

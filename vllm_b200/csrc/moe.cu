@@ -192,6 +192,109 @@ grouped_topk_kernel(const float* __restrict__ logits, const TX* __restrict__ x, 
     for (int j = lane; j < k; j += 32) out_w[(int64_t)t * k + j] *= scale / (wsum + 1e-20f);
 }
 
+// The same for given logits of up to 32 EL experts: a warp per token, its experts in registers, a maximum in one instruction (of keys that order as the
+// numbers do); a CTA per token spent its time on barriers and on two-step exchanges.  us, before and so: 24 tokens, 6 of 32 in 4 groups 5.1 and 2.5, 6900
+// tokens 21 and 6.8; 8 of 256 in 8 groups 7.1 and 7.9, 6900 tokens 39 and 23.
+VB_DEVICE uint32_t order_key(float x) {            // NaN and what is left out order as -inf: 0x007fffff
+  const uint32_t b = __float_as_uint(x + 0.f);
+  return x != x ? 0x007fffffu : (b >> 31) ? ~b : b | 0x80000000u;
+}
+constexpr uint32_t NONE_KEY = 0x007fffffu;
+template <typename TL, int EL>
+__global__ void __launch_bounds__(128)
+grouped_topk_warp_kernel(const TL* __restrict__ logits, const float* __restrict__ bias, float* __restrict__ out_w, int* __restrict__ out_ids, int n_tokens,
+                         int E, int k, int n_group, int keep, int group_top2, int softmax, int renorm, float scale) {
+  pdl_trigger();
+  pdl_wait();
+  const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= n_tokens) return;
+  constexpr unsigned ALL = 0xffffffffu;
+  float score[EL];
+  uint32_t choice[EL];
+#pragma unroll
+  for (int i = 0; i < EL; ++i) score[i] = lane + 32 * i < E ? to_f32(logits[(int64_t)t * E + lane + 32 * i]) : -INFINITY;
+  if (softmax) {
+    float mx = -INFINITY, sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < EL; ++i) mx = fmaxf(mx, score[i]);
+    mx = warp_max(mx);
+#pragma unroll
+    for (int i = 0; i < EL; ++i) {
+      score[i] = lane + 32 * i < E ? expf(score[i] - mx) : 0.f;
+      sum += score[i];
+    }
+    const float inv = 1.f / warp_sum(sum);
+#pragma unroll
+    for (int i = 0; i < EL; ++i) score[i] *= inv;
+  } else {
+#pragma unroll
+    for (int i = 0; i < EL; ++i) score[i] = 1.f / (1.f + expf(-score[i]));
+  }
+  int group[EL];
+#pragma unroll
+  for (int i = 0; i < EL; ++i) {
+    const int e = lane + 32 * i;
+    choice[i] = e < E ? order_key(score[i] + (bias ? bias[e] : 0.f)) : NONE_KEY;
+    group[i] = e < E ? e / (E / n_group) : -1;
+  }
+  // the largest key among the lanes' and the first place that has it
+  auto first = [&](uint32_t key, int place, uint32_t& top) {
+    top = __reduce_max_sync(ALL, key);
+    return (int)__reduce_min_sync(ALL, key == top ? (unsigned)place : 0x7fffffffu);
+  };
+  auto own = [&](int g, int but, uint32_t& key, int& place) {      // of this lane's in group g (-1: all), without one
+    key = NONE_KEY; place = 0x7fffffff;
+#pragma unroll
+    for (int i = 0; i < EL; ++i) {
+      const int e = lane + 32 * i;
+      if (choice[i] > key && e != but && (g < 0 || group[i] == g)) { key = choice[i]; place = e; }
+    }
+  };
+  auto number = [](uint32_t key) { return __uint_as_float((key >> 31) ? key & 0x7fffffffu : ~key); };
+  uint32_t key, top;
+  int place;
+  if (n_group > 1) {
+    const bool two = group_top2 && E / n_group > 1;
+    uint32_t mine = NONE_KEY;                      // of group `lane`
+    for (int g = 0; g < n_group; ++g) {
+      own(g, -1, key, place);
+      const int p = first(key, place, top);
+      float s = number(top);
+      if (two) {
+        own(g, p, key, place);
+        s += number(__reduce_max_sync(ALL, key));
+      }
+      if (lane == g) mine = order_key(s);
+    }
+    unsigned kept = 0;
+    for (int n = 0; n < keep; ++n) {
+      const int g = first(lane < n_group && !((kept >> lane) & 1u) ? mine : NONE_KEY, lane, top);
+      if (top != NONE_KEY) kept |= 1u << g;
+    }
+#pragma unroll
+    for (int i = 0; i < EL; ++i)
+      if (group[i] >= 0 && !((kept >> group[i]) & 1u)) choice[i] = NONE_KEY;
+  }
+  float wsum = 0.f, my_w = 0.f;
+  int my_id = 0;
+  for (int j = 0; j < k; ++j) {
+    own(-1, -1, key, place);
+    int e = first(key, place, top);
+    if (top == NONE_KEY) e = 0;                    // fewer than k candidates: cannot happen for a valid configuration
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < EL; ++i)
+      if (i == e >> 5) { s = score[i]; if ((e & 31) == lane) choice[i] = NONE_KEY; }
+    s = __shfl_sync(ALL, s, e & 31);
+    wsum += s;
+    if (lane == j) { my_w = s; my_id = e; }
+  }
+  if (lane < k) {
+    out_w[(int64_t)t * k + lane] = my_w * (renorm ? scale / (wsum + 1e-20f) : scale);
+    out_ids[(int64_t)t * k + lane] = my_id;
+  }
+}
+
 // Grouped GEMM on the CUDA cores for what the tcgen05 kernel (gemm_tc.cu) does not take — fp32, or rows that are not
 // 16-byte multiples:  y[r, n] = act(sum_k x[tok(r), k] * w[e(r), n, k]), rows sorted by expert.  64 x 64 tiles; grid.y
 // enumerates (expert, row tile) pairs, found from `offs` on the device.
@@ -574,6 +677,16 @@ EXPORT int vb_moe_grouped_topk(const float* logits, const void* x, int x_f32, co
   if (E < 1 || E > 4096 || k < 1 || k > E || n_group < 1 || E % n_group || keep < 1 || keep > n_group) return -1;
   if (!logits && !x) return -1;
   const bool given = logits || !w;
+  if (given && (E <= 128 || (E <= 256 && n_tokens >= 1024)) && n_group <= 32 && k <= 32) {          // eight experts to a lane: where there are warps enough
+    const dim3 grid((n_tokens + 3) / 4);
+#define GW(TL, EL) vb_launch(moe::grouped_topk_warp_kernel<TL, EL>, grid, dim3(128), 0, st, reinterpret_cast<const TL*>(logits ? (const void*)logits : x), bias, out_w, out_ids, n_tokens, E, k, n_group, keep, group_top2, softmax, renorm, scale)
+#define GE(TL) do { if (E <= 32) GW(TL, 1); else if (E <= 64) GW(TL, 2); else if (E <= 128) GW(TL, 4); else GW(TL, 8); } while (0)
+    if (logits) GE(float);
+    else DISPATCH_DTYPE(dtype, T, GE(T));
+#undef GE
+#undef GW
+    return (int)cudaGetLastError();
+  }
   const size_t smem = (size_t)(2 * E + n_group + (given ? 0 : H)) * sizeof(float);
   if (smem > 48 * 1024) return -3;
   const int thr = given ? (E > 128 ? 256 : 64) : (E > 32 ? 512 : 256);
