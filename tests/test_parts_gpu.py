@@ -100,3 +100,25 @@ def test_a_warp_per_token_chooses_as_a_block(E, groups, keep, k, scoring, biased
         w = s[t, ids[:n]]
         want = w * 2.5 / s32[t, ids].sum().double()
         assert torch.allclose(a[0][t, :n].double(), want, rtol=1e-5, atol=1e-12)
+
+
+@pytest.mark.parametrize("E,k", [(1, 1), (8, 2), (32, 32), (33, 4), (64, 8), (129, 6), (512, 32)])
+@pytest.mark.parametrize("renorm", [False, True])
+def test_softmax_router(E, k, renorm):
+    """Equal logits (the first expert wins), a row whose other experts round to nothing, one with NaN."""
+    from vllm_b200.ops import cuda as cu
+    g = torch.Generator(device="cuda").manual_seed(E)
+    lg = torch.randint(-3, 4, (70, E), device="cuda", generator=g).float()
+    lg[1] = -200.0
+    lg[1, E // 2] = 0.0
+    w, ids = cu.topk_softmax(lg, k, renorm)
+    want = lg.double().softmax(-1)
+    order = lg.sort(dim=-1, descending=True, stable=True).indices[:, :k]
+    assert torch.equal(ids.long(), order)
+    p = want.gather(1, order)
+    p = p / p.sum(-1, keepdim=True) if renorm else p
+    # a quick exponential (2^-21 of it and 2^-23 of its argument, at most 6 here) and sums of up to 512 numbers in 32 bits
+    assert torch.allclose(w.double(), p, rtol=2.0 ** -17, atol=1e-30)
+    if E > 1:
+        lg[2, 0] = float("nan")
+        assert int(cu.topk_softmax(lg, 1, renorm)[1][2]) != 0
