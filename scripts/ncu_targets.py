@@ -72,6 +72,17 @@ if which in ("latent", "all"):
     up, down = (torch.randn(*s, device="cuda", dtype=dt) * 0.02 for s in ((32, 1408, 2048), (32, 2048, 1408)))
     wt, ids = _routing(4096, 32, 6)
     rep(lambda: moe.expert_rows_plain(x, up, down, ids, "relu2", None))
+if which in ("steps", "all"):
+    # decode steps: experts whose weights are streamed, products of one input, log-probabilities, the routers (prompts too) and the sort by expert
+    xs, offs = torch.randn(144, 2048, device="cuda", dtype=dt) * 0.1, (torch.arange(33, device="cuda") * 144 // 32).int()
+    w13, w2 = (torch.randn(*s, device="cuda", dtype=dt) * 0.02 for s in ((32, 1536, 2048), (32, 2048, 768)))
+    rep(lambda: cu.gemm_experts(cu.gemm_experts(xs, w13, offs, 16, "silu"), w2, offs, 16))
+    ws = [torch.randn(n, 2048, device="cuda", dtype=dt) * 0.02 for n in (4096, 512, 512)]
+    rep(lambda: cu.linear_parts(xs[:24], ws, [None] * 3, [128, None, None]))
+    rep(lambda: cu.logprobs(torch.randn(24, 32000, device="cuda").to(dt), torch.zeros(24, dtype=torch.int64, device="cuda"), 5))
+    lg = torch.randn(6900, 32, device="cuda").to(dt)
+    rep(lambda: cu.moe_align(cu.topk_softmax(lg, 6, True)[1], 32))
+    rep(lambda: cu.grouped_topk(lg, 6, 4, 2, True))
 if which in ("scan", "all"):
     # Legelix: scans of prompts (1024 tokens each) and of a decode batch, at the sizes of a 2048-wide model
     from vllm_b200.forward_context import AttentionMetadata

@@ -7,9 +7,9 @@ Behavioural reference: the reference's MRV2 runner
 
 Design (ours):
 * request state lives in NumPy arrays indexed by a dense row; per-step inputs
-  (ids, positions, slot mapping, seq lens, block table) are produced with
-  vectorised NumPy into double-buffered *pinned* staging buffers and copied with
-  async H2D copies into *static* device buffers — the buffers CUDA graphs replay on;
+  (ids, positions, slot mapping, seq lens, block table) are expanded on the device
+  from a few integers per request, uploaded with the sampler's inputs in one copy out of
+  *pinned* staging sets, into *static* device buffers — the buffers CUDA graphs replay on;
 * decode-only steps replay a full-step CUDA graph per padded batch bucket
   (forward + logits + fused sampling), everything else runs eagerly;
 * sampled ids stay on the device in ``last_sampled`` (indexed by row); with async
