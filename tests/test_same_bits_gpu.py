@@ -1,0 +1,26 @@
+"""What a kernel for some sizes or some company computes is, bit for bit, what the kernel for the others computes."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M", [1, 24, 64, 100, 128])
+@pytest.mark.parametrize("K,parts", [(2048, [(1536, "silu", False), (32, None, False), (1, None, False)]), (2048, [(4096, 128, False), (512, None, False), (512, None, True)]),
+                                     (1024, [(2048, 64, True), (256, None, True), (255, None, True), (8, None, False)]), (2048, [(1024, None, False), (576, None, False)]),
+                                     (576, [(4992, None, True), (128, "silu", False)]), (4096, [(128, None, False), (13000, None, False)])])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_products_together_and_alone(M, K, parts, dtype):
+    """Products that share a launch add their partial sums as each does alone: more and fewer CTAs of a cluster than a matrix has sums."""
+    from vllm_b200.ops import cuda as cu
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    x = torch.randn(M, K, device="cuda", generator=g).to(dtype)
+    ws = [(torch.randn(n, K, device="cuda", generator=g) * K ** -0.5).to(dtype) for n, _, _ in parts]
+    bs = [torch.randn(n, device="cuda", generator=g).to(dtype) if b else None for n, _, b in parts]
+    got = cu.linear_parts(x, ws, bs, [f for _, f, _ in parts])
+    assert got is not None or (M > 64 and len(parts) == 2 and K == 4096)         # (there no cluster holds the sums of 103 tiles)
+    for y, w, b, (n, f, _) in zip(got or [], ws, bs, parts):
+        alone = cu.gemm_tc(x, w, b, act=int(f == "silu"))
+        if isinstance(f, int):
+            alone = alone.view(M, -1, 2, f).permute(2, 0, 1, 3).reshape(2, M, -1)
+        assert torch.equal(y, alone)

@@ -56,13 +56,17 @@ struct Params {
 
 // Several matrices of one K applied to the same rows (SWAP only): the tiles of part i are those from first[i] on along grid x.  A decode step's
 // small products cost 3.5 to 5 us each whatever they read (launch, first bytes, exchange of the splits), so those of one input go together.  Of a
-// captured step, for 24 rows of 2048: 1536 gated, 32 and 1 outputs 4.9 us (4.4, 3.9 and 3.6 in turn); 4096, 512 and 512, the first ones split into
-// queries and gates, 8.6 (8.2, 5.7 and 3.8, and 5.5 for the two copies).
+// captured step, for 24 rows of 2048: 1536 gated, 32 and 1 outputs 5.4 us (4.9, 3.7 and 3.7 in turn); 4096, 512 and 512, the first ones split into
+// queries and gates, 9.6 (6.8, 3.9 and 3.9, and 5.5 for the two copies).  With one number of sums for all of a launch those were 5.2 and 7.4, and the
+// results other ones than alone.
 constexpr int MAX_PARTS = 4;
 struct Parts {
   CUtensorMap map[MAX_PARTS];
   int first[MAX_PARTS], N[MAX_PARTS], act[MAX_PARTS];
   int run[MAX_PARTS];      // not 0: the outputs are pairs of runs of this many; the first runs of all rows lie before the second runs, [2, M, N / 2]
+  // Partial sums of a part's outputs, as many as the plan gives its matrix alone, added in the same order: a result does not depend on what shares its
+  // launch.  A CTA of a cluster has one or several of them, each in columns of tensor memory (and then a piece of shared memory) of its own.
+  int splits[MAX_PARTS];
   void* y[MAX_PARTS];
   const void* bias[MAX_PARTS];
 };
@@ -116,10 +120,18 @@ gemm_kernel(const __grid_constant__ A a, const __grid_constant__ CUtensorMap tma
       }
     return y + (size_t)m * N + n;
   };
-  const int kb0 = split * p.k_blocks_per_split;
   const int total_kb = (p.K + BK - 1) / BK;
-  const int nkb = max(0, min(p.k_blocks_per_split, total_kb - kb0));
-  constexpr uint32_t TMEM_COLS = BN <= 32 ? 32 : (BN <= 64 ? 64 : (BN <= 128 ? 128 : 256));
+  int splits = p.splits, per_split = p.k_blocks_per_split, sums = 1;           // sums: of this CTA
+  if constexpr (PARTS) {
+    splits = a.splits[part];
+    per_split = (total_kb + splits - 1) / splits;
+    sums = (splits + p.splits - 1) / p.splits;
+  }
+  const int kb0 = split * sums * per_split;
+  const int nkb = max(0, min(sums * per_split, total_kb - kb0));
+  uint32_t tmem_cols = BN <= 32 ? 32 : (BN <= 64 ? 64 : (BN <= 128 ? 128 : 256));
+  if constexpr (PARTS)
+    while (tmem_cols < (uint32_t)(sums * BN)) tmem_cols <<= 1;
 
 #define VB_TRACE(i) do { if (p.trace) p.trace[((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * 16 + (i)] = clock64(); } while (0)
   if (threadIdx.x == 0) VB_TRACE(0);
@@ -172,7 +184,7 @@ gemm_kernel(const __grid_constant__ A a, const __grid_constant__ CUtensorMap tma
     mbar_init(tmem_full, 1);
     mbar_fence_init();
   }
-  if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
+  if (warp == 1) tmem_alloc(tmem_slot, tmem_cols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -218,8 +230,11 @@ gemm_kernel(const __grid_constant__ A a, const __grid_constant__ CUtensorMap tma
   } else if (warp == 1) {
     // ===== MMA issuer
     const uint32_t idesc = umma_idesc_f16(TM, BN, DTypeOf<T>::v == DT_BF16);
-    for (int kb = 0; kb < nkb; ++kb) {
+    uint32_t acc = tmem_base;
+    int of_sum = 0;                                // blocks that the accumulator has
+    for (int kb = 0; kb < nkb; ++kb, ++of_sum) {
       const int s = kb % STAGES;
+      if (PARTS && of_sum == per_split) { of_sum = 0; acc += BN; }
       mbar_wait(&full[s], (kb / STAGES) & 1);
       tc_fence_after();
       __syncwarp();
@@ -229,7 +244,7 @@ gemm_kernel(const __grid_constant__ A a, const __grid_constant__ CUtensorMap tma
         const uint64_t da = umma_desc_sw128(a_src), db = umma_desc_sw128(a_src + L::A_BYTES);
 #pragma unroll
         for (int k = 0; k < BK / 16; ++k)   // UMMA_K = 16 → advance 32 B inside the swizzle span
-          warp_umma_f16(tmem_base, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) != 0);
+          warp_umma_f16(acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (of_sum | k) != 0);
         warp_umma_commit(&empty[s]);                 // frees the smem slot once these MMAs retire
         if (kb == nkb - 1) { warp_umma_commit(tmem_full); if (lane == 0) VB_TRACE(4); }
       }
@@ -247,21 +262,21 @@ gemm_kernel(const __grid_constant__ A a, const __grid_constant__ CUtensorMap tma
       tc_fence_after();
     }
     if (threadIdx.x == 64) VB_TRACE(5);
-    auto load_chunk = [&](int c, float (&v)[CH]) {
-      if (nkb == 0) {
+    auto load_chunk = [&](int c, float (&v)[CH], int sum = 0) {
+      if (nkb <= sum * per_split) {
 #pragma unroll
         for (int j = 0; j < CH; ++j) v[j] = 0.f;
         return;
       }
       if constexpr (CH == 32) {
         uint32_t r[32];
-        tmem_ld_32x32(t_row + c, r);
+        tmem_ld_32x32(t_row + sum * BN + c, r);
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
       } else {
         uint32_t r[16];
-        tmem_ld_32x16(t_row + c, r);
+        tmem_ld_32x16(t_row + sum * BN + c, r);
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
@@ -274,12 +289,13 @@ gemm_kernel(const __grid_constant__ A a, const __grid_constant__ CUtensorMap tma
       // fp32 partial in its OWN shared memory (the operand ring is idle once tmem_full fired) — part 1 of 2, the
       // reduction itself follows the cluster barrier below.
       float* red = reinterpret_cast<float*>(stage_base);
-      for (int c = 0; c < BN; c += CH) {
-        float v[CH];
-        load_chunk(c, v);
+      for (int sum = 0; sum < sums; ++sum)
+        for (int c = 0; c < BN; c += CH) {
+          float v[CH];
+          load_chunk(c, v, sum);
 #pragma unroll
-        for (int j = 0; j < CH; ++j) red[(c + j) * TM + row] = v[j];
-      }
+          for (int j = 0; j < CH; ++j) red[(sum * BN + c + j) * TM + row] = v[j];
+        }
       if (threadIdx.x == 64) VB_TRACE(6);
       do_store = false;
     }
@@ -288,6 +304,13 @@ gemm_kernel(const __grid_constant__ A a, const __grid_constant__ CUtensorMap tma
       for (int c = 0; c < BN; c += CH) {
         float v[CH];
         load_chunk(c, v);
+        if constexpr (PARTS)
+          for (int sum = 1; sum < sums; ++sum) {
+            float more[CH];
+            load_chunk(c, more, sum);
+#pragma unroll
+            for (int j = 0; j < CH; ++j) v[j] += more[j];
+          }
         if (SWAP && p.red_acc) {
           // fused combine: acc[token(row), n] += w(row) * y[row, n]   (lanes = 32 consecutive n → 128-byte bursts)
           const int n = a_tile * TM + row;
@@ -374,6 +397,15 @@ gemm_kernel(const __grid_constant__ A a, const __grid_constant__ CUtensorMap tma
         const int per = (units + p.splits - 1) / p.splits;
         const int u_end = min(units, (split + 1) * per);
         const uint32_t red_s = smem_u32(stage_base);
+        uint32_t from[8];                                          // PARTS: where the sums of the tile are
+        if constexpr (PARTS) {
+          int cta = 0, sum = 0;
+#pragma unroll
+          for (int r = 0; r < 8; ++r) {
+            from[r] = dsmem_addr(red_s + (uint32_t)(sum * BN * TM * 4), (uint32_t)(r < splits ? cta : 0));
+            if (++sum == sums) { sum = 0; ++cta; }
+          }
+        }
         // two units per pass: all DSMEM loads of both are in flight before the first add
         for (int u0 = split * per + et; u0 < u_end; u0 += 2 * EPI_THREADS) {
           float4 x[2][8];
@@ -381,10 +413,13 @@ gemm_kernel(const __grid_constant__ A a, const __grid_constant__ CUtensorMap tma
           for (int h = 0; h < 2; ++h) {
             const int u = u0 + h * EPI_THREADS;
             if (u < u_end) {
-              const uint32_t off = red_s + (uint32_t)((u / (TM / 4)) * TM + (u % (TM / 4)) * 4) * 4u;
+              const uint32_t off = (PARTS ? 0 : red_s) + (uint32_t)((u / (TM / 4)) * TM + (u % (TM / 4)) * 4) * 4u;
 #pragma unroll
               for (int r = 0; r < 8; ++r)
-                if (r < p.splits) x[h][r] = ld_dsmem_f32x4(dsmem_addr(off, (uint32_t)r));
+                if (r < splits) {
+                  if constexpr (PARTS) x[h][r] = ld_dsmem_f32x4(from[r] + off);
+                  else x[h][r] = ld_dsmem_f32x4(dsmem_addr(off, (uint32_t)r));
+                }
             }
           }
 #pragma unroll
@@ -395,7 +430,7 @@ gemm_kernel(const __grid_constant__ A a, const __grid_constant__ CUtensorMap tma
             float4 acc = x[h][0];
 #pragma unroll
             for (int r = 1; r < 8; ++r)
-              if (r < p.splits) { acc.x += x[h][r].x; acc.y += x[h][r].y; acc.z += x[h][r].z; acc.w += x[h][r].w; }
+              if (r < splits) { acc.x += x[h][r].x; acc.y += x[h][r].y; acc.z += x[h][r].z; acc.w += x[h][r].w; }
             const int n = a_tile * TM + rq * 4;
             float o[4] = {acc.x, acc.y, acc.z, acc.w};
             if (act == 1) {      // (gate, up) pairs are adjacent features: two outputs per unit
@@ -433,7 +468,7 @@ gemm_kernel(const __grid_constant__ A a, const __grid_constant__ CUtensorMap tma
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
+  if (warp == 1) tmem_dealloc(tmem_base, tmem_cols);
   if (threadIdx.x == 0) VB_TRACE(10);
 #undef VB_TRACE
 }
@@ -595,18 +630,18 @@ EXPORT int vb_gemm_tc2(const void* x, const void* w, const void* bias, void* y, 
   }
 }
 
-// y[i] = act(x w[i]^T + bias[i]) for n matrices [N[i], K] at once, M <= 128 rows; act as above (0 or 1), splits from the plan for all their tiles
-// run[i] (act 0, a multiple of 4): see Parts
-EXPORT int vb_gemm_tc_parts(const void* x, const void* const* w, const void* const* bias, void* const* y, const int* N, const int* act, const int* run, int n,
-                            int M, int K, int64_t x_stride, int bn, int splits, int dtype, cudaStream_t st) {
+// y[i] = act(x w[i]^T + bias[i]) for n matrices [N[i], K] at once, M <= 128 rows; act as above (0 or 1); splits[i] as the plan gives matrix i, by clusters of
+// `ctas`; run[i] (act 0, a multiple of 4): see Parts.  -3: the sums of a CTA do not fit.
+EXPORT int vb_gemm_tc_parts(const void* x, const void* const* w, const void* const* bias, void* const* y, const int* N, const int* act, const int* run, const int* splits,
+                            int n, int M, int K, int64_t x_stride, int bn, int ctas, int dtype, cudaStream_t st) {
   using namespace gemm;
-  if (dtype == DT_F32 || K % 8 != 0 || n < 1 || n > MAX_PARTS || M < 1 || M > bn || bn > 128 || bn % 16 || splits < 1 || splits > 8) return -1;
+  if (dtype == DT_F32 || K % 8 != 0 || n < 1 || n > MAX_PARTS || M < 1 || M > bn || bn > 128 || bn % 16 || ctas < 1 || ctas > 8) return -1;
   const bool bf16 = dtype == DT_BF16;
   Parts ta = {};
   CUtensorMap tb;
   Params p = {};
-  p.M = M; p.K = K; p.splits = splits; p.red_k = 1; p.red_world = 1; p.red_per = 1;
-  p.k_blocks_per_split = ((K + BK - 1) / BK + splits - 1) / splits;
+  p.M = M; p.K = K; p.splits = ctas; p.red_k = 1; p.red_world = 1; p.red_per = 1;
+  const int ring = (bn <= 64 ? 8 : 6) * (TM * BK * 2 + bn * BK * 2);
   int rc, tiles = 0;
   for (int i = 0; i < MAX_PARTS; ++i) {
     ta.first[i] = i < n ? tiles : INT32_MAX;
@@ -614,11 +649,14 @@ EXPORT int vb_gemm_tc_parts(const void* x, const void* const* w, const void* con
     if (act[i] && (act[i] != 1 || bias[i] || (N[i] & 3) || run[i])) return -1;
     if (run[i] < 0 || run[i] % 4 || (run[i] && N[i] % (2 * run[i]))) return -1;
     if ((rc = make_tmap(&ta.map[i], w[i], N[i], K, K, TM, bf16))) return rc;
-    ta.N[i] = N[i]; ta.act[i] = act[i]; ta.run[i] = run[i]; ta.y[i] = y[i]; ta.bias[i] = bias[i];
+    if (splits[i] < 1 || splits[i] > 8) return -1;
+    const int sums = (splits[i] + ctas - 1) / ctas;
+    if (sums * bn > 512 || (ctas > 1 && sums * bn * TM * 4 > ring)) return -3;
+    ta.N[i] = N[i]; ta.act[i] = act[i]; ta.run[i] = run[i]; ta.y[i] = y[i]; ta.bias[i] = bias[i]; ta.splits[i] = splits[i];
     tiles += (N[i] + TM - 1) / TM;
   }
   if ((rc = make_tmap(&tb, x, M, K, x_stride, bn, bf16))) return rc;
-  const dim3 grid(tiles, 1, splits);
+  const dim3 grid(tiles, 1, ctas);
 #define GOP(BNV, ST)                                                                     \
     if (bf16) return launch<__nv_bfloat16, BNV, ST, true>(ta, tb, p, grid, st);          \
     else return launch<__half, BNV, ST, true>(ta, tb, p, grid, st);

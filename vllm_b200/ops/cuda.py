@@ -1091,14 +1091,39 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     return torch.nn.functional.linear(x, weight, bias)
 
 
-_gemm_parts = _sig("vb_gemm_tc_parts", _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i, _i, _i, _vp)
-MAX_PARTS, PARTS_ROWS, PARTS_TILES = 4, 128, 132        # as many tiles as have a CTA each: beyond that two to an SM, which only the single product has
+_gemm_parts = _sig("vb_gemm_tc_parts", _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i, _i, _i, _vp)
+_max_clusters = _sig("vb_gemm_max_active_clusters", _i)
+# as many tiles as have a CTA each, by the ceiling of csrc/gemm_tc.cu's own plan: beyond that two share an SM, which only the single product's form does
+MAX_PARTS, PARTS_ROWS, PARTS_TILES = 4, 128, 132
+_parts_plans: dict[tuple, Optional[tuple]] = {}
+
+
+def _parts_plan(M: int, K: int, Ns: tuple) -> Optional[tuple]:
+    """(columns of a tile, partial sums of each matrix, CTAs of a cluster) for ``linear_parts``, or None.  The sums are those of the matrix alone,
+    so that its result is the same bits; of the cluster sizes that run at a time and hold the sums, the one whose busiest CTA reads least."""
+    key = (M, K, Ns)
+    if key not in _parts_plans:
+        plans = [_plan(M, n, K) for n in Ns]
+        bn, splits, tiles, blocks = plans[0][1], [p[2] for p in plans], sum(-(-n // 128) for n in Ns), -(-K // 64)
+        best = None
+        for c in range(1, 9):
+            if c > max(splits) or tiles * c > PARTS_TILES or (c > 1 and tiles > _max_clusters(c)):
+                break
+            sums = [-(-s // c) for s in splits]
+            # columns of tensor memory; shared memory of the operands' ring, which the sums of a cluster pass through
+            if max(sums) * bn > 512 or (c > 1 and max(sums) * bn * 512 > (8 if bn <= 64 else 6) * 128 * (128 + bn)):
+                continue
+            most = max(q * -(-blocks // s) for q, s in zip(sums, splits))
+            if best is None or most < best[0]:
+                best = (most, c)
+        _parts_plans[key] = None if best is None or any(p[1] != bn or not p[0] for p in plans) else (bn, splits, best[1])
+    return _parts_plans[key]
 
 
 def linear_parts(x: torch.Tensor, weights, biases, forms) -> Optional[list]:
     """x W_i^T (+ b_i) for up to four matrices in one launch, for rows that ``linear`` would give to ``gemm_tc`` one product at a time.  ``forms``: None;
     "silu" (W's rows interleave gate and up, the result is silu(gate) * up); or n (the outputs alternate between two results in runs of n: a tensor of
-    both).  None = not covered."""
+    both).  Every result is what its product alone gives, bit for bit.  None = not covered."""
     x2 = x.reshape(-1, x.shape[-1])
     M, K = x2.shape
     tiles = sum(-(-w.shape[0] // 128) for w in weights)
@@ -1111,12 +1136,15 @@ def linear_parts(x: torch.Tensor, weights, biases, forms) -> Optional[list]:
         if (f == "silu" and (N % 4 or b is not None)) or (isinstance(f, int) and (f % 4 or N % (2 * f))) or (b is not None and b.dtype != x.dtype):
             return None
         outs.append(torch.empty((2, M, N // 2) if isinstance(f, int) else (M, N // 2 if f == "silu" else N), dtype=x.dtype, device=x.device))
-    _, bn, splits, _, _ = _plan(M, tiles * 128, K)
+    plan = _parts_plan(M, K, tuple(w.shape[0] for w in weights))
+    if plan is None:
+        return None
+    bn, splits, ctas = plan
     n = len(weights)
     ptrs, ints = ctypes.c_void_p * n, _i * n
     _check(_gemm_parts(x2.data_ptr(), ptrs(*[w.data_ptr() for w in weights]), ptrs(*[_p(b) for b in biases]), ptrs(*[y.data_ptr() for y in outs]),
                        ints(*[w.shape[0] for w in weights]), ints(*[int(f == "silu") for f in forms]),
-                       ints(*[f if isinstance(f, int) else 0 for f in forms]), n, M, K, x2.stride(0), bn, splits, _DT[x.dtype], _st()),
+                       ints(*[f if isinstance(f, int) else 0 for f in forms]), ints(*splits), n, M, K, x2.stride(0), bn, ctas, _DT[x.dtype], _st()),
            f"linear_parts(M={M},N={[w.shape[0] for w in weights]},K={K})")
     lead = x.shape[:-1]
     return [y.view((2,) + lead + (-1,)) if isinstance(f, int) else y.view(lead + (-1,)) for y, f in zip(outs, forms)]
