@@ -24,3 +24,24 @@ def test_products_together_and_alone(M, K, parts, dtype):
         if isinstance(f, int):
             alone = alone.view(M, -1, 2, f).permute(2, 0, 1, 3).reshape(2, M, -1)
         assert torch.equal(y, alone)
+
+
+@pytest.mark.parametrize("R,I,K,E", [(48, 512, 1024, 16), (144, 768, 2048, 32), (7, 64, 192, 300), (300, 128, 64, 2), (1000, 192, 128, 9)])
+@pytest.mark.parametrize("act", ["silu", "gelu", "gelu_tanh"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_experts_streamed_and_by_tiles(R, I, K, E, act, dtype):
+    """Hidden rows and outputs of a few rows per expert are those of the product by tiles with the activation behind it."""
+    from vllm_b200.ops import cuda as cu
+    from vllm_b200.ops import moe
+    g = torch.Generator(device="cuda").manual_seed(R + E)
+    x = torch.randn(R, K, device="cuda", generator=g).to(dtype)
+    w13 = (torch.randn(E, 2 * I, K, device="cuda", generator=g) * K ** -0.5).to(dtype)
+    w2 = (torch.randn(E, K, I, device="cuda", generator=g) * I ** -0.5).to(dtype)
+    ids = torch.randint(0, E, (R, 1), device="cuda", generator=g, dtype=torch.int32)
+    tok, inv, offs = cu.moe_align(ids, E)
+    xs, bn = cu.moe_gather(x, tok), moe._tile_width(R, E)
+    want = cu.act_and_mul(cu.gemm_tc_grouped(xs, w13, offs, bn), act)
+    for width in (16, 32, 64, 128):
+        assert torch.equal(cu.gemm_experts(xs, w13, offs, width, act, rounded=True), want)
+    rows, where = moe.grouped_rows(x, w13, w2, ids, act, None)
+    assert torch.equal(rows[where.long()], cu.gemm_tc_grouped(want, w2, offs, bn)[inv.long()])

@@ -1,5 +1,7 @@
 // Grouped GEMM of decode steps:  Y[r, :] = X[r, :] · W[e(r)]^T  for a few rows per expert, sorted by expert; gated: Y[r, n] = act(X[r, :] · W[e, n]^T) *
-// (X[r, :] · W[e, I + n]^T), the activation in 32 bits between the accumulator and the one rounding.
+// (X[r, :] · W[e, I + n]^T), the activation in 32 bits between the accumulator and the one rounding, or (`rounded`) between numbers that are rounded first:
+// bit for bit what the product by tiles (gemm_tc.cu) and the activation behind it (norm_act.cu) give, so that neither a batch's size nor the choice of the
+// kernel shows in a token's hidden row.
 //
 // Bound by the weights, which are read once.  gemm_tc.cu gives every tile of 128 weight rows a CTA, two to an SM: each begins with a look for its
 // expert's rows and a first wait for memory and ends with a drain in which its half of the SM loads nothing.  Here a CTA stays on its SM
@@ -24,7 +26,7 @@ struct Params {
   int E, N, K;             // N: rows of an expert's weight (gated: 2 I)
   int tiles;               // per expert: of 128 rows, gated: of 64 + 64
   int second;              // weight rows between the two halves of a tile: 64 or I
-  int act;
+  int act, rounded;
   int ahead;
   // sums (not gated): acc[token of row r, :] += weight of r * product, in 32 bits; a row's (token, slot) pair is row_pair[r]
   float* acc;
@@ -180,7 +182,8 @@ experts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
             const int n = et & 63, col = a * (TM / 2) + n;
             if (col < p.second)
               for (int j = et >> 6; j < min(CH, rows - c); j += 2) {
-                const float g = xch[j * TM + n], up = xch[j * TM + 64 + n];
+                float g = xch[j * TM + n], up = xch[j * TM + 64 + n];
+                if (p.rounded) { g = to_f32(from_f32<T>(g)); up = to_f32(from_f32<T>(up)); }
                 const float x = p.act == ACT_SILU ? act_fn<ACT_SILU>(g) : p.act == ACT_GELU ? act_fn<ACT_GELU>(g) : act_fn<ACT_GELU_TANH>(g);
                 y[(int64_t)(row + c + j) * p.second + col] = from_f32<T>(x * up);
               }
@@ -238,8 +241,8 @@ static int launch(const CUtensorMap& tw, const CUtensorMap& tx, const Params& p,
 }  // namespace ge
 
 // x [R, K] rows sorted by expert (offs[e] .. offs[e + 1]), w [E, N, K]; act < 0: y [R, N], or sums into acc where given; act 0 silu, 1 gelu, 2 gelu by
-// tanh: w's rows are N / 2 gates and N / 2 ups (N / 2 a multiple of 64), y [R, N / 2].  bn: 16, 32, 64 or 128 rows of an expert at a time.
-EXPORT int vb_gemm_experts(const void* x, const void* w, void* y, const int* offs, int* error, int R, int N, int K, int E, int bn, int act, int ahead,
+// tanh: w's rows are N / 2 gates and N / 2 ups (N / 2 a multiple of 64), y [R, N / 2]; rounded: gates and ups are rounded first.  bn: 16, 32, 64 or 128 rows of an expert at a time.
+EXPORT int vb_gemm_experts(const void* x, const void* w, void* y, const int* offs, int* error, int R, int N, int K, int E, int bn, int act, int rounded, int ahead,
                            float* acc, const int* row_pair, const float* pair_w, int k, int H, int num_sms, int dtype, cudaStream_t st) {
   using namespace ge;
   if (R == 0) return 0;
@@ -250,7 +253,7 @@ EXPORT int vb_gemm_experts(const void* x, const void* w, void* y, const int* off
   int rc;
   if ((rc = tmap(&tw, w, (int64_t)E * N, K, TM / 2, bf16)) || (rc = tmap(&tx, x, R, K, bn, bf16))) return rc;
   Params p;
-  p.y = y; p.offs = offs; p.E = E; p.N = N; p.K = K; p.act = act; p.ahead = ahead; p.error = error;
+  p.y = y; p.offs = offs; p.E = E; p.N = N; p.K = K; p.act = act; p.rounded = rounded; p.ahead = ahead; p.error = error;
   p.acc = acc; p.row_pair = row_pair; p.pair_w = pair_w; p.k = k; p.H = H;
   p.tiles = gated ? N / 128 : (N + TM - 1) / TM;
   p.second = gated ? N / 2 : TM / 2;

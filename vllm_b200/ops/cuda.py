@@ -1361,18 +1361,20 @@ def gemm_tc_grouped(xs: torch.Tensor, w: torch.Tensor, offs: torch.Tensor, bn: i
     return y
 
 
-_gemm_experts = _sig("vb_gemm_experts", _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _vp)
+_gemm_experts = _sig("vb_gemm_experts", _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _i, _i, _i, _i, _vp)
 
 
-def gemm_experts(xs: torch.Tensor, w: torch.Tensor, offs: torch.Tensor, bn: int, act: Optional[str] = None, sums: Optional[tuple] = None):
+def gemm_experts(xs: torch.Tensor, w: torch.Tensor, offs: torch.Tensor, bn: int, act: Optional[str] = None, sums: Optional[tuple] = None,
+                 rounded: bool = False):
     """``gemm_grouped`` for a few rows per expert, weights streamed by one block per SM (csrc/gemm_experts.cu).  ``bn``: 16, 32, 64 or 128 rows of an
-    expert at a time.  ``sums`` = (address of the fp32 accumulator, sorted_pair, pair_w, k): the rows are added up there, times their weights."""
+    expert at a time.  ``sums`` = (address of the fp32 accumulator, sorted_pair, pair_w, k): the rows are added up there, times their weights.
+    ``rounded``: gates and ups are rounded before the activation, which gives the bits of ``act_and_mul(gemm_tc_grouped(...))``."""
     R, K = xs.shape
     E, N, _ = w.shape
     assert xs.is_contiguous() and w.is_contiguous() and xs.dtype == w.dtype and w.shape[2] == K
     y = None if sums else torch.empty((R, N if act is None else N // 2), dtype=xs.dtype, device=xs.device)
     acc, pair, pw, k = sums or (None, None, None, 1)
-    _check(_gemm_experts(xs.data_ptr(), w.data_ptr(), _p(y), offs.data_ptr(), _error_flag(xs.device), R, N, K, E, bn, _GATED_ACT[act], int(R >= 3 * E), acc,
+    _check(_gemm_experts(xs.data_ptr(), w.data_ptr(), _p(y), offs.data_ptr(), _error_flag(xs.device), R, N, K, E, bn, _GATED_ACT[act], int(rounded), int(R >= 3 * E), acc,
                          _p(pair), _p(pw), k, N, num_sms(), _DT[xs.dtype], _st()), f"gemm_experts(R={R},N={N},K={K},E={E})")
     return y
 

@@ -34,7 +34,7 @@ def grouped_rows(x, w13, w2, topk_ids, act, expert_map):
     bn = _tile_width(R, E)
     if streamed(R, w13, act):
         bn = _stream_width(bn)
-        return cu.gemm_experts(cu.gemm_experts(cu.moe_gather(x, sorted_tok), w13, offs, bn, act), w2, offs, bn), inv
+        return cu.gemm_experts(cu.gemm_experts(cu.moe_gather(x, sorted_tok), w13, offs, bn, act, rounded=True), w2, offs, bn), inv
     flat = flat_grid(R, E, bn)
     h = cu.gemm_tc_grouped(cu.moe_gather(x, sorted_tok), w13, offs, bn, flat=flat)
     return cu.gemm_tc_grouped(cu.act_and_mul(h, act), w2, offs, bn, flat=flat), inv
@@ -46,7 +46,8 @@ def streamed(R: int, w13, act) -> bool:
     the others and little else to read meanwhile.  us of both products, gemm_tc.cu (with the activation between them) → gemm_experts.cu: 2048 x 768, 32
     experts, 6 of them for each of 4 tokens 35 → 35, 8 tokens 42 → 38, 24 58 → 49, 128 64 → 55 (the weights' bytes take 47); 8 of 2048 x 2048, 2 for each of 4
     tokens 32 → 35, 8 38 → 37, 16 41 → 36, 128 48 → 41 (31); 16 of 1024 x 512, 4 for each of 4 tokens 17 → 14, 64 30 → 16 (8); 128 of 2048 x 768, 8
-    for each of 4 tokens 56 → 54, 16 134 → 121, 128 203 → 185 (187).  Not in batch-invariant mode, which rounds the hidden rows before the activation."""
+    for each of 4 tokens 56 → 54, 16 134 → 121, 128 203 → 185 (187).  The hidden
+    rows have the same bits either way.  Not in batch-invariant mode, where no kernel is chosen by the number of rows."""
     from vllm_b200.ops import cuda as cu
     E, N, _ = w13.shape
     return act in cu._GATED_ACT and N % 128 == 0 and E <= cu.GROUPED_MAX_EXPERTS and (R >= 3 * E or R >= E >= 16) and not cu.batch_invariant()
@@ -241,7 +242,7 @@ def fused_moe_reduce_norm(x, w13, w2, topk_w, topk_ids, act, expert_map, residua
         bn += 16
     stream = streamed(R, w13, act)
     if stream:
-        a = cu.gemm_experts(xs, w13, offs, _stream_width(bn), act)
+        a = cu.gemm_experts(xs, w13, offs, _stream_width(bn), act, rounded=True)
     else:
         a = cu.act_and_mul(cu.gemm_tc_grouped(xs, w13, offs, bn), act)
     pw = topk_w.to(torch.float32).contiguous()
