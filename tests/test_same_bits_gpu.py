@@ -45,3 +45,27 @@ def test_experts_streamed_and_by_tiles(R, I, K, E, act, dtype):
         assert torch.equal(cu.gemm_experts(xs, w13, offs, width, act, rounded=True), want)
     rows, where = moe.grouped_rows(x, w13, w2, ids, act, None)
     assert torch.equal(rows[where.long()], cu.gemm_tc_grouped(want, w2, offs, bn)[inv.long()])
+
+
+@pytest.mark.parametrize("E,groups,keep", [(40, 1, 1), (64, 4, 3), (96, 4, 2), (128, 8, 4), (129, 3, 2), (160, 8, 3), (256, 1, 1), (256, 32, 8)])
+@pytest.mark.parametrize("scoring,biased,top2", [("softmax", False, "max"), ("softmax", True, "top2"), ("sigmoid", True, "top2")])
+@pytest.mark.parametrize("renorm", [False, True])
+def test_router_of_few_and_many_tokens(E, groups, keep, scoring, biased, top2, renorm):
+    """A warp per token and a block per token: by the number of tokens above 128 experts, by that of the choices (32 and 33) at all sizes."""
+    from vllm_b200.ops import cuda as cu
+    g = torch.Generator(device="cuda").manual_seed(E + keep)
+    lg = torch.randn(1100, E, device="cuda", generator=g) * 3
+    bias = torch.randn(E, device="cuda", generator=g) * 0.1 if biased else None
+    if biased:
+        bias[1::5] = float("-inf")                   # experts that are never chosen
+    lg[3, ::7], lg[4], lg[5, 2] = float("-inf"), float("-inf"), float("nan")
+    if groups > 1:
+        lg[6:9, :E // groups - 1] = float("-inf")    # one candidate in a group
+    for t in (lg, lg.bfloat16()):
+        few = [cu.grouped_topk(t[a:a + 100], 8, groups, keep, renorm, scoring, bias, 2.5, top2) for a in range(0, 1100, 100)]
+        many = cu.grouped_topk(t, 8, groups, keep, renorm, scoring, bias, 2.5, top2)
+        assert torch.equal(torch.cat([f[1] for f in few]), many[1])
+        assert torch.equal(torch.cat([f[0] for f in few]).view(torch.int32), many[0].view(torch.int32))
+        if E > 33:
+            a, b = (cu.grouped_topk(t, k, groups, keep, False, scoring, bias, 1.0, top2) for k in (32, 33))
+            assert torch.equal(a[1], b[1][:, :32]) and torch.equal(a[0].view(torch.int32), b[0][:, :32].contiguous().view(torch.int32))

@@ -193,7 +193,7 @@ grouped_topk_kernel(const float* __restrict__ logits, const TX* __restrict__ x, 
     for (int j = lane; j < k; j += 32) out_w[(int64_t)t * k + j] *= scale / (wsum + 1e-20f);
 }
 
-// The same for given logits of up to 32 EL experts: a warp per token, its experts in registers, a maximum in one instruction (of keys that order as the
+// The same, to the bit, for given logits of up to 32 EL experts: a warp per token, its experts in registers, a maximum in one instruction (of keys that order as the
 // numbers do); a CTA per token spent its time on barriers and on two-step exchanges.  us, before and so: 24 tokens, 6 of 32 in 4 groups 5.1 and 2.5, 6900
 // tokens 21 and 6.8; 8 of 256 in 8 groups 7.1 and 7.9, 6900 tokens 39 and 23.
 VB_DEVICE uint32_t order_key(float x) {            // NaN and what is left out order as -inf: 0x007fffff
@@ -215,16 +215,24 @@ grouped_topk_warp_kernel(const TL* __restrict__ logits, const float* __restrict_
 #pragma unroll
   for (int i = 0; i < EL; ++i) score[i] = lane + 32 * i < E ? to_f32(logits[(int64_t)t * E + lane + 32 * i]) : -INFINITY;
   if (softmax) {
-    float mx = -INFINITY, sum = 0.f;
+    float mx = -INFINITY;
 #pragma unroll
     for (int i = 0; i < EL; ++i) mx = fmaxf(mx, score[i]);
     mx = warp_max(mx);
 #pragma unroll
-    for (int i = 0; i < EL; ++i) {
-      score[i] = lane + 32 * i < E ? expf(score[i] - mx) : 0.f;
-      sum += score[i];
-    }
-    const float inv = 1.f / warp_sum(sum);
+    for (int i = 0; i < EL; ++i) score[i] = lane + 32 * i < E ? expf(score[i] - mx) : 0.f;
+    // the sum in the order of the block's warps (64 threads up to 128 experts, 256 beyond) and of its sum over them: the same bits
+    float part[EL];
+#pragma unroll
+    for (int i = 0; i < EL; ++i) part[i] = EL == 4 && i < 2 ? score[i] + score[i + 2] : score[i];
+    constexpr int PARTS = EL == 4 ? 2 : EL;
+#pragma unroll
+    for (int i = 0; i < PARTS; ++i) part[i] = warp_sum(part[i]);
+#pragma unroll
+    for (int o = PARTS / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < o; ++i) part[i] += part[i + o];
+    const float inv = 1.f / part[0];
 #pragma unroll
     for (int i = 0; i < EL; ++i) score[i] *= inv;
   } else {
@@ -257,6 +265,7 @@ grouped_topk_warp_kernel(const TL* __restrict__ logits, const float* __restrict_
   if (n_group > 1) {
     const bool two = group_top2 && E / n_group > 1;
     uint32_t mine = NONE_KEY;                      // of group `lane`
+    bool low = false;                              // its score is -inf: such a group is neither chosen nor left out, as in the block
     for (int g = 0; g < n_group; ++g) {
       own(g, -1, key, place);
       const int p = first(key, place, top);
@@ -265,13 +274,14 @@ grouped_topk_warp_kernel(const TL* __restrict__ logits, const float* __restrict_
         own(g, p, key, place);
         s += number(__reduce_max_sync(ALL, key));
       }
-      if (lane == g) mine = order_key(s);
+      if (lane == g) { mine = order_key(s); low = s == -INFINITY; }
     }
     unsigned kept = 0;
     for (int n = 0; n < keep; ++n) {
       const int g = first(lane < n_group && !((kept >> lane) & 1u) ? mine : NONE_KEY, lane, top);
       if (top != NONE_KEY) kept |= 1u << g;
     }
+    kept |= __ballot_sync(ALL, low);
 #pragma unroll
     for (int i = 0; i < EL; ++i)
       if (group[i] >= 0 && !((kept >> group[i]) & 1u)) choice[i] = NONE_KEY;
