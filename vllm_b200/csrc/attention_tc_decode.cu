@@ -17,7 +17,6 @@
 // The weights keep 16 more bits in a second product, P = hi + lo: 2 % of the time, and the error against 64 bits is that of the result's own
 // rounding (bf16, 33 to 2000 tokens: 0.00165; with 16-bit weights 0.0017 to 0.0022, as before).  CAP: capped scores.
 #include "attention_prompt.cuh"
-#include "warp_mma.cuh"
 
 namespace fmha_dec {
 
@@ -55,6 +54,22 @@ struct Params {
   const float* sinks;      // optional [Hq] logits in the softmax denominator that have no key
   float out_scale;         // factor of the output
 };
+
+VB_DEVICE void ldsm4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+template <typename T> VB_DEVICE void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1);
+template <> VB_DEVICE void mma16816<__nv_bfloat16>(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <> VB_DEVICE void mma16816<__half>(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// an 8 x 8 matrix of 16-bit values, two to a lane, with rows and columns exchanged
+VB_DEVICE uint32_t turn8(uint32_t x) { uint32_t r; asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(x)); return r; }
+VB_DEVICE float ld_dsmem_f32(uint32_t addr) { float v; asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr)); return v; }
 
 // NT: groups of eight query rows
 template <typename T, int NT, bool CAP, typename F>
@@ -208,7 +223,10 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
         uint32_t keep[2] = {0xffffffffu, 0xffffffffu};        // of tokens c0, c0 + 1 of either group of eight
         if (cut) {
 #pragma unroll
-          for (int j = 0; j < 2; ++j) keep[j] = keep2(tok + j * 8 + c0, kv_begin, kv_end);
+          for (int j = 0; j < 2; ++j) {
+            const int t = tok + j * 8 + c0;
+            keep[j] = (t >= kv_begin && t < kv_end ? 0xffffu : 0u) | (t + 1 >= kv_begin && t + 1 < kv_end ? 0xffff0000u : 0u);
+          }
         }
 #pragma unroll
         for (int i = 0; i < D / 16; ++i) {
@@ -315,21 +333,25 @@ static int launch(const CUtensorMap& tk, const CUtensorMap& tv, const Params& p,
     if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return -21;
     set = true;
   }
-  return (int)vb_launch_parts(k, dim3(p.parts * B, p.Hkv), dim3(F::NUM_THREADS), (size_t)smem, st, p.parts, tk, tv, p);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.parts * B, p.Hkv); cfg.blockDim = dim3(F::NUM_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (p.parts > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = p.parts; attr[n].val.clusterDim.y = 1; attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (vb_pdl_enabled()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
+  cfg.attrs = attr; cfg.numAttrs = n;
+  return (int)cudaLaunchKernelEx(&cfg, k, tk, tv, p);
 }
 
 }  // namespace fmha_dec
-
-// clusters of `parts` CTAs of the form Few that run at a time
-EXPORT int vb_fmha_decode_clusters(int parts) {
-  using namespace fmha_dec;
-  auto k = fmha_decode_kernel<__nv_bfloat16, 1, false, Few>;
-  const int smem = Few::STAGES * STAGE_BYTES + 8 * ROW_BYTES + 1024;
-  if (parts < 1 || parts > MAX_PARTS || cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, Few::STAGES * STAGE_BYTES + 16 * ROW_BYTES + 1024) != cudaSuccess ||
-      cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-    return -1;
-  return vb_max_clusters(k, dim3(Few::NUM_THREADS), (size_t)smem, parts);
-}
 
 // q [B, Hq, 128] (rows start on 4 bytes), out [B, Hq, 128]; parts: key ranges per (request, kv head), a cluster of CTAs (1 to 16).
 // `error` (device int, may be null) becomes 1 when a wait inside the kernel ran into its limit.

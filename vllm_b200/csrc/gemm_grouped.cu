@@ -12,7 +12,7 @@
 // Warps: 0 TMA producer, 1 MMA issuer (pairs: of the first CTA), 2..5 epilogue (thread = row).
 #include "act.cuh"
 #include "pair_mma.cuh"
-#include "warp_mma.cuh"
+#include "cluster.cuh"
 
 namespace gg {
 

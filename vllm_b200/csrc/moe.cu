@@ -4,7 +4,7 @@
 // Reference counterparts: csrc/moe/topk_softmax_kernels.cu, moe_align_sum_kernels.cu, moe_permute_unpermute_op.cu
 // (here: routing probabilities + top-k in one warp per token; counting sort of (token, slot) pairs by expert with
 // an inverse map; weighted un-permute that sums a token's k expert outputs in a fixed order → deterministic).
-#include "warp_mma.cuh"
+#include "cluster.cuh"
 
 namespace moe {
 

@@ -6,7 +6,7 @@
 // One CTA per row; logits are read once with 16-byte loads straight from the LM-head output
 // dtype (no fp32 staging copy); the noise is a counter-based hash of (seed, step, token) so
 // the result is independent of launch geometry and reproducible per request seed.
-#include "warp_mma.cuh"
+#include "cluster.cuh"
 
 namespace {
 

@@ -387,15 +387,6 @@ def decode_splits(B: int, Hkv: int, max_seq_len: int, block_size: int) -> int:
 # 8 / 2 heads 24.3 and 7.2 (17.4), 2 x 1000 of 16 / 4 8.8 and 5.6 (9.7), 8 x 1000 9.1 and 7.7 (10.9), 16 x 4000 27.3 and 24.9 (27.3), 8 x 16000 of 16 / 1
 # 128 and 24 (87), 1 x 40 of 8 / 2 3.1 (4.8).
 MAX_PARTS, SPLIT_PAGES = 16, 32
-_decode_clusters, _mla_clusters = _sig("vb_fmha_decode_clusters", _i), _sig("vb_mla_clusters", _i)
-
-
-@functools.lru_cache(maxsize=None)
-def clusters_at_a_time(mla: bool, parts: int) -> int:
-    """How many clusters of so many CTAs run together: a cluster stays within one of the groups of SMs (16 to 20 of them), so six CTAs each for 24
-    requests would take two rounds."""
-    n = (_mla_clusters if mla else _decode_clusters)(parts)
-    return n if n >= 0 else num_sms() // parts                   # (no device to ask)
 
 
 def decode_parts(B: int, Hkv: int, max_seq_len: int) -> int:
@@ -405,7 +396,7 @@ def decode_parts(B: int, Hkv: int, max_seq_len: int) -> int:
     if envs.VLLM_B200_ATTN_SPLITS > 0:
         return min(envs.VLLM_B200_ATTN_SPLITS, MAX_PARTS)
     n, pages = max(B * Hkv, 1), -(-max(max_seq_len, 1) // 64)
-    return next((p for p in (8, 4, 2) if n * p <= num_sms() and pages * p > SPLIT_PAGES and n <= clusters_at_a_time(False, p)), 1)
+    return next((p for p in (8, 4, 2) if n * p <= num_sms() and pages * p > SPLIT_PAGES), 1)
 
 
 def decode_form(ctas: int) -> int:
@@ -596,14 +587,15 @@ def merge_attn_states(o1, lse1, o2, lse2):
     return out, lse
 
 
-_mla_decode = _sig("vb_mla_decode3", _vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i64, _i64,
-                   _i64, _i64, _i64, _i, _i, _i, _i, _i, _f, _i, _vp)
+_mla_decode = _sig("vb_mla_decode2", _vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i64, _i64,
+                   _i64, _i64, _i64, _i, _i, _i, _i, _f, _i, _vp)
 _mla_prefill = _sig("vb_mla_prefill3", _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i64, _i, _i, _i, _i, _i, _i, _i64, _i64,
                     _i64, _i64, _i64, _i64, _i64, _i, _i, _f, _i, _i, _i, _i, _vp)
 _mla_simt = _sig("vb_mla_simt", _vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _i, _i, _i, _i, _i, _i, _i64, _i64, _i64, _i64, _i64,
                  _i64, _i, _f, _i, _vp)
 _latent_rope = _sig("vb_latent_rope_cache2", _vp, _vp, _i64, _i64, _i, _i, _i, _i, _vp, _f, _vp, _vp, _i, _vp, _i64, _vp, _i, _i, _vp)
 _latent_norm = _sig("vb_latent_norm_cache", _vp, _i64, _i, _vp, _vp, _i, _vp, _vp, _vp, _i64, _vp, _i, _f, _i, _vp)
+_mla_ws: dict[int, tuple] = {}
 _kernel_error: dict[int, torch.Tensor] = {}
 
 
@@ -639,40 +631,49 @@ def check_kernel_error(device: torch.device) -> None:
             raise RuntimeError(KERNEL_GAVE_UP)
 
 
-MLA_SPLIT_TILES = 2      # rows of so many tiles of 64 tokens stay with one CTA
-
-
-def mla_decode_splits(B: int, H: int, max_seq_len: int) -> int:
-    """Token ranges per (request, sixteen heads) of csrc/mla_decode.cu, the CTAs of a cluster: one CTA per SM (its shared memory), one round.
-    us with the best of 1 to 8 splits of the tcgen05 kernel before (in brackets as captured steps split) and so: 24 requests of 60 to 924 tokens, 16
-    heads 20.6 (35.5) and 13.3, 8 x 1000 18.5 (35.8) and 11.0, 1 x 4000 37.0 (111) and 18.7, 64 x 1024 37.9 and 25.1, 256 x 1024 119 and 64, of 128
-    heads 64 x 1024 128 and 117, 1 x 32000 123 and 100; R = 128 without rope 64 x 1024 15.3 and 12.0."""
+def mla_decode_splits(B: int, H: int, max_seq_len: int, least: int = 512) -> int:
     if batch_invariant():
         return 1
     forced = envs.VLLM_B200_ATTN_SPLITS
     if forced > 0:
-        return min(forced, MAX_PARTS)
-    n = max(B * -(-H // 16), 1)
-    return next((p for p in range(min(8, num_sms() // n, -(-max_seq_len // 64)), 1, -1) if n <= clusters_at_a_time(True, p)), 1)
+        return forced
+    groups = (H + 31) // 32 if H > 16 else 1
+    ctas = max(B * groups, 1)
+    s = max(1, min(16, num_sms() // ctas))           # one CTA per SM (170 KB smem): stay inside ONE wave
+    return max(1, min(s, max_seq_len // least))     # every split should still stream >= 8 tiles (windows: 4)
 
 
 def mla_decode_tc(q_nope_abs, q_pe, kv_cache, block_table, seq_lens, scale, max_seq_len: int, num_splits: int = 0,
                   return_lse: bool = False, sliding_window: Optional[int] = None, wide: bool = False):
-    """MLA decode on the tensor cores (csrc/mla_decode.cu): q_nope_abs [B, H, R], q_pe [B, H, P] or None, cache [blocks, BS, R + P].  ``wide``: the
+    """tcgen05 MLA decode (csrc/mla_decode.cu): q_nope_abs [B, H, R], q_pe [B, H, P] or None, cache [blocks, BS, R + P].  ``wide``: the
     softmax weights keep 16 more bits."""
     B, H, R = q_nope_abs.shape
     P = 0 if q_pe is None else q_pe.shape[-1]
     assert kv_cache.shape[-1] == R + P and q_nope_abs.stride(-1) == 1 and (q_pe is None or q_pe.stride(-1) == 1)
     dev = q_nope_abs.device
-    parts = min(num_splits, MAX_PARTS) or mla_decode_splits(B, H, min(max_seq_len, sliding_window or max_seq_len))
+    splits = num_splits or (mla_decode_splits(B, H, min(max_seq_len, sliding_window), 256) if sliding_window else
+                            mla_decode_splits(B, H, max_seq_len))
     out = torch.empty((B, H, R), dtype=q_nope_abs.dtype, device=dev)
     lse = torch.empty((B, H), dtype=torch.float32, device=dev) if return_lse else None
+    po = pl = None
+    if splits > 1:
+        key = dev.index or 0
+        need = B * H * splits
+        ws = _mla_ws.get(key)
+        if ws is None or ws[1].numel() < need:
+            if torch.cuda.is_current_stream_capturing():
+                raise RuntimeError("MLA split-KV workspace must be allocated before CUDA-graph capture")
+            n = max(need, 64 * 128 * 4)
+            ws = _mla_ws[key] = (torch.empty(n * 512, dtype=torch.float32, device=dev),
+                                 torch.empty(n, dtype=torch.float32, device=dev))
+        po, pl = ws
+    err = kernel_error_flag(dev)
     _check(_mla_decode(q_nope_abs.data_ptr(), _p(q_pe), kv_cache.data_ptr(), kv_cache.shape[0],
-                       block_table.data_ptr(), seq_lens.data_ptr(), out.data_ptr(), _p(lse), _error_flag(dev), B,
+                       block_table.data_ptr(), seq_lens.data_ptr(), out.data_ptr(), _p(po), _p(pl), _p(lse), err.data_ptr(), B,
                        H, R, P, kv_cache.shape[1], q_nope_abs.stride(0), q_nope_abs.stride(1),
                        q_pe.stride(0) if P else 0, q_pe.stride(1) if P else 0,
-                       out.stride(0), block_table.stride(0), parts, 0 if num_splits else MLA_SPLIT_TILES, sliding_window or 0, int(wide), scale,
-                       _DT[q_nope_abs.dtype], _st()), f"mla_decode(B={B},H={H},R={R})")
+                       out.stride(0), block_table.stride(0), splits, sliding_window or 0, int(wide), scale, _DT[q_nope_abs.dtype], _st()),
+           f"mla_decode(B={B},H={H},R={R})", 2 if splits > 1 else 1)
     return (out, lse) if return_lse else out
 
 
@@ -781,7 +782,8 @@ def mla_attention(q_nope_abs, q_pe, kv_cache, md, scale, kv_lora_rank, sliding_w
     kernel of csrc/latent.cu, which needs no host lengths either."""
     R = q_nope_abs.shape[-1]
     if md.decode_only and R == kv_lora_rank and _mla_tc_ok(q_nope_abs, q_pe, kv_cache):
-        return mla_decode_tc(q_nope_abs, q_pe, kv_cache, md.block_table, md.seq_lens, scale, md.max_seq_len, sliding_window=sliding_window)
+        return mla_decode_tc(q_nope_abs, q_pe, kv_cache, md.block_table, md.seq_lens, scale, md.max_seq_len,
+                             md.num_splits or 0, sliding_window=sliding_window)
     B = md.num_reqs
     return mla_simt(q_nope_abs, q_pe, kv_cache, md.block_table, md.seq_lens[:B],
                     None if md.decode_only else md.query_start_loc, scale, sliding_window)
