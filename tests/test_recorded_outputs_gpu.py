@@ -10,7 +10,9 @@ import torch
 
 pytestmark = pytest.mark.gpu
 HERE = os.path.dirname(__file__)
-CASES = {"deepseek": ("deepseek", 12, 20, 90, 5, False), "deepseek long": ("deepseek", 3, 500, 700, 3, False)}
+CASES = {"llama": ("llama", 12, 20, 90, 5, False), "llama long": ("llama", 3, 500, 700, 3, False), "llama fp8": ("llama", 12, 20, 90, 5, True),
+         "gemma2": ("gemma2", 12, 20, 90, 5, False), "gemma2 long": ("gemma2", 3, 500, 700, 3, False), "mixtral": ("mixtral", 12, 20, 90, 5, False),
+         "deepseek": ("deepseek", 12, 20, 90, 5, False), "deepseek long": ("deepseek", 3, 500, 700, 3, False), "qwen3next": ("qwen3next", 12, 20, 90, 5, False)}
 
 
 def outputs(name):

@@ -94,8 +94,8 @@ _paged_attention_ex = _sig("vb_paged_attention_ex", _vp, _vp, _vp, _vp, _vp, _vp
                            _i64, _i64, _i, _i, _i, _f, _f, _f, _i, _i, _i, _vp, _vp, _i, _vp)
 _fmha_tc = _sig("vb_fmha_tc4", _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i64, _i64, _i,
                 _i, _i, _f, _f, _i, _i, _i, _vp, _f, _i, _i, _i, _vp)
-_fmha_tc_decode = _sig("vb_fmha_tc_decode3", _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i64, _i, _i, _i, _i, _i, _f, _f, _i, _vp,
-                       _f, _i, _vp)
+_fmha_tc_decode = _sig("vb_fmha_tc_decode2", _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i64, _i,
+                       _i, _i, _f, _f, _i, _vp, _f, _i, _vp)
 _any_attention = _sig("vb_any_attention", _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i64, _i64, _i, _i, _i,
                       _i, _f, _f, _f, _vp, _vp, _i, _vp)
 _merge_states = _sig("vb_merge_attn_states", _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _vp)
@@ -381,32 +381,6 @@ def decode_splits(B: int, Hkv: int, max_seq_len: int, block_size: int) -> int:
     return max(1, min(s, pages))
 
 
-# How csrc/attention_tc_decode.cu divides a decode step.  Parts of the keys are CTAs of one cluster; merging them takes 1.2 us, so they are taken where
-# one CTA per (request, kv head) leaves SMs idle, and the kernel leaves what has SPLIT_PAGES / parts pages or fewer to one CTA.  us in a graph with
-# caches larger than L2, one part and this rule (in brackets the tcgen05 kernel of before, with the better of one and two splits): 1 x 4000 tokens of
-# 8 / 2 heads 24.3 and 7.2 (17.4), 2 x 1000 of 16 / 4 8.8 and 5.6 (9.7), 8 x 1000 9.1 and 7.7 (10.9), 16 x 4000 27.3 and 24.9 (27.3), 8 x 16000 of 16 / 1
-# 128 and 24 (87), 1 x 40 of 8 / 2 3.1 (4.8).
-MAX_PARTS, SPLIT_PAGES = 16, 32
-
-
-def decode_parts(B: int, Hkv: int, max_seq_len: int) -> int:
-    """Key ranges per (request, kv head) of csrc/attention_tc_decode.cu, the CTAs of a cluster."""
-    if batch_invariant():
-        return 1
-    if envs.VLLM_B200_ATTN_SPLITS > 0:
-        return min(envs.VLLM_B200_ATTN_SPLITS, MAX_PARTS)
-    n, pages = max(B * Hkv, 1), -(-max(max_seq_len, 1) // 64)
-    return next((p for p in (8, 4, 2) if n * p <= num_sms() and pages * p > SPLIT_PAGES), 1)
-
-
-def decode_form(ctas: int) -> int:
-    """Pages on their way per CTA and CTAs per SM (Few, Some, Many): a page takes 1.6 us to come, so a CTA that has its SM to itself keeps six on
-    the way; with several per SM one's start is hidden by the others.  us for Few, Some, Many, and before: 24 requests of 60 to 924 tokens, 16 / 4
-    heads (96 CTAs) 9.3, 12.1, 13.8 (11.5); 64 of 60 to 532 (256) 13.9, 11.5, 12.5 (14.6); 64 x 1024, 32 / 8 (512) 52.2, 47.7, 51.7 (48.4); 256 x 500
-    (2048) 99.9, 90.5, 85.6 (87.6).  (With weights of one part; the second adds 0.2 to 0.5.)"""
-    return 0 if ctas <= num_sms() else 1 if ctas <= 6 * num_sms() else 2
-
-
 _SIMT_SHAPES = {(128, 64), (64, 64), (32, 64), (128, 32), (128, 16), (64, 32), (64, 16), (256, 32), (32, 32), (32, 16)}
 
 
@@ -445,21 +419,19 @@ def paged_attention(q, kv_cache, md, scale, sliding_window=None, logits_soft_cap
         assert tc_attention_ok(D, DV, G) and BS == 64 and alibi_slopes is None, "tensor-core attention: D=128, 64-token pages, no ALiBi"
         # batch-invariant mode: a decode row takes the varlen kernel it would take inside a mixed batch
         decode = md.decode_only and not (batch_invariant() and md.query_start_loc is not None)
-        if decode and G <= 16 and (G & (G - 1)) == 0 and causal:
-            reach = min(x for x in (md.max_seq_len, sliding_window, chunk_size) if x)
-            parts = min(md.num_splits, MAX_PARTS) or decode_parts(md.num_reqs, Hkv, reach)
-            rc = _fmha_tc_decode(q.data_ptr(), kv_cache.data_ptr(), kv_cache.shape[0], bt.data_ptr(), md.seq_lens.data_ptr(), out.data_ptr(),
-                                 _p(lse), _error_flag(q.device), md.num_reqs, Hq, Hkv, q.stride(0), out.stride(0), bt.stride(0), parts,
-                                 0 if md.num_splits else SPLIT_PAGES, decode_form(md.num_reqs * Hkv * parts),
-                                 sliding_window or 0, scale, logits_soft_cap, chunk_size, _p(sinks), out_scale, _DT[q.dtype], _st())
-            _check(rc, f"fmha_tc_decode(G={G})")
-            return (out, lse) if return_lse else out
-        # (a captured step knows no lengths: those of a typical context)
-        typical = min(md.max_seq_len, 4096) if torch.cuda.is_current_stream_capturing() else md.max_seq_len
-        splits = (md.num_splits or decode_splits(md.num_reqs, Hkv, typical, 128)) if decode else 1
+        splits = (md.num_splits or decode_splits(md.num_reqs, Hkv, md.max_seq_len, 128)) if decode else 1
         if chunk_size and chunk_size <= 4096:
             splits = 1                                   # a chunk is all that a query reads
         ws = _get_attn_ws(md.num_reqs, Hq, D, splits, q.device) if splits > 1 else None
+        if decode and G <= 16 and (G & (G - 1)) == 0 and causal:
+            # swap-AB decode kernel: KV tokens on the MMA M axis
+            rc = _fmha_tc_decode(q.data_ptr(), kv_cache.data_ptr(), kv_cache.shape[0], bt.data_ptr(),
+                                 md.seq_lens.data_ptr(), out.data_ptr(), _p(ws.part_out) if ws else None,
+                                 _p(ws.part_lse) if ws else None, _p(lse), md.num_reqs, Hq, Hkv, q.stride(0),
+                                 out.stride(0), bt.stride(0), splits, sliding_window or 0, scale, logits_soft_cap, chunk_size,
+                                 _p(sinks), out_scale, _DT[q.dtype], _st())
+            _check(rc, f"fmha_tc_decode(G={G})", 2 if splits > 1 else 1)
+            return (out, lse) if return_lse else out
         rc = _fmha_tc(q.data_ptr(), kv_cache.data_ptr(), kv_cache.shape[0], bt.data_ptr(), md.seq_lens.data_ptr(),
                       None if decode else md.query_start_loc.data_ptr(), out.data_ptr(),
                       _p(ws.part_out) if ws else None, _p(ws.part_lse) if ws else None, _p(lse), _error_flag(q.device),
