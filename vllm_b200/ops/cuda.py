@@ -1068,7 +1068,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
 _gemm_parts = _sig("vb_gemm_tc_parts", _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i, _i, _i, _vp)
 _max_clusters = _sig("vb_gemm_max_active_clusters", _i)
 # as many tiles as have a CTA each, by the ceiling of csrc/gemm_tc.cu's own plan: beyond that two share an SM, which only the single product's form does
-MAX_PARTS, PARTS_ROWS, PARTS_TILES = 4, 128, 132
+PARTS_MATRICES, PARTS_ROWS, PARTS_TILES = 4, 128, 132
 _parts_plans: dict[tuple, Optional[tuple]] = {}
 
 
@@ -1101,7 +1101,7 @@ def linear_parts(x: torch.Tensor, weights, biases, forms) -> Optional[list]:
     x2 = x.reshape(-1, x.shape[-1])
     M, K = x2.shape
     tiles = sum(-(-w.shape[0] // 128) for w in weights)
-    if (not 0 < M <= PARTS_ROWS or not 1 < len(weights) <= MAX_PARTS or tiles > PARTS_TILES or envs.VLLM_B200_GEMM_SK or batch_invariant()
+    if (not 0 < M <= PARTS_ROWS or not 1 < len(weights) <= PARTS_MATRICES or tiles > PARTS_TILES or envs.VLLM_B200_GEMM_SK or batch_invariant()
             or not all(w.shape[1] == K and _tc_ok(x2, w) for w in weights)):
         return None
     outs = []
