@@ -2,7 +2,7 @@
 
     VLLM_BATCH_INVARIANT=1 python scripts/batch_invariance_check.py [--model llama-3-8b] [--tp 1]
 
-Generates from one prompt (a) alone, (b) first in a batch of 48 unrelated prompts of mixed length, (c) last in that batch,
+Generates from one prompt (a) alone, (b) first in a batch of 62 unrelated prompts of mixed length, (c) last in that batch,
 (d) arriving while the others are mid-decode, and compares the sampled-token logprobs bit for bit.  Prints one JSON
 line: {"invariant": bool, "max_abs_diff": {...}}.  Without the flag the same script reports how far the default
 dispatch drifts (split-K / split-KV / in-switch reductions), which is the number the mode exists to remove.
@@ -29,7 +29,7 @@ def main():
     V = llm.llm_engine.vllm_config.model_config.vocab_size
     sp = SamplingParams(max_tokens=a.tokens, temperature=0.0, ignore_eos=True, logprobs=1)
     needle = {"prompt_token_ids": [(17 * i + 3) % (V - 10) + 5 for i in range(301)]}
-    others = [{"prompt_token_ids": [(31 * i + 7 * j) % (V - 10) + 5 for j in range(16 + 61 * (i % 9))]} for i in range(48)]
+    others = [{"prompt_token_ids": [(31 * i + 7 * j) % (V - 10) + 5 for j in range(16 + 61 * (i % 9))]} for i in range(62)]
 
     def lps(out):
         o = out.outputs[0]

@@ -546,13 +546,13 @@ EXPORT int vb_row_lse(const void* logits, int64_t row_stride, int B, int V, floa
   return (int)cudaGetLastError();
 }
 
-// k <= V; rows 16-byte aligned (row_stride a multiple of 16 bytes)
-EXPORT int vb_logprobs(const void* logits, int64_t row_stride, int B, int V, const int64_t* sampled, int k, int* out, int dtype, cudaStream_t st) {
+// k <= V; rows 16-byte aligned (row_stride a multiple of 16 bytes).  alone: a CTA per row whatever B and k are, as the two forms add in different orders
+EXPORT int vb_logprobs(const void* logits, int64_t row_stride, int B, int V, const int64_t* sampled, int k, int* out, int alone, int dtype, cudaStream_t st) {
   if (B == 0) return 0;
   if (k < 0 || k > V) return -1;
   // Clusters for up to 7.5 M values: beyond that there are rows enough for all SMs, and a CTA per row has less to exchange, while k is small (its
   // cost grows with k).  us for k = 5, clusters and CTAs: 128 rows of 32000 15 and 24, 256 29 and 24, 512 56 and 44; 64 rows of 102400 44 and 50, 128 79 and 58.
-  if (B <= INT32_MAX / 8 && V <= 8 * 32 * 1024 && k <= 64 && (k > 8 || (int64_t)B * V <= 7500000)) {
+  if (!alone && B <= INT32_MAX / 8 && V <= 8 * 32 * 1024 && k <= 64 && (k > 8 || (int64_t)B * V <= 7500000)) {
     // the smallest CTAs of which eight hold a row
     const int threads = V <= 8 * 32 * 256 ? 256 : V <= 8 * 32 * 512 ? 512 : 1024, parts = (V + threads * 32 - 1) / (threads * 32);
     const size_t smem = (size_t)2 * (threads / 32 + 1) * k * 4;

@@ -21,7 +21,7 @@ MoE combine            ``red.add.f32`` epilogue into per-token accumulators     
 NCCL fallbacks         library's size-dependent algorithm / protocol               tree + Simple, one channel, no NVLS / CollNet
 =====================  =========================================================  ==========================================
 
-Per-row kernels (LayerNorm; RoPE; activation; sampling: one row per CTA) are already invariant.  Not covered: products of
+Per-row kernels (LayerNorm; RoPE; activation; sampling: one row per CTA, log-probabilities too, in this mode) are already invariant.  Not covered: products of
 more than 256 rows in 16 bits, whose kernel the library picks by the rows; MLA decode rows inside a mixed batch (they take
 the prefill path), FP4 weight-only GEMMs, LoRA shrink/expand split over slots.
 
