@@ -60,7 +60,7 @@ class EngineCore:
         self.batch_queue_size = n_batches
         self.step_fn: Callable = self.step if self.batch_queue is None else self.step_with_batch_queue
         self._aborts_since_step: list[str] = []
-        self._ahead = False
+        self._ahead = self._ahead_ends = False
 
     def _initialize_kv_caches(self):
         t0 = time.perf_counter()
@@ -97,10 +97,10 @@ class EngineCore:
         if sp is not None and sp.structured_outputs is not None:
             so_req = self.structured_output_manager.make_request(req.request_id, sp.structured_outputs)
         r = Request.from_engine_core_request(req, self.block_hasher, so_req)
-        if self._ahead and not self._steps_ahead(r):
-            raise RuntimeError("a request that is sampled with host state cannot join steps that run ahead")
         if len(r.prompt_token_ids) >= self.vllm_config.scheduler_config.max_model_len:
             raise ValueError(f"prompt of {len(r.prompt_token_ids)} tokens exceeds max_model_len")
+        if self._ahead and not self._steps_ahead(r):
+            self._ahead_ends = True     # what is in flight comes back first, then steps are synchronous
         self.scheduler.add_request(r)
 
     def _restore_mm(self, req) -> None:
@@ -156,7 +156,10 @@ class EngineCore:
         bq = self.batch_queue
         assert bq is not None
         scheduled = False
-        if len(bq) < self.batch_queue_size and self.scheduler.has_requests():
+        if self._ahead_ends and not bq:
+            self._set_ahead(False)
+            return self.step()
+        if not self._ahead_ends and len(bq) < self.batch_queue_size and self.scheduler.has_requests():
             so = self.scheduler.schedule()
             if so.total_num_scheduled_tokens > 0 or so.finished_req_ids:
                 so.grammar_bitmask = self.scheduler.get_grammar_bitmask(so)
@@ -178,7 +181,7 @@ class EngineCore:
     # ------------------------------------------------------- one step ahead
     def start_ahead(self) -> bool:
         """For a caller that steps until all its requests are done: the next step is scheduled and launched while the device works on this one,
-        as with ``async_scheduling``, until ``stop_ahead``.  Only where a step needs nothing from the host but its tokens: one worker in
+        as with ``async_scheduling``, until ``stop_ahead`` or a request that does not allow it.  Only where a step needs nothing from the host but its tokens: one worker in
         this process, no speculation or connector, and requests without per-token host state.  False: steps stay synchronous."""
         from vllm_b200.executor import UniProcExecutor
         s = self.scheduler
@@ -197,7 +200,7 @@ class EngineCore:
                 and not sp.bad_words_token_ids and sp.min_tokens == 0 and not sp.stop and not sp.extra_args)
 
     def _set_ahead(self, on: bool) -> None:
-        self._ahead = on
+        self._ahead, self._ahead_ends = on, False
         self.batch_queue, self.batch_queue_size = (deque(maxlen=2), 2) if on else (None, 1)
         self.step_fn = self.step_with_batch_queue if on else self.step
         self.scheduler.async_scheduling = on
