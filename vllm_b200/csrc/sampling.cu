@@ -176,11 +176,12 @@ __global__ void __launch_bounds__(1024) logprobs_kernel(const T* __restrict__ lo
 
 // The same for vocabularies of up to 8 x 32 x THREADS tokens: a row is a cluster's, 32 x THREADS values of it a CTA's, 32 a thread's, which holds
 // them in registers for all passes.  The k likeliest are among the values that reach the k-th of the maxima of 2 k groups and more: hardly more than k
-// of them, which the CTAs list and the first one ranks by comparing each with each.  Where the lists are too short for that (equal
-// values, rows that are masked for the most part), a warp takes its k likeliest one by one, the CTA merges its warps' lists, the first CTA those of
-// the cluster.  What bounds it is the chain of exchanges, not the 1.5 MB
-// of 24 such rows: us for k = 5, here and with a CTA per row, 1 row of 32000 6.9 and 15.2, 24 rows 7.5 and 15.7, 24 rows of 102400 18 and 36, of
-// 256000 32 and 89; for k = 64, 1 row of 32000 11 and 136.  Rows of one value, which take the second way: 24 of 32000 24 and 17.
+// of them, which the CTAs list and the first one ranks by comparing each with each.  Where the lists are too short for that (equal values, or the likeliest
+// next to each other in a few groups), a CTA lists what is above the bound and the first k that are equal; with too many above it the bound is the
+// largest of the CTAs' own k-th maxima of 256 groups.  Where the lists are still too short, a warp takes its k likeliest one by one, the CTA merges its
+// warps' lists, the first CTA those of the cluster.  What bounds it is the chain of exchanges, not the 1.5 MB of 24 such rows: us for k = 5, here and with
+// a CTA per row, 1 row of 32000 6.9 and 15.2, 24 rows 7.5 and 15.7, 24 rows of 102400 18 and 36, of 256000 32 and 89; for k = 64, 1 row of 32000
+// 11 and 136.  Rows of one value and ascending ones: 24 of 32000 13 and 17, 17 and 16.
 template <typename T, int THREADS>
 __global__ void __launch_bounds__(THREADS) logprobs_cluster_kernel(const T* __restrict__ logits, int64_t row_stride, int V,
                                                                    const int64_t* __restrict__ sampled, int k, int* __restrict__ out, int parts) {
@@ -190,8 +191,10 @@ __global__ void __launch_bounds__(THREADS) logprobs_cluster_kernel(const T* __re
   int* li = reinterpret_cast<int*>(lp_smem + (WARPS + 1) * k);
   __shared__ float red[32];
   __shared__ float part[2];                          // of the CTA: maximum, sum of exponentials
-  __shared__ float groups[128], row_groups[256];     // maxima of the CTA's groups, of the row's
-  __shared__ int count[2];                           // of the CTA: tokens above the sampled one, listed values
+  __shared__ float groups[128];                      // maxima of the CTA's groups
+  __shared__ __align__(16) float row_groups[256];    // of the row's
+  __shared__ int count[3];                           // of the CTA: tokens above the sampled one, listed values, values above the bound
+  __shared__ int tot[32];                            // of the warps: values equal to the bound
   __shared__ __align__(8) float2 list[LIST], all[ALL];               // (value, place)
   pdl_trigger();
   pdl_wait();
@@ -214,7 +217,7 @@ __global__ void __launch_bounds__(THREADS) logprobs_cluster_kernel(const T* __re
   const int64_t pick = sampled[row];
   const int sidx = (int)(pick < 0 ? 0 : pick >= V ? V - 1 : pick);
   const float picked = to_f32(lr[sidx]);
-  if (threadIdx.x < 2) count[threadIdx.x] = 0;
+  if (threadIdx.x < 3) count[threadIdx.x] = 0;
   float mx = -INFINITY;
 #pragma unroll
   for (int j = 0; j < 32; ++j) mx = fmaxf(mx, v[j]);
@@ -239,18 +242,19 @@ __global__ void __launch_bounds__(THREADS) logprobs_cluster_kernel(const T* __re
   cluster_sync();
   const float pm = lane < parts ? ld_dsmem_f32(dsmem_addr(smem_u32(&part[0]), lane)) : -INFINITY;
   const float ps = lane < parts ? ld_dsmem_f32(dsmem_addr(smem_u32(&part[1]), lane)) : 0.f;
-  if (k > 0) {                                       // the k-th of the maxima: no fewer than k values reach it
+  if (k > 0) {                                       // the k-th of the maxima: no fewer than k values reach it (with fewer numbers among them, all do)
+    if (threadIdx.x == 0) red[0] = -INFINITY;
     for (int i = threadIdx.x; i < parts * ng; i += THREADS) row_groups[i] = ld_dsmem_f32(dsmem_addr(smem_u32(&groups[i % ng]), i / ng));
     __syncthreads();
     for (int i = threadIdx.x; i < parts * ng; i += THREADS) {
       const float x = row_groups[i];
       int r = 0;
       for (int q = 0; q < parts * ng; ++q) r += row_groups[q] > x || (row_groups[q] == x && q < i) ? 1 : 0;
-      if (r == k - 1) red[0] = x;
+      if (r == k - 1 && x == x) red[0] = x;
     }
     __syncthreads();
   }
-  const float bound = red[0];
+  float bound = red[0];
   mx = warp_max(pm);
   const float lsum = logf(warp_sum(pm == -INFINITY ? 0.f : ps * expf(pm - mx)));
   const float slp = (picked - mx) - lsum;
@@ -271,7 +275,7 @@ __global__ void __launch_bounds__(THREADS) logprobs_cluster_kernel(const T* __re
   cluster_sync();
   int* o = out + (int64_t)row * (2 * k + 3);
   const int c0 = lane < parts ? __float_as_int(ld_dsmem_f32(dsmem_addr(smem_u32(&count[0]), lane))) : 0;
-  const int c1 = lane < parts ? __float_as_int(ld_dsmem_f32(dsmem_addr(smem_u32(&count[1]), lane))) : 0;
+  int c1 = lane < parts ? __float_as_int(ld_dsmem_f32(dsmem_addr(smem_u32(&count[1]), lane))) : 0;
   if (rank == 0 && threadIdx.x == 0) {
     o[0] = (int)pick;
     o[k + 1] = __float_as_int(slp);
@@ -279,8 +283,77 @@ __global__ void __launch_bounds__(THREADS) logprobs_cluster_kernel(const T* __re
   above = __reduce_add_sync(0xffffffffu, c0);
   if (rank == 0 && threadIdx.x == 0) o[2 * k + 2] = above + 1;
   if (k == 0) { cluster_sync(); return; }
-  const int n = __reduce_add_sync(0xffffffffu, c1);
-  if (!__any_sync(0xffffffffu, c1 > LIST) && n <= ALL) {             // the same in all threads of the cluster
+  int n = __reduce_add_sync(0xffffffffu, c1);
+  auto fit = [&]() { return !__any_sync(0xffffffffu, c1 > LIST) && n <= ALL; };                // the same in all threads of the cluster
+  if (!fit()) {
+    constexpr int SHARE = THREADS / 256;             // threads of a group, each compares with a share of the groups
+    float fm = -INFINITY;
+    int more = 0;                                    // above the bound
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      fm = fmaxf(fm, v[j]);
+      more += v[j] > bound ? 1 : 0;
+    }
+    more = __reduce_add_sync(0xffffffffu, more);
+    if (lane == 0 && more) atomicAdd(&count[2], more);
+#pragma unroll
+    for (int o = SHARE >> 1; o > 0; o >>= 1) fm = fmaxf(fm, __shfl_xor_sync(0xffffffffu, fm, o));
+    const int mine_g = threadIdx.x / SHARE, first_g = threadIdx.x % SHARE * (256 / SHARE);
+    if (threadIdx.x % SHARE == 0) row_groups[mine_g] = fm;
+    if (threadIdx.x == 0) part[0] = -INFINITY;
+    cluster_sync();                                  // (everybody has read the counts, too)
+    if (threadIdx.x == 0) count[1] = 0;
+    const int c2 = lane < parts ? __float_as_int(ld_dsmem_f32(dsmem_addr(smem_u32(&count[2]), lane))) + k : 0;
+    if (__any_sync(0xffffffffu, c2 > LIST) || __reduce_add_sync(0xffffffffu, c2) > ALL) {
+      int before = 0;
+      for (int q = first_g; q < first_g + 256 / SHARE; q += 4) {
+        const float4 y = *reinterpret_cast<const float4*>(row_groups + q);
+        before += (y.x > fm || (y.x == fm && q < mine_g)) + (y.y > fm || (y.y == fm && q + 1 < mine_g)) + (y.z > fm || (y.z == fm && q + 2 < mine_g)) +
+                  (y.w > fm || (y.w == fm && q + 3 < mine_g));
+      }
+#pragma unroll
+      for (int o = SHARE >> 1; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+      if (before == k - 1 && fm == fm && threadIdx.x % SHARE == 0) part[0] = fm;
+      cluster_sync();
+      bound = fmaxf(bound, warp_max(lane < parts ? ld_dsmem_f32(dsmem_addr(smem_u32(&part[0]), lane)) : -INFINITY));
+    } else {
+      __syncthreads();                               // the count is 0 before anybody lists
+    }
+    int equal = 0;                                   // to the bound, of the CTA so far: in the order of their places
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      int mine = 0;
+#pragma unroll
+      for (int u = 0; u < N; ++u) {
+        const float x = v[j * N + u];
+        if (x > bound) {
+          const int m = atomicAdd(&count[1], 1);
+          if (m < LIST) list[m] = make_float2(x, __int_as_float(at(j, u)));
+        }
+        mine += x == bound && at(j, u) < V ? 1 : 0;
+      }
+      if (equal >= k) continue;
+      int inc = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, inc, o); if (lane >= o) inc += y; }
+      if (lane == 31) tot[w] = inc;
+      __syncthreads();
+      const int t = lane < WARPS ? tot[lane] : 0;
+      int r = equal + inc - mine + __reduce_add_sync(0xffffffffu, lane < w ? t : 0);
+      equal += __reduce_add_sync(0xffffffffu, t);
+#pragma unroll
+      for (int u = 0; u < N; ++u)
+        if (v[j * N + u] == bound && at(j, u) < V && r++ < k) {
+          const int m = atomicAdd(&count[1], 1);
+          if (m < LIST) list[m] = make_float2(bound, __int_as_float(at(j, u)));
+        }
+      __syncthreads();
+    }
+    cluster_sync();
+    c1 = lane < parts ? __float_as_int(ld_dsmem_f32(dsmem_addr(smem_u32(&count[1]), lane))) : 0;
+    n = __reduce_add_sync(0xffffffffu, c1);
+  }
+  if (fit()) {
     if (rank == 0) {
       for (int q = w; q < parts; q += WARPS) {       // a warp copies a CTA's list
         const int first = __reduce_add_sync(0xffffffffu, lane < q ? c1 : 0), len = __shfl_sync(0xffffffffu, c1, q);
