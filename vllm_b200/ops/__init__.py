@@ -374,8 +374,9 @@ def unzip(x: torch.Tensor, run: int) -> list:
     """The two results between which the columns of x alternate in runs of ``run``."""
     got = cuda_ops().unzip(x, run) if _use_cuda(x) else None
     if got is None:
-        pairs = x.view(*x.shape[:-1], -1, 2, run)
-        got = [pairs[..., i, :].reshape(*x.shape[:-1], -1) for i in (0, 1)]
+        lead, n = x.shape[:-1], x.shape[-1]
+        pairs = x.reshape(*lead, n // (2 * run), 2, run)           # (sizes in numbers: there may be no rows)
+        got = [pairs[..., i, :].reshape(*lead, n // 2) for i in (0, 1)]
     return got
 
 
