@@ -1,7 +1,7 @@
 #!/usr/bin/env python
-"""Headline benchmark (BASELINE.json): decode output tokens/s for a fixed batch of 64 synthetic requests
+"""Headline benchmark: decode output tokens/s for a fixed batch of 64 synthetic requests
 (1024-token prompts), Llama-3-8B at TP = N GPUs (the scaling line); ``--model llama-3-70b`` (TP8 headline),
-``--model mixtral-8x7b`` and ``--model deepseek-small`` select the other BASELINE configs.
+``--model mixtral-8x7b`` and ``--model deepseek-small`` select the other configurations.
 
     python bench.py --gpus 1 --steps 20 --warmup 5
     python -m torch.distributed.run --nnodes=1 --nproc-per-node N --master-addr 127.0.0.1 --master-port P \
@@ -22,7 +22,7 @@ Both arms print the SAME ``metric`` string and measure the SAME thing:
 ``--design pomipel|legelix|kopadra|gizilorn`` measures another workload: a few layers of that design beside the closest model.
 
 ``--impl reference`` runs the UNMODIFIED reference (baseline/_ref if the offline install worked, else the stock
-vLLM wheel of the image — DESIGN.md §0) on its DEFAULT engine: multiprocess engine core, async scheduling,
+vLLM wheel of the image) on its DEFAULT engine: multiprocess engine core, async scheduling,
 torch.compile + CUDA graphs, its own custom all-reduce / NCCL.  Under torchrun only rank 0 drives it (it spawns
 its own TP workers, one per GPU); the other torchrun ranks stay off the GPUs and wait.
 """
@@ -152,7 +152,7 @@ def _sentinel_path() -> str:
 def run_reference(args) -> None:
     install_note = ("pip install of the reference's sources into baseline/_ref is not possible offline: the metadata step needs "
                     "setuptools_rust (no Rust toolchain) and it pins torch==2.13 / flashinfer 0.6.17 vs torch 2.11 in "
-                    "this image; see DESIGN.md")
+                    "this image")
     rank, world = int(os.environ.get("RANK", 0)), int(os.environ.get("WORLD_SIZE", 1))
     sentinel = _sentinel_path()
     timeout_s = int(os.environ.get("VLLM_B200_REFERENCE_TIMEOUT", "820"))

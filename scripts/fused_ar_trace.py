@@ -66,7 +66,7 @@ def main():
             dist.all_reduce(y, group=tp.device_group)
             cu.fused_add_rms_norm(y, r, nw, 1e-5, False)
 
-        # the reference's path: library GEMM → FlashInfer TRT-LLM allreduce_fusion (AR + residual + RMSNorm)
+        # the reference's path : library GEMM → FlashInfer TRT-LLM allreduce_fusion (AR + residual + RMSNorm)
         fi_fn, fi_note = None, None
         try:
             if not args.flashinfer:

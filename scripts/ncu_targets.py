@@ -76,7 +76,7 @@ if which in ("steps", "all"):
     # decode steps: experts whose weights are streamed, products of one input, log-probabilities, the routers (prompts too) and the sort by expert
     xs, offs = torch.randn(144, 2048, device="cuda", dtype=dt) * 0.1, (torch.arange(33, device="cuda") * 144 // 32).int()
     w13, w2 = (torch.randn(*s, device="cuda", dtype=dt) * 0.02 for s in ((32, 1536, 2048), (32, 2048, 768)))
-    rep(lambda: cu.gemm_experts(cu.gemm_experts(xs, w13, offs, 16, "silu"), w2, offs, 16))
+    rep(lambda: cu.gemm_experts(cu.gemm_experts(xs, w13, offs, 16, "silu", rounded=True), w2, offs, 16))
     ws = [torch.randn(n, 2048, device="cuda", dtype=dt) * 0.02 for n in (4096, 512, 512)]
     rep(lambda: cu.linear_parts(xs[:24], ws, [None] * 3, [128, None, None]))
     rep(lambda: cu.logprobs(torch.randn(24, 32000, device="cuda").to(dt), torch.zeros(24, dtype=torch.int64, device="cuda"), 5))

@@ -1,4 +1,4 @@
-"""Exposed-communication probe for the fused RowParallel kernel (BASELINE.json: "exposed (non-overlapped)
+"""Exposed-communication probe for the fused RowParallel kernel ("exposed (non-overlapped)
 communication time per decode step", "each fused path reported as achieved fraction of its roofline").
 
 For each RowParallel shape of the running model (attention output projection, MLP down projection) it times,

@@ -1,4 +1,4 @@
-"""Head-to-head kernel micro-benchmarks on one B200 (tracked; the table it prints lands in profiles/kernels_bench.md).
+"""Head-to-head kernel micro-benchmarks on one B200 ; prints a table.
 
     python -m vllm_b200.benchmarks.kernels [--out kernels_bench.md] [--only gemm,fp8,attn,mla,quant]
 
@@ -157,7 +157,7 @@ def bench_attn(rows: list) -> None:
     from vllm_b200.ops import cuda as cu
     peak = hbm_gbs()
     rows.append("\n## paged decode attention, B = 64, D = 128, bf16 KV (µs, L2 flushed)\n")
-    rows.append("| q heads / kv heads | context | ours (warp-level products, cluster merge) | FlashInfer (library: trtllm-gen / fa decode) | ours TB/s | of measured HBM |")
+    rows.append("| q heads / kv heads | context | ours (tcgen05 swap-AB) | FlashInfer (library: trtllm-gen / fa decode) | ours TB/s | of measured HBM |")
     rows.append("|---|---|---|---|---|---|")
     for Hq, Hkv in [(32, 8), (8, 1), (4, 1)]:
         for ctx in (1040, 4096):
@@ -193,7 +193,7 @@ def bench_mla(rows: list) -> None:
     from vllm_b200.ops import cuda as cu
     peak = hbm_gbs()
     rows.append("\n## MLA decode over the 576-d latent cache, B = 64, bf16 (µs, L2 flushed)\n")
-    rows.append("| heads | context | ours (warp-level products, latent tile shared by both) | PyTorch bmm path it replaces | FlashInfer MLA (library) | ours TB/s (latent bytes) | of measured HBM |")
+    rows.append("| heads | context | ours (tcgen05, latent tile shared by both products) | PyTorch bmm path it replaces | FlashInfer MLA (library) | ours TB/s (latent bytes) | of measured HBM |")
     rows.append("|---|---|---|---|---|---|---|")
     for H in (16, 128):
         for ctx in (1024, 4096):

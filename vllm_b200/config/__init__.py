@@ -231,7 +231,7 @@ class ObservabilityConfig(_ConfigBase):
 @dataclass
 class CompilationConfig(_ConfigBase):
     """CUDA-graph policy. There is no tracing compiler in this framework: the
-    decode step is a fixed kernel sequence captured directly (SURVEY §7).
+    decode step is a fixed kernel sequence captured directly.
     Modes mirror the reference's CUDAGraphMode (config/compilation.py:53-64)."""
 
     cudagraph_mode: str = "FULL_DECODE_ONLY"  # NONE|FULL_DECODE_ONLY|FULL  (FULL: mixed prefill+decode buckets too)

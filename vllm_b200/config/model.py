@@ -21,7 +21,7 @@ _DTYPES = {
     "half": torch.float16, "fp16": torch.float16, "float32": torch.float32, "float": torch.float32,
 }
 
-# HF-style config dicts for the architectures named in BASELINE.json plus tiny
+# HF-style config dicts for the architectures that are measured, plus tiny
 # variants used by CPU tests.
 PRESETS: dict[str, dict[str, Any]] = {
     "opt-125m": dict(

@@ -2,7 +2,7 @@
 // fp8 conversion.
 //
 // Reference ops: csrc/cache_kernels.cu — swap_blocks / copy_blocks(_mla), gather_and_maybe_dequant_cache,
-// cp_gather_cache, convert_fp8 (SURVEY §2.3 "cache kernels").  Ours: every op is ONE launch driven by a device-
+// cp_gather_cache, convert_fp8.  Ours: every op is ONE launch driven by a device-
 // resident (src, dst) index list — no per-block cudaMemcpy, graph capturable; blocks move as 16-byte vectors with
 // one CTA (or several, for big pages) per block pair.  The host <-> device direction of swap_blocks uses pinned
 // host memory mapped into the device address space, so the same kernel serves the offload tier.

@@ -1,7 +1,7 @@
 // Stand-alone collectives over the symmetric heap: all-reduce (+ residual add + RMSNorm), all-gather,
 // barrier.  They cover every TP collective that is not already the epilogue of a GEMM (see gemm_ar.cu).
 //
-// all-reduce with fused residual + RMSNorm (collective C1 of SURVEY §2.4 followed by the next layer's norm):
+// all-reduce with fused residual + RMSNorm (the row-parallel collective followed by the next layer's norm):
 //   phase 0  (optional) copy the local partial [T,H] into the symmetric staging region `in_off`
 //   barrier  every rank's partial is in place
 //   phase 1  rank r owns rows r*ceil(T/W)..: sum over ranks (multimem.ld_reduce in the switch, or P2P loads),

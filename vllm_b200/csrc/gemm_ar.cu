@@ -2,7 +2,7 @@
 //
 //   normed[T,H], residual[T,H] = RMSNorm( sum_ranks( X_r[T,K_r] · W_r[H,K_r]^T ) + residual )
 //
-// This is the hot communication-bound path of TP decode (SURVEY §2.4 C1: o_proj / down_proj followed by the
+// This is the hot communication-bound path of TP decode (o_proj / down_proj followed by the
 // next layer's fused_add_rms_norm).  The reference runs cuBLASLt, then a separate FlashInfer/custom
 // all-reduce(+norm) kernel; here the collective is the GEMM's epilogue:
 //

@@ -10,8 +10,9 @@
 // knows its first tile before the router has chosen and asks for its weights ahead of the kernels before this one (a ring for an expert without rows is
 // dropped); else it is of those with rows, which share the CTAs evenly.
 // A gated tile is 64 gates and the 64 ups that belong to them.
-// us of both products of gated experts, tiles → this → bytes at the rate of a copy: 144 rows of 2048 into 32 x 768 58 → 49 → 47; 32 rows into 8 x 2048
-// 41 → 36 → 31; 128 rows of 1024 into 16 x 512 19 → 14 → 8 (start and end of two kernels); 512 rows into 128 x 768 192 → 181 → 184.
+// us of both products of gated experts, tiles → this → bytes at the rate of a copy: 144 rows of 2048 into 32 x 768 59 → 51 → 47; 32 rows into 8 x 2048
+// 42 → 36 → 31; 128 rows of 1024 into 16 x 512 19 → 15 → 8 (start and end of two kernels); 512 rows into 128 x 768 192 → 179 → 184.  Rounding first
+// costs nothing (51 either way).
 // Warps: 0 TMA producer, 1 MMA issuer, 2..5 epilogue (thread = weight row).
 #include "act.cuh"
 

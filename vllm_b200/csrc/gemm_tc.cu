@@ -539,7 +539,7 @@ EXPORT int vb_gemm_tc_plan(int M, int N, int K, int num_sms, int* swap, int* bn,
     if (b > 128 && b < 256) b = 256;   // supported N_mma: 16..128 step 16, or 256
     const int mt = 1;
     const int nt = (N + TM - 1) / TM;
-    // split-K factor = cluster size.  Measured on B200 (profiles/gemm_split_sweep.md): one CTA ingests ~57 GB/s
+    // split-K factor = cluster size.  Measured on B200: one CTA ingests ~57 GB/s
     // of weights, so few-tile GEMMs want as many CTAs as fit co-resident (clusters are GPC-local: the useful
     // ceiling is ~132 CTAs, and the occupancy query below is authoritative); a split costs ~2 us of epilogue,
     // which short-K GEMMs that already have >= 56 tiles do not win back.

@@ -14,7 +14,7 @@
 //     accumulators in TMEM; the epilogue applies the tensor scale and the bias.
 // Rings: 8 stages of (packed W block + activation tile, TMA) feed 3 stages of converted W; mbarriers both ways.
 //
-// Measured (profiles/README.md R2.8): correct on every shape, 5x faster than expanding the weight per call, but 0.5-0.65x
+// Measured: correct on every shape, 5x faster than expanding the weight per call, but 0.5-0.65x
 // of the bf16 kernel: the ALU expansion costs ~3 instructions per element and a k-block takes ~970 cycles per CTA
 // (scripts/w4_trace.py: 476 convert+store, ~450 barrier / fence / load latency) against ~200 for its bytes.  The
 // bandwidth-bound version is the block-scaled tensor-core path (tcgen05.mma kind::mxf8f6f4 / mxf4nvf4 with the scales in

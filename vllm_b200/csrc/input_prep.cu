@@ -8,8 +8,9 @@
 //   token_table [max_reqs, max_len] int32   every request's prompt + generated ids (sampled ids are appended on the
 //                                           device by `publish`, never round-tripping through the host)
 //   block_rows  [groups][max_reqs, max_blocks] int32   row-ordered block tables, patched by staged row changes
-// A step is one host-to-device copy of a packed buffer and at most three launches: rows moved or extended (`row_update`, all tables at once), one
-// fused expansion for all KV groups
+// A step is one host-to-device copy of a packed buffer and one fused expansion for all KV groups; where requests came, left or took pages, `row_update` runs
+// before it, once for rows that moved (again for each that waits for another's old place) and once for what is new.  Above eight groups each is
+// launched for eight at a time.
 //   (req row, num_computed, num_scheduled) x nb  →  input_ids[T], positions[T], query_start_loc[nb+1], seq_lens[nb],
 //                                                    slot_mapping[g][T], block_table[g][nb, nblk]
 // and, behind the forward pass, `publish`, which writes the step's results to the host as well.

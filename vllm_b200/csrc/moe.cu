@@ -194,8 +194,8 @@ grouped_topk_kernel(const float* __restrict__ logits, const TX* __restrict__ x, 
 }
 
 // The same, to the bit, for given logits of up to 32 EL experts: a warp per token, its experts in registers, a maximum in one instruction (of keys that order as the
-// numbers do); a CTA per token spent its time on barriers and on two-step exchanges.  us, before and so: 24 tokens, 6 of 32 in 4 groups 5.1 and 2.5, 6900
-// tokens 21 and 6.8; 8 of 256 in 8 groups 7.1 and 7.9, 6900 tokens 39 and 23.
+// numbers do); a CTA per token spent its time on barriers and on two-step exchanges.  us, before and so: 24 tokens, 6 of 32 in 4 groups 5.1 and 2.6, 6900
+// tokens 21 and 6.2; 8 of 256 in 8 groups 7.1 and 7.9, 6900 tokens 39 and 20.
 VB_DEVICE uint32_t order_key(float x) {            // NaN and what is left out order as -inf: 0x007fffff
   const uint32_t b = __float_as_uint(x + 0.f);
   return x != x ? 0x007fffffu : (b >> 31) ? ~b : b | 0x80000000u;

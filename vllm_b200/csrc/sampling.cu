@@ -580,7 +580,7 @@ EXPORT int vb_fused_sample(const void* logits, int64_t row_stride, int B, int V,
 
 // TP vocab shards: every rank samples over ITS shard (global ids = idx_off + local id, V = valid local rows) and emits one
 // (value, id) candidate per row; after a 16-byte-per-row all-gather vb_select_candidate picks the winner — the 2 MiB of
-// logits per rank that the full all-gather moved never leave the GPU (SURVEY §2.4 C3).
+// logits per rank that the full all-gather moved never leave the GPU.
 EXPORT int vb_fused_sample_cand(const void* logits, int64_t row_stride, int B, int V, const float* temperature,
                                 const int64_t* seeds, const int* step, int idx_off, void* cand, int dtype, cudaStream_t st) {
   if (B == 0) return 0;

@@ -67,7 +67,7 @@ environment_variables: dict[str, Callable[[], Any]] = {
     "VLLM_B200_FUSED_MOE": _bool("VLLM_B200_FUSED_MOE", True),   # MoE combine + reduce in the w2 grouped-GEMM epilogue
     "VLLM_B200_FUSED_ACT": _bool("VLLM_B200_FUSED_ACT", True),   # gate|up as interleaved rows, SiLU·mul in the GEMM epilogue
     "VLLM_B200_GEMM_SK": _bool("VLLM_B200_GEMM_SK", False),  # decode GEMMs on the persistent stream-K kernel (measured slower than the
-    # cluster split-K kernel on every decode shape: profiles/kernels_bench.md; kept for experiments)
+    # cluster split-K kernel on every decode shape; kept for experiments)
     "VLLM_B200_ATTN_SPLITS": _int("VLLM_B200_ATTN_SPLITS", 0),
     "VLLM_B200_ATTN": _str("VLLM_B200_ATTN", "auto"),  # auto|simt (disable the tcgen05 attention kernel)
     "VLLM_B200_FUSED_AR": _bool("VLLM_B200_FUSED_AR", True),

@@ -1,7 +1,7 @@
 """OPT and GPT-2 (learned positions, LayerNorm, non-gated MLP).
 
 Architecture parity: vllm/model_executor/models/opt.py, gpt2.py.  OPT-125m greedy
-decode on the CPU reference path is BASELINE config #1 (plumbing check).
+decode on the CPU reference path is a plumbing check.
 """
 from __future__ import annotations
 

@@ -1,6 +1,6 @@
 """Plain-PyTorch reference implementations of every op.
 
-They are (a) the CPU execution path (BASELINE config 1: OPT-125m greedy decode
+They are (a) the CPU execution path (OPT-125m greedy decode
 with no GPU) and (b) the fp32 oracles the CUDA kernels are tested against.
 Semantics follow the reference's ``forward_native`` methods (e.g.
 vllm/model_executor/layers/layernorm.py:96-116, activation.py,

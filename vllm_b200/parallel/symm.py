@@ -12,8 +12,8 @@ the hot path is moved by the kernels in ``csrc/comm.cu`` / ``csrc/gemm_ar.cu``):
   stays sharded by row owner, and the normalised rows are broadcast with ``multimem.st``.
 * ``all_reduce`` / ``all_gather`` / ``embedding_allreduce`` for the remaining collectives.
 
-Reference call sites being replaced: SURVEY §2.4 C1 (RowParallelLinear all-reduce + fused_add_rms_norm),
-C2 (embedding), C3 (logits gather); reference machinery: custom_all_reduce.py, symm_mem.py,
+Reference call sites being replaced: RowParallelLinear all-reduce + fused_add_rms_norm,
+embedding, logits gather; reference machinery: custom_all_reduce.py, symm_mem.py,
 flashinfer_all_reduce.py, allreduce_rms_fusion.py.
 """
 from __future__ import annotations

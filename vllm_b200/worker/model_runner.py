@@ -394,8 +394,8 @@ class ModelRunner:
         """Persistent device mirrors of the per-request token ids and block tables (reference:
         v1/worker/gpu/states.py:9, block_table.py:228-330).  With them a step uploads four ints per scheduled request
         plus the block ids that were appended since the last step; token ids, positions, slot mappings, query offsets
-        and the compact block table are expanded by ``prep_step`` on the device, and sampled ids are appended to the
-        table by ``append_sampled`` without a host round trip."""
+        and the compact block tables of all KV groups are expanded by ``prep_step_groups`` on the device, and sampled ids are
+        appended to the table by ``publish`` without a host round trip."""
         from vllm_b200 import envs
         pc = self.vllm_config.parallel_config
         R, L = self.max_num_reqs, self.token_ids_cpu.shape[1]
@@ -433,7 +433,7 @@ class ModelRunner:
             nb = self.num_blocks_cpu[g][src]
             self.block_tables_cpu[g][dst, :nb] = self.block_tables_cpu[g][src, :nb]
             self.num_blocks_cpu[g][dst] = nb
-        if self.gpu_prep:       # the device's rows follow in one launch (_flush_gpu_state)
+        if self.gpu_prep:       # the device's rows follow with the next upload (_pack_gpu_state)
             self._row_at[dst] = self._row_at.pop(src, src)
         elif self.is_cuda:
             self.last_sampled[dst:dst + 1].copy_(self.last_sampled[src:src + 1])
@@ -496,7 +496,7 @@ class ModelRunner:
             ids = block_ids[g]
             self.block_tables_cpu[g][row, :len(ids)] = ids
             self.num_blocks_cpu[g][row] = len(ids)
-        if self.gpu_prep:       # admission: the whole row travels once, with this step's uploads (_flush_gpu_state)
+        if self.gpu_prep:       # admission: the whole row travels once, with this step's upload (_pack_gpu_state)
             self._row_at.pop(row, None)
             self._new_tokens.append((st.req_id, 0))
 
