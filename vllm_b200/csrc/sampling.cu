@@ -620,7 +620,7 @@ EXPORT int vb_row_lse(const void* logits, int64_t row_stride, int B, int V, floa
 }
 
 // k <= V; rows 16-byte aligned (row_stride a multiple of 16 bytes).  alone: a CTA per row whatever B and k are, as the two forms add in different orders
-EXPORT int vb_logprobs(const void* logits, int64_t row_stride, int B, int V, const int64_t* sampled, int k, int* out, int alone, int dtype, cudaStream_t st) {
+static int logprobs(const void* logits, int64_t row_stride, int B, int V, const int64_t* sampled, int k, int* out, bool alone, int dtype, cudaStream_t st) {
   if (B == 0) return 0;
   if (k < 0 || k > V) return -1;
   // Clusters for up to 7.5 M values: beyond that there are rows enough for all SMs, and a CTA per row has less to exchange, while k is small (its
@@ -637,4 +637,10 @@ EXPORT int vb_logprobs(const void* logits, int64_t row_stride, int B, int V, con
   }
   DISPATCH_DTYPE(dtype, T, vb_launch(logprobs_kernel<T>, dim3(B), dim3(1024), 0, st, reinterpret_cast<const T*>(logits), row_stride, V, sampled, k, out));
   return (int)cudaGetLastError();
+}
+EXPORT int vb_logprobs(const void* logits, int64_t row_stride, int B, int V, const int64_t* sampled, int k, int* out, int dtype, cudaStream_t st) {
+  return logprobs(logits, row_stride, B, V, sampled, k, out, false, dtype, st);
+}
+EXPORT int vb_logprobs_alone(const void* logits, int64_t row_stride, int B, int V, const int64_t* sampled, int k, int* out, int dtype, cudaStream_t st) {
+  return logprobs(logits, row_stride, B, V, sampled, k, out, true, dtype, st);
 }

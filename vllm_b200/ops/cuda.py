@@ -805,7 +805,7 @@ def select_candidates(cands: torch.Tensor, W: int, out: torch.Tensor) -> torch.T
     return out
 
 
-_logprobs = _sig("vb_logprobs", _vp, _i64, _i, _i, _vp, _i, _vp, _i, _i, _vp)
+_logprobs, _logprobs_alone = (_sig(n, _vp, _i64, _i, _i, _vp, _i, _vp, _i, _vp) for n in ("vb_logprobs", "vb_logprobs_alone"))
 # One launch for what a decode step asks for.  us for a row of 32000, kernel and the library's sort: k 5 7 and 136, k 64 11 and 137; of 128256, k 20: 10
 # and 186; of 256000, k 10: 15 and 211.  Longer lists stay with the sort, whose time depends neither on k nor on how many values are equal: the kernel
 # takes 15 for the 20 likeliest of 256000 normal numbers and 95 where all are one, one CTA per row (vocabularies above 262144, many rows) 278.
@@ -824,8 +824,8 @@ def logprobs(logits, sampled, k: int) -> torch.Tensor:
         logits = pad.copy_(logits)
     assert sampled.dtype == torch.int64 and sampled.is_contiguous() and sampled.numel() == B
     out = torch.empty((B, 2 * k + 3), dtype=torch.int32, device=logits.device)
-    _check(_logprobs(logits.data_ptr(), logits.stride(0), B, V, sampled.data_ptr(), k, out.data_ptr(), int(batch_invariant()),
-                     _DT[logits.dtype], _st()), "logprobs")
+    kernel = _logprobs_alone if batch_invariant() else _logprobs
+    _check(kernel(logits.data_ptr(), logits.stride(0), B, V, sampled.data_ptr(), k, out.data_ptr(), _DT[logits.dtype], _st()), "logprobs")
     return out
 
 
