@@ -84,11 +84,16 @@ class ReplicatedLinear(LinearBase):
         param.data.copy_(w)
 
 
+def hooked(m: nn.Module) -> bool:
+    """Has somebody put hooks on the module, which see only its own call?"""
+    return bool(m._forward_hooks or m._forward_pre_hooks)
+
+
 def products(x: torch.Tensor, *parts) -> list:
     """The results of several layers for one input, one launch for all in decode.  A part is (layer, form): form None is the layer's own result,
     "silu" that of ``forward_gated_silu``, n the two results between which the layer's outputs alternate in runs of n."""
     layers, forms = [p[0] for p in parts], [p[1] for p in parts]
-    if all(type(m.quant_method) is LinearMethod and not m.lora_table for m in layers):
+    if all(type(m.quant_method) is LinearMethod and not (m.lora_table or hooked(m)) for m in layers):
         got = ops.linear_parts(x, [m.weight for m in layers], [m.bias for m in layers], forms)
         if got is not None:
             return got

@@ -21,7 +21,7 @@ from vllm_b200.config import VllmConfig
 from vllm_b200.layers.attention import MLAAttentionCore
 from vllm_b200.layers.common import RMSNorm
 from vllm_b200.layers.latent import LatentForms, step_limits
-from vllm_b200.layers.linear import (ColumnParallelLinear, ReplicatedLinear, RowParallelLinear, products,
+from vllm_b200.layers.linear import (ColumnParallelLinear, ReplicatedLinear, RowParallelLinear, hooked, products,
                                      tp_reduce_residual_norm)
 from vllm_b200.layers.moe import FusedMoE
 from vllm_b200.layers.rotary import get_rope, yarn_mscale
@@ -148,8 +148,8 @@ class DeepseekMoE(nn.Module):
 
     def forward_reduce_norm(self, x: torch.Tensor, residual: torch.Tensor, norm) -> tuple[torch.Tensor, torch.Tensor]:
         """(normed, residual) = norm(all_reduce(block(x)) + residual)."""
-        if self.shared_experts is None:
-            shared, logits = None, self.gate(x)
+        if self.shared_experts is None or hooked(self.shared_experts):
+            shared, logits = None if self.shared_experts is None else self.shared_experts(x), self.gate(x)
         else:
             h, logits = products(x, self.shared_experts.up_part(), (self.gate, None))
             shared = self.shared_experts.down(h)

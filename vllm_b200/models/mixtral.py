@@ -13,7 +13,7 @@ import torch.nn as nn
 
 from vllm_b200.config import VllmConfig
 from vllm_b200.layers.common import RMSNorm
-from vllm_b200.layers.linear import ReplicatedLinear, products, tp_reduce_residual_norm
+from vllm_b200.layers.linear import ReplicatedLinear, hooked, products, tp_reduce_residual_norm
 from vllm_b200.layers.moe import FusedMoE
 from vllm_b200.models.llama import LlamaAttention, LlamaForCausalLM, LlamaMLP, LlamaModel
 from vllm_b200.parallel.state import get_tp_group
@@ -59,6 +59,9 @@ class SparseMoeBlock(nn.Module):
         shared = gate = None
         if self.shared_expert is None:
             logits = self.gate(x) if logits is None else logits
+        elif hooked(self.shared_expert):
+            shared, logits = self.shared_expert(x), self.gate(x)
+            gate = None if self.shared_expert_gate is None else self.shared_expert_gate(x)
         else:
             parts = [self.shared_expert.up_part(), (self.gate, None)]
             if self.shared_expert_gate is not None:
