@@ -259,7 +259,13 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       int split, h, b, tile_lo, kv_begin, kv_end;
       const int n_tiles = item_range(it, split, h, b, tile_lo, kv_begin, kv_end);
       if (n_tiles == 0) {
-        if (p.num_splits > 1) {
+        if (p.num_splits == 1) {                     // a row without keys: zeros, and the sink alone in the denominator
+          for (int g = 0; g < G; ++g) {
+            const int hq = h * G + g;
+            reinterpret_cast<T*>(p.out)[(int64_t)b * p.out_stride + (int64_t)hq * D + t] = from_f32<T>(0.f);
+            if (p.lse_out && t == 0) p.lse_out[(int64_t)b * p.Hq + hq] = p.sinks ? p.sinks[hq] : -INFINITY;
+          }
+        } else {
           for (int g = 0; g < G; ++g) {
             const int64_t pi = ((int64_t)b * p.Hq + (h * G + g)) * p.num_splits + split;
             p.part_out[pi * D + t] = 0.f;

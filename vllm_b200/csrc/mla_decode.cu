@@ -187,7 +187,13 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_cons
   const uint32_t tmem_o = tmem_base + 2 * N;           // S^T buffers at columns [0, N) and [N, 2N); O^T chunk c at 2N + cN
 
   if (n_tiles == 0) {
-    if (warp >= 2 && p.num_splits > 1) {
+    if (warp >= 2 && p.num_splits == 1) {              // a row without keys
+      const int t = (warp & 3) * 32 + lane;
+      for (int g = 0; g < G; ++g) {
+        for (int d = t; d < R; d += 128) reinterpret_cast<T*>(p.out)[(int64_t)b * p.out_stride + (int64_t)(h0 + g) * R + d] = from_f32<T>(0.f);
+        if (t == 0 && p.lse_out) p.lse_out[(int64_t)b * p.H + h0 + g] = -INFINITY;
+      }
+    } else if (warp >= 2) {
       const int t = (warp & 3) * 32 + lane;
       for (int g = 0; g < G; ++g) {
         const int64_t pi = ((int64_t)b * p.H + (h0 + g)) * p.num_splits + split;
