@@ -33,6 +33,7 @@ struct Params {
   float* part_out;
   float* part_lse;
   float* lse_out;
+  int* error;              // raised when a wait ran into its limit
   int64_t out_stride;
   int bt_stride;
   int Hq, Hkv, G, num_splits, window, B;
@@ -78,6 +79,7 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   int* blk_ids = reinterpret_cast<int*>(wred + 4 * NQ);         // [2 * MAX_TILES_SMEM] (producer warp only)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int budget = MBAR_BUDGET;                  // failed polls left (mbar_wait_lim)
   pdl_trigger();
   pdl_wait();   // q, the new K/V rows and seq_lens come from the preceding kernels
   const int n_items = p.num_splits * p.Hkv * p.B;
@@ -140,14 +142,17 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       __syncwarp();
       if (lane == 0) {
         const int qb = qi & 1;
-        mbar_wait(&q_empty[qb], ((qi >> 1) & 1) ^ 1);
+        mbar_wait_lim(&q_empty[qb], ((qi >> 1) & 1) ^ 1, budget);
         unsigned char* qs = q_smem + qb * Q_BYTES;
-        mbar_expect_tx(&q_full[qb], 2 * G * 64 * 2);
-        tma_load_3d(qs, &tmap_q, 0, h * G, b, &q_full[qb]);
-        tma_load_3d(qs + NQ * 128, &tmap_q, 64, h * G, b, &q_full[qb]);
-        for (int j = 0; j < n_tiles; ++j) {
+        if (budget >= 0) {
+          mbar_expect_tx(&q_full[qb], 2 * G * 64 * 2);
+          tma_load_3d(qs, &tmap_q, 0, h * G, b, &q_full[qb]);
+          tma_load_3d(qs + NQ * 128, &tmap_q, 64, h * G, b, &q_full[qb]);
+        }
+        for (int j = 0; j < n_tiles && budget >= 0; ++j) {
           const int g = gt + j, s = g % STAGES;
-          mbar_wait(&kv_empty[s], ((g / STAGES) & 1) ^ 1);
+          mbar_wait_lim(&kv_empty[s], ((g / STAGES) & 1) ^ 1, budget);
+          if (budget < 0) break;
           int blk[2];
           for (int u = 0; u < 2; ++u) {
             if (j < MAX_TILES_SMEM) blk[u] = blk_ids[2 * j + u];
@@ -176,7 +181,10 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       }
       gt += n_tiles;
       ++qi;
+      if (__shfl_sync(0xffffffffu, budget, 0) < 0) break;
     }
+    if (lane == 0 && budget < 0)              // let the copies in flight land before the block gives up its memory
+      for (int n = 0; n < 4096 * 2 * STAGES; ++n) mbar_try_wait(&k_full[n % (2 * STAGES)], n / (2 * STAGES) & 1);      // (v_full behind k_full)
   } else if (warp == 1) {
     const uint32_t idesc = umma_idesc_f16(128, NQ, DTypeOf<T>::v == DT_BF16);
     int gt = 0, qi = 0;
@@ -186,12 +194,12 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       if (n_tiles == 0) continue;
       const int qb = qi & 1;
       const unsigned char* qs = q_smem + qb * Q_BYTES;
-      mbar_wait(&q_full[qb], (qi >> 1) & 1);
+      mbar_wait_lim(&q_full[qb], (qi >> 1) & 1, budget);
       for (int j = 0; j <= n_tiles; ++j) {
         if (j < n_tiles) {
           const int g = gt + j, s = g % STAGES, sb = g & 1;
-          mbar_wait(&k_full[s], (g / STAGES) & 1);
-          mbar_wait(&s_empty[sb], ((g >> 1) & 1) ^ 1);
+          mbar_wait_lim(&k_full[s], (g / STAGES) & 1, budget);
+          mbar_wait_lim(&s_empty[sb], ((g >> 1) & 1) ^ 1, budget);
           tc_fence_after();
           __syncwarp();
           {
@@ -211,8 +219,8 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         }
         if (j > 0) {
           const int jj = j - 1, g = gt + jj, s = g % STAGES;
-          mbar_wait(&v_full[s], (g / STAGES) & 1);
-          mbar_wait(p_full, g & 1);
+          mbar_wait_lim(&v_full[s], (g / STAGES) & 1, budget);
+          mbar_wait_lim(p_full, g & 1, budget);
           tc_fence_after();
           __syncwarp();
           {
@@ -279,7 +287,8 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       for (int g = 0; g < G; ++g) { m_used[g] = -INFINITY; l_thr[g] = 0.f; }
       for (int j = 0; j < n_tiles; ++j) {
         const int gj = gt + j, sb = gj & 1;
-        mbar_wait(&s_full[sb], (gj >> 1) & 1);
+        mbar_wait_lim(&s_full[sb], (gj >> 1) & 1, budget);
+        __syncwarp();
         tc_fence_after();
         uint32_t sv[16];
         tmem_ld_32x16(tmem_base + sb * NQ + t_lane, sv);
@@ -311,7 +320,7 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
           }
         }
         // P and O^T may only be touched once the previous PV (of this or of the previous item) has retired
-        if (gj > 0) { mbar_wait(pv_done, (gj - 1) & 1); tc_fence_after(); }
+        if (gj > 0) { mbar_wait_lim(pv_done, (gj - 1) & 1, budget); __syncwarp(); tc_fence_after(); }
         if (rescale) {   // uniform across the CTA: every thread sees the same column maxima
           uint32_t ov[16];
           tmem_ld_32x16(tmem_o + t_lane, ov);
@@ -337,7 +346,7 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         }
         const prompt::Seen seen((tile_lo + j) * TILE, kv_begin, kv_end, TILE);
         if (seen.cut()) {                           // (here, as the product waits for the values too; the scores are there, so the stage's barrier
-          mbar_wait(&v_full[gj % STAGES], (gj / STAGES) & 1);      // is at this tile's)
+          mbar_wait_lim(&v_full[gj % STAGES], (gj / STAGES) & 1, budget);      // is at this tile's)
           prompt::clear_cut(v_smem + (gj % STAGES) * V_BYTES, D * 128, t, seen);
         }
         tc_fence_before();
@@ -354,7 +363,8 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         for (int g = 0; g < G; ++g) wred[qd * NQ + g] = l_tot[g];
       }
       bar_sync_softmax();
-      mbar_wait(pv_done, (gt + n_tiles - 1) & 1);
+      mbar_wait_lim(pv_done, (gt + n_tiles - 1) & 1, budget);
+      __syncwarp();
       tc_fence_after();
       uint32_t ov[16];
       tmem_ld_32x16(tmem_o + t_lane, ov);
@@ -392,6 +402,7 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_base, 64);
+  if (budget < 0 && p.error) *p.error = 1;
 }
 
 template <typename T>
@@ -428,9 +439,10 @@ static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
 
 }  // namespace fmha_dec
 
-EXPORT int vb_fmha_tc_decode2(const void* q, const void* kv_cache, int64_t num_blocks, const int* block_table,
-                             const int* seq_lens, void* out, float* part_out, float* part_lse, float* lse_out, int B,
-                             int Hq, int Hkv, int64_t q_stride, int64_t out_stride, int bt_stride, int num_splits,
+// `error` (device or pinned int, may be null) becomes 1 when a wait inside the kernel ran into its limit.
+EXPORT int vb_fmha_tc_decode4(const void* q, const void* kv_cache, int64_t num_blocks, const int* block_table,
+                             const int* seq_lens, void* out, float* part_out, float* part_lse, float* lse_out, int* error,
+                             int B, int Hq, int Hkv, int64_t q_stride, int64_t out_stride, int bt_stride, int num_splits,
                              int window, float scale, float soft_cap, int chunk, const float* sinks, float out_scale, int dtype,
                              cudaStream_t st) {
   using namespace fmha_dec;
@@ -444,7 +456,7 @@ EXPORT int vb_fmha_tc_decode2(const void* q, const void* kv_cache, int64_t num_b
   const CUtensorMapDataType dt = bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   Params p;
   p.block_table = block_table; p.seq_lens = seq_lens; p.out = out; p.part_out = part_out; p.part_lse = part_lse;
-  p.lse_out = lse_out; p.out_stride = out_stride; p.bt_stride = bt_stride; p.Hq = Hq; p.Hkv = Hkv; p.G = G;
+  p.lse_out = lse_out; p.error = error; p.out_stride = out_stride; p.bt_stride = bt_stride; p.Hq = Hq; p.Hkv = Hkv; p.G = G;
   p.num_splits = num_splits; p.window = window; p.scale_log2 = scale * 1.4426950408889634f; p.B = B;
   p.chunk = chunk; p.sinks = sinks; p.out_scale = out_scale;
   p.ku = soft_cap > 0.f ? scale / soft_cap : 0.f; p.c2 = soft_cap * 1.4426950408889634f;

@@ -94,7 +94,7 @@ _paged_attention_ex = _sig("vb_paged_attention_ex", _vp, _vp, _vp, _vp, _vp, _vp
                            _i64, _i64, _i, _i, _i, _f, _f, _f, _i, _i, _i, _vp, _vp, _i, _vp)
 _fmha_tc = _sig("vb_fmha_tc4", _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i64, _i64, _i,
                 _i, _i, _f, _f, _i, _i, _i, _vp, _f, _i, _i, _i, _vp)
-_fmha_tc_decode = _sig("vb_fmha_tc_decode2", _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i64, _i,
+_fmha_tc_decode = _sig("vb_fmha_tc_decode4", _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i64, _i64, _i,
                        _i, _i, _f, _f, _i, _vp, _f, _i, _vp)
 _any_attention = _sig("vb_any_attention", _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _i64, _i64, _i, _i, _i,
                       _i, _f, _f, _f, _vp, _vp, _i, _vp)
@@ -427,7 +427,7 @@ def paged_attention(q, kv_cache, md, scale, sliding_window=None, logits_soft_cap
             # swap-AB decode kernel: KV tokens on the MMA M axis
             rc = _fmha_tc_decode(q.data_ptr(), kv_cache.data_ptr(), kv_cache.shape[0], bt.data_ptr(),
                                  md.seq_lens.data_ptr(), out.data_ptr(), _p(ws.part_out) if ws else None,
-                                 _p(ws.part_lse) if ws else None, _p(lse), md.num_reqs, Hq, Hkv, q.stride(0),
+                                 _p(ws.part_lse) if ws else None, _p(lse), _error_flag(q.device), md.num_reqs, Hq, Hkv, q.stride(0),
                                  out.stride(0), bt.stride(0), splits, sliding_window or 0, scale, logits_soft_cap, chunk_size,
                                  _p(sinks), out_scale, _DT[q.dtype], _st())
             _check(rc, f"fmha_tc_decode(G={G})", 2 if splits > 1 else 1)
@@ -639,9 +639,8 @@ def mla_decode_tc(q_nope_abs, q_pe, kv_cache, block_table, seq_lens, scale, max_
             ws = _mla_ws[key] = (torch.empty(n * 512, dtype=torch.float32, device=dev),
                                  torch.empty(n, dtype=torch.float32, device=dev))
         po, pl = ws
-    err = kernel_error_flag(dev)
     _check(_mla_decode(q_nope_abs.data_ptr(), _p(q_pe), kv_cache.data_ptr(), kv_cache.shape[0],
-                       block_table.data_ptr(), seq_lens.data_ptr(), out.data_ptr(), _p(po), _p(pl), _p(lse), err.data_ptr(), B,
+                       block_table.data_ptr(), seq_lens.data_ptr(), out.data_ptr(), _p(po), _p(pl), _p(lse), _error_flag(dev), B,
                        H, R, P, kv_cache.shape[1], q_nope_abs.stride(0), q_nope_abs.stride(1),
                        q_pe.stride(0) if P else 0, q_pe.stride(1) if P else 0,
                        out.stride(0), block_table.stride(0), splits, sliding_window or 0, int(wide), scale, _DT[q_nope_abs.dtype], _st()),
