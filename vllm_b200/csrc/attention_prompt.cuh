@@ -82,12 +82,9 @@ template <int KS, int VS> struct Bars {
   }
   // a producer that gave up: let its copies in flight land before the block gives up its memory
   VB_DEVICE void drain() {
-    for (int s = 0; s < KS; ++s)
-      for (int n = 0; n < 4096 && !(mbar_try_wait(&k_full[s], 0) || mbar_try_wait(&k_full[s], 1)); ++n) {}
-    for (int s = 0; s < VS; ++s)
-      for (int n = 0; n < 4096 && !(mbar_try_wait(&v_full[s], 0) || mbar_try_wait(&v_full[s], 1)); ++n) {}
-    for (int t = 0; t < 2; ++t)
-      for (int n = 0; n < 4096 && !(mbar_try_wait(&edge[t], 0) || mbar_try_wait(&edge[t], 1)); ++n) {}
+    mbar_let_land(k_full, KS);
+    mbar_let_land(v_full, VS);
+    mbar_let_land(edge, 2);
   }
 };
 

@@ -144,10 +144,8 @@ talk_fold_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         if (++j == n_tiles) { j = 0; ++ci; }
       }
       if (budget < 0 && rank == 0) {            // let the copies in flight land before the pair gives up its memory
-        for (int s = 0; s < K_STAGES; ++s)
-          for (int n = 0; n < 4096 && !(mbar_try_wait(&k_full[s], 0) || mbar_try_wait(&k_full[s], 1)); ++n) {}
-        for (int s = 0; s < V_STAGES; ++s)
-          for (int n = 0; n < 4096 && !(mbar_try_wait(&v_full[s], 0) || mbar_try_wait(&v_full[s], 1)); ++n) {}
+        mbar_let_land(k_full, K_STAGES);
+        mbar_let_land(v_full, V_STAGES);
       }
     }
   } else if (warp == 1) {

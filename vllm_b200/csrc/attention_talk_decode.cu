@@ -137,8 +137,7 @@ talk_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         prev[0] = blk[0]; prev[1] = blk[1];
       }
       if (budget < 0) {                          // let the copies in flight land before the block gives up its memory
-        for (int s = 0; s < SLOTS; ++s)
-          for (int i = 0; i < 4096 && !(mbar_try_wait(&full[s], 0) || mbar_try_wait(&full[s], 1)); ++i) {}
+        mbar_let_land(full, SLOTS);
       }
     }
   } else if (warp == 1) {

@@ -184,7 +184,7 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       if (__shfl_sync(0xffffffffu, budget, 0) < 0) break;
     }
     if (lane == 0 && budget < 0)              // let the copies in flight land before the block gives up its memory
-      for (int n = 0; n < 4096 * 2 * STAGES; ++n) mbar_try_wait(&k_full[n % (2 * STAGES)], n / (2 * STAGES) & 1);      // (v_full behind k_full)
+      mbar_let_land(k_full, 2 * STAGES);       // (v_full behind k_full)
   } else if (warp == 1) {
     const uint32_t idesc = umma_idesc_f16(128, NQ, DTypeOf<T>::v == DT_BF16);
     int gt = 0, qi = 0;

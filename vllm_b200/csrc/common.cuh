@@ -150,6 +150,11 @@ VB_DEVICE void mbar_wait_lim(uint64_t* bar, uint32_t parity, int& budget) {
   while (!mbar_try_wait(bar, parity))
     if (--budget < 0) break;
 }
+// Of a producer that gave up: some time for the copies in flight on its n barriers to land.  Of a barrier's two parities one is always that of a phase that
+// has ended, so no answer of a poll ends this; the poll of the phase that has not suspends.
+VB_DEVICE void mbar_let_land(uint64_t* bars, int n) {
+  for (int i = 0; i < 4096 * n; ++i) mbar_try_wait(bars + i % n, i / n & 1);
+}
 
 // ------------------------------------------------- PTX: bulk / tensor copies
 // 1-D bulk copy global → shared, completion counted on an mbarrier (bytes % 16 == 0)

@@ -119,8 +119,7 @@ experts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant
           }
       }
       if (budget < 0)                        // let the copies in flight land before the block gives up its memory
-        for (int s = 0; s < STAGES; ++s)
-          for (int n = 0; n < 4096 && !(mbar_try_wait(&full[s], 0) || mbar_try_wait(&full[s], 1)); ++n) {}
+        mbar_let_land(full, STAGES);
     }
   } else if (warp == 1) {
     const uint32_t idesc = umma_idesc_f16(TM, BN, DTypeOf<T>::v == DT_BF16);

@@ -236,8 +236,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_qn, const __grid_cons
         }
       }
       if (budget < 0) {                         // let the copies in flight land before the block gives up its memory
-        for (int i = 0; i < STAGES * NKB; ++i)
-          for (int n = 0; n < 4096 && !mbar_try_wait(&kv_full[i], 0) && !mbar_try_wait(&kv_full[i], 1); ++n) {}
+        mbar_let_land(kv_full, STAGES * NKB);
       }
     }
   } else if (warp == 1) {
